@@ -36,6 +36,12 @@ struct DevBuf {
     if (e == cudaSuccess) bytes = n;
     return e;
   }
+  // As ensure, zeroed on `s` whenever it is newly allocated.
+  cudaError_t ensure_zeroed(size_t n, cudaStream_t s) {
+    if (n <= bytes) return cudaSuccess;
+    cudaError_t e = ensure(n);
+    return e == cudaSuccess ? cudaMemsetAsync(p, 0, n, s) : e;
+  }
   void release() {
     if (p) cudaFree(p);
     p = nullptr;
@@ -118,7 +124,7 @@ struct jpxlg_ref {
   jpxlg_ctx* ctx = nullptr;
   int device = 0;
   int w = 0, h = 0, nscales = 0;
-  SsimScale scales[6];
+  SsimScale scales[kMaxScales];
   void* block = nullptr;  // one allocation holding every scale's planes
 };
 
@@ -178,9 +184,10 @@ void stage_end(jpxlg_ctx* ctx) {
   ctx->open_stage = -1;
 }
 
-// The blur kernels of one SSIMULACRA2 scale, each under its own stage: the
-// row pass, the column ripple, the column outputs; the rest of the metric
-// (positive XYB, downscaling, the final sums) stays under JPXLG_STAGE_SSIM.
+// The blur kernels of SSIMULACRA2, each under its own stage: the row pass and
+// the column outputs (the column ripple's stage is empty: its scan runs
+// inside the column pass); the rest of the metric (positive XYB, downscaling,
+// the final sums) stays under JPXLG_STAGE_SSIM.
 void ssim_stage_hook(void* user, int part) {
   jpxlg_ctx* ctx = static_cast<jpxlg_ctx*>(user);
   static const int kNext[4] = {JPXLG_STAGE_SSIM_ROWS, JPXLG_STAGE_SSIM_COL_RIPPLE,
@@ -532,55 +539,71 @@ int render_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const int32_t* qcoeff,
   return rc;
 }
 
+// The scratch of the metric over scales of the given sizes: the row pass's
+// planes (nq per channel) and the column pass's scan buffer.
+int ensure_blur_scratch(jpxlg_ctx* ctx, const int (*dims)[2], int n, int nq) {
+  size_t planes = 0, carry = kBlurCarryHeader;
+  for (int s = 0; s < n; ++s) {
+    planes += 3 * nq * blur_plane_floats(dims[s][0], dims[s][1]);
+    carry += blur_carry_bytes(dims[s][0], dims[s][1], 3);
+  }
+  CK(ctx->hpl.ensure(planes * sizeof(float)));
+  CK(ctx->bcarry.ensure_zeroed(carry, ctx->stream));
+  return JPXLG_OK;
+}
+
+// Floats of three w x h planes, rounded so that what follows stays 16-byte
+// aligned.
+size_t plane_set_floats(int w, int h) { return (3 * (size_t)w * h + 3) & ~(size_t)3; }
+
 // Candidate side of SSIMULACRA2 against `ref`: cand_dev is the candidate's
 // linear RGB; cand_xyb (optional) its positive XYB, when the producer of the
-// pixels already formed it.  Each pyramid level keeps linear RGB (for the
-// next level) and positive XYB (for the tile kernel).
+// pixels already formed it.
 int score_device(jpxlg_ctx* ctx, const jpxlg_ref* ref, const float* cand_dev,
                  const float* cand_xyb, double* out_dev) {
-  const int w = ref->w, h = ref->h;
-  size_t pyr = 0;
-  for (int s = 1; s < ref->nscales; ++s) pyr += 6 * (size_t)ref->scales[s].w * ref->scales[s].h;
+  const int w = ref->w, h = ref->h, ns = ref->nscales;
+  int dims[kMaxScales][2], ctas[kMaxScales], pixels[kMaxScales];
+  size_t pyr = 0, ctas_total = 0;
+  for (int s = 0; s < ns; ++s) {
+    dims[s][0] = ref->scales[s].w;
+    dims[s][1] = ref->scales[s].h;
+    if (s > 0) pyr += plane_set_floats(dims[s][0], dims[s][1]);
+    ctas[s] = blur_partial_rows(dims[s][0], dims[s][1]);
+    ctas_total += (size_t)ctas[s];
+    pixels[s] = dims[s][0] * dims[s][1];
+  }
   CK(ctx->pyr.ensure(std::max<size_t>(pyr, 1) * sizeof(float)));
-  size_t ctas_total = 0;
-  for (int s = 0; s < ref->nscales; ++s)
-    ctas_total += (size_t)blur_partial_rows(ref->scales[s].w, ref->scales[s].h);
   CK(ctx->partial.ensure(ctas_total * 18 * sizeof(DF)));
-  CK(ctx->hpl.ensure(9 * (size_t)w * h * sizeof(float)));
-  CK(ctx->bcarry.ensure(blur_carry_floats(w, h) * sizeof(float)));
-  int ctas[6], pixels[6];
-  stage_begin(ctx, JPXLG_STAGE_SSIM);
-  uint64_t k = 0;
+  int rc = ensure_blur_scratch(ctx, dims, ns, 3);
+  if (rc) return rc;
+  PyramidOut po{};
+  BlurScale bs[kMaxScales];
   if (!cand_xyb) {
     CK(ctx->cxyb.ensure(3 * (size_t)w * h * sizeof(float)));
-    launch_positive_xyb(cand_dev, ctx->cxyb.as<float>(), (size_t)w * h, ctx->num_sms, ctx->stream);
-    ++k;
-    cand_xyb = ctx->cxyb.as<float>();
+    po.xyb[0] = ctx->cxyb.as<float>();
   }
-  const float* cur = cand_dev;
-  const float* cur_xyb = cand_xyb;
   float* next = ctx->pyr.as<float>();
   DF* part = ctx->partial.as<DF>();
-  for (int s = 0; s < ref->nscales; ++s) {
+  for (int s = 0; s < ns; ++s) {
     const SsimScale& rs = ref->scales[s];
     if (s > 0) {
-      const size_t ns = (size_t)rs.w * rs.h;
-      launch_downscale3(cur, ref->scales[s - 1].w, ref->scales[s - 1].h, next, next + 3 * ns,
-                        ctx->stream);
-      ++k;
-      cur = next;
-      cur_xyb = next + 3 * ns;
-      next += 6 * ns;
+      po.xyb[s] = next;
+      next += plane_set_floats(rs.w, rs.h);
     }
-    ctas[s] = launch_score_scale(cur_xyb, rs, ctx->hpl.as<float>(), ctx->bcarry.as<float>(), 0,
-                                 3, part, ctx->d_words, ctx->stream, ssim_stage_hook,
-                                 ctx);  // the hook counts its kernels
-    pixels[s] = rs.w * rs.h;
+    bs[s] = {rs.w, rs.h, s == 0 && cand_xyb ? cand_xyb : po.xyb[s], rs.xyb, rs.mu, rs.s11, part};
     part += (size_t)ctas[s] * 18;
   }
-  k += launch_score_finish(ctx->partial.as<DF>(), ctas, ref->nscales, pixels, out_dev,
-                           ctx->stream);
-  int rc = after_launch(ctx, k);
+  stage_begin(ctx, JPXLG_STAGE_SSIM);
+  uint64_t k = 0;
+  if (!cand_xyb || ns > 1) {
+    launch_pyramid(cand_dev, w, h, po, ns, ctx->stream);
+    ++k;
+  }
+  // the hook counts the blur's kernels
+  launch_score_scales(bs, ns, 0, 3, ctx->hpl.as<float>(), ctx->bcarry.p, ctx->d_words,
+                      ctx->stream, ssim_stage_hook, ctx);
+  k += launch_score_finish(ctx->partial.as<DF>(), ctas, ns, pixels, out_dev, ctx->stream);
+  rc = after_launch(ctx, k);
   stage_end(ctx);
   return rc;
 }
@@ -1008,12 +1031,12 @@ int jpxlg_reconstruct(jpxlg_ctx* ctx, const jpxlg_layout* L, const jpxlg_plan* p
 namespace {
 
 // reference.rs:90: the scales (keep halving while the current one is at
-// least 8x8) and the floats of a reference's planes (per scale: the RGB
-// level, XYB, mu and sigma11, 3 planes each).
-int ref_layout(int w, int h, int dims[6][2], size_t* total) {
+// least 8x8) and the floats of a reference's planes (per scale: positive
+// XYB, mu and sigma11, 3 planes each).
+int ref_layout(int w, int h, int dims[kMaxScales][2], size_t* total) {
   int cw = w, ch = h, ns = 0;
   *total = 0;
-  for (int s = 0; s < 6; ++s) {
+  for (int s = 0; s < kMaxScales; ++s) {
     if (s > 0) {
       if (cw < 8 || ch < 8) break;
       cw = (cw + 1) / 2;
@@ -1021,7 +1044,7 @@ int ref_layout(int w, int h, int dims[6][2], size_t* total) {
     }
     dims[s][0] = cw;
     dims[s][1] = ch;
-    *total += 9 * (size_t)cw * ch + 3 * (size_t)cw * ch;
+    *total += 3 * plane_set_floats(cw, ch);
     ++ns;
   }
   return ns;
@@ -1038,7 +1061,7 @@ int ref_check(jpxlg_ctx* ctx, int w, int h) {
 // Fills R (w, h, device set) in `block` (ref_layout's floats): the pyramid,
 // positive XYB and the blurred moments of every scale.
 int ref_fill(jpxlg_ctx* ctx, jpxlg_ref* R, void* block, const float* rgb, uint32_t mem) {
-  int dims[6][2];
+  int dims[kMaxScales][2];
   size_t total;
   const int w = R->w, h = R->h;
   const int ns = ref_layout(w, h, dims, &total);
@@ -1046,40 +1069,31 @@ int ref_fill(jpxlg_ctx* ctx, jpxlg_ref* R, void* block, const float* rgb, uint32
   R->block = block;
   float* cursor = (float*)block;
   const size_t n0 = (size_t)w * h;
-  CK(ctx->hpl.ensure(9 * n0 * sizeof(float)));
-  CK(ctx->bcarry.ensure(blur_carry_floats(w, h) * sizeof(float)));
-  CK(ctx->out.ensure(3 * n0 * sizeof(float)));
+  int rc = ensure_blur_scratch(ctx, dims, ns, 2);
+  if (rc) return rc;
   const float* src = rgb;
   if (mem == JPXLG_MEM_HOST) {
+    CK(ctx->out.ensure(3 * n0 * sizeof(float)));
     CK(cudaMemcpyAsync(ctx->out.p, rgb, 3 * n0 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     src = ctx->out.as<float>();
   }
-  uint64_t k = 0;
-  const float* level = src;
+  PyramidOut po{};
+  BlurScale bs[kMaxScales];
   for (int s = 0; s < ns; ++s) {
     SsimScale& sc = R->scales[s];
     sc.w = dims[s][0];
     sc.h = dims[s][1];
-    const size_t n = (size_t)sc.w * sc.h;
-    float* rgb_s = cursor;
-    cursor += 3 * n;
-    if (s > 0) {
-      launch_downscale3(level, dims[s - 1][0], dims[s - 1][1], rgb_s, nullptr, ctx->stream);
-      ++k;
-      level = rgb_s;
-    }
+    const size_t set = plane_set_floats(sc.w, sc.h);
     sc.xyb = cursor;
-    cursor += 3 * n;
-    sc.mu = cursor;
-    cursor += 3 * n;
-    sc.s11 = cursor;
-    cursor += 3 * n;
-    launch_positive_xyb(level, sc.xyb, n, ctx->num_sms, ctx->stream);
-    launch_ref_moments(sc.xyb, sc.mu, sc.s11, ctx->hpl.as<float>(), ctx->bcarry.as<float>(), sc.w,
-                       sc.h, ctx->d_words, ctx->stream);
-    k += 1 + 2;
+    sc.mu = cursor + set;
+    sc.s11 = cursor + 2 * set;
+    cursor += 3 * set;
+    po.xyb[s] = sc.xyb;
+    bs[s] = {sc.w, sc.h, sc.xyb, sc.xyb, sc.mu, sc.s11, nullptr};
   }
-  return after_launch(ctx, k);
+  launch_pyramid(src, w, h, po, ns, ctx->stream);
+  launch_ref_moments(bs, ns, ctx->hpl.as<float>(), ctx->bcarry.p, ctx->d_words, ctx->stream);
+  return after_launch(ctx, 3);
 }
 
 }  // namespace
@@ -1096,7 +1110,7 @@ int jpxlg_ssim2_ref_create(jpxlg_ctx* ctx, const float* rgb, int w, int h, uint3
   R->device = ctx->device;
   R->w = w;
   R->h = h;
-  int dims[6][2];
+  int dims[kMaxScales][2];
   size_t total;
   ref_layout(w, h, dims, &total);
   void* block = nullptr;
@@ -1173,7 +1187,7 @@ int jpxlg_score_pair(jpxlg_ctx* ctx, const float* ref_rgb, const float* cand_rgb
   R.device = ctx->device;
   R.w = w;
   R.h = h;
-  int dims[6][2];
+  int dims[kMaxScales][2];
   size_t total;
   ref_layout(w, h, dims, &total);
   CK(ctx->pair_ref.ensure(total * sizeof(float)));
@@ -1471,32 +1485,35 @@ extern "C" int jpxlg_batch_probe(jpxlg_ctx* ctx, int n_items, const jpxlg_batch_
 // cudaFree.
 //
 // Capacity: reference frames up to kStaticMaxSide x kStaticMaxSide.  For a
-// 2048 x 2048 frame the workspace holds the linear pyramid of scales 1..5,
-// 3 * (1024^2 + 512^2 + 256^2 + 128^2 + 64^2) = 4,190,208 floats; the
-// current scale's candidate positive XYB, 3 * 2048^2 = 12,582,912 floats;
-// the row pass of one channel (three planes), 12,582,912 floats; the column
-// pass's segment responses and entry states of one channel,
-// 2 x 64 segments x 18 x 2048 = 4,718,592 floats; and the partial sums, one
-// row of 18 double-float sums per 32 x 32 tile of each scale,
-// 4096 + 1024 + 256 + 64 + 16 + 4 = 5,460 rows: 137 MB in all.  Every count grows with width and height, so any frame within the
-// side limit fits.
-// Channels are scored one after another so that the row pass needs one
-// channel's planes.
+// 2048 x 2048 frame the workspace holds the candidate's positive XYB at every
+// level, 3 * 2048^2 = 12,582,912 floats and
+// 3 * (1024^2 + 512^2 + 256^2 + 128^2 + 64^2) = 4,190,208 floats; the row
+// pass of one channel and scale (three planes), 12,582,912 floats; the column
+// pass's scan buffer for one channel and scale, 16 + 32 segments x 6 x 2048
+// words of four floats = 1,572,880 floats; and the partial sums, one row of
+// 18 double-float sums per 32 x 32 tile of each scale,
+// 4096 + 1024 + 256 + 64 + 16 + 4 = 5,460 rows: 125 MB in all.  Every count
+// grows with width and height (a plane set or a row-pass row rounded up to 16
+// bytes included), so any frame within the side limit fits.
+// Channels and scales are scored one after another so that the row pass needs
+// one channel's planes of one scale.
 //
-// Nothing in the scratch has to start at zero: each call writes every level,
-// plane and partial row before reading it.  There is one scratch per device,
-// so calls whose work overlaps on a device (two streams, two contexts, or
-// two host threads) race on it; callers serialise them.
+// Nothing in the scratch but the scan buffer has to start at zero: each call
+// writes every level, plane and partial row before reading it.  The scan
+// buffer starts zeroed with the module and is used for nothing else.  There
+// is one scratch per device, so calls whose work overlaps on a device (two
+// streams, two contexts, or two host threads) race on it; callers serialise
+// them.
 namespace {
 
 constexpr int kStaticMaxSide = 2048;
 constexpr size_t kStaticPyrFloats = 4190208;
 constexpr size_t kStaticPlaneFloats = (size_t)kStaticMaxSide * kStaticMaxSide;
 constexpr size_t kStaticPartialRows = 5460;
-constexpr size_t kStaticCarryFloats = 4718592;
-// pyramid, positive XYB, row pass, segment states
+constexpr size_t kStaticCarryFloats = 1572880;
+// positive XYB levels, row pass, scan buffer
 constexpr size_t kStaticFloats = kStaticPyrFloats + 6 * kStaticPlaneFloats + kStaticCarryFloats;
-constexpr size_t kStaticFloatBytes = kStaticFloats * sizeof(float);  // a multiple of 256
+constexpr size_t kStaticFloatBytes = kStaticFloats * sizeof(float);  // a multiple of 64
 constexpr size_t kStaticScratchBytes = kStaticFloatBytes + kStaticPartialRows * 18 * sizeof(DF);
 constexpr int kStaticMaxDevices = 64;
 
@@ -1539,45 +1556,41 @@ extern "C" int jpxlg_ssim2_score_static(jpxlg_ctx* ctx, const jpxlg_ref* ref,
   int rc = static_scratch(ctx, &scratch);
   if (rc) return rc;
   // Every region checked against its capacity at run time, not only through
-  // the side limit: the pyramid, the partial-sum rows, and per scale the
-  // candidate's positive XYB and one channel's row-pass planes (three planes
-  // each) and its column-pass carry (a third of the three channels').
+  // the side limit: the positive XYB levels, the partial-sum rows, and per
+  // scale one channel's row-pass planes (three) and scan buffer.
   size_t pyr = 0, rows = 0;
-  bool fits = true;
+  bool fits = 3 * (size_t)ref->w * ref->h <= 3 * kStaticPlaneFloats;
   for (int s = 0; s < ref->nscales; ++s) {
     const SsimScale& rs = ref->scales[s];
-    if (s > 0) pyr += 3 * (size_t)rs.w * rs.h;
+    if (s > 0) pyr += plane_set_floats(rs.w, rs.h);
     rows += (size_t)blur_partial_rows(rs.w, rs.h);
-    fits = fits && (size_t)rs.w * rs.h <= kStaticPlaneFloats &&
-           blur_carry_floats(rs.w, rs.h) / 3 <= kStaticCarryFloats;
+    fits = fits && blur_plane_floats(rs.w, rs.h) <= kStaticPlaneFloats &&
+           kBlurCarryHeader + blur_carry_bytes(rs.w, rs.h, 1) <= kStaticCarryFloats * sizeof(float);
   }
   if (!fits || pyr > kStaticPyrFloats || rows > kStaticPartialRows)
     return fail(ctx, JPXLG_ERR_ARGUMENT, "static scoring scratch too small for %dx%d", ref->w,
                 ref->h);
-  float* next = (float*)scratch;
-  float* xyb = next + kStaticPyrFloats;
-  float* hpl = xyb + 3 * kStaticPlaneFloats;
+  float* xyb0 = (float*)scratch;
+  float* next = xyb0 + 3 * kStaticPlaneFloats;
+  float* hpl = next + kStaticPyrFloats;
   float* carry = hpl + 3 * kStaticPlaneFloats;
   DF* part0 = (DF*)(scratch + kStaticFloatBytes);
   DF* part = part0;
-  const float* cur = linear_rgb_dev;
-  int ctas[6], pixels[6];
-  uint64_t k = 0;
+  int ctas[kMaxScales], pixels[kMaxScales];
+  PyramidOut po{};
   for (int s = 0; s < ref->nscales; ++s) {
     const SsimScale& rs = ref->scales[s];
-    if (s > 0) {
-      launch_downscale3(cur, ref->scales[s - 1].w, ref->scales[s - 1].h, next, xyb, ctx->stream);
-      ++k;
-      cur = next;
-      next += 3 * (size_t)rs.w * rs.h;
-    } else {
-      launch_positive_xyb(cur, xyb, (size_t)rs.w * rs.h, ctx->num_sms, ctx->stream);
-      ++k;
-    }
-    for (int c = 0; c < 3; ++c) {
-      ctas[s] = launch_score_scale(xyb, rs, hpl, carry, c, 1, part, ctx->d_words, ctx->stream);
-      k += kScoreScaleKernels;
-    }
+    po.xyb[s] = s == 0 ? xyb0 : next;
+    if (s > 0) next += plane_set_floats(rs.w, rs.h);
+  }
+  launch_pyramid(linear_rgb_dev, ref->w, ref->h, po, ref->nscales, ctx->stream);
+  uint64_t k = 1;
+  for (int s = 0; s < ref->nscales; ++s) {
+    const SsimScale& rs = ref->scales[s];
+    const BlurScale bs{rs.w, rs.h, po.xyb[s], rs.xyb, rs.mu, rs.s11, part};
+    for (int c = 0; c < 3; ++c)
+      k += launch_score_scales(&bs, 1, c, 1, hpl, carry, ctx->d_words, ctx->stream);
+    ctas[s] = blur_partial_rows(rs.w, rs.h);
     pixels[s] = rs.w * rs.h;
     part += (size_t)ctas[s] * 18;
   }

@@ -70,7 +70,6 @@ void launch_mul_table(uint32_t global_scale, float* table, cudaStream_t s);
 // Per-device kernel attributes (dynamic shared memory above 48 KB); call once
 // per device with it current, before any launch or stream capture.
 cudaError_t configure_encode_kernels();
-cudaError_t configure_ssim_kernels();
 
 void upload_dct_constants(const float* iv4, const float* iv8, const float* iv16,
                           const float* scale_f, cudaStream_t s);
@@ -165,41 +164,55 @@ struct SsimScale {
   float* mu;    // [3][w*h]
   float* s11;   // [3][w*h]
 };
+constexpr int kMaxScales = 6;
 // The blur's constants (taps, resonators) into constant memory.
 void upload_blur_consts(cudaStream_t s);
 // Widest frame the row pass stages in shared memory (a line plus its output).
 constexpr int kBlurMaxWidth = 8192;
-size_t blur_row_smem(int w);
 cudaError_t configure_blur_kernels();
-// Rows of partial sums one scale writes (one per 32 x 32 tile), and the
-// floats of the column pass's segment-state scratch for three channels.
+// Rows of partial sums one scale writes (one per 32 x 32 tile).
 int blur_partial_rows(int w, int h);
-size_t blur_carry_floats(int w, int h);
-// 2x2 mean of linear RGB planes; xyb (optional) receives the result's
-// positive XYB planes.
-void launch_downscale3(const float* in, int w, int h, float* out, float* xyb, cudaStream_t s);
-void launch_positive_xyb(const float* rgb, float* xyb, size_t n, int num_sms, cudaStream_t s);
-// Reference side of one scale: mu = blur(xyb), s11 = blur(xyb * xyb) per
-// channel; hpl (6 w*h planes) and carry (blur_carry_floats) are scratch; a
-// column-scan wait that runs out raises kDevBlurTimeout in err.  Three
-// launches: the row pass, the column flags' reset, the column pass.
-void launch_ref_moments(const float* xyb, float* mu, float* s11, float* hpl, float* carry, int w,
-                        int h, uint32_t* err, cudaStream_t s);
-// Candidate side of one scale for channels c0 .. c0+nch-1: cand_xyb is the
-// candidate's positive XYB [3][w*h]; hpl (3 * nch w*h planes) and carry
-// (blur_carry_floats) are scratch; partial receives one row of 18
-// double-float sums (8 bytes each) per 32 x 32 tile, each channel filling
-// its six.  Returns the number of rows (blur_partial_rows).
-struct DF;
-// Called between a scale's launches when the caller times them: part 0
-// before the row pass, 1 after it, 2 before the column pass (its flags'
-// reset and its kernel, which runs the ripple's segment scan inside), 3
-// after it.  Two kernels per scale (kScoreScaleKernels).
+// Floats of one row-pass plane (rows padded to a 16-byte pitch).
+size_t blur_plane_floats(int w, int h);
+// Bytes of one scale's segment states in the column pass's scan buffer, which
+// also holds kBlurCarryHeader bytes.  The buffer is zeroed when it is
+// allocated and carries its launches' epoch from then on.
+constexpr size_t kBlurCarryHeader = 64;
+size_t blur_carry_bytes(int w, int h, int nch);
+// The pyramid of a linear RGB frame as positive XYB planes: level s
+// (ceil-halved s times by 2x2 means, edge replicated) into xyb[s], levels
+// 1 .. n-1, and level 0 where xyb[0] is not null.
+struct PyramidOut {
+  float* xyb[kMaxScales];
+};
+void launch_pyramid(const float* rgb, int w, int h, const PyramidOut& out, int n, cudaStream_t s);
+// One scale of the blur: positive XYB x (the candidate's, or the reference's
+// own for its moments), the reference's r, and mu and sigma11 (written by
+// launch_ref_moments, read by launch_score_scales).
+struct BlurScale {
+  int w, h;
+  const float* x;  // [3][w*h]
+  const float* r;  // [3][w*h]
+  float* mu;       // [3][w*h]
+  float* s11;      // [3][w*h]
+  DF* partial;     // blur_partial_rows rows of 18 sums (scoring only)
+};
+// Reference side of every scale: mu = blur(x), s11 = blur(x * x) per channel;
+// hpl (6 row-pass planes per scale) and carry (blur_carry_bytes, summed, plus
+// the header) are scratch; a column-scan wait that runs out raises
+// kDevBlurTimeout in err.  Two launches: the row pass, the column pass.
+void launch_ref_moments(const BlurScale* scales, int n, float* hpl, void* carry, uint32_t* err,
+                        cudaStream_t s);
+// Candidate side of every scale for channels c0 .. c0+nch-1; hpl (3 * nch
+// row-pass planes per scale) and carry are scratch; each scale's partial
+// receives one row of 18 double-float sums (8 bytes each) per 32 x 32 tile,
+// each channel filling its six.  Returns the number of launches (two).
+// The hook is called between the launches when the caller times them: part 0
+// before the row pass, 1 after it, 2 before the column pass, 3 after it.
 using ScaleHook = void (*)(void* user, int part);
-constexpr int kScoreScaleKernels = 2;
-int launch_score_scale(const float* cand_xyb, const SsimScale& ref, float* hpl, float* carry,
-                       int c0, int nch, DF* partial, uint32_t* err, cudaStream_t s,
-                       ScaleHook hook = nullptr, void* user = nullptr);
+int launch_score_scales(const BlurScale* scales, int n, int c0, int nch, float* hpl, void* carry,
+                        uint32_t* err, cudaStream_t s, ScaleHook hook = nullptr,
+                        void* user = nullptr);
 // Two launches (the per-scale sums, then the score); returns 2.  The sums
 // overwrite row 0 of each scale's partial rows.
 int launch_score_finish(DF* partials, const int* ctas_per_scale, int nscales,

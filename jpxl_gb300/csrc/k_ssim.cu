@@ -1,7 +1,7 @@
 // k_ssim.cu — sm_103a kernels of SSIMULACRA2 (jpxl-perceptual) besides the
 // blur (k_blur.cu):
-//   S1 k_downscale3        pyramid.rs:19 2x2 mean, edge replicated
-//   S2 k_positive_xyb      color.rs:66 positive XYB (reproducible cube root)
+//   S1, S2 k_pyramid       pyramid.rs:19 2x2 means, edge replicated, and
+//                          color.rs:66 positive XYB (reproducible cube root)
 //   S5 k_score_reduce      the partial rows' sums per scale and quantity
 //      k_score_finish      norms, 108 weights, remap (ssimulacra2.rs:509/:531)
 //
@@ -16,57 +16,89 @@
 
 namespace jpxlg {
 
-// S1 — one output pixel per thread, all three channels; with `xyb` set the
-// pixel's positive XYB (S2) is written too, for the scale's candidate side.
-__global__ void __launch_bounds__(256) k_downscale3(const float* __restrict__ in, int w, int h,
-                                                    float* __restrict__ out,
-                                                    float* __restrict__ xyb) {
-  const int ow = (w + 1) / 2, oh = (h + 1) / 2;
-  const size_t ip = (size_t)w * h, op = (size_t)ow * oh;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ow * oh; i += gridDim.x * blockDim.x) {
-    int ox = i % ow, oy = i / ow;
-    int x0 = min(2 * ox, w - 1), x1 = min(2 * ox + 1, w - 1);
-    int y0 = min(2 * oy, h - 1), y1 = min(2 * oy + 1, h - 1);
-    float v[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float* p = in + ip * c;
-      float a = p[(size_t)y0 * w + x0], b = p[(size_t)y0 * w + x1];
-      float cc = p[(size_t)y1 * w + x0], d = p[(size_t)y1 * w + x1];
-      v[c] = (a + b + cc + d) * 0.25f;
-      out[op * c + i] = v[c];
-    }
-    if (xyb) {
-      float o[3];
-      positive_xyb(v[0], v[1], v[2], o);
-      xyb[i] = o[0];
-      xyb[op + i] = o[1];
-      xyb[2 * op + i] = o[2];
-    }
-  }
-}
+// S1 — the pyramid of one frame in one launch: a CTA takes a 64 x 64 tile
+// of the source, whose 2x2 means at every level (edge replicated,
+// pyramid.rs:19) depend on that tile alone, and keeps each level in shared
+// memory for the next; only the levels' positive XYB (S2) goes to memory.
+// Bound by the cube roots (issue slots of the ALU and FMA pipes).  Measured
+// at 2048x2048: 24.5 us for levels 1..5 against 39.9 us in five launches.
+constexpr int kPyrTile = 64;
+constexpr int kPyrThreads = 256;
 
-void launch_downscale3(const float* in, int w, int h, float* out, float* xyb, cudaStream_t s) {
-  int n = ((w + 1) / 2) * ((h + 1) / 2);
-  dim3 grid(std::max(1, std::min((n + 255) / 256, 4096)));
-  k_downscale3<<<grid, 256, 0, s>>>(in, w, h, out, xyb);
-}
-
-__global__ void __launch_bounds__(256) k_positive_xyb(const float* __restrict__ rgb,
-                                                      float* __restrict__ xyb, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(kPyrThreads) k_pyramid(const float* __restrict__ rgb, int w,
+                                                         int h, PyramidOut out, int n) {
+  __shared__ float lev[3][kPyrTile / 2][kPyrTile / 2 + 1];
+  __shared__ float lev2[3][kPyrTile / 4][kPyrTile / 4 + 1];
+  const int t = threadIdx.x;
+  const int x0 = blockIdx.x * kPyrTile, y0 = blockIdx.y * kPyrTile;
+  const size_t plane = (size_t)w * h;
+  auto put = [](float* dst, size_t np, size_t p, const float* v) {
     float o[3];
-    positive_xyb(rgb[i], rgb[n + i], rgb[2 * n + i], o);
-    xyb[i] = o[0];
-    xyb[n + i] = o[1];
-    xyb[2 * n + i] = o[2];
+    positive_xyb(v[0], v[1], v[2], o);
+    dst[p] = o[0];
+    dst[np + p] = o[1];
+    dst[2 * np + p] = o[2];
+  };
+  if (out.xyb[0]) {
+    for (int i = t; i < kPyrTile * kPyrTile; i += kPyrThreads) {
+      const int gx = x0 + i % kPyrTile, gy = y0 + i / kPyrTile;
+      if (gx >= w || gy >= h) continue;
+      const size_t p = (size_t)gy * w + gx;
+      const float v[3] = {rgb[p], rgb[plane + p], rgb[2 * plane + p]};
+      put(out.xyb[0], plane, p, v);
+    }
+  }
+  // Level 1 from the source.
+  int lw = (w + 1) / 2, lh = (h + 1) / 2;
+  if (n > 1)
+    for (int i = t; i < kPyrTile * kPyrTile / 4; i += kPyrThreads) {
+      const int lx = i % (kPyrTile / 2), ly = i / (kPyrTile / 2);
+      const int gx = x0 / 2 + lx, gy = y0 / 2 + ly;
+      if (gx >= lw || gy >= lh) continue;
+      const int sx0 = 2 * gx, sx1 = min(2 * gx + 1, w - 1);
+      const size_t ra = (size_t)(2 * gy) * w, rb = (size_t)min(2 * gy + 1, h - 1) * w;
+      float v[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float* p = rgb + plane * c;
+        v[c] = (p[ra + sx0] + p[ra + sx1] + p[rb + sx0] + p[rb + sx1]) * 0.25f;
+        lev[c][ly][lx] = v[c];
+      }
+      put(out.xyb[1], (size_t)lw * lh, (size_t)gy * lw + gx, v);
+    }
+  // The smaller levels from the one before, which alternates between the two
+  // shared tiles.
+  for (int s = 2; s < n; ++s) {
+    __syncthreads();
+    const int pw = lw, ph = lh, side = kPyrTile >> s;
+    lw = (lw + 1) / 2;
+    lh = (lh + 1) / 2;
+    const int bx = x0 >> s, by = y0 >> s;
+    if (t < side * side) {
+      const int lx = t % side, ly = t / side, gx = bx + lx, gy = by + ly;
+      if (gx < lw && gy < lh) {
+        const int a0 = 2 * lx, a1 = min(2 * gx + 1, pw - 1) - 2 * bx;
+        const int b0 = 2 * ly, b1 = min(2 * gy + 1, ph - 1) - 2 * by;
+        float v[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (s & 1) {
+            v[c] = (lev2[c][b0][a0] + lev2[c][b0][a1] + lev2[c][b1][a0] + lev2[c][b1][a1]) * 0.25f;
+            lev[c][ly][lx] = v[c];
+          } else {
+            v[c] = (lev[c][b0][a0] + lev[c][b0][a1] + lev[c][b1][a0] + lev[c][b1][a1]) * 0.25f;
+            lev2[c][ly][lx] = v[c];
+          }
+        }
+        put(out.xyb[s], (size_t)lw * lh, (size_t)gy * lw + gx, v);
+      }
+    }
   }
 }
 
-void launch_positive_xyb(const float* rgb, float* xyb, size_t n, int num_sms, cudaStream_t s) {
-  int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)num_sms * 8);
-  k_positive_xyb<<<std::max(1, blocks), 256, 0, s>>>(rgb, xyb, n);
+void launch_pyramid(const float* rgb, int w, int h, const PyramidOut& out, int n, cudaStream_t s) {
+  const dim3 grid((w + kPyrTile - 1) / kPyrTile, (h + kPyrTile - 1) / kPyrTile);
+  k_pyramid<<<grid, kPyrThreads, 0, s>>>(rgb, w, h, out, n);
 }
 
 // S5 — ssimulacra2.rs:391 WEIGHTS (the metric's data table), :509
