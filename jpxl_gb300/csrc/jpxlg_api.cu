@@ -633,6 +633,7 @@ int jpxlg_ctx_create(int device, uint32_t flags, jpxlg_ctx** out) {
   } while (0)
   CKC(cudaSetDevice(device));
   CKC(configure_encode_kernels());
+  CKC(configure_render_kernels());
   CKC(configure_blur_kernels());
   CKC(configure_tc_kernels());
   CKC(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));

@@ -70,6 +70,7 @@ void launch_mul_table(uint32_t global_scale, float* table, cudaStream_t s);
 // Per-device kernel attributes (dynamic shared memory above 48 KB); call once
 // per device with it current, before any launch or stream capture.
 cudaError_t configure_encode_kernels();
+cudaError_t configure_render_kernels();
 
 void upload_dct_constants(const float* iv4, const float* iv8, const float* iv16,
                           const float* scale_f, cudaStream_t s);

@@ -8,6 +8,7 @@
 // jpxl-core kernels it calls; -fmad=false keeps every unfused product.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "jpxlg_common.cuh"
 #include "jpxlg_internal.h"
@@ -603,34 +604,67 @@ void launch_render_varblocks(const RenderArgs& a, const uint32_t* const* lists, 
 // in row-major order from 0, kernel from GaborKernel::new (:111, with FMA).
 // ---------------------------------------------------------------------------
 
-constexpr int kGT = 32;
-__global__ void __launch_bounds__(256) k_gaborish(const float* __restrict__ in,
-                                                  float* __restrict__ out, int w, int h,
-                                                  float centre, float edge, float corner) {
-  __shared__ float t[kGT + 2][kGT + 3];
+// A thread forms V columns of kGabRun rows, keeping three rows of its V + 2
+// columns in registers: 16-byte reads and writes where the rows are aligned
+// (V = 4), one column a lane otherwise.  The columns' shared edges come from
+// the L1.  Bound: memory latency and issue slots (18 operations a sample).
+// Measured at 2048x2048: 47.7 -> 21.8 us (0.68 of the copy rate for its 101
+// MB; 32 x 32 tiles in shared memory before).
+constexpr int kGabRun = 8;
+constexpr int kGabThreads = 128;
+
+template <int V>
+__global__ void __launch_bounds__(kGabThreads) k_gaborish(const float* __restrict__ in,
+                                                          float* __restrict__ out, int w, int h,
+                                                          float centre, float edge, float corner) {
   const size_t plane = (size_t)w * h;
   in += plane * blockIdx.z;
   out += plane * blockIdx.z;
-  const int x0 = blockIdx.x * kGT, y0 = blockIdx.y * kGT;
-  for (int i = threadIdx.x; i < (kGT + 2) * (kGT + 2); i += blockDim.x) {
-    int lx = i % (kGT + 2), ly = i / (kGT + 2);
-    int gx = mirror1d(x0 + lx - 1, w), gy = mirror1d(y0 + ly - 1, h);
-    t[ly][lx] = in[(size_t)gy * w + gx];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kGT * kGT; i += blockDim.x) {
-    int lx = i % kGT, ly = i / kGT;
-    int gx = x0 + lx, gy = y0 + ly;
-    if (gx >= w || gy >= h) continue;
-    float acc = 0.0f;
+  const int x = V * (blockIdx.x * kGabThreads + threadIdx.x), y0 = blockIdx.y * kGabRun;
+  if (x >= w) return;
+  const int xl = mirror1d(x - 1, w), xr = mirror1d(x + V, w);
+  float r[3][V + 2];
+  auto fetch = [&](float* row, int y) {
+    const float* p = in + (size_t)mirror1d(y, h) * w;
+    row[0] = __ldg(p + xl);
+    if constexpr (V == 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p + x));
+      row[1] = v.x;
+      row[2] = v.y;
+      row[3] = v.z;
+      row[4] = v.w;
+    } else {
+      row[1] = __ldg(p + x);
+    }
+    row[V + 1] = __ldg(p + xr);
+  };
+  fetch(r[0], y0 - 1);
+  fetch(r[1], y0);
 #pragma unroll
-    for (int dy = -1; dy <= 1; ++dy)
+  for (int i = 0; i < kGabRun; ++i) {
+    if (y0 + i >= h) return;
+    fetch(r[2], y0 + i + 1);
+    float o[V];
 #pragma unroll
-      for (int dx = -1; dx <= 1; ++dx) {
-        float wt = (dx == 0 && dy == 0) ? centre : ((dx == 0 || dy == 0) ? edge : corner);
-        acc = __fmaf_rn(wt, t[ly + 1 + dy][lx + 1 + dx], acc);
-      }
-    out[(size_t)gy * w + gx] = acc;
+    for (int k = 0; k < V; ++k) {
+      float acc = 0.0f;
+#pragma unroll
+      for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+          const float wt = dx == 1 && dy == 1 ? centre : (dx == 1 || dy == 1 ? edge : corner);
+          acc = __fmaf_rn(wt, r[dy][k + dx], acc);
+        }
+      o[k] = acc;
+    }
+    float* q = out + (size_t)(y0 + i) * w + x;
+    if constexpr (V == 4) *reinterpret_cast<float4*>(q) = make_float4(o[0], o[1], o[2], o[3]);
+    else *q = o[0];
+#pragma unroll
+    for (int k = 0; k < V + 2; ++k) {
+      r[0][k] = r[1][k];
+      r[1][k] = r[2][k];
+    }
   }
 }
 
@@ -638,8 +672,14 @@ void launch_gaborish(const float* in, float* out, int w, int h, cudaStream_t s) 
   const float w1 = 0.115169525f, w2 = 0.061248592f;
   float unnorm = fmaf(4.0f, w2, fmaf(4.0f, w1, 1.0f));
   float scale = 1.0f / unnorm;
-  dim3 grid((w + kGT - 1) / kGT, (h + kGT - 1) / kGT, 3);
-  k_gaborish<<<grid, 256, 0, s>>>(in, out, w, h, scale, w1 * scale, w2 * scale);
+  const bool vec = w % 4 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+  const int cols = kGabThreads * (vec ? 4 : 1);
+  const dim3 grid((w + cols - 1) / cols, (h + kGabRun - 1) / kGabRun, 3);
+  auto run = [&](auto* kernel) {
+    kernel<<<grid, kGabThreads, 0, s>>>(in, out, w, h, scale, w1 * scale, w2 * scale);
+  };
+  if (vec) run(k_gaborish<4>);
+  else run(k_gaborish<1>);
 }
 
 // ---------------------------------------------------------------------------
@@ -651,96 +691,235 @@ void launch_gaborish(const float* in, float* out, int w, int h, cudaStream_t s) 
 // pixel.  Mirrored padding of 3.
 // ---------------------------------------------------------------------------
 
-constexpr int kET = 32;
-constexpr int kEP = 3;
-constexpr int kES = kET + 2 * kEP;
+// A tap and its opposite take one distance: with
+// d_k(p) = sum |t(p+q) - t(p+k+q)| over the cross q (channels outside),
+// d_-k(p) = sum |t(p+q) - t(p-k+q)| has d_k(p-k)'s terms in the same order,
+// |a - b| being |b - a| to the bit.  So step 0's twelve taps need six
+// distance fields and step 1's four need two.  A CTA forms the fields of a
+// 64 x 24 region in shared memory, a thread six rows of one column: each
+// |t - t'| of a column serves the three crosses above one another that hold
+// it, and the lanes' consecutive columns read without conflicts.  It then
+// weighs the taps of the region's inner pixels (a field is read at most two
+// to the left and above, and one to the right).
+// Bound: issue slots (67 %: FMA pipe, reads and the weights' ALU together).
+// Measured, the three steps: 2048x2048 225 -> 155 us, 1920x1080 111 -> 86,
+// 501x333 33 -> 27 (a thread per pixel and every tap's own distance before).
+// Runs of four or eight rows and regions of 20 to 40 rows measured 160 to
+// 166 us at 2048x2048; taller regions leave 1920x1080 a nearly empty wave.
+constexpr int kEpfCols = 64;                     // region columns, a thread each
+constexpr int kEpfRun = 6;                       // region rows of a thread
+constexpr int kEpfRows = 4 * kEpfRun;            // region rows
+constexpr int kEpfThreads = kEpfCols * kEpfRows / kEpfRun;
+constexpr int kEpfTileW = kEpfCols + 8;          // 16-byte columns around the region
+constexpr int kEpfTileH = kEpfRows + 4;          // region rows -1 .. kEpfRows + 2
 
 template <int STEP>
-__global__ void __launch_bounds__(256, 3) k_epf(const float* __restrict__ in, float* __restrict__ out,
-                                             const float* __restrict__ sigma, int w, int h,
-                                             float step_mul4) {
-  __shared__ float t[3][kES][kES + 1];
-  const size_t plane = (size_t)w * h;
-  const int x0 = blockIdx.x * kET, y0 = blockIdx.y * kET;
-  for (int i = threadIdx.x; i < kES * kES; i += blockDim.x) {
-    int lx = i % kES, ly = i / kES;
-    int gx = mirror1d(x0 + lx - kEP, w), gy = mirror1d(y0 + ly - kEP, h);
-    size_t p = (size_t)gy * w + gx;
-    t[0][ly][lx] = in[p];
-    t[1][ly][lx] = in[plane + p];
-    t[2][ly][lx] = in[2 * plane + p];
-  }
-  __syncthreads();
-  const int bw = (w + 7) / 8;
-  const float scale[3] = {40.0f, 5.0f, 3.5f};
-  for (int i = threadIdx.x; i < kET * kET; i += blockDim.x) {
-    int lx = i % kET, ly = i / kET;
-    int gx = x0 + lx, gy = y0 + ly;
-    if (gx >= w || gy >= h) continue;
-    const int cx = lx + kEP, cy = ly + kEP;
-    size_t p = (size_t)gy * w + gx;
-    float bs = sigma[(size_t)(gy / 8) * bw + gx / 8];
-    if (bs < 0.3f) {
-      out[p] = t[0][cy][cx];
-      out[plane + p] = t[1][cy][cx];
-      out[2 * plane + p] = t[2][cy][cx];
-      continue;
-    }
-    const float inv_sigma = step_mul4 / bs;
-    const int rx = gx % 8, ry = gy % 8;
-    const bool at_border = ry == 0 || ry == 7 || rx == 0 || rx == 7;
-    const float pos_mul = at_border ? 2.0f / 3.0f : 1.0f;
-    float sum_w = 0.0f, acc0 = 0.0f, acc1 = 0.0f, acc2 = 0.0f;
-    constexpr int NT = STEP == 0 ? 13 : 5;
-    // J.4.4 kernels: the 5-pixel cross, plus the diagonals and +-2 for step 0.
-    constexpr int tkx[13] = {0, -1, 1, 0, 0, 1, 1, -1, -1, -2, 2, 0, 0};
-    constexpr int tky[13] = {0, 0, 0, -1, 1, -1, 1, 1, -1, 0, 0, 2, -2};
-    auto dist = [&](int kx, int ky) {
-      float d = 0.0f;
+struct EpfSmem {
+  static constexpr int kFields = STEP == 0 ? 6 : (STEP == 1 ? 2 : 0);
+  // Pixels written: the region's columns 2 .. 61 and rows from 2 where fields
+  // are read to their left, right and above, all of it in step 2.
+  static constexpr int kEdge = STEP < 2 ? 2 : 0;
+  static constexpr int kOutW = STEP < 2 ? kEpfCols - 4 : kEpfCols, kOutH = kEpfRows - kEdge;
+  static constexpr int kBlocksW = kOutW / 8 + 2, kBlocksH = kOutH / 8 + 2;
+  float t[3][kEpfTileH][kEpfTileW];
+  float d[kFields > 0 ? kFields : 1][kFields > 0 ? kEpfRows : 1][kEpfCols];
+  float sigma[kBlocksH][kBlocksW], inv[kBlocksH][kBlocksW];  // of the 8x8 blocks under the tile
+};
+
+__device__ __forceinline__ constexpr float epf_scale(int c) {
+  return c == 0 ? 40.0f : (c == 1 ? 5.0f : 3.5f);
+}
+
+// The distance fields of a thread's run of rows of region column x from row
+// y (t's origin is region row -1, column -2): fields (1,0), (0,1) and, for
+// step 0, (1,1), (-1,1), (2,0), (0,2).  Row by row, a cross's north, centre
+// row and south terms enter its sum in the order centre, west, east, north,
+// south.
+template <int STEP>
+__device__ __forceinline__ void epf_fields(EpfSmem<STEP>& sm, int x, int y) {
+  constexpr int NF = EpfSmem<STEP>::kFields;
+  constexpr int kAhead = STEP == 0 ? 2 : 1;  // rows a tap reaches down
+  constexpr int fx[6] = {1, 0, 1, -1, 2, 0}, fy[6] = {0, 1, 1, 1, 0, 2};
+  float d[NF][kEpfRun];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (STEP == 2) {
-          d = __fmaf_rn(fabsf(t[c][cy][cx] - t[c][cy + ky][cx + kx]), scale[c], d);
-        } else {
-          const int ix[5] = {0, -1, 1, 0, 0}, iy[5] = {0, 0, 0, -1, 1};
+  for (int k = 0; k < NF; ++k)
 #pragma unroll
-          for (int q = 0; q < 5; ++q) {
-            float av = t[c][cy + iy[q]][cx + ix[q]];
-            float bv = t[c][cy + ky + iy[q]][cx + kx + ix[q]];
-            d = __fmaf_rn(fabsf(av - bv), scale[c], d);
-          }
-        }
-      }
-      return d;
+    for (int i = 0; i < kEpfRun; ++i) d[k][i] = 0.0f;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float s = epf_scale(c);
+    float r[kAhead + 1][6];  // columns x - 2 .. x + 3
+    auto fetch = [&](float* row, int j) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) row[i] = sm.t[c][y + j][x + i];
     };
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) fetch(r[j], j);
+    float north[NF];
+#pragma unroll
+    for (int j = 0; j < kEpfRun + 2; ++j) {  // run row j - 1
+      if (j + kAhead < kEpfRun + 2 + kAhead) fetch(r[kAhead], j + kAhead);
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        auto diff = [&](int q) { return fabsf(r[0][q] - r[fy[k]][q + fx[k]]); };
+        const float centre = diff(2);
+        if (j >= 2) d[k][j - 2] = __fmaf_rn(centre, s, d[k][j - 2]);
+        if (j >= 1 && j <= kEpfRun) {
+          float& a = d[k][j - 1];
+          a = __fmaf_rn(centre, s, a);
+          a = __fmaf_rn(diff(1), s, a);
+          a = __fmaf_rn(diff(3), s, a);
+          a = __fmaf_rn(north[k], s, a);
+        }
+        north[k] = centre;
+      }
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k)
+#pragma unroll
+        for (int i = 0; i < 6; ++i) r[k][i] = r[k + 1][i];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NF; ++k)
+#pragma unroll
+    for (int i = 0; i < kEpfRun; ++i) sm.d[k][y + i][x] = d[k][i];
+}
+
+template <int STEP>
+__global__ void __launch_bounds__(kEpfThreads, STEP == 0 ? 3 : 4)
+    k_epf(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ sigma,
+          int w, int h, float step_mul4) {
+  extern __shared__ __align__(16) unsigned char epf_smem[];
+  EpfSmem<STEP>& sm = *reinterpret_cast<EpfSmem<STEP>*>(epf_smem);
+  const size_t plane = (size_t)w * h;
+  using Smem = EpfSmem<STEP>;
+  constexpr int kEdge = Smem::kEdge;
+  const int x0 = blockIdx.x * Smem::kOutW, y0 = blockIdx.y * Smem::kOutH;
+  // Tile columns x0-4 .., region rows -1 ..: 16 bytes at a time inside the frame,
+  // else mirrored at its borders, a warp per row.
+  const int tx0 = x0 - 4, ty0 = y0 - kEdge - 1;
+  if (tx0 >= 0 && ty0 >= 0 && tx0 + kEpfTileW <= w && ty0 + kEpfTileH <= h && (w & 3) == 0 &&
+      (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
+    constexpr int kVec = kEpfTileW / 4;
+    const float* src = in + (size_t)ty0 * w + tx0;
+    for (int i = threadIdx.x; i < 3 * kEpfTileH * kVec; i += kEpfThreads) {
+      const int v = i % kVec, r = i / kVec, c = r / kEpfTileH, ly = r - c * kEpfTileH;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.t[c][ly][4 * v]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                   "l"(src + plane * c + (size_t)ly * w + 4 * v)
+                   : "memory");
+    }
+  } else {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int gx[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) gx[i] = mirror1d(tx0 + lane + 32 * i, w);
+    for (int r = warp; r < 3 * kEpfTileH; r += kEpfThreads / 32) {
+      const int c = r / kEpfTileH, ly = r - c * kEpfTileH;
+      const float* row = in + plane * c + (size_t)mirror1d(ty0 + ly, h) * w;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        if (32 * i + lane < kEpfTileW) {
+          const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.t[c][ly][32 * i + lane]);
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(row + gx[i])
+                       : "memory");
+        }
+    }
+  }
+  const int bw = (w + 7) / 8, bh = (h + 7) / 8;
+  constexpr int kBW = Smem::kBlocksW, kBH = Smem::kBlocksH;
+  if (threadIdx.x < kBW * kBH) {
+    const int bx = x0 / 8 + threadIdx.x % kBW, by = y0 / 8 + threadIdx.x / kBW;
+    const float bs = bx < bw && by < bh ? __ldg(sigma + (size_t)by * bw + bx) : 1.0f;
+    sm.sigma[0][threadIdx.x] = bs;
+    sm.inv[0][threadIdx.x] = step_mul4 / bs;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  const int rx = threadIdx.x % kEpfCols, ry = threadIdx.x / kEpfCols * kEpfRun;
+  if constexpr (STEP < 2) {
+    epf_fields<STEP>(sm, rx, ry);
+    __syncthreads();
+  }
+  const int gx = x0 - kEdge + rx;
+  if (rx < kEdge || rx >= kEdge + Smem::kOutW || gx >= w) return;
+  // J.4.4 taps: the 5-pixel cross, plus the diagonals and +-2 for step 0.
+  constexpr int NT = STEP == 0 ? 13 : 5;
+  constexpr int tkx[13] = {0, -1, 1, 0, 0, 1, 1, -1, -1, -2, 2, 0, 0};
+  constexpr int tky[13] = {0, 0, 0, -1, 1, -1, 1, 1, -1, 0, 0, 2, -2};
+  // The field of each tap and where it is read: at the pixel for the
+  // field's own tap, at the pixel plus the tap for the opposite one.
+  constexpr int fld[13] = {0, 0, 0, 1, 1, 3, 2, 3, 2, 4, 4, 5, 5};
+  constexpr bool opp[13] = {false, true,  false, true, false, true, false,
+                            false, true,  true,  false, false, true};
+  const bool side = (gx & 7) == 0 || (gx & 7) == 7;
+  const int bcol = gx / 8 - x0 / 8;
+#pragma unroll 1
+  for (int i = 0; i < kEpfRun; ++i) {
+    const int cy = ry + i, gy = y0 - kEdge + cy;
+    if (cy < kEdge || gy >= h) continue;
+    auto at = [&](int c, int dx, int dy) { return sm.t[c][cy + 1 + dy][rx + 4 - kEdge + dx]; };
+    const int brow = gy / 8 - y0 / 8;
+    const float inv_sigma = sm.inv[brow][bcol];
+    const float pos_mul = side || (gy & 7) == 0 || (gy & 7) == 7 ? 2.0f / 3.0f : 1.0f;
+    auto dist = [&](int tp) {
+      if constexpr (STEP == 2) {
+        float d = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          d = __fmaf_rn(fabsf(at(c, 0, 0) - at(c, tkx[tp], tky[tp])), epf_scale(c), d);
+        return d;
+      } else {
+        return sm.d[fld[tp]][cy + (opp[tp] ? tky[tp] : 0)][rx + (opp[tp] ? tkx[tp] : 0)];
+      }
+    };
+    // A zero distance weighs exactly 1 through the same expression (sigma is
+    // at least 0.3, so its inverse is finite); fmaxf takes 0 for a NaN.
     auto weight = [&](float d) {
-      float sd = pos_mul * d;
-      if (sd == 0.0f) return 1.0f;
-      float v = __fmaf_rn(sd, -inv_sigma, 1.0f);
-      return v > 0.0f ? v : 0.0f;
+      return fmaxf(__fmaf_rn(pos_mul * d, -inv_sigma, 1.0f), 0.0f);
     };
     // The centre tap's distance sums |s - s| over the centre's own patch:
     // exactly 0 (weight 1) when every sample there is finite, not a number
     // otherwise.  The next tap's distance takes |s - s'| of the same samples
     // with positive scales, so it is finite only if they all are; then the
     // centre's terms are skipped, else evaluated as written.
-    const float d1 = dist(tkx[1], tky[1]);
-    float wts[NT];
-    wts[0] = isfinite(d1) ? 1.0f : weight(dist(0, 0));
-    wts[1] = weight(d1);
+    const float d1 = dist(1);
+    float w0 = 1.0f;
+    if (!isfinite(d1)) {
+      float d = 0.0f;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < (STEP == 2 ? 1 : 5); ++k) {
+          constexpr int ix[5] = {0, -1, 1, 0, 0}, iy[5] = {0, 0, 0, -1, 1};
+          const float v = at(c, ix[k], iy[k]);
+          d = __fmaf_rn(fabsf(v - v), epf_scale(c), d);
+        }
+      w0 = weight(d);
+    }
+    float sum_w = 0.0f, acc[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int tp = 0; tp < NT; ++tp) {
-      const int kx = tkx[tp], ky = tky[tp];
-      const float wt = tp < 2 ? wts[tp] : weight(dist(kx, ky));
+      const float wt = tp == 0 ? w0 : weight(tp == 1 ? d1 : dist(tp));
       sum_w += wt;
-      acc0 = __fmaf_rn(t[0][cy + ky][cx + kx], wt, acc0);
-      acc1 = __fmaf_rn(t[1][cy + ky][cx + kx], wt, acc1);
-      acc2 = __fmaf_rn(t[2][cy + ky][cx + kx], wt, acc2);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) acc[c] = __fmaf_rn(at(c, tkx[tp], tky[tp]), wt, acc[c]);
     }
-    out[p] = acc0 / sum_w;
-    out[plane + p] = acc1 / sum_w;
-    out[2 * plane + p] = acc2 / sum_w;
+    const bool copy = sm.sigma[brow][bcol] < 0.3f;
+    const size_t p = (size_t)gy * w + gx;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out[plane * c + p] = copy ? at(c, 0, 0) : acc[c] / sum_w;
   }
+}
+
+cudaError_t configure_render_kernels() {
+  auto allow = [](auto* kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  cudaError_t e;
+  if ((e = allow(k_epf<0>, sizeof(EpfSmem<0>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<1>, sizeof(EpfSmem<1>))) != cudaSuccess) return e;
+  return allow(k_epf<2>, sizeof(EpfSmem<2>));
 }
 
 void launch_epf_step(int step, const float* in, float* out, const float* sigma, int w, int h,
@@ -750,10 +929,15 @@ void launch_epf_step(int step, const float* in, float* out, const float* sigma, 
   float sc = step == 0 ? 0.9f : (step == 1 ? 1.0f : 6.5f);
   float sm = 1.65f * sc;
   float num = sm * 4.0f * (1.0f - sqrtf(0.5f));
-  dim3 grid((w + kET - 1) / kET, (h + kET - 1) / kET);
-  if (step == 0) k_epf<0><<<grid, 256, 0, s>>>(in, out, sigma, w, h, num);
-  else if (step == 1) k_epf<1><<<grid, 256, 0, s>>>(in, out, sigma, w, h, num);
-  else k_epf<2><<<grid, 256, 0, s>>>(in, out, sigma, w, h, num);
+  auto run = [&](auto* kernel, auto smem) {
+    using Smem = decltype(smem);
+    const dim3 grid((w + Smem::type::kOutW - 1) / Smem::type::kOutW,
+                    (h + Smem::type::kOutH - 1) / Smem::type::kOutH);
+    kernel<<<grid, kEpfThreads, sizeof(typename Smem::type), s>>>(in, out, sigma, w, h, num);
+  };
+  if (step == 0) run(k_epf<0>, std::common_type<EpfSmem<0>>{});
+  else if (step == 1) run(k_epf<1>, std::common_type<EpfSmem<1>>{});
+  else run(k_epf<2>, std::common_type<EpfSmem<2>>{});
 }
 
 // ---------------------------------------------------------------------------
