@@ -76,6 +76,7 @@ struct jpxlg_ctx {
   uint64_t launches = 0;
   // tables
   float* d_dq = nullptr;
+  std::vector<float> h_dq;  // the dequantization matrices, as on the device
   std::map<int, float*> lut;          // sRGB -> linear per source depth
   std::map<int, DepthTable> depth;    // output depth classifiers
   // small device words
@@ -87,7 +88,7 @@ struct jpxlg_ctx {
   // workspace
   DevBuf rgb, xyb, pre, coeff, dyhf, qcoeff, lfs, dylf, lfq, cflx, cflb;
   DevBuf planes, aux, sigma, out, llf;
-  DevBuf lf_part, lf_seed, cfl_tile, cover, cover_map;
+  DevBuf lf_part, lf_seed, cfl_tile, cover_map;
   DevBuf pyr, partial, score, cxyb, hpl, bcarry;
   DevBuf pair_ref;  // the reference side of jpxlg_score_pair, kept across calls
   // stage timers
@@ -634,6 +635,7 @@ int jpxlg_ctx_create(int device, uint32_t flags, jpxlg_ctx** out) {
   CKC(cudaSetDevice(device));
   CKC(configure_encode_kernels());
   CKC(configure_render_kernels());
+  CKC(configure_cover_kernels());
   CKC(configure_blur_kernels());
   CKC(configure_tc_kernels());
   CKC(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
@@ -650,7 +652,8 @@ int jpxlg_ctx_create(int device, uint32_t flags, jpxlg_ctx** out) {
   CKC(cudaMemset(c->d_lf, 0, 4 * sizeof(int)));
   CKC(cudaMallocHost(&c->h_words, 16 * sizeof(uint32_t)));
   CKC(cudaMallocHost(&c->h_score, 128 * sizeof(double)));
-  std::vector<float> dq(3 * kDequantTableFloats);
+  std::vector<float>& dq = c->h_dq;
+  dq.resize(3 * kDequantTableFloats);
   build_dequant_tables(dq.data());
   CKC(cudaMalloc(&c->d_dq, dq.size() * sizeof(float)));
   CKC(cudaMemcpy(c->d_dq, dq.data(), dq.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -685,8 +688,7 @@ int jpxlg_ctx_destroy(jpxlg_ctx* ctx) {
   DevBuf* bufs[] = {&ctx->rgb,    &ctx->xyb,   &ctx->pre,     &ctx->coeff,   &ctx->dyhf,
                     &ctx->qcoeff, &ctx->lfs,   &ctx->dylf,    &ctx->lfq,     &ctx->cflx,
                     &ctx->cflb,   &ctx->planes, &ctx->aux,    &ctx->sigma,   &ctx->out,
-                    &ctx->lf_part, &ctx->lf_seed, &ctx->cfl_tile, &ctx->cover,
-                    &ctx->cover_map, &ctx->pyr,  &ctx->pair_ref, &ctx->partial,
+                    &ctx->lf_part, &ctx->lf_seed, &ctx->cfl_tile, &ctx->cover_map, &ctx->pyr,  &ctx->pair_ref, &ctx->partial,
                     &ctx->score,  &ctx->cxyb,   &ctx->hpl,   &ctx->bcarry, &ctx->llf};
   for (DevBuf* b : bufs) b->release();
   for (auto& m : ctx->marks) {
@@ -1276,7 +1278,6 @@ extern "C" int jpxlg_select_blocks(jpxlg_ctx* ctx, int width, int height, const 
   const float* pre = nullptr;
   rc = transform_frame(ctx, g, src, bits, p, &pre);
   if (rc) return rc;
-  CK(ctx->cover.ensure(cover_scratch_bytes(g)));
   uint8_t* map = block_map;
   if (mem == JPXLG_MEM_HOST) {
     CK(ctx->cover_map.ensure(nb));
@@ -1293,8 +1294,7 @@ extern "C" int jpxlg_select_blocks(jpxlg_ctx* ctx, int width, int height, const 
   a.scale[0] = mul * host_qm_multiplier(p->x_qm_scale);
   a.scale[1] = mul;
   a.scale[2] = mul * host_qm_multiplier(p->b_qm_scale);
-  std::vector<float> dq(3 * kDequantTableFloats);
-  build_dequant_tables(dq.data());
+  const std::vector<float>& dq = ctx->h_dq;
   for (int c = 0; c < 3; ++c) {
     double sum = 0.0;
     uint32_t count = 0;
@@ -1311,7 +1311,6 @@ extern "C" int jpxlg_select_blocks(jpxlg_ctx* ctx, int width, int height, const 
       a.w[s][c] = a.lambda[c] * ((double)(side * side) * 1.0);
     }
   }
-  cover_bind_scratch(&a, ctx->cover.p);
   a.map = map;
   a.fallbacks = ctx->d_words + 3;
   a.err = ctx->d_words;

@@ -24,70 +24,95 @@ __device__ __forceinline__ float bias_adjust(int32_t q, float bias) { return bia
 
 // quantize.rs:1400 HfQuantizer::choose (nearest reconstruction, ties to the
 // smaller magnitude) with step = scale * matrix and the zero threshold
-// 0.5 * bias * step, both formed as quantize.rs:334 forms them.
-//
-// The reference centres its candidates {0, e-1, e, e+1} on
-// e = clamp_round(target / step).  The winner is always within one of
-// target / step (a reconstruction bias_adjust(q) * step lies within 0.08
-// steps of q * step), so a centre taken from target * (1 / step), which can
-// differ from e by one only next to a half-integer, yields a candidate set
-// holding the same winner, and the exact error comparison below picks it.
-// `rstep` is 1.0f / step, formed once per cell by the caller.  Quotients
-// near the 2^20 range limit, where the reference's error condition is
-// decided, take the exact division.
-__device__ __forceinline__ int32_t choose(float target, float step, float rstep, float bias,
-                                          uint32_t* err, float* recon) {
+// 0.5 * bias * step, both formed as quantize.rs:334 forms them, as it stands:
+// candidates {0, e-1, e, e+1} around e = clamp_round(target / step), of which
+// only e and its neighbour on the target's side can win, reconstruction
+// levels increasing with q.  Out of line: choose below takes it for quotients
+// beyond its table, for steps that are not positive and finite and for
+// targets that are not finite, where the error conditions are decided.
+static __device__ __noinline__ int32_t choose_general(float target, float step, float bias,
+                                                      uint32_t* err, float* recon) {
+  *recon = 0.0f;
   if (!(isfinite(step) && step > 0.0f)) {
     raise_error(err, kDevBadStep);
-    *recon = 0.0f;
     return 0;
   }
-  float thr = 0.5f * bias * step;
-  if (fabsf(target) <= thr) {
-    *recon = bias_adjust(0, bias) * step;
-    return 0;
-  }
+  if (fabsf(target) <= 0.5f * bias * step) return 0;
   int32_t e;
-  const float va = target * rstep;
-  if (fabsf(va) < 1048000.0f) {
-    e = (int32_t)(signbit(va) ? va - 0.5f : va + 0.5f);
-  } else if (!clamp_round(target / step, &e)) {
+  if (!clamp_round(target / step, &e)) {
     raise_error(err, kDevQuantRange);
-    *recon = 0.0f;
     return 0;
   }
-  // Reconstruction levels increase with q, so of {e-1, e, e+1} only e and
-  // its neighbour on the target's side can be nearest; the third is strictly
-  // farther.  Candidates in the reference's update rule: q = 0 first (its
-  // level is 0, error |target|), then the pair in increasing q.
   const float re = bias_adjust(e, bias) * step;
   const int32_t nb = re < target ? e + 1 : e - 1;
   const float rn = bias_adjust(nb, bias) * step;
+  // Candidates in the reference's update rule: q = 0 first (its level is 0,
+  // error |target|), then the pair in increasing q; |q| > 2^20 is outside
+  // its range.
   int32_t best = 0;
   float best_err = fabsf(target);
-  float best_recon = 0.0f;
-  const int32_t q_lo = min(e, nb), q_hi = max(e, nb);
-  const float r_lo = e < nb ? re : rn, r_hi = e < nb ? rn : re;
-  // (|q| > 2^20 is outside the reference's candidate range; only the exact
-  // path near the limit can reach it.)
-  if (abs(q_lo) <= (1 << 20)) {
-    const float er = fabsf(r_lo - target);
-    if (er < best_err || (er == best_err && abs(q_lo) < abs(best))) {
-      best = q_lo;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int32_t cand = (i == 0) == (e < nb) ? e : nb;
+    const float r = (i == 0) == (e < nb) ? re : rn, er = fabsf(r - target);
+    if (abs(cand) <= (1 << 20) &&
+        (er < best_err || (er == best_err && abs(cand) < abs(best)))) {
+      best = cand;
       best_err = er;
-      best_recon = r_lo;
+      *recon = r;
     }
   }
-  if (abs(q_hi) <= (1 << 20)) {
-    const float er = fabsf(r_hi - target);
-    if (er < best_err || (er == best_err && abs(q_hi) < abs(best))) {
-      best = q_hi;
-      best_err = er;
-      best_recon = r_hi;
-    }
-  }
-  *recon = best_recon;
   return best;
+}
+
+// Entry e of channel c: bias_adjust (reconstruct.rs:50, channel c's bias) at
+// e - 1, e and e + 1 (0 at -1), from the host (upload_dct_constants).
+constexpr int kLevelN = 256;
+extern __device__ float4 g_levels[3][kLevelN];
+
+// 1 / step to an ulp, for choose's centre.
+__device__ __forceinline__ float approx_rcp(float step) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(step));
+  return r;
+}
+
+// choose_general for channel c, with rstep within a few ulps of 1 / step.
+//
+// Everything in it is odd in the target (ties go to the smaller magnitude on
+// either side), so it works on a = |target|.  The levels around a are those
+// of the floor and the ceiling of a / step: a level lies at most 0.08 steps
+// below its integer.  The centre e, a / step rounded with an error of a few
+// 2^-24 of it, is one of the two; the level of e tells which, and one table
+// entry holds the other's level too.  The lower level wins ties; zero, a
+// third candidate, never beats a lower level above it (that level lies
+// below 2a), and the threshold test decides zero against the first.
+__device__ __forceinline__ int32_t choose(int c, float target, float step, float rstep,
+                                          uint32_t* err, float* recon) {
+  const float bias = c_quant_bias[c];
+  const float a = fabsf(target), va = a * rstep;
+  if (!(va < (float)kLevelN - 0.5f && step > 0.0f && step < __int_as_float(0x7f800000)))
+    return choose_general(target, step, bias, err, recon);
+  const int32_t e = (int32_t)(va + 0.5f);
+  const float4 v = __ldg(&g_levels[c][e]);
+  const float re = v.y * step;
+  const bool up = re < a;  // e is the floor
+  const float ro = (up ? v.z : v.x) * step;
+  const float lo = up ? re : ro, hi = up ? ro : re;
+  const bool upper = fabsf(hi - a) < fabsf(lo - a);
+  int32_t q = (up ? e : e - 1) + (upper ? 1 : 0);
+  float r = upper ? hi : lo;
+  if (a <= 0.5f * bias * step) {
+    q = 0;
+    r = 0.0f;
+  }
+  const bool neg = target < 0.0f;
+  *recon = neg ? 0.0f - r : r;  // +0 for zero
+  return neg ? -q : q;
+}
+__device__ __forceinline__ int32_t choose(int c, float target, float step, uint32_t* err,
+                                          float* recon) {
+  return choose(c, target, step, approx_rcp(step), err, recon);
 }
 
 __device__ __forceinline__ uint32_t residual_bits(int32_t q) {

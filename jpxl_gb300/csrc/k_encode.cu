@@ -515,10 +515,12 @@ int launch_precondition(const float* in, float* out, int w, int h, cudaStream_t 
 // Shared quantization rules (jpxl-encode-policy quantize.rs)
 // ---------------------------------------------------------------------------
 
-__constant__ float c_quant_bias[3] = {1.0f - 0.054650073f, 1.0f - 0.0700545f,
-                                      1.0f - 0.049935103f};
+constexpr float kQuantBiasX = 1.0f - 0.054650073f, kQuantBiasY = 1.0f - 0.0700545f,
+                kQuantBiasB = 1.0f - 0.049935103f;
+__constant__ float c_quant_bias[3] = {kQuantBiasX, kQuantBiasY, kQuantBiasB};
 
 __device__ float g_bias_quot[kBiasQuotN];
+__device__ float4 g_levels[3][kLevelN];
 
 // quantize.rs:199 LfQuantizer::quantize with extra_precision 0.
 __device__ __forceinline__ int32_t lf_quantize(float target, float m, uint32_t* err) {
@@ -662,7 +664,6 @@ __global__ void __launch_bounds__(128) k_fdct_luma(EncArgs a, const uint32_t* __
       hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[(size_t)by * geo.bw + bx]);
   const float scale = mul * a.qs.qm[1];
   const float* m = a.dq + kDequantTableFloats + dq_offset(dq_slot(N == 8 ? 0 : (N == 16 ? 4 : 5)));
-  const float bias = c_quant_bias[1];
   // The luma coefficients go through this thread's own row of T so that the
   // quantization loop need not be unrolled N times.
 #pragma unroll
@@ -675,9 +676,9 @@ __global__ void __launch_bounds__(128) k_fdct_luma(EncArgs a, const uint32_t* __
     float recon;
     const float step = scale * __ldg(&m[cell]);
     if (k < n && j < n) {
-      recon = bias_adjust(0, bias) * step;
+      recon = bias_adjust(0, c_quant_bias[1]) * step;
     } else {
-      q = choose(T[g][j][k], step, 1.0f / step, bias, a.err, &recon);
+      q = choose(1, T[g][j][k], step, a.err, &recon);
     }
     a.qcoeff[cplane + ci] = q;
     a.dyhf[ci] = recon;
@@ -988,10 +989,10 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_tile_bits(EncArgs a,
         for (int c = 0; c < 4; ++c) {
           if (c < ncx)
             bits[0][c] += residual_bits(
-                choose(x - kx[c] * dy, step_x, rstep_x, c_quant_bias[0], a.err, &rc));
+                choose(0, x - kx[c] * dy, step_x, rstep_x, a.err, &rc));
           if (c < ncb)
             bits[1][c] += residual_bits(
-                choose(b - kb[c] * dy, step_b, rstep_b, c_quant_bias[2], a.err, &rc));
+                choose(2, b - kb[c] * dy, step_b, rstep_b, a.err, &rc));
         }
       }
     }
@@ -1289,7 +1290,6 @@ __global__ void __launch_bounds__(128) k_quant_chroma(EncArgs a, const uint32_t*
   for (int c = 0; c <= 2; c += 2) {
     const float scale = mul * a.qs.qm[c];
     const float* m = a.dq + c * kDequantTableFloats + off;
-    const float bias = c_quant_bias[c];
 #pragma unroll 4
     for (int k = 0; k < N; ++k) {
       const size_t ci = (size_t)(y0 + k) * geo.W8 + x0 + j;
@@ -1298,7 +1298,7 @@ __global__ void __launch_bounds__(128) k_quant_chroma(EncArgs a, const uint32_t*
         float target = a.coeff[cplane * c + ci] - k_hf[c] * a.dyhf[ci];
         float rc;
         const float step = scale * __ldg(&m[k * N + j]);
-        q = choose(target, step, 1.0f / step, bias, a.err, &rc);
+        q = choose(c, target, step, a.err, &rc);
       }
       a.qcoeff[cplane * c + ci] = q;
     }
@@ -1377,6 +1377,17 @@ void upload_dct_constants(const float* iv4, const float* iv8, const float* iv16,
   quot[0] = 0.0f;
   for (int q = 1; q < kBiasQuotN; ++q) quot[q] = 0.145f / (float)q;
   cudaMemcpyToSymbolAsync(g_bias_quot, quot, sizeof quot, 0, cudaMemcpyHostToDevice, s);
+  // bias_adjust of q and its neighbours, evaluated as bias_adjust_q does.
+  static const float bias[3] = {kQuantBiasX, kQuantBiasY, kQuantBiasB};
+  static float4 levels[3][kLevelN];
+  for (int c = 0; c < 3; ++c) {
+    auto level = [&](int q) {
+      return q <= 0 ? 0.0f : (q == 1 ? 1.0f * bias[c] : (float)q - 0.145f / (float)q);
+    };
+    for (int q = 0; q < kLevelN; ++q)
+      levels[c][q] = make_float4(level(q - 1), level(q), level(q + 1), 0.0f);
+  }
+  cudaMemcpyToSymbolAsync(g_levels, levels, sizeof levels, 0, cudaMemcpyHostToDevice, s);
 }
 
 }  // namespace jpxlg
