@@ -88,7 +88,7 @@ struct jpxlg_ctx {
   // workspace
   DevBuf rgb, xyb, pre, coeff, dyhf, qcoeff, lfs, dylf, lfq, cflx, cflb;
   DevBuf planes, aux, sigma, out, llf;
-  DevBuf lf_part, lf_seed, cfl_tile, cover_map;
+  DevBuf lf_part, lf_seed, cover_map;
   DevBuf pyr, partial, score, cxyb, hpl, bcarry;
   DevBuf pair_ref;  // the reference side of jpxlg_score_pair, kept across calls
   // stage timers
@@ -372,7 +372,6 @@ int encode_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const void* rgb_dev, in
   CK(ctx->dylf.ensure(nb * sizeof(float)));
   CK(ctx->lf_seed.ensure(4 * sizeof(int)));
   CK(ctx->lf_part.ensure(kCflScratchBytes));
-  CK(ctx->cfl_tile.ensure(cfl_tile_scratch_bytes(g.tw * g.th)));
   const float* pre = nullptr;
   int rc = transform_frame(ctx, g, rgb_dev, bits, p, &pre);
   if (rc) return rc;
@@ -416,20 +415,14 @@ int encode_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const void* rgb_dev, in
   }
   stage_end(ctx);
   if (rc) return rc;
+  // The tiles' factors and chroma in one kernel: JPXLG_STAGE_QUANT_CHROMA
+  // stays empty.
   stage_begin(ctx, JPXLG_STAGE_CFL);
   {
-    const int chains[2] = {2, 1};  // the tile chain on the context's stream, the LF one beside
+    const int chains[2] = {2, 1};  // the tiles on the context's stream, the LF chain beside
     const ClassStreams cs = class_fork(ctx, chains, 2);
-    rc = after_launch(ctx, launch_cfl(a, ctx->lf_seed.as<int>(), ctx->lf_part.p,
-                                      ctx->cfl_tile.p, cs.s[0], cs.s[1]));
-    class_join(ctx, cs);
-  }
-  stage_end(ctx);
-  if (rc) return rc;
-  stage_begin(ctx, JPXLG_STAGE_QUANT_CHROMA);
-  {
-    const ClassStreams cs = class_fork(ctx, L->counts, 3);
-    rc = after_launch(ctx, launch_quant_chroma(a, L->lists, L->counts, cs.s));
+    rc = after_launch(ctx, launch_cfl_chroma(a, ctx->lf_seed.as<int>(), ctx->lf_part.p, cs.s[0],
+                                             cs.s[1]));
     class_join(ctx, cs);
   }
   stage_end(ctx);
@@ -688,7 +681,7 @@ int jpxlg_ctx_destroy(jpxlg_ctx* ctx) {
   DevBuf* bufs[] = {&ctx->rgb,    &ctx->xyb,   &ctx->pre,     &ctx->coeff,   &ctx->dyhf,
                     &ctx->qcoeff, &ctx->lfs,   &ctx->dylf,    &ctx->lfq,     &ctx->cflx,
                     &ctx->cflb,   &ctx->planes, &ctx->aux,    &ctx->sigma,   &ctx->out,
-                    &ctx->lf_part, &ctx->lf_seed, &ctx->cfl_tile, &ctx->cover_map, &ctx->pyr,  &ctx->pair_ref, &ctx->partial,
+                    &ctx->lf_part, &ctx->lf_seed, &ctx->cover_map, &ctx->pyr,  &ctx->pair_ref, &ctx->partial,
                     &ctx->score,  &ctx->cxyb,   &ctx->hpl,   &ctx->bcarry, &ctx->llf};
   for (DevBuf* b : bufs) b->release();
   for (auto& m : ctx->marks) {

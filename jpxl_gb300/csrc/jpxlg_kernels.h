@@ -87,15 +87,11 @@ int launch_fdct_luma(const EncArgs& a, const uint32_t* const* lists, const int* 
 // LF CfL partials: kLfCtas CTAs, each 7 double-float sums and 8 bit counts.
 constexpr int kLfCtas = 128;
 constexpr size_t kCflScratchBytes = (size_t)kLfCtas * (7 * 8 + 8 * 4);
-// Per-tile CfL scratch: 8 double-float sums and 2 seeds per 64x64 tile.
-inline size_t cfl_tile_scratch_bytes(int ntiles) { return (size_t)ntiles * (8 * 8 + 2 * 4); }
-// The per-tile chain runs on s, the LF factors' chain on lf_s (it reads
-// only the LF planes); the caller joins lf_s back before the factors are
-// read.
-int launch_cfl(const EncArgs& a, int* lf_seeds, void* lf_scratch, void* tile_scratch,
-               cudaStream_t s, cudaStream_t lf_s);
-int launch_quant_chroma(const EncArgs& a, const uint32_t* const* lists, const int* counts,
-                        const cudaStream_t* s);
+// CfL estimation and the chroma quantization: the tiles' kernel on s, the
+// LF factors' chain and the chroma LF on lf_s (it reads only the LF planes);
+// the caller joins lf_s back.  Returns the number of kernels.
+int launch_cfl_chroma(const EncArgs& a, int* lf_seeds, void* lf_scratch, cudaStream_t s,
+                      cudaStream_t lf_s);
 
 void launch_render_varblocks(const RenderArgs& a, const uint32_t* const* lists,
                              const int* counts, const cudaStream_t* s);

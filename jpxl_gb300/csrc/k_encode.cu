@@ -2,12 +2,13 @@
 //   K1 k_srgb_to_xyb       RGB8/RGB16 -> LUT -> linear -> XYB planes
 //   K2 k_precondition      12 fused Jacobi steps of the inverse Gaborish
 //   K3 k_fdct_luma<N>      gather + DCT_2D + LF samples + luma quantization
-//   K4 k_cfl_*             chroma-from-luma factor estimation
-//   K5 k_quant_chroma<N>   X/B quantization against reconstructed luma
+//   K4 k_cfl_*             chroma-from-luma factor estimation, and with it
+//   K5                     X/B quantization against reconstructed luma
 // Each kernel restates the reference arithmetic it replaces (cited per
 // kernel) in the reference's operation order; the build uses -fmad=false.
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 
 #include "jpxlg_common.cuh"
 #include "jpxlg_internal.h"
@@ -668,20 +669,24 @@ __global__ void __launch_bounds__(128) k_fdct_luma(EncArgs a, const uint32_t* __
   // quantization loop need not be unrolled N times.
 #pragma unroll
   for (int k = 0; k < N; ++k) T[g][j][k] = v[k];
-#pragma unroll 2
-  for (int k = 0; k < N; ++k) {
-    const int cell = k * N + j;
-    const size_t ci = (size_t)(y0 + k) * geo.W8 + x0 + j;
-    int32_t q = 0;
-    float recon;
-    const float step = scale * __ldg(&m[cell]);
-    if (k < n && j < n) {
-      recon = bias_adjust(0, c_quant_bias[1]) * step;
-    } else {
-      q = choose(1, T[g][j][k], step, a.err, &recon);
+#pragma unroll 1
+  for (int k0 = 0; k0 < N; k0 += 4) {
+    float target[4], step[4], recon[4];
+    int32_t q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      target[i] = T[g][j][k0 + i];
+      step[i] = scale * __ldg(&m[(k0 + i) * N + j]);
+      // the LLF corner: level 0, from a target under every threshold
+      if (k0 + i < n && j < n) target[i] = 0.0f;
     }
-    a.qcoeff[cplane + ci] = q;
-    a.dyhf[ci] = recon;
+    choose_n<4>(1, target, step, a.err, q, recon);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const size_t ci = (size_t)(y0 + k0 + i) * geo.W8 + x0 + j;
+      a.qcoeff[cplane + ci] = q[i];
+      a.dyhf[ci] = recon[i];
+    }
   }
 }
 
@@ -757,306 +762,366 @@ __device__ int best_factor(const RegSums& s, float base, double slack_yy, double
   return best;
 }
 
+// best_factor by eight lanes (a lane per candidate; `sub` is the lane's place
+// among them, the group aligned): the candidates' energies are independent,
+// and the choice goes over them in the same order afterwards.
+__device__ __forceinline__ int best_factor_lanes(unsigned mask, int sub, const RegSums& s,
+                                                 float base, double slack_yy, double slack_yc,
+                                                 double slack_cc, bool* robust) {
+  int star_cand = 0;
+  *robust = true;
+  double energy = 0.0;
+  if (s.s_yy > 0.0) {
+    const double cf = 84.0;
+    const double k_ls = s.s_yc / s.s_yy;
+    const double star = (k_ls - (double)base) * cf;
+    const double dk = (slack_yc + fabs(k_ls) * slack_yy) / s.s_yy;
+    const double dstar = cf * dk * 1.01 + 1e-12 * (1.0 + fabs(star));
+    const double kk = fabs(k_ls) + 2.0;
+    const double e_round = 8.0 * 1.1102230246251565e-16 *
+                           (s.s_cc + slack_cc + 2.0 * kk * (fabs(s.s_yc) + slack_yc) +
+                            kk * kk * (s.s_yy + slack_yy));
+    const double tie = e_round * cf * cf / (2.0 * s.s_yy);
+    const double dist = fabs((star - floor(star)) - 0.5);
+    if (dist <= dstar + tie || !isfinite(star)) *robust = false;
+    long long c = (long long)round(star) + (sub - 2);
+    c = c < -128 ? -128 : (c > 127 ? 127 : c);
+    star_cand = sub < 5 ? (int)c : 0;
+    const double k = (double)((float)base + (float)star_cand / 84.0f);
+    energy = s.s_cc - 2.0 * k * s.s_yc + k * k * s.s_yy;
+  }
+  int best = 0;
+  double best_e = 0.0;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    const int cand = __shfl_sync(mask, star_cand, i, 8);
+    const double e = __shfl_sync(mask, energy, i, 8);
+    const int ac = cand < 0 ? -cand : cand, ab = best < 0 ? -best : best;
+    if (i == 0 || e < best_e || (e == best_e && ac < ab)) {
+      best = cand;
+      best_e = e;
+    }
+  }
+  return s.s_yy > 0.0 ? best : 0;  // as best_factor: all terms zero
+}
+
 __device__ __forceinline__ uint32_t factor_bits(int32_t f) {
   if (f == 0) return 0;
   uint32_t af = (uint32_t)(f < 0 ? -f : f);
   return (32u - __clz(af)) + 2u;
 }
 
-// Whether coefficient-image cell (px, py) is in the n x n LLF corner of its
-// varblock; *lg = log2 of the varblock side in blocks (DCT8 0, DCT16 1,
-// DCT32 2).  Square varblocks only (the encoder's cover); origins are
-// naturally aligned, so positions within the varblock are masks.
-__device__ __forceinline__ bool cell_is_llf(const uint8_t* map, int bw, int px, int py, int* lg) {
-  const int sel = map[(size_t)(py >> 3) * bw + (px >> 3)] & 0x1f;
-  const int l = sel == 0 ? 0 : (sel == 4 ? 1 : 2);
-  *lg = l;
-  const int mask = (8 << l) - 1;
-  return (px & mask) < (1 << l) && (py & mask) < (1 << l);
-}
-
 constexpr int kCflThreads = 256;
 
-// Per 64x64 tile in three kernels: (1) the HF regression sums (X and B
-// against source Y) in double-float, one CTA per tile; (2) the seeds, one
-// thread per tile and channel, so that the f64 arithmetic of best_factor and
-// its robustness bound overlaps across tiles instead of holding a CTA at a
-// barrier; (3) the residual bit costs of the candidate windows and the
-// choice, one CTA per tile.
+// One CTA per 64x64 tile, from the coefficients to the quantized chroma:
+// (1) the HF regression sums (X and B against source Y) in double-float;
+// (2) the seeds; (3) the residual bit costs of the candidate windows and the
+// choice; (4) K5, the X and B cells against the chosen factors.  The tile's
+// four planes arrive once, by cp.async, and stay in shared memory; the
+// steps' latencies (the seeds' f64 chain above all) hide behind the SM's
+// other tiles.
+// Bound: issue slots (ten quantizer choices a cell).  Measured, with the LF
+// chain beside it: MEASURED_CFL
+constexpr int kCflSide = 64;
+struct CflSmem {
+  float p[4][kCflSide][kCflSide];        // X, Y, B coefficients, reconstructed luma
+  float step[2][64], rstep[2][64];       // baseline quantizer, DCT8x8 cells
+  float mul[64];                         // hf multiplier of each 8x8 block's varblock
+  uint8_t lg[64];                        // log2 of its side in blocks
+  DF part[kCflThreads / 32][8];
+  uint32_t bits[kCflThreads / 32][8];
+  int seed[2], factor[2];
+};
 
-// (1) sums[tile][8]: s_yy, s_yx, s_xx, s_yb, s_bb, sum|yx|, sum|yb|, count.
-__global__ void __launch_bounds__(kCflThreads) k_cfl_tile_sums(EncArgs a, DF* __restrict__ sums) {
-  __shared__ DF s_part[kCflThreads / 32][8];
-  const Geo& geo = a.geo;
-  const int tx = blockIdx.x, ty = blockIdx.y;
-  const int tile = ty * geo.tw + tx;
-  if (*a.not_gray == 0u || !a.cfl_enabled) return;
-  const size_t cplane = (size_t)geo.W8 * geo.H8;
-  const int px0 = tx * 64, py0 = ty * 64;
-  const int pw = min(64, geo.W8 - px0), ph = min(64, geo.H8 - py0);
-  // Thread t covers column (t % 64) of rows t/64, t/64 + 4, ... of the tile:
-  // coalesced rows, no divisions.
-  DF syy{0, 0}, syx{0, 0}, sxx{0, 0}, syb{0, 0}, sbb{0, 0};
-  float ayx = 0.0f, ayb = 0.0f, cnt = 0.0f;
-  {
-    const int col = threadIdx.x % 64;
-    if (col < pw) {
-      const int px = px0 + col;
-      for (int row = threadIdx.x / 64; row < ph; row += kCflThreads / 64) {
-        const int py = py0 + row;
-        int lg;
-        if (cell_is_llf(a.block_map, geo.bw, px, py, &lg)) continue;
-        size_t ci = (size_t)py * geo.W8 + px;
-        float y = a.coeff[cplane + ci];
-        float x = a.coeff[ci];
-        float b = a.coeff[2 * cplane + ci];
-        syy = df_add(syy, df_two_prod(y, y));
-        syx = df_add(syx, df_two_prod(y, x));
-        sxx = df_add(sxx, df_two_prod(x, x));
-        syb = df_add(syb, df_two_prod(y, b));
-        sbb = df_add(sbb, df_two_prod(b, b));
-        ayx += fabsf(y * x);
-        ayb += fabsf(y * b);
-        cnt += 1.0f;
-      }
-    }
-  }
-  // One fixed-order reduction: a butterfly per warp, then the warps in order.
-  DF v[8] = {syy, syx, sxx, syb, sbb, DF{ayx, 0.0f}, DF{ayb, 0.0f}, DF{cnt, 0.0f}};
-  const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+// Eight double-float sums over a warp in the order of an xor butterfly, each
+// step handing half of the remaining quantities to the partner lane.  Every
+// fourth lane ends with the total of quantity *q = lane >> 2.
+__device__ __forceinline__ DF warp_sum8(DF* v, int lane, int* q) {
+  const unsigned full = 0xffffffffu;
+  auto swap = [&](DF x, int o) {
+    return DF{__shfl_xor_sync(full, x.hi, o), __shfl_xor_sync(full, x.lo, o)};
+  };
+  int base = 0;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const DF t = df_warp_sum(v[q]);
-    if (lane == 0) s_part[wid][q] = t;
+  for (int o = 16, n = 4; o >= 4; o >>= 1, n >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const DF keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+      v[i] = df_add(keep, swap(send, o));
+    }
+    base += up ? n : 0;
   }
-  __syncthreads();
-  if (threadIdx.x < 8) {
-    DF t = s_part[0][threadIdx.x];
-    for (int i = 1; i < kCflThreads / 32; ++i) t = df_add(t, s_part[i][threadIdx.x]);
-    sums[(size_t)tile * 8 + threadIdx.x] = t;
-  }
+  DF x = v[0];
+  x = df_add(x, swap(x, 2));
+  x = df_add(x, swap(x, 1));
+  *q = base;
+  return x;
 }
 
-// (2) seeds[tile][2] from the sums; a seed the bound cannot settle is
-// recomputed from the tile's coefficients in the reference's order
-// (varblocks in raster order of their origins within the tile, then
-// coefficient rows and columns).
-__global__ void __launch_bounds__(128) k_cfl_tile_seeds(EncArgs a, const DF* __restrict__ sums,
-                                                        int* __restrict__ seeds) {
+__global__ void __launch_bounds__(kCflThreads, 3) k_cfl_tile(const __grid_constant__ EncArgs a) {
+  extern __shared__ __align__(16) unsigned char cfl_smem[];
+  CflSmem& sm = *reinterpret_cast<CflSmem*>(cfl_smem);
   const Geo& geo = a.geo;
-  const int ntiles = geo.tw * geo.th;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 2 * ntiles) return;
-  const int tile = i >> 1, ch = i & 1;
-  if (*a.not_gray == 0u || !a.cfl_enabled) {
-    seeds[i] = 0;
-    return;
-  }
-  const DF* t = sums + (size_t)tile * 8;
-  const double t_syy = df_value(t[0]), t_syc = df_value(t[ch == 0 ? 1 : 3]);
-  const double t_scc = df_value(t[ch == 0 ? 2 : 4]), t_ayc = df_value(t[ch == 0 ? 5 : 6]);
-  const double t_cnt = df_value(t[7]);
-  // Distance of the double-float tree sum and of the reference's sequential
-  // f64 sum from the exact sum, relative to sum|t| (the |t| sums are f32
-  // estimates; the factor 2 covers their error).
-  const double gam = 2.0 * (t_cnt + 64.0) * (2.2737367544323206e-13 + 1.1102230246251565e-16);
-  const float base = ch == 0 ? 0.0f : 1.0f;
-  int seed = 0;
-  bool robust = true;
-  if (t_cnt > 0.0) {
-    RegSums r{t_syy, t_syc, t_scc, t_ayc, t_cnt};
-    seed = best_factor(r, base, gam * t_syy, gam * t_ayc, gam * t_scc, &robust);
-  }
-  if (!robust) {
-    atomicAdd(a.cfl_fallbacks, 1u);
-    const size_t cplane = (size_t)geo.W8 * geo.H8;
-    const int tx = tile % geo.tw, ty = tile / geo.tw;
-    const int px0 = tx * 64, py0 = ty * 64;
-    const int pw = min(64, geo.W8 - px0), ph = min(64, geo.H8 - py0);
-    const float* cc = a.coeff + (ch == 0 ? 0 : 2 * cplane);
-    RegSums r{0, 0, 0, 0, 0};
-    for (int by = py0 / 8; by < (py0 + ph) / 8; ++by)
-      for (int bx = px0 / 8; bx < (px0 + pw) / 8; ++bx) {
-        uint8_t e = a.block_map[(size_t)by * geo.bw + bx];
-        if (!(e & 0x80)) continue;
-        int sel = e & 0x1f;
-        int nb = sel == 0 ? 1 : (sel == 4 ? 2 : 4), side = nb * 8;
-        for (int row = 0; row < side; ++row)
-          for (int col = (row < nb ? nb : 0); col < side; ++col) {
-            size_t ci = (size_t)(by * 8 + row) * geo.W8 + bx * 8 + col;
-            double y = (double)a.coeff[cplane + ci];
-            double c = (double)cc[ci];
-            r.s_yy += y * y;
-            r.s_yc += y * c;
-            r.s_cc += c * c;
-            r.n += 1.0;
-          }
-      }
-    bool unused;
-    seed = r.n > 0 ? best_factor(r, base, 0, 0, 0, &unused) : 0;
-  }
-  seeds[i] = seed;
-}
-
-// (3) Residual bits of every candidate through the DCT8x8 baseline quantizer
-// (cells folded onto the 8x8 grid, lib.rs:3585), then the choice.
-__global__ void __launch_bounds__(kCflThreads, 4) k_cfl_tile_bits(EncArgs a,
-                                                               const int* __restrict__ seeds) {
-  __shared__ uint32_t s_bits[kCflThreads / 32][8];
-  __shared__ float s_step[2][64], s_rstep[2][64];
-  const Geo& geo = a.geo;
-  const int tx = blockIdx.x, ty = blockIdx.y;
-  const int tile = ty * geo.tw + tx;
-  if (*a.not_gray == 0u || !a.cfl_enabled) {
-    if (threadIdx.x == 0) {
-      a.cfl_x[tile] = 0;
-      a.cfl_b[tile] = 0;
-    }
-    return;
-  }
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int tx = blockIdx.x, ty = blockIdx.y, tile = ty * geo.tw + tx;
   const size_t cplane = (size_t)geo.W8 * geo.H8;
-  const int px0 = tx * 64, py0 = ty * 64;
-  const int pw = min(64, geo.W8 - px0), ph = min(64, geo.H8 - py0);
-  // lib.rs:3735 factor_candidates(seed, -128, 127): seed-1, seed, seed+1
-  // clamped and de-duplicated, then 0 if absent (every thread forms both).
-  int cands[2][4], ncand[2];
-  const int seed[2] = {seeds[2 * tile], seeds[2 * tile + 1]};
-#pragma unroll
-  for (int ch = 0; ch < 2; ++ch) {
-    int nc = 0;
-    for (int d = -1; d <= 1; ++d) {
-      int v = min(max(seed[ch] + d, -128), 127);
-      bool dup = false;
-      for (int i = 0; i < nc; ++i) dup |= cands[ch][i] == v;
-      if (!dup) cands[ch][nc++] = v;
-    }
-    bool has0 = false;
-    for (int i = 0; i < nc; ++i) has0 |= cands[ch][i] == 0;
-    if (!has0) cands[ch][nc++] = 0;
-    ncand[ch] = nc;
+  const int px0 = tx * kCflSide, py0 = ty * kCflSide;
+  const int pw = min(kCflSide, geo.W8 - px0), ph = min(kCflSide, geo.H8 - py0);
+  const size_t origin = (size_t)py0 * geo.W8 + px0;
+  for (int i = t; i < 4 * kCflSide * kCflSide / 4; i += kCflThreads) {
+    const int x = 4 * (i % (kCflSide / 4)), y = i / (kCflSide / 4) % kCflSide,
+              c = i / (kCflSide * kCflSide / 4);
+    if (x >= pw || y >= ph) continue;
+    const float* src = (c < 3 ? a.coeff + cplane * c : a.dyhf) + origin + (size_t)y * geo.W8 + x;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.p[c][y][x]);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
   }
-  // Steps of the 64 folded cells and their reciprocals, per channel.
-  if (threadIdx.x < 128) {
-    const int ch = threadIdx.x / 64, cell = threadIdx.x % 64;
+  // Each block's varblock (square, naturally aligned: its origin is the
+  // block position with the low bits cleared).
+  if (t < 64) {
+    const int bx = px0 / 8 + t % 8, by = py0 / 8 + t / 8;
+    int l = 0;
+    float mul = 1.0f;
+    if (bx < geo.bw && by < geo.bh) {
+      const int sel = a.block_map[(size_t)by * geo.bw + bx] & 0x1f;
+      l = sel == 0 ? 0 : (sel == 4 ? 1 : 2);
+      const int clear = ~((1 << l) - 1);
+      mul = hf_multiplier(a.mul_table, a.qs.global_scale,
+                          a.hf_mul[(size_t)(by & clear) * geo.bw + (bx & clear)]);
+    }
+    sm.lg[t] = (uint8_t)l;
+    sm.mul[t] = mul;
+  }
+  // Baseline steps of the 64 folded cells and their reciprocals.
+  if (t >= 128) {
+    const int ch = (t - 128) / 64, cell = t % 64;
     const float scale = a.base_mul * a.qs.qm[ch == 0 ? 0 : 2];
     const float st = scale * a.dq[(ch == 0 ? 0 : 2) * kDequantTableFloats + cell];
-    s_step[ch][cell] = st;
-    s_rstep[ch][cell] = 1.0f / st;
+    sm.step[ch][cell] = st;
+    sm.rstep[ch][cell] = 1.0f / st;
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  uint32_t bits[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-  float kx[4], kb[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    kx[i] = 0.0f + (float)cands[0][i < ncand[0] ? i : 0] / 84.0f;
-    kb[i] = 1.0f + (float)cands[1][i < ncand[1] ? i : 0] / 84.0f;
-  }
-  const bool need_x = seed[0] != 0, need_b = seed[1] != 0;
-  const int ncx = need_x ? ncand[0] : 0, ncb = need_b ? ncand[1] : 0;
-  if (need_x || need_b) {
-    const int col = threadIdx.x % 64;
-    if (col < pw) {
-      const int px = px0 + col;
-      // Each row's block-map entry and three samples are loaded a row ahead
-      // of its quantizer evaluations, so that their latency overlaps them.
-      struct Cell {
-        uint8_t sel;
-        float dy, x, b;
-      };
-      auto fetch = [&](int row) {
-        const int py = py0 + row;
-        const size_t ci = (size_t)py * geo.W8 + px;
-        return Cell{a.block_map[(size_t)(py >> 3) * geo.bw + (px >> 3)], a.dyhf[ci], a.coeff[ci],
-                    a.coeff[2 * cplane + ci]};
-      };
-      int row = threadIdx.x / 64;
-      Cell nxt = row < ph ? fetch(row) : Cell{0, 0.0f, 0.0f, 0.0f};
-      for (; row < ph; row += kCflThreads / 64) {
-        const int py = py0 + row;
-        const Cell cur = nxt;
-        if (row + kCflThreads / 64 < ph) nxt = fetch(row + kCflThreads / 64);
-        // cell_is_llf on the prefetched block-map entry.
-        const int sel = cur.sel & 0x1f;
-        const int lg = sel == 0 ? 0 : (sel == 4 ? 1 : 2);
-        const int mask = (8 << lg) - 1;
-        if ((px & mask) < (1 << lg) && (py & mask) < (1 << lg)) continue;
-        const int cell8 = ((py & mask) >> lg) * 8 + ((px & mask) >> lg);
-        const float dy = cur.dy, x = cur.x, b = cur.b;
-        const float step_x = s_step[0][cell8], rstep_x = s_rstep[0][cell8];
-        const float step_b = s_step[1][cell8], rstep_b = s_rstep[1][cell8];
-        float rc;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (c < ncx)
-            bits[0][c] += residual_bits(
-                choose(0, x - kx[c] * dy, step_x, rstep_x, a.err, &rc));
-          if (c < ncb)
-            bits[1][c] += residual_bits(
-                choose(2, b - kb[c] * dy, step_b, rstep_b, a.err, &rc));
-        }
+  const bool on = *a.not_gray != 0u && a.cfl_enabled;
+  // Thread t covers column t % 64 of rows t / 64, t / 64 + 4, ...
+  const int col = t % kCflSide, row0 = t / kCflSide;
+  constexpr int kStep = kCflThreads / kCflSide;
+  int seed[2] = {0, 0};
+  if (on) {
+    // (1) s_yy, s_yx, s_xx, s_yb, s_bb, sum|yx|, sum|yb|, count.
+    DF v[8] = {};
+    if (col < pw)
+#pragma unroll 2
+      for (int row = row0; row < ph; row += kStep) {
+        const int l = sm.lg[(row >> 3) * 8 + (col >> 3)], mask = (8 << l) - 1;
+        if ((col & mask) < (1 << l) && (row & mask) < (1 << l)) continue;  // LLF
+        const float x = sm.p[0][row][col], y = sm.p[1][row][col], b = sm.p[2][row][col];
+        v[0] = df_add(v[0], df_two_prod(y, y));
+        v[1] = df_add(v[1], df_two_prod(y, x));
+        v[2] = df_add(v[2], df_two_prod(x, x));
+        v[3] = df_add(v[3], df_two_prod(y, b));
+        v[4] = df_add(v[4], df_two_prod(b, b));
+        v[5].hi += fabsf(y * x);
+        v[6].hi += fabsf(y * b);
+        v[7].hi += 1.0f;
       }
+    int q;
+    const DF w = warp_sum8(v, lane, &q);
+    if ((lane & 3) == 0) sm.part[warp][q] = w;
+    __syncthreads();
+    // (2) Eight lanes for X's seed, eight for B's; a seed the bound cannot
+    // settle is recomputed from the tile's coefficients in the reference's
+    // order (varblocks in raster order of their origins within the tile,
+    // then coefficient rows and columns).
+    if (warp == 0) {
+      DF sum = sm.part[0][lane & 7];
+      for (int i = 1; i < kCflThreads / 32; ++i) sum = df_add(sum, sm.part[i][lane & 7]);
+      const double value = df_value(sum);
+      auto total = [&](int k) { return __shfl_sync(0xffffffffu, value, k); };
+      const int ch = lane >> 3 & 1;
+      const double t0 = total(0), t1 = total(1), t2 = total(2), t3 = total(3), t4 = total(4),
+                   t5 = total(5), t6 = total(6), t7 = total(7);
+      RegSums r{t0, ch ? t3 : t1, ch ? t4 : t2, ch ? t6 : t5, t7};
+      // Distance of the double-float tree sum and of the reference's
+      // sequential f64 sum from the exact sum, relative to sum|t| (the |t|
+      // sums are f32 estimates; the factor 2 covers their error).
+      const double gam = 2.0 * (r.n + 64.0) * (2.2737367544323206e-13 + 1.1102230246251565e-16);
+      bool robust;
+      int sd = best_factor_lanes(0xffffffffu, lane & 7, r, ch ? 1.0f : 0.0f, gam * r.s_yy,
+                                 gam * r.a_yc, gam * r.s_cc, &robust);
+      if (!(r.n > 0.0)) sd = 0;
+      else if (!robust && (lane & 7) == 0 && lane < 16) {
+        atomicAdd(a.cfl_fallbacks, 1u);
+        RegSums e{0, 0, 0, 0, 0};
+        for (int by = 0; by < ph / 8; ++by)
+          for (int bx = 0; bx < pw / 8; ++bx) {
+            const uint8_t m = a.block_map[(size_t)(py0 / 8 + by) * geo.bw + px0 / 8 + bx];
+            if (!(m & 0x80)) continue;
+            const int nb = 1 << sm.lg[by * 8 + bx], side = nb * 8;
+            for (int row = 0; row < side; ++row)
+              for (int cc = (row < nb ? nb : 0); cc < side; ++cc) {
+                const double y = (double)sm.p[1][by * 8 + row][bx * 8 + cc];
+                const double c = (double)sm.p[ch ? 2 : 0][by * 8 + row][bx * 8 + cc];
+                e.s_yy += y * y;
+                e.s_yc += y * c;
+                e.s_cc += c * c;
+                e.n += 1.0;
+              }
+          }
+        bool unused;
+        sd = e.n > 0 ? best_factor(e, ch ? 1.0f : 0.0f, 0, 0, 0, &unused) : 0;
+      }
+      if ((lane & 7) == 0 && lane < 16) sm.seed[ch] = sd;
     }
+    __syncthreads();
+    seed[0] = sm.seed[0];
+    seed[1] = sm.seed[1];
   }
-  // Integer sums (exact in any order): butterflies, then warps in order.
-  // A tile holds at most 4096 cells of at most 22 bits, so 32 bits suffice.
-  {
-    uint32_t v[8];
+  // (3) Residual bits of every candidate through the DCT8x8 baseline quantizer
+  // (cells folded onto the 8x8 grid, lib.rs:3585), then the choice.
+  // lib.rs:3735 factor_candidates(seed, -128, 127): seed-1, seed, seed+1
+  // clamped and de-duplicated, then 0 if absent (every thread forms both).
+  if (seed[0] != 0 || seed[1] != 0) {
+    int cands[2][4], ncand[2];
+#pragma unroll
+    for (int ch = 0; ch < 2; ++ch) {
+      int nc = 0;
+      for (int d = -1; d <= 1; ++d) {
+        int v = min(max(seed[ch] + d, -128), 127);
+        bool dup = false;
+        for (int i = 0; i < nc; ++i) dup |= cands[ch][i] == v;
+        if (!dup) cands[ch][nc++] = v;
+      }
+      bool has0 = false;
+      for (int i = 0; i < nc; ++i) has0 |= cands[ch][i] == 0;
+      if (!has0) cands[ch][nc++] = 0;
+      ncand[ch] = nc;
+    }
+    uint32_t bits[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    float kx[4], kb[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      kx[i] = 0.0f + (float)cands[0][i < ncand[0] ? i : 0] / 84.0f;
+      kb[i] = 1.0f + (float)cands[1][i < ncand[1] ? i : 0] / 84.0f;
+    }
+    if (col < pw)
+#pragma unroll 1
+      for (int row = row0; row < ph; row += kStep) {
+        const int l = sm.lg[(row >> 3) * 8 + (col >> 3)], mask = (8 << l) - 1;
+        if ((col & mask) < (1 << l) && (row & mask) < (1 << l)) continue;  // LLF
+        const int cell8 = ((row & mask) >> l) * 8 + ((col & mask) >> l);
+        const float x = sm.p[0][row][col], b = sm.p[2][row][col], dy = sm.p[3][row][col];
+        const float step_x = sm.step[0][cell8], rstep_x = sm.rstep[0][cell8];
+        const float step_b = sm.step[1][cell8], rstep_b = sm.rstep[1][cell8];
+        auto cost = [&](int ch, float v, const float* k, float step, float rstep) {
+          bool ok = true;
+          uint32_t n[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const Choice q(ch, v - k[c] * dy, step, rstep);
+            ok = ok && q.ok;
+            n[c] = q.bits();
+          }
+          if (!ok)
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+              float rc;
+              n[c] = residual_bits(
+                  choose_general(v - k[c] * dy, step, c_quant_bias[ch], a.err, &rc));
+            }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) bits[ch / 2][c] += n[c];
+        };
+        if (seed[0] != 0) cost(0, x, kx, step_x, rstep_x);
+        if (seed[1] != 0) cost(2, b, kb, step_b, rstep_b);
+      }
+    // Integer sums, exact in any order.  A tile holds at most 4096 cells of at
+    // most 22 bits, so 32 bits suffice.
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      v[q] = bits[q / 4][q % 4];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+      const uint32_t v = __reduce_add_sync(0xffffffffu, bits[q / 4][q % 4]);
+      if (lane == 0) sm.bits[warp][q] = v;
     }
-    const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) s_bits[wid][q] = v[q];
     __syncthreads();
-  }
-  if (threadIdx.x % 32 == 0 && threadIdx.x < 64) {
-    const int ch = threadIdx.x / 32;
-    unsigned long long tot[4];
-    for (int c = 0; c < 4; ++c) {
-      unsigned long long t = 0;
-      for (int i = 0; i < kCflThreads / 32; ++i) t += s_bits[i][ch * 4 + c];
-      tot[c] = t;
-    }
-    int result = 0;
-    if (seed[ch] != 0) {
-      // lib.rs:3966 refine_hf_factor: cost(0) first, then each non-zero
-      // candidate needs residual + factor bits strictly below (ties to the
-      // smaller magnitude).
-      unsigned long long best_cost = 0;
-      for (int c = 0; c < ncand[ch]; ++c)
-        if (cands[ch][c] == 0) best_cost = tot[c];
-      int best_f = 0;
-      for (int c = 0; c < ncand[ch]; ++c) {
-        int f = cands[ch][c];
-        if (f == 0) continue;
-        unsigned long long fb = factor_bits(f);
-        unsigned long long cutoff = best_cost > fb ? best_cost - fb : 0;
-        if (tot[c] > cutoff) continue;
-        unsigned long long cost = tot[c] + fb;
-        int af = f < 0 ? -f : f, ab = best_f < 0 ? -best_f : best_f;
-        if (cost < best_cost || (cost == best_cost && af < ab)) {
-          best_cost = cost;
-          best_f = f;
-        }
+    if (lane == 0 && warp < 2) {
+      const int ch = warp;
+      uint32_t tot[4];
+      for (int c = 0; c < 4; ++c) {
+        tot[c] = 0;
+        for (int i = 0; i < kCflThreads / 32; ++i) tot[c] += sm.bits[i][ch * 4 + c];
       }
-      result = best_f;
+      int result = 0;
+      if (seed[ch] != 0) {
+        // lib.rs:3966 refine_hf_factor: cost(0) first, then each non-zero
+        // candidate needs residual + factor bits strictly below (ties to the
+        // smaller magnitude).
+        unsigned long long best_cost = 0;
+        for (int c = 0; c < ncand[ch]; ++c)
+          if (cands[ch][c] == 0) best_cost = tot[c];
+        int best_f = 0;
+        for (int c = 0; c < ncand[ch]; ++c) {
+          int f = cands[ch][c];
+          if (f == 0) continue;
+          unsigned long long fb = factor_bits(f);
+          unsigned long long cutoff = best_cost > fb ? best_cost - fb : 0;
+          if (tot[c] > cutoff) continue;
+          unsigned long long cost = tot[c] + fb;
+          int af = f < 0 ? -f : f, ab = best_f < 0 ? -best_f : best_f;
+          if (cost < best_cost || (cost == best_cost && af < ab)) {
+            best_cost = cost;
+            best_f = f;
+          }
+        }
+        result = best_f;
+      }
+      sm.factor[ch] = result;
     }
-    if (ch == 0) a.cfl_x[tile] = (int8_t)result;
-    else a.cfl_b[tile] = (int8_t)result;
+  } else if (t < 2) {
+    sm.factor[t] = 0;
+  }
+  __syncthreads();
+  if (t < 2) (t == 0 ? a.cfl_x : a.cfl_b)[tile] = (int8_t)sm.factor[t];
+  // (4) K5 — the HF half of lib.rs:3237 quantize_square_varblock for chroma:
+  // targets c - k*dY (no FMA), nearest choice; the LLF corners stay zero.
+  if (col >= pw) return;
+  const float k_x = 0.0f + (float)sm.factor[0] / 84.0f, k_b = 1.0f + (float)sm.factor[1] / 84.0f;
+  const float qm_x = a.qs.qm[0], qm_b = a.qs.qm[2];
+#pragma unroll 2
+  for (int row = row0; row < ph; row += kStep) {
+    const int blk = (row >> 3) * 8 + (col >> 3);
+    const int l = sm.lg[blk], mask = (8 << l) - 1, k = row & mask, j = col & mask;
+    int32_t qx = 0, qb = 0;
+    if (!(k < (1 << l) && j < (1 << l))) {
+      const float mul = sm.mul[blk], dy = sm.p[3][row][col];
+      const float* m = a.dq + dq_offset(l) + (k << (3 + l)) + j;  // slots 0, 1, 2: the squares
+      const float step_x = mul * qm_x * __ldg(m);
+      const float step_b = mul * qm_b * __ldg(m + 2 * kDequantTableFloats);
+      const float vx = sm.p[0][row][col] - k_x * dy, vb = sm.p[2][row][col] - k_b * dy;
+      const Choice cx(0, vx, step_x, approx_rcp(step_x)), cb(2, vb, step_b, approx_rcp(step_b));
+      qx = cx.q(vx);
+      qb = cb.q(vb);
+      if (!(cx.ok && cb.ok)) {
+        float rc;
+        qx = choose_general(vx, step_x, c_quant_bias[0], a.err, &rc);
+        qb = choose_general(vb, step_b, c_quant_bias[2], a.err, &rc);
+      }
+    }
+    const size_t ci = origin + (size_t)row * geo.W8 + col;
+    a.qcoeff[ci] = qx;
+    a.qcoeff[2 * cplane + ci] = qb;
   }
 }
 
-// Frame-wide LF pair (lib.rs:3831 refine_lf_factors) in four kernels: the
-// regression sums of every LF sample as per-CTA double-float partials across
-// the GPU; one CTA folding them in a fixed order into the two seeds (with the
-// sequential fallback in the reference's LF-group / band / varblock / cell
-// order when a seed is not robust); the residual bit costs of both candidate
-// windows as per-CTA partials; one CTA folding those and making the joint
-// choice.
+// Frame-wide LF pair (lib.rs:3831 refine_lf_factors) and the chroma LF in
+// three kernels: the regression sums of every LF sample as per-CTA
+// double-float partials across the GPU; the two seeds, which every CTA forms
+// from the partials (with the sequential fallback in the reference's LF-group
+// / band / varblock / cell order when a seed is not robust), and the residual
+// bit costs of both candidate windows as per-CTA partials; the joint choice,
+// which every CTA makes from those, and the LF half of lib.rs:3237 for X and
+// B against it.  Forming a small sum again in each CTA costs less than the
+// launches of single-CTA kernels between.
 constexpr int kLfThreads = 256;
 
 __device__ void lf_candidates(int seed, int* c, int* nc_out) {
@@ -1108,70 +1173,77 @@ __global__ void __launch_bounds__(kLfThreads) k_cfl_lf_sums(EncArgs a, DF* part)
   }
 }
 
-__global__ void __launch_bounds__(64) k_cfl_lf_seed(EncArgs a, const DF* part, int* seeds) {
-  __shared__ double s_t[7];
+// The seeds from the partial sums, by a whole CTA (all of it calls); the
+// first CTA counts a fallback.
+__device__ void cfl_lf_seeds(const EncArgs& a, const DF* part, int seeds[2]) {
+  __shared__ double s_t[8];
+  __shared__ int s_seed[2];
   const Geo& geo = a.geo;
-  if (cfl_off(a)) {
-    if (threadIdx.x == 0) {
-      seeds[0] = 0;
-      seeds[1] = 0;
-    }
-    return;
-  }
-  if (threadIdx.x < 7) {
-    DF t = part[threadIdx.x];
-    for (int c = 1; c < kLfCtas; ++c) t = df_add(t, part[c * 7 + threadIdx.x]);
-    s_t[threadIdx.x] = df_value(t);
+  const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+  if (wid < 7) {
+    DF t = part[lane * 7 + wid];
+    for (int c = lane + 32; c < kLfCtas; c += 32) t = df_add(t, part[c * 7 + wid]);
+    t = df_warp_sum(t);
+    if (lane == 0) s_t[wid] = df_value(t);
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
   const size_t nb = (size_t)geo.bw * geo.bh;
-  const double* t = s_t;
-  const double n = (double)nb;
-  const double gam = 2.0 * (n + 64.0) * (2.2737367544323206e-13 + 1.1102230246251565e-16);
-  bool rx, rb;
-  RegSums sx{t[0], t[1], t[2], t[5], n}, sb{t[0], t[3], t[4], t[6], n};
-  int seed_x = best_factor(sx, 0.0f, gam * t[0], gam * t[5], gam * t[2], &rx);
-  int seed_b = best_factor(sb, 1.0f, gam * t[0], gam * t[6], gam * t[4], &rb);
-  if (!rx || !rb) {
-    atomicAdd(a.cfl_fallbacks, 1u);
-    RegSums qx{0, 0, 0, 0, n}, qb{0, 0, 0, 0, n};
-    const int G = 256;
-    const int gw = (geo.bw + G - 1) / G, gh = (geo.bh + G - 1) / G;
-    for (int gy = 0; gy < gh; ++gy)
-      for (int gx = 0; gx < gw; ++gx) {
-        int by0 = gy * G, bx0 = gx * G;
-        int gbh = min(G, geo.bh - by0), gbw = min(G, geo.bw - bx0);
-        for (int trow = 0; trow < (gbh + 7) / 8; ++trow)
-          for (int by = by0 + trow * 8; by < min(by0 + trow * 8 + 8, by0 + gbh); ++by)
-            for (int bx = bx0; bx < bx0 + gbw; ++bx) {
-              uint8_t e = a.block_map[(size_t)by * geo.bw + bx];
-              if (!(e & 0x80)) continue;
-              int sel = e & 0x1f, nbk = sel == 0 ? 1 : (sel == 4 ? 2 : 4);
-              for (int i = 0; i < nbk * nbk; ++i) {
-                size_t bi = (size_t)(by + i / nbk) * geo.bw + bx + i % nbk;
-                double y = a.lfs[nb + bi], x = a.lfs[bi], b = a.lfs[2 * nb + bi];
-                qx.s_yy += y * y; qx.s_yc += y * x; qx.s_cc += x * x;
-                qb.s_yy += y * y; qb.s_yc += y * b; qb.s_cc += b * b;
-              }
-            }
+  if (wid == 0) {
+    const double* t = s_t;
+    const double n = (double)nb;
+    const double gam = 2.0 * (n + 64.0) * (2.2737367544323206e-13 + 1.1102230246251565e-16);
+    const int ch = lane >> 3 & 1;
+    const RegSums r{t[0], ch ? t[3] : t[1], ch ? t[4] : t[2], ch ? t[6] : t[5], n};
+    bool robust;
+    int seed = best_factor_lanes(0xffffffffu, lane & 7, r, ch ? 1.0f : 0.0f, gam * r.s_yy,
+                                 gam * r.a_yc, gam * r.s_cc, &robust);
+    if (__any_sync(0xffffffffu, !robust)) {
+      if (blockIdx.x == 0 && lane == 0) atomicAdd(a.cfl_fallbacks, 1u);
+      if ((lane & 7) == 0 && lane < 16) {
+        RegSums e{0, 0, 0, 0, n};
+        const int G = 256;
+        const int gw = (geo.bw + G - 1) / G, gh = (geo.bh + G - 1) / G;
+        for (int gy = 0; gy < gh; ++gy)
+          for (int gx = 0; gx < gw; ++gx) {
+            int by0 = gy * G, bx0 = gx * G;
+            int gbh = min(G, geo.bh - by0), gbw = min(G, geo.bw - bx0);
+            for (int trow = 0; trow < (gbh + 7) / 8; ++trow)
+              for (int by = by0 + trow * 8; by < min(by0 + trow * 8 + 8, by0 + gbh); ++by)
+                for (int bx = bx0; bx < bx0 + gbw; ++bx) {
+                  uint8_t m = a.block_map[(size_t)by * geo.bw + bx];
+                  if (!(m & 0x80)) continue;
+                  int sel = m & 0x1f, nbk = sel == 0 ? 1 : (sel == 4 ? 2 : 4);
+                  for (int i = 0; i < nbk * nbk; ++i) {
+                    size_t bi = (size_t)(by + i / nbk) * geo.bw + bx + i % nbk;
+                    double y = a.lfs[nb + bi], c = a.lfs[(ch ? 2 * nb : 0) + bi];
+                    e.s_yy += y * y;
+                    e.s_yc += y * c;
+                    e.s_cc += c * c;
+                  }
+                }
+          }
+        bool unused;
+        seed = best_factor(e, ch ? 1.0f : 0.0f, 0, 0, 0, &unused);
       }
-    bool r;
-    seed_x = best_factor(qx, 0.0f, 0, 0, 0, &r);
-    seed_b = best_factor(qb, 1.0f, 0, 0, 0, &r);
+    }
+    if ((lane & 7) == 0 && lane < 16) s_seed[ch] = seed;
   }
-  seeds[0] = seed_x;
-  seeds[1] = seed_b;
+  __syncthreads();
+  seeds[0] = s_seed[0];
+  seeds[1] = s_seed[1];
 }
 
 // Residual bits of every candidate per CTA: [kLfCtas][8] (X candidates 0..3,
 // B candidates 0..3).  At most 2^16 * 22 bits per CTA fit in 32 bits for
 // frames up to 2^28 LF samples.
-__global__ void __launch_bounds__(kLfThreads) k_cfl_lf_bits(EncArgs a, const int* seeds,
-                                                            uint32_t* part) {
+__global__ void __launch_bounds__(kLfThreads) k_cfl_lf_bits(EncArgs a, const DF* sums,
+                                                            int* seeds_out, uint32_t* part) {
   __shared__ uint32_t s_w[kLfThreads / 32][8];
   if (cfl_off(a)) return;
   const size_t nb = (size_t)a.geo.bw * a.geo.bh;
+  int seeds[2];
+  cfl_lf_seeds(a, sums, seeds);
+  if (blockIdx.x == 0 && threadIdx.x < 2) seeds_out[threadIdx.x] = seeds[threadIdx.x];
   int cand[2][4], ncand[2];
   lf_candidates(seeds[0], cand[0], &ncand[0]);
   lf_candidates(seeds[1], cand[1], &ncand[1]);
@@ -1207,101 +1279,60 @@ __global__ void __launch_bounds__(kLfThreads) k_cfl_lf_bits(EncArgs a, const int
   }
 }
 
-__global__ void __launch_bounds__(32) k_cfl_lf_pick(EncArgs a, const int* seeds,
-                                                    const uint32_t* part) {
+// The joint choice (every CTA, from the partial costs), then the LF half of
+// lib.rs:3237 quantize_square_varblock for X and B: targets c - k_lf*dY_lf.
+__global__ void __launch_bounds__(kLfThreads) k_cfl_lf_quant(EncArgs a, const int* seeds,
+                                                             const uint32_t* part) {
   __shared__ unsigned long long s_cost[8];
-  int* out = a.lf_factors;
-  if (cfl_off(a)) {
+  __shared__ int s_factor[2];
+  const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+  if (!cfl_off(a)) {
+    static_assert(kLfThreads / 32 == 8, "a warp per candidate cost");
+    uint32_t t = 0;  // 2^16 x 22 bits per partial: a lane's four fit
+    for (int c = lane; c < kLfCtas; c += 32) t += part[c * 8 + wid];
+    unsigned long long v = t;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) s_cost[wid] = v;
+    __syncthreads();
     if (threadIdx.x == 0) {
-      out[0] = 0;
-      out[1] = 0;
+      int cand[2][4], ncand[2];
+      lf_candidates(seeds[0], cand[0], &ncand[0]);
+      lf_candidates(seeds[1], cand[1], &ncand[1]);
+      const unsigned long long* cost0 = s_cost;
+      const unsigned long long* cost1 = s_cost + 4;
+      unsigned long long nx = 0, nbb = 0;
+      for (int c = 0; c < ncand[0]; ++c) if (cand[0][c] == 0) { nx = cost0[c]; break; }
+      for (int c = 0; c < ncand[1]; ++c) if (cand[1][c] == 0) { nbb = cost1[c]; break; }
+      int bx = 0, bbf = 0;
+      unsigned long long best = nx + nbb;
+      for (int i = 0; i < ncand[0]; ++i)
+        for (int j = 0; j < ncand[1]; ++j) {
+          int fx = cand[0][i], fb = cand[1][j];
+          unsigned long long c = cost0[i] + cost1[j];
+          if (fx != 0 || fb != 0) c += 50ull + factor_bits(fx) + factor_bits(fb);
+          int mag = abs(fx) + abs(fb), bmag = abs(bx) + abs(bbf);
+          if (c < best || (c == best && mag < bmag)) {
+            bx = fx;
+            bbf = fb;
+            best = c;
+          }
+        }
+      s_factor[0] = bx;
+      s_factor[1] = bbf;
     }
-    return;
+  } else if (threadIdx.x < 2) {
+    s_factor[threadIdx.x] = 0;
   }
-  if (threadIdx.x < 8) {
-    unsigned long long t = 0;
-    for (int c = 0; c < kLfCtas; ++c) t += part[c * 8 + threadIdx.x];
-    s_cost[threadIdx.x] = t;
-  }
-  __syncwarp();
-  if (threadIdx.x != 0) return;
-  int cand[2][4], ncand[2];
-  lf_candidates(seeds[0], cand[0], &ncand[0]);
-  lf_candidates(seeds[1], cand[1], &ncand[1]);
-  const unsigned long long* cost0 = s_cost;
-  const unsigned long long* cost1 = s_cost + 4;
-  unsigned long long nx = 0, nbb = 0;
-  for (int c = 0; c < ncand[0]; ++c) if (cand[0][c] == 0) { nx = cost0[c]; break; }
-  for (int c = 0; c < ncand[1]; ++c) if (cand[1][c] == 0) { nbb = cost1[c]; break; }
-  int bx = 0, bbf = 0;
-  unsigned long long best = nx + nbb;
-  for (int i = 0; i < ncand[0]; ++i)
-    for (int j = 0; j < ncand[1]; ++j) {
-      int fx = cand[0][i], fb = cand[1][j];
-      unsigned long long c = cost0[i] + cost1[j];
-      if (fx != 0 || fb != 0) c += 50ull + factor_bits(fx) + factor_bits(fb);
-      int mag = abs(fx) + abs(fb), bmag = abs(bx) + abs(bbf);
-      if (c < best || (c == best && mag < bmag)) {
-        bx = fx;
-        bbf = fb;
-        best = c;
-      }
-    }
-  out[0] = bx;
-  out[1] = bbf;
-}
-
-// ---------------------------------------------------------------------------
-// K5 — chroma half of lib.rs:3237 quantize_square_varblock: LF targets
-// c - k_lf*dY_lf, HF targets c - k_hf*dY_hf (no FMA), nearest choice.
-// ---------------------------------------------------------------------------
-
-template <int N>
-__global__ void __launch_bounds__(128) k_quant_chroma(EncArgs a, const uint32_t* __restrict__ list,
-                                                      int count) {
-  constexpr int VPB = 128 / N;
-  constexpr int n = N / 8;
-  const int g = threadIdx.x / N, j = threadIdx.x % N;
-  const int vi = blockIdx.x * VPB + g;
-  if (vi >= count) return;
-  const uint32_t packed = list[vi];
-  const int bx = packed & 0xffff, by = packed >> 16;
-  const int x0 = bx * 8, y0 = by * 8;
-  const Geo& geo = a.geo;
-  const size_t cplane = (size_t)geo.W8 * geo.H8;
-  const size_t bplane = (size_t)geo.bw * geo.bh;
-  const int tile = (by / 8) * geo.tw + bx / 8;
-  const int fx = a.lf_factors[0], fb = a.lf_factors[1];
-  const float k_lf[3] = {0.0f + (float)fx / 84.0f, 0.0f, 1.0f + (float)fb / 84.0f};
-  const float k_hf[3] = {0.0f + (float)a.cfl_x[tile] / 84.0f, 0.0f,
-                         1.0f + (float)a.cfl_b[tile] / 84.0f};
-  // LF: n*n samples, thread j < n*n takes sample j.
-  if (j < n * n) {
-    size_t bi = (size_t)(by + j / n) * geo.bw + bx + j % n;
-    float dy = a.dylf[bi];
-    for (int c = 0; c <= 2; c += 2) {
-      float target = a.lfs[bplane * c + bi] - k_lf[c] * dy;
-      a.lfq[bplane * c + bi] = lf_quantize(target, a.qs.m_dc[c], a.err);
-    }
-  }
-  const float mul =
-      hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[(size_t)by * geo.bw + bx]);
-  const int off = dq_offset(dq_slot(N == 8 ? 0 : (N == 16 ? 4 : 5)));
-  for (int c = 0; c <= 2; c += 2) {
-    const float scale = mul * a.qs.qm[c];
-    const float* m = a.dq + c * kDequantTableFloats + off;
-#pragma unroll 4
-    for (int k = 0; k < N; ++k) {
-      const size_t ci = (size_t)(y0 + k) * geo.W8 + x0 + j;
-      int32_t q = 0;
-      if (!(k < n && j < n)) {
-        float target = a.coeff[cplane * c + ci] - k_hf[c] * a.dyhf[ci];
-        float rc;
-        const float step = scale * __ldg(&m[k * N + j]);
-        q = choose(c, target, step, a.err, &rc);
-      }
-      a.qcoeff[cplane * c + ci] = q;
-    }
+  __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x < 2) a.lf_factors[threadIdx.x] = s_factor[threadIdx.x];
+  const float k_x = 0.0f + (float)s_factor[0] / 84.0f, k_b = 1.0f + (float)s_factor[1] / 84.0f;
+  const size_t nb = (size_t)a.geo.bw * a.geo.bh;
+  for (size_t i = (size_t)blockIdx.x * kLfThreads + threadIdx.x; i < nb;
+       i += (size_t)gridDim.x * kLfThreads) {
+    const float dy = a.dylf[i];
+    a.lfq[i] = lf_quantize(a.lfs[i] - k_x * dy, a.qs.m_dc[0], a.err);
+    a.lfq[2 * nb + i] = lf_quantize(a.lfs[2 * nb + i] - k_b * dy, a.qs.m_dc[2], a.err);
   }
 }
 
@@ -1324,32 +1355,18 @@ int launch_luma_from_image(const EncArgs& a, const uint32_t* const* lists, const
   return k;
 }
 
-int launch_cfl(const EncArgs& a, int* lf_seeds, void* lf_scratch, void* tile_scratch,
-               cudaStream_t s, cudaStream_t lf_s) {
-  dim3 tiles(a.geo.tw, a.geo.th);
-  const int ntiles = a.geo.tw * a.geo.th;
-  DF* tile_sums = (DF*)tile_scratch;
-  int* tile_seeds = (int*)((char*)tile_scratch + (size_t)ntiles * 8 * sizeof(DF));
-  k_cfl_tile_sums<<<tiles, kCflThreads, 0, s>>>(a, tile_sums);
-  k_cfl_tile_seeds<<<(2 * ntiles + 127) / 128, 128, 0, s>>>(a, tile_sums, tile_seeds);
-  k_cfl_tile_bits<<<tiles, kCflThreads, 0, s>>>(a, tile_seeds);
+int launch_cfl_chroma(const EncArgs& a, int* lf_seeds, void* lf_scratch, cudaStream_t s,
+                      cudaStream_t lf_s) {
+  k_cfl_tile<<<dim3(a.geo.tw, a.geo.th), kCflThreads, sizeof(CflSmem), s>>>(a);
   DF* sums = (DF*)lf_scratch;
   uint32_t* bits = (uint32_t*)((char*)lf_scratch + kLfCtas * 7 * sizeof(DF));
-  // The LF factors' chain reads only the LF planes: on its own stream.
+  // The LF chain reads only the LF planes: on its own stream.
   k_cfl_lf_sums<<<kLfCtas, kLfThreads, 0, lf_s>>>(a, sums);
-  k_cfl_lf_seed<<<1, 64, 0, lf_s>>>(a, sums, lf_seeds);
-  k_cfl_lf_bits<<<kLfCtas, kLfThreads, 0, lf_s>>>(a, lf_seeds, bits);
-  k_cfl_lf_pick<<<1, 32, 0, lf_s>>>(a, lf_seeds, bits);
-  return 7;
-}
-
-int launch_quant_chroma(const EncArgs& a, const uint32_t* const* lists, const int* counts,
-                        const cudaStream_t* s) {
-  int k = 0;
-  if (counts[0]) { k_quant_chroma<8><<<(counts[0] + 15) / 16, 128, 0, s[0]>>>(a, lists[0], counts[0]); ++k; }
-  if (counts[1]) { k_quant_chroma<16><<<(counts[1] + 7) / 8, 128, 0, s[1]>>>(a, lists[1], counts[1]); ++k; }
-  if (counts[2]) { k_quant_chroma<32><<<(counts[2] + 3) / 4, 128, 0, s[2]>>>(a, lists[2], counts[2]); ++k; }
-  return k;
+  k_cfl_lf_bits<<<kLfCtas, kLfThreads, 0, lf_s>>>(a, sums, lf_seeds, bits);
+  const size_t nb = (size_t)a.geo.bw * a.geo.bh;
+  const int ctas = (int)std::min<size_t>((nb + kLfThreads - 1) / kLfThreads, kLfCtas);
+  k_cfl_lf_quant<<<ctas, kLfThreads, 0, lf_s>>>(a, lf_seeds, bits);
+  return 4;
 }
 
 __global__ void k_mul_table(uint32_t global_scale, float* table) {
@@ -1362,8 +1379,11 @@ void launch_mul_table(uint32_t global_scale, float* table, cudaStream_t s) {
 }
 
 cudaError_t configure_encode_kernels() {
-  return cudaFuncSetAttribute(k_precondition, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)kPreRingSmem);
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_precondition, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPreRingSmem);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_cfl_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(CflSmem));
 }
 
 void upload_dct_constants(const float* iv4, const float* iv8, const float* iv16,
@@ -1384,8 +1404,17 @@ void upload_dct_constants(const float* iv4, const float* iv8, const float* iv16,
     auto level = [&](int q) {
       return q <= 0 ? 0.0f : (q == 1 ? 1.0f * bias[c] : (float)q - 0.145f / (float)q);
     };
-    for (int q = 0; q < kLevelN; ++q)
-      levels[c][q] = make_float4(level(q - 1), level(q), level(q + 1), 0.0f);
+    for (int q = 0; q < kLevelN; ++q) {
+        uint32_t packed = 0;
+        for (int i = 0; i < 3; ++i) {
+          uint32_t m = (uint32_t)std::max(q - 1 + i, 0), n = 0;
+          while (m >> n) ++n;
+          packed |= (n ? n + 1 : 0) << (8 * i);  // residual_bits
+        }
+        float w;
+        std::memcpy(&w, &packed, sizeof w);
+        levels[c][q] = make_float4(level(q - 1), level(q), level(q + 1), w);
+    }
   }
   cudaMemcpyToSymbolAsync(g_levels, levels, sizeof levels, 0, cudaMemcpyHostToDevice, s);
 }

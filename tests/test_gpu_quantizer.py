@@ -1,7 +1,7 @@
 """The quantizer's nearest-reconstruction choice and the cover search built
 on it, bit for bit against the restatement: quantizers from so coarse that
 every coefficient falls under the zero threshold to so fine that quotients
-leave the table of levels (256 and beyond) and then the working range, where
+leave the table of levels (1024 and beyond) and then the working range, where
 both refuse, on noise, whose coefficients
 spread over all of them; frames of one block, of partial 32x32 regions and
 of odd sizes."""
