@@ -125,7 +125,7 @@ void launch_epf_step(int step, const float* in, float* out, const float* sigma, 
 // pxyb (optional, out_kind 3 only): also the SSIMULACRA2 positive XYB planes
 // of the output pixels.
 // bracket (out_kind 3, more than 256 levels): per level (the threshold
-// below, the threshold above, the level's value).
+// below, the threshold above, the level's value); levels: the levels' values.
 void launch_colour_out(const float* xyb, int w, int h, int out_kind, const float* thresholds,
                        const float* levels, const float4* bracket, int nlevels, void* out,
                        float* pxyb, int num_sms, cudaStream_t s);

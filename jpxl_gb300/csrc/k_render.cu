@@ -912,16 +912,6 @@ __global__ void __launch_bounds__(kEpfThreads, STEP == 0 ? 3 : 4)
   }
 }
 
-cudaError_t configure_render_kernels() {
-  auto allow = [](auto* kernel, size_t bytes) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  };
-  cudaError_t e;
-  if ((e = allow(k_epf<0>, sizeof(EpfSmem<0>))) != cudaSuccess) return e;
-  if ((e = allow(k_epf<1>, sizeof(EpfSmem<1>))) != cudaSuccess) return e;
-  return allow(k_epf<2>, sizeof(EpfSmem<2>));
-}
-
 void launch_epf_step(int step, const float* in, float* out, const float* sigma, int w, int h,
                      cudaStream_t s) {
   // restoration.rs:356 epf_inv_sigma: step_multiplier * 4 * (1 - sqrt(0.5)) / sigma,
@@ -959,23 +949,29 @@ __device__ __forceinline__ int level_of(float x, const float* thr, int n) {
   return lo;
 }
 
-// The linear value of x's level among n + 1 levels, for deep outputs
-// (65536 levels): the level is first estimated from the transfer curve with
-// the fast powf (its error, a few ulp, moves the estimate by well under one
-// level), then confirmed against the exact thresholds around it, stepping by
-// one where the estimate sits on the wrong side; one 16-byte load of the
-// bracket table per try gives both thresholds and the level's value.  The
-// binary search remains the fallback.  The thresholds decide, so the result
-// is exactly the bisected level's.
-__device__ __forceinline__ float level_value_bracketed(float x, const float4* __restrict__ br,
-                                                       const float* __restrict__ thr,
-                                                       const float* __restrict__ levels, int n,
-                                                       float maxv) {
+// x's level among 0 .. maxv, estimated from the transfer curve with the fast
+// powf.  The scaled code's error is below 1e-6 of maxv; where the code is
+// further than `margin` from a half-integer the estimate is the bisected
+// level (whose own curve and scaling round within 0.004 of a code at 16
+// bits) and *certain is set.  Not for values that are not finite.
+__device__ __forceinline__ int level_estimate(float x, float maxv, float margin, bool* certain) {
+  const float a = fabsf(x);
+  const float e = a <= 0.0031308f ? 12.92f * a : 1.055f * __powf(a, 1.0f / 2.4f) - 0.055f;
+  const float s = (x < 0.0f ? -e : e) * maxv;
+  const float k = rintf(s);
+  *certain = fabsf(s - k) < 0.5f - margin;
+  return (int)fminf(fmaxf(k, 0.0f), maxv);
+}
+
+// The linear value of x's level for deep outputs (more than 256 levels) where
+// the bracket of the estimated level does not hold x: stepping by one, then
+// by binary search.  The thresholds decide, so the result is exactly the
+// bisected level's.
+static __device__ __noinline__ float level_value_search(float x, int est,
+                                                        const float4* __restrict__ br,
+                                                        const float* __restrict__ thr,
+                                                        const float* __restrict__ levels, int n) {
   if (!isfinite(x)) return __ldg(&levels[0]);
-  float a = fabsf(x);
-  float e = a <= 0.0031308f ? 12.92f * a : 1.055f * __powf(a, 1.0f / 2.4f) - 0.055f;
-  float s = rintf((x < 0.0f ? -e : e) * maxv);
-  int est = (int)fminf(fmaxf(s, 0.0f), maxv);
 #pragma unroll 1
   for (int it = 0; it < 4; ++it) {
     const float4 v = __ldg(&br[est]);
@@ -986,22 +982,33 @@ __device__ __forceinline__ float level_value_bracketed(float x, const float4* __
   return __ldg(&levels[level_of(x, thr, n)]);
 }
 
+// Bound: issue slots (the powf's, the metric's cube roots).  An 8-bit level
+// searches its thresholds only next to a half-integer (1 in 400), and a
+// deeper pixel's three bracket entries are loaded at once.  Measured:
+// 2048x2048 to 16-bit levels and the metric's XYB 77 -> 64 us, 1920x1080 to
+// 8 bits 31.5 -> 18.4.  A byte per level beside the curve in shared memory,
+// in place of the table's gathers: 65 to 77, not kept.
+constexpr int kColourThreads = 256;
+
 template <int KIND>
-__global__ void __launch_bounds__(256) k_colour_out(const float* __restrict__ xyb, size_t n,
-                                                    const float* __restrict__ thr,
-                                                    const float* __restrict__ levels,
-                                                    const float4* __restrict__ bracket, int nlev,
-                                                    void* __restrict__ out,
-                                                    float* __restrict__ pxyb) {
+__global__ void __launch_bounds__(kColourThreads, 6)
+    k_colour_out(const float* __restrict__ xyb, size_t n, const float* __restrict__ thr,
+                 const float* __restrict__ levels, const float4* __restrict__ bracket, int nlev,
+                 void* __restrict__ out, float* __restrict__ pxyb) {
   __shared__ float s_thr[255];
   __shared__ float s_lev[256];
-  if (KIND == 2 || (KIND == 3 && nlev <= 256)) {
+  const bool shallow = KIND == 2 || (KIND == 3 && nlev <= 256);
+  if (shallow) {
     for (int i = threadIdx.x; i < nlev - 1; i += blockDim.x) s_thr[i] = thr[i];
     for (int i = threadIdx.x; i < nlev; i += blockDim.x) s_lev[i] = levels[i];
     __syncthreads();
   }
-  const float* T = (nlev <= 256) ? s_thr : thr;
-  const float* LV = (nlev <= 256) ? s_lev : levels;
+  const float maxv = (float)(nlev - 1), margin = 1e-3f + 1e-6f * maxv;
+  auto shallow_level = [&](float x) {
+    bool certain;
+    const int k = level_estimate(x, maxv, margin, &certain);
+    return certain ? k : level_of(x, s_thr, nlev - 1);
+  };
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     float x = xyb[i], y = xyb[n + i], b = xyb[2 * n + i];
@@ -1036,19 +1043,30 @@ __global__ void __launch_bounds__(256) k_colour_out(const float* __restrict__ xy
       }
     } else if (KIND == 2) {
       uint8_t* o = (uint8_t*)out;
-      o[3 * i] = (uint8_t)level_of(rgb[0], T, nlev - 1);
-      o[3 * i + 1] = (uint8_t)level_of(rgb[1], T, nlev - 1);
-      o[3 * i + 2] = (uint8_t)level_of(rgb[2], T, nlev - 1);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) o[3 * i + q] = (uint8_t)shallow_level(rgb[q]);
     } else {
       float lin[3];
-      if (nlev <= 256) {
+      if (shallow) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) lin[q] = LV[level_of(rgb[q], T, nlev - 1)];
+        for (int q = 0; q < 3; ++q) lin[q] = s_lev[shallow_level(rgb[q])];
       } else {
-        const float maxv = (float)(nlev - 1);
+        // One 16-byte load of the bracket table gives a level's thresholds and
+        // value, the three channels' at once.
+        int k[3];
+        float4 v[3];
 #pragma unroll
-        for (int q = 0; q < 3; ++q)
-          lin[q] = level_value_bracketed(rgb[q], bracket, T, LV, nlev - 1, maxv);
+        for (int q = 0; q < 3; ++q) {
+          bool unused;
+          k[q] = level_estimate(rgb[q], maxv, margin, &unused);
+          v[q] = __ldg(&bracket[k[q]]);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          lin[q] = v[q].z;
+          if (!(v[q].x <= rgb[q] && rgb[q] < v[q].y))
+            lin[q] = level_value_search(rgb[q], k[q], bracket, thr, levels, nlev - 1);
+        }
       }
       float* o = (float*)out;
       o[i] = lin[0];
@@ -1070,21 +1088,26 @@ __global__ void __launch_bounds__(256) k_colour_out(const float* __restrict__ xy
 void launch_colour_out(const float* xyb, int w, int h, int out_kind, const float* thresholds,
                        const float* levels, const float4* bracket, int nlevels, void* out,
                        float* pxyb, int num_sms, cudaStream_t s) {
-  size_t n = (size_t)w * h;
-  int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)num_sms * 8);
-  if (blocks < 1) blocks = 1;
-  if (out_kind == 1)
-    k_colour_out<1><<<blocks, 256, 0, s>>>(xyb, n, thresholds, levels, bracket, nlevels, out,
-                                           nullptr);
-  else if (out_kind == 2)
-    k_colour_out<2><<<blocks, 256, 0, s>>>(xyb, n, thresholds, levels, bracket, nlevels, out,
-                                           nullptr);
-  else if (out_kind == 4)
-    k_colour_out<4><<<blocks, 256, 0, s>>>(xyb, n, thresholds, levels, bracket, nlevels, out,
-                                           nullptr);
-  else
-    k_colour_out<3><<<blocks, 256, 0, s>>>(xyb, n, thresholds, levels, bracket, nlevels, out,
-                                           pxyb);
+  const size_t n = (size_t)w * h;
+  const int blocks = (int)std::max<size_t>(
+      1, std::min<size_t>((n + kColourThreads - 1) / kColourThreads, (size_t)num_sms * 16));
+  auto run = [&](auto* kernel, float* px) {
+    kernel<<<blocks, kColourThreads, 0, s>>>(xyb, n, thresholds, levels, bracket, nlevels, out, px);
+  };
+  if (out_kind == 1) run(k_colour_out<1>, nullptr);
+  else if (out_kind == 2) run(k_colour_out<2>, nullptr);
+  else if (out_kind == 4) run(k_colour_out<4>, nullptr);
+  else run(k_colour_out<3>, pxyb);
+}
+
+cudaError_t configure_render_kernels() {
+  auto allow = [](auto* kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  cudaError_t e;
+  if ((e = allow(k_epf<0>, sizeof(EpfSmem<0>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<1>, sizeof(EpfSmem<1>))) != cudaSuccess) return e;
+  return allow(k_epf<2>, sizeof(EpfSmem<2>));
 }
 
 // ---------------------------------------------------------------------------

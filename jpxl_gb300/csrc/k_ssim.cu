@@ -21,11 +21,12 @@ namespace jpxlg {
 // pyramid.rs:19) depend on that tile alone, and keeps each level in shared
 // memory for the next; only the levels' positive XYB (S2) goes to memory.
 // Bound by the cube roots (issue slots of the ALU and FMA pipes).  Measured
-// at 2048x2048: 24.5 us for levels 1..5 against 39.9 us in five launches.
+// at 2048x2048: 24.5 us for levels 1..5 against 39.9 us in five launches; with
+// level 0, 4096x3072: 154 us (182 in six launches; 189 at four CTAs an SM).
 constexpr int kPyrTile = 64;
 constexpr int kPyrThreads = 256;
 
-__global__ void __launch_bounds__(kPyrThreads) k_pyramid(const float* __restrict__ rgb, int w,
+__global__ void __launch_bounds__(kPyrThreads, 6) k_pyramid(const float* __restrict__ rgb, int w,
                                                          int h, PyramidOut out, int n) {
   __shared__ float lev[3][kPyrTile / 2][kPyrTile / 2 + 1];
   __shared__ float lev2[3][kPyrTile / 4][kPyrTile / 4 + 1];
