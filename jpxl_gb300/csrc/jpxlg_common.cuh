@@ -7,6 +7,8 @@
 // written out exactly where the reference calls mul_add.
 #pragma once
 #include <cstdint>
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 #include "jpxlg_defs.cuh"
@@ -377,6 +379,158 @@ __device__ __forceinline__ void idct_1d(float* v) {
   const float f = __fsqrt_rn((float)N);
 #pragma unroll
   for (int i = 0; i < N; ++i) v[i] *= f;
+}
+
+// ---- one DCT shared by a group of warps (N = 16, 32) ------------------------
+// A 1-D transform of N points falls apart into dot products: with
+// i = (2u + 1) 2^t, the odd half of level t of the recursion is dct_iv of
+// N >> (t + 1) points, each output of which is independent of the others.
+// N / 4 "shares" of four outputs each cover a transform: shares
+// 0 .. N/8 - 1 the odd half of level 0, the next N/16 level 1, and so on; the
+// last one holds levels of two points and the final pair.  A warp takes one
+// share of 32 (or 2 x 16) columns, so a 32-point transform is a few hundred
+// instructions in each of eight warps instead of fifteen hundred in one, and
+// no warp's code is long.  The operations and their order are those of dct_ii
+// and dct_iii above.
+
+// Scaling by sqrt(1/2) once per level, as the recursion applies it.
+template <int T>
+__device__ __forceinline__ float scale_half(float v) {
+#pragma unroll
+  for (int i = 0; i < T; ++i) v = v * kSqrtHalf;
+  return v;
+}
+
+// acc[i] = sum over n of iv<M>(u0 + i, n) x[n], n in order from 0.
+template <int M>
+__device__ __forceinline__ void iv_dot4(int u0, const float* x, float* acc) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i] = 0.0f;
+#pragma unroll
+  for (int n = 0; n < M; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = acc[i] + iv_coef<M>(u0 + i, n) * x[n];
+}
+
+// Forward: share `g` of the N-point transform of get(0 .. N-1); put(index,
+// value) receives its four outputs, scaled as dct_1d.
+template <int N, typename Get, typename Put>
+__device__ __forceinline__ void dct_share(int g, Get get, Put put) {
+  const float f = 1.0f / __fsqrt_rn((float)N);
+  float e[N / 2];  // the running even half, from level 1 on
+  if (g < N / 8) {
+    float d[N / 2], acc[4];
+#pragma unroll
+    for (int n = 0; n < N / 2; ++n) d[n] = get(n) - get(N - 1 - n);
+    iv_dot4<N / 2>(4 * g, d, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) put(2 * (4 * g + i) + 1, scale_half<1>(acc[i]) * f);
+    return;
+  }
+#pragma unroll
+  for (int n = 0; n < N / 2; ++n) e[n] = get(n) + get(N - 1 - n);
+  g -= N / 8;
+  if (N >= 16 && g < N / 16) {
+    float d[N / 4], acc[4];
+#pragma unroll
+    for (int n = 0; n < N / 4; ++n) d[n] = e[n] - e[N / 2 - 1 - n];
+    iv_dot4<N / 4>(4 * g, d, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) put(2 * (2 * (4 * g + i) + 1), scale_half<2>(acc[i]) * f);
+    return;
+  }
+#pragma unroll
+  for (int n = 0; n < N / 4; ++n) e[n] = e[n] + e[N / 2 - 1 - n];
+  g -= N / 16;
+  if constexpr (N == 32) {
+    if (g < 1) {
+      float d[4], acc[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) d[n] = e[n] - e[7 - n];
+      iv_dot4<4>(0, d, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) put(4 * (2 * i + 1), scale_half<3>(acc[i]) * f);
+      return;
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) e[n] = e[n] + e[7 - n];
+  }
+  // four points left: dct_ii<4>
+  constexpr int T = N == 32 ? 3 : 2;  // levels above
+  float odd[2] = {e[0] - e[3], e[1] - e[2]};
+  dct_iv<2>(odd);
+  float even[2] = {e[0] + e[3], e[1] + e[2]};
+  dct_ii_2(even);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    put((N / 4) * (2 * k), scale_half<T + 1>(even[k]) * f);
+    put((N / 4) * (2 * k + 1), scale_half<T + 1>(odd[k]) * f);
+  }
+}
+
+// Inverse, first half: share `g`'s dot products from get(0 .. N-1) into
+// put(row, value): the odd half of level t at rows N - (N >> t) ..., the last
+// pair in rows N - 2, N - 1.
+template <int N, typename Get, typename Put>
+__device__ __forceinline__ void idct_share(int g, Get get, Put put) {
+  auto level = [&](auto lt, int share) {
+    constexpr int t = decltype(lt)::value, M = N >> (t + 1);
+    float x[M], acc[4];
+#pragma unroll
+    for (int n = 0; n < M; ++n) x[n] = scale_half<t + 1>(get((2 * n + 1) << t));
+    iv_dot4<M>(4 * share, x, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) put(N - (N >> t) + 4 * share + i, acc[i]);
+  };
+  if (g < N / 8) {
+    level(std::integral_constant<int, 0>{}, g);
+    return;
+  }
+  g -= N / 8;
+  if (g < N / 16) {
+    level(std::integral_constant<int, 1>{}, g);
+    return;
+  }
+  g -= N / 16;
+  if constexpr (N == 32) {
+    if (g < 1) {
+      level(std::integral_constant<int, 2>{}, 0);
+      return;
+    }
+  }
+  constexpr int T = N == 32 ? 4 : 3;
+  float odd[2] = {scale_half<T>(get(N / 4)), scale_half<T>(get(3 * N / 4))};
+  dct_iv<2>(odd);
+  float even[2] = {scale_half<T>(get(0)), scale_half<T>(get(N / 2))};
+  dct_ii_2(even);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    put(N - 4 + k, odd[k]);
+    put(N - 2 + k, even[k]);
+  }
+}
+
+// Inverse, second half: outputs k and N - 1 - k (k < N / 2) from the rows of
+// idct_share, scaled as idct_1d.
+template <int N, typename Get>
+__device__ __forceinline__ void idct_pair(int k, Get get, float* lo, float* hi) {
+  // the even half at k, from the last pair outwards
+  auto fold = [](int i, int m) { return i < m ? i : 2 * m - 1 - i; };
+  int at[4];  // position within the half of level t
+  constexpr int kLevels = N == 32 ? 4 : 3;
+  at[0] = k;
+#pragma unroll
+  for (int t = 1; t < kLevels; ++t) at[t] = fold(at[t - 1], N >> (t + 1));
+  // innermost: two points
+  float even = get(N - 2 + at[kLevels - 1]);
+#pragma unroll
+  for (int t = kLevels - 1; t >= 1; --t) {
+    const float odd = get(N - (N >> t) + at[t]);
+    even = at[t - 1] < (N >> (t + 1)) ? even + odd : even - odd;
+  }
+  const float odd = get(at[0]), f = __fsqrt_rn((float)N);
+  *lo = (even + odd) * f;
+  *hi = (even - odd) * f;
 }
 
 // ---- LF rectangles (dct.rs:956 on the LLF corner of a varblock) -------------

@@ -114,7 +114,7 @@ int launch_render_tc(const RenderArgs& a, const uint32_t* const* lists, const in
 int launch_llf_sigma(const RenderArgs& a, const uint32_t* const* lists, const int* counts,
                      float* const* llf, const cudaStream_t* s);
 // Luma LF and HF quantization of the square varblocks from a coefficient
-// image the split-precision forward transform wrote (k_fdct_luma without its
+// image the split-precision forward transform wrote (k_fdct8 and k_fdct_sq without their
 // own transform).
 int launch_luma_from_image(const EncArgs& a, const uint32_t* const* lists, const int* counts,
                            const cudaStream_t* s);

@@ -57,7 +57,7 @@ __device__ __forceinline__ int cover_dq(int s) {
 
 // Forward DCT_2D of the N x N candidates along a strip: row of blocks `row`
 // of channel c.  Lane l transforms column l, then row l % N of block l / N
-// (k_fdct_luma's order); the strip is this warp's alone.
+// (dct_1d's order); the strip is this warp's alone.
 template <int N>
 __device__ __forceinline__ void cover_strip(CoverSmem& sm, int c, int row, int lane) {
   constexpr int S = N == 8 ? 0 : (N == 16 ? 1 : 2);

@@ -1,7 +1,7 @@
 // k_encode.cu — sm_103a kernels of the encoder's transform path:
 //   K1 k_srgb_to_xyb       RGB8/RGB16 -> LUT -> linear -> XYB planes
 //   K2 k_precondition      12 fused Jacobi steps of the inverse Gaborish
-//   K3 k_fdct_luma<N>      gather + DCT_2D + LF samples + luma quantization
+//   K3 k_fdct8, k_fdct_sq<N>  gather + DCT_2D + LF samples + luma quantization
 //   K4 k_cfl_*             chroma-from-luma factor estimation, and with it
 //   K5                     X/B quantization against reconstructed luma
 // Each kernel restates the reference arithmetic it replaces (cited per
@@ -550,154 +550,239 @@ __device__ __forceinline__ int32_t lf_quantize(float target, float m, uint32_t* 
   return q;
 }
 
-// forward.rs:779 lf_from_llf_into for an n x n (n = 1, 2, 4) LLF corner:
-// divide by scale_f(y)*scale_f(x), then IDCT_2D.
-__device__ __forceinline__ void lf_from_llf(const float* llf, int n, float* lf) {
-  const float* sf = &c_scale_f[(n == 1 ? 0 : (n == 2 ? 1 : 2)) * 8];
-  float work[16];
-  for (int y = 0; y < n; ++y)
-    for (int x = 0; x < n; ++x) work[y * n + x] = llf[y * n + x] / (sf[y] * sf[x]);
-  if (n == 1) {
-    lf[0] = work[0];  // a 1x1 IDCT_2D multiplies by sqrt(1) twice
-    lf[0] = lf[0] * 1.0f * 1.0f;
-    return;
-  }
-  // dct.rs:982 idct_2d_in_place on an n x n square: scratch = work;
-  // column pass; transpose; column pass.
-  float col[4], t[16];
-  for (int c = 0; c < n; ++c) {
-    for (int r = 0; r < n; ++r) col[r] = work[r * n + c];
-    if (n == 2) idct_1d<2>(col); else idct_1d<4>(col);
-    for (int r = 0; r < n; ++r) work[r * n + c] = col[r];
-  }
-  for (int r = 0; r < n; ++r)
-    for (int c = 0; c < n; ++c) t[c * n + r] = work[r * n + c];
-  for (int c = 0; c < n; ++c) {
-    for (int r = 0; r < n; ++r) col[r] = t[r * n + c];
-    if (n == 2) idct_1d<2>(col); else idct_1d<4>(col);
-    for (int r = 0; r < n; ++r) lf[r * n + c] = col[r];
-  }
-}
-
 // ---------------------------------------------------------------------------
-// K3 — forward transform of every square varblock of size N (policy
-// lib.rs:3008 gather_square with edge replication; forward.rs:451
-// forward_dct_rc = dct.rs:956 DCT_2D), LF samples (lib.rs:3100
-// lf_samples_of), and the luma half of lib.rs:3237 quantize_square_varblock:
-// LF quantize + reconstruct, HF choose + reconstruct.
+// K3 — forward transform of every square varblock (policy lib.rs:3008
+// gather_square with edge replication; forward.rs:451 forward_dct_rc =
+// dct.rs:956 DCT_2D), LF samples (lib.rs:3100 lf_samples_of; forward.rs:779
+// lf_from_llf_into), and the luma half of lib.rs:3237
+// quantize_square_varblock: LF quantize + reconstruct, HF choose +
+// reconstruct.
 //
-// N threads per varblock: thread j transforms column j, then (after a shared
-// memory transpose) row j, ending with column j of the coefficient matrix,
-// which it writes to column bx*8+j of the coefficient image (coalesced).
+// 8 x 8: eight lanes per block, four blocks per warp; lane j transforms
+// column j, then (through shared memory, its own warp only) row j, ending
+// with column j of the coefficient matrix, which it writes to column bx*8+j
+// of the coefficient image.  The three channels go together: their loads are
+// in flight at once and no barrier of the block is needed.
+// FROM_IMAGE: the split-precision forward transform has written all three
+// channels' coefficients already.
 // ---------------------------------------------------------------------------
 
-template <int N, bool FROM_IMAGE = false>
-__global__ void __launch_bounds__(128) k_fdct_luma(EncArgs a, const uint32_t* __restrict__ list,
-                                                   int count) {
-  constexpr int VPB = 128 / N;  // varblocks per CTA
-  constexpr int n = N / 8;
-  __shared__ float T[VPB][N][N + 1];
-  __shared__ float LL[VPB][3][16];
-  const int g = threadIdx.x / N, j = threadIdx.x % N;
-  const int vi = blockIdx.x * VPB + g;
+template <bool FROM_IMAGE>
+__global__ void __launch_bounds__(128) k_fdct8(EncArgs a, const uint32_t* __restrict__ list,
+                                               int count) {
+  __shared__ float T[16][3][8][9];
+  const int g = threadIdx.x / 8, j = threadIdx.x % 8;
+  const int vi = blockIdx.x * 16 + g;
   const bool active = vi < count;
-  uint32_t packed = active ? list[vi] : 0u;
+  const uint32_t packed = list[active ? vi : count - 1];  // idle lanes repeat the last block
   const int bx = packed & 0xffff, by = packed >> 16;
   const int x0 = bx * 8, y0 = by * 8;
   const Geo& geo = a.geo;
   const size_t plane = (size_t)geo.w * geo.h;
   const size_t cplane = (size_t)geo.W8 * geo.H8;
-  // Six passes (three channels x column and row transforms) through one copy
-  // of the transform: the loop stays rolled so that a 32-point transform is
-  // not inlined six times past the instruction cache.  Luma runs last, so
-  // its coefficients are in v when the loop ends.
-  float v[N];
+  const size_t cell0 = (size_t)y0 * geo.W8 + x0 + j;
+  const float mul =
+      hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[(size_t)by * geo.bw + bx]);
+  float v[3][8];
   if constexpr (FROM_IMAGE) {
-    // The split-precision forward transform has written all three channels'
-    // coefficients: column j of the luma matrix, and the LLF corners.
-    if (active) {
 #pragma unroll
-      for (int k = 0; k < N; ++k) v[k] = a.coeff[cplane + (size_t)(y0 + k) * geo.W8 + x0 + j];
-      if (j < n) {
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+      for (int k = 0; k < 8; ++k)
+        if (c == 1 || k == 0) v[c][k] = a.coeff[cplane * c + cell0 + (size_t)k * geo.W8];
+  } else {
+    const int xx = min(x0 + j, geo.w - 1);
 #pragma unroll
-          for (int k = 0; k < n; ++k)
-            LL[g][c][k * n + j] = a.coeff[cplane * c + (size_t)(y0 + k) * geo.W8 + x0 + j];
-      }
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        v[c][r] = a.pre[plane * c + (size_t)min(y0 + r, geo.h - 1) * geo.w + xx];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      dct_1d<8>(v[c]);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) T[g][c][r][j] = v[c][r];
     }
-    __syncthreads();
-  }
-#pragma unroll 1
-  for (int pass = 0; pass < (FROM_IMAGE ? 0 : 6); ++pass) {
-    const int c = pass < 2 ? 0 : (pass < 4 ? 2 : 1);
-    if (active) {
-      if ((pass & 1) == 0) {
-        const float* p = a.pre + plane * c;
-        const int xx = min(x0 + j, geo.w - 1);
+    __syncwarp();
 #pragma unroll
-        for (int r = 0; r < N; ++r) v[r] = p[(size_t)min(y0 + r, geo.h - 1) * geo.w + xx];
-      } else {
+    for (int c = 0; c < 3; ++c) {
 #pragma unroll
-        for (int k = 0; k < N; ++k) v[k] = T[g][j][k];
-      }
-      dct_1d<N>(v);
-      if ((pass & 1) == 0) {
-#pragma unroll
-        for (int r = 0; r < N; ++r) T[g][r][j] = v[r];
-      } else {
-#pragma unroll
-        for (int k = 0; k < N; ++k) a.coeff[cplane * c + (size_t)(y0 + k) * geo.W8 + x0 + j] = v[k];
-        if (j < n) {
-#pragma unroll
-          for (int k = 0; k < n; ++k) LL[g][c][k * n + j] = v[k];
-        }
-      }
+      for (int k = 0; k < 8; ++k) v[c][k] = T[g][c][j][k];
+      dct_1d<8>(v[c]);
     }
-    __syncthreads();
+    if (active)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a.coeff[cplane * c + cell0 + (size_t)k * geo.W8] = v[c][k];
   }
   if (!active) return;
-  // LF samples of all three channels and the luma LF quantization.
-  const size_t bplane = (size_t)geo.bw * geo.bh;
-  if (j < 3) {
-    float lf[16];
-    lf_from_llf(LL[g][j], n, lf);
-    for (int i = 0; i < n * n; ++i) {
-      size_t bi = (size_t)(by + i / n) * geo.bw + bx + i % n;
-      a.lfs[bplane * j + bi] = lf[i];
-      if (j == 1) {
-        int32_t q = lf_quantize(lf[i], a.qs.m_dc[1], a.err);
+  // LF samples of all three channels (a 1 x 1 inverse: the coefficient) and
+  // the luma LF quantization.
+  if (j == 0) {
+    const size_t bplane = (size_t)geo.bw * geo.bh, bi = (size_t)by * geo.bw + bx;
+    const float sf2 = c_scale_f[0] * c_scale_f[0];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float lf = v[c][0] / sf2;
+      a.lfs[bplane * c + bi] = lf;
+      if (c == 1) {
+        const int32_t q = lf_quantize(lf, a.qs.m_dc[1], a.err);
         a.lfq[bplane + bi] = q;
         a.dylf[bi] = a.qs.m_dc[1] * (float)q / 1.0f;
       }
     }
   }
-  // Luma HF: cells (k, j) of column j; the n x n LLF corner stays zero.
-  const float mul =
-      hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[(size_t)by * geo.bw + bx]);
+  // Luma HF: cells (k, j) of column j; the LLF cell stays zero: level 0, from
+  // a target under every threshold.
+  if (j == 0) v[1][0] = 0.0f;
   const float scale = mul * a.qs.qm[1];
-  const float* m = a.dq + kDequantTableFloats + dq_offset(dq_slot(N == 8 ? 0 : (N == 16 ? 4 : 5)));
-  // The luma coefficients go through this thread's own row of T so that the
-  // quantization loop need not be unrolled N times.
+  const float* m = a.dq + kDequantTableFloats + dq_offset(dq_slot(0));
+  // Through this lane's own column of T, so that the choice is not inlined
+  // twice.
 #pragma unroll
-  for (int k = 0; k < N; ++k) T[g][j][k] = v[k];
+  for (int k = 0; k < 8; ++k) T[g][1][j][k] = v[1][k];
 #pragma unroll 1
-  for (int k0 = 0; k0 < N; k0 += 4) {
+  for (int k0 = 0; k0 < 8; k0 += 4) {
     float target[4], step[4], recon[4];
     int32_t q[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      target[i] = T[g][j][k0 + i];
-      step[i] = scale * __ldg(&m[(k0 + i) * N + j]);
-      // the LLF corner: level 0, from a target under every threshold
-      if (k0 + i < n && j < n) target[i] = 0.0f;
+      target[i] = T[g][1][j][k0 + i];
+      step[i] = scale * __ldg(&m[(k0 + i) * 8 + j]);
     }
     choose_n<4>(1, target, step, a.err, q, recon);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const size_t ci = (size_t)(y0 + k0 + i) * geo.W8 + x0 + j;
+      const size_t ci = cell0 + (size_t)(k0 + i) * geo.W8;
       a.qcoeff[cplane + ci] = q[i];
       a.dyhf[ci] = recon[i];
+    }
+  }
+}
+
+// K3, N = 16 and 32 — the same block by N / 4 warps, a share of each column
+// per warp and the three channels together through each phase: the split of
+// k_render_sq, for the same reason (the luma stage at 1920x1080: 47 us, now
+// 34; at 64x64 14.9, now 13.3).
+template <int N, bool FROM_IMAGE = false>
+__global__ void __launch_bounds__(8 * N) k_fdct_sq(EncArgs a, const uint32_t* __restrict__ list,
+                                                   int count) {
+  constexpr int kShares = N / 4, VPB = 32 / N, n = N / 8;
+  constexpr int kRows = FROM_IMAGE ? 1 : N;
+  __shared__ float A[VPB][3][kRows][N + 1], B[VPB][3][kRows][N + 1];
+  __shared__ float LL[VPB][3][16];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int g = lane / N, j = lane % N;
+  const int vi = blockIdx.x * VPB + g;
+  const bool active = vi < count;
+  const uint32_t packed = list[active ? vi : count - 1];  // an idle half repeats the last block
+  const int bx = packed & 0xffff, by = packed >> 16;
+  const int x0 = bx * 8, y0 = by * 8;
+  const Geo& geo = a.geo;
+  const size_t plane = (size_t)geo.w * geo.h;
+  const size_t cplane = (size_t)geo.W8 * geo.H8;
+  const float mul =
+      hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[(size_t)by * geo.bw + bx]);
+  float target[4];
+  if constexpr (FROM_IMAGE) {
+    // The split-precision forward transform has written all three channels'
+    // coefficients.
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = 4 * warp + i;
+      target[i] = a.coeff[cplane + (size_t)(y0 + k) * geo.W8 + x0 + j];
+      if (k < n && j < n)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          LL[g][c][k * n + j] = a.coeff[cplane * c + (size_t)(y0 + k) * geo.W8 + x0 + j];
+    }
+    __syncthreads();
+  } else {
+    const int xx = min(x0 + j, geo.w - 1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 4 * warp + i;
+        A[g][c][r][j] = a.pre[plane * c + (size_t)min(y0 + r, geo.h - 1) * geo.w + xx];
+      }
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c)
+      dct_share<N>((warp + 3 * c) % kShares, [&](int i) { return A[g][c][i][j]; },
+                   [&](int k, float v) { B[g][c][k][j] = v; });
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c)
+      dct_share<N>((warp + 3 * c) % kShares, [&](int i) { return B[g][c][j][i]; },
+                   [&](int k, float v) { A[g][c][k][j] = v; });
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = 4 * warp + i;
+      target[i] = A[g][1][k][j];
+      if (k < n && j < n)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) LL[g][c][k * n + j] = A[g][c][k][j];
+      if (active)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          a.coeff[cplane * c + (size_t)(y0 + k) * geo.W8 + x0 + j] = A[g][c][k][j];
+    }
+  }
+  // Luma HF: cells (k, j) of column j; the n x n LLF corner stays zero.
+  if (active) {
+    const float scale = mul * a.qs.qm[1];
+    const float* m = a.dq + kDequantTableFloats + dq_offset(dq_slot(N == 16 ? 4 : 5));
+    float step[4], recon[4];
+    int32_t q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = 4 * warp + i;
+      step[i] = scale * __ldg(&m[k * N + j]);
+      // the LLF corner: level 0, from a target under every threshold
+      if (k < n && j < n) target[i] = 0.0f;
+    }
+    choose_n<4>(1, target, step, a.err, q, recon);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const size_t ci = (size_t)(y0 + 4 * warp + i) * geo.W8 + x0 + j;
+      a.qcoeff[cplane + ci] = q[i];
+      a.dyhf[ci] = recon[i];
+    }
+  }
+  // LF samples of all three channels: IDCT_2D of the n x n LLF corner over its
+  // scale factors (one lane per column, then per row) and the luma LF quantization, by the warp that holds the corner.
+  if (warp != 0) return;
+  __syncwarp();
+  const int lg = lane / (3 * n), c = lane / n % 3, k = lane % n;
+  const int lv = blockIdx.x * VPB + lg;
+  const bool on = lane < VPB * 3 * n && lv < count;
+  const float* sf = &c_scale_f[(n == 2 ? 1 : 2) * 8];
+  float v[n];
+  if (on) {
+#pragma unroll
+    for (int r = 0; r < n; ++r) v[r] = LL[lg][c][r * n + k] / (sf[r] * sf[k]);
+    idct_1d<n>(v);
+#pragma unroll
+    for (int r = 0; r < n; ++r) LL[lg][c][r * n + k] = v[r];
+  }
+  __syncwarp();
+  if (!on) return;
+#pragma unroll
+  for (int r = 0; r < n; ++r) v[r] = LL[lg][c][k * n + r];
+  idct_1d<n>(v);
+  const uint32_t pk = list[lv];
+  const size_t bplane = (size_t)geo.bw * geo.bh;
+#pragma unroll
+  for (int r = 0; r < n; ++r) {
+    const size_t bi = (size_t)((pk >> 16) + r) * geo.bw + (pk & 0xffff) + k;
+    a.lfs[bplane * c + bi] = v[r];
+    if (c == 1) {
+      const int32_t lq = lf_quantize(v[r], a.qs.m_dc[1], a.err);
+      a.lfq[bplane + bi] = lq;
+      a.dylf[bi] = a.qs.m_dc[1] * (float)lq / 1.0f;
     }
   }
 }
@@ -1352,18 +1437,18 @@ int launch_fdct_luma(const EncArgs& a, const uint32_t* const* lists, const int* 
                      const cudaStream_t* s) {
   // square classes: 0 -> DCT8, 1 -> DCT16, 2 -> DCT32, each on its stream
   int k = 0;
-  if (counts[0]) { k_fdct_luma<8><<<(counts[0] + 15) / 16, 128, 0, s[0]>>>(a, lists[0], counts[0]); ++k; }
-  if (counts[1]) { k_fdct_luma<16><<<(counts[1] + 7) / 8, 128, 0, s[1]>>>(a, lists[1], counts[1]); ++k; }
-  if (counts[2]) { k_fdct_luma<32><<<(counts[2] + 3) / 4, 128, 0, s[2]>>>(a, lists[2], counts[2]); ++k; }
+  if (counts[0]) { k_fdct8<false><<<(counts[0] + 15) / 16, 128, 0, s[0]>>>(a, lists[0], counts[0]); ++k; }
+  if (counts[1]) { k_fdct_sq<16><<<(counts[1] + 1) / 2, 128, 0, s[1]>>>(a, lists[1], counts[1]); ++k; }
+  if (counts[2]) { k_fdct_sq<32><<<counts[2], 256, 0, s[2]>>>(a, lists[2], counts[2]); ++k; }
   return k;
 }
 
 int launch_luma_from_image(const EncArgs& a, const uint32_t* const* lists, const int* counts,
                            const cudaStream_t* s) {
   int k = 0;
-  if (counts[0]) { k_fdct_luma<8, true><<<(counts[0] + 15) / 16, 128, 0, s[0]>>>(a, lists[0], counts[0]); ++k; }
-  if (counts[1]) { k_fdct_luma<16, true><<<(counts[1] + 7) / 8, 128, 0, s[1]>>>(a, lists[1], counts[1]); ++k; }
-  if (counts[2]) { k_fdct_luma<32, true><<<(counts[2] + 3) / 4, 128, 0, s[2]>>>(a, lists[2], counts[2]); ++k; }
+  if (counts[0]) { k_fdct8<true><<<(counts[0] + 15) / 16, 128, 0, s[0]>>>(a, lists[0], counts[0]); ++k; }
+  if (counts[1]) { k_fdct_sq<16, true><<<(counts[1] + 1) / 2, 128, 0, s[1]>>>(a, lists[1], counts[1]); ++k; }
+  if (counts[2]) { k_fdct_sq<32, true><<<counts[2], 256, 0, s[2]>>>(a, lists[2], counts[2]); ++k; }
   return k;
 }
 

@@ -1,5 +1,5 @@
 // k_render.cu — sm_103a kernels of the plan renderer / decoder tail:
-//   R1 k_render_vb<R,C>  dequantize, HF CfL, LLF from the LF planes, IDCT_2D,
+//   R1 k_render8, k_render_sq<N>, k_render_vb<R,C>  dequantize, HF CfL, LLF from the LF planes, IDCT_2D,
 //                        in-frame scatter and the per-block EPF sigma
 //   R2 k_gaborish        J.3 3x3 with FMA, mirrored borders
 //   R3 k_epf<step>       J.4 steps 0/1/2
@@ -336,7 +336,8 @@ __global__ void __launch_bounds__(128) k_render_vb(RenderArgs a, const uint32_t*
   // Dequantize landscape column x = j of each channel (plan-render
   // lib.rs:913: adjusted * (mul*qm) * matrix, left to right).
   float dY[CR];
-  // compact dequant slot of this shape (Table I.4 indices 0,4,5,6,7,8)
+  // compact dequant slot of this shape (the plain squares up to 32 have kernels
+  // of their own)
   constexpr int slot = KIND == 1 ? 6
                        : KIND == 2 ? 9
                        : KIND == 3 ? 10
@@ -344,12 +345,11 @@ __global__ void __launch_bounds__(128) k_render_vb(RenderArgs a, const uint32_t*
                        : KIND >= 6 ? 12
                        : (R == 64 && C == 64) ? 7
                        : (T == 64) ? 8
-                       : (R == C) ? (R == 8 ? 0 : (R == 16 ? 1 : 2))
-                                  : (CC == 16 ? 3 : (CR == 8 ? 4 : 5));
+                                   : (CC == 16 ? 3 : (CR == 8 ? 4 : 5));
   const int off = dq_offset(slot);
-  // The channel loop stays rolled, and for square shapes both IDCT passes
-  // run through one copy of the transform: a 32-point transform inlined six
-  // times does not fit the instruction cache.
+  // The channel loop stays rolled, and for 64 x 64 both IDCT passes run
+  // through one copy of the transform: inlined six times it does not fit the
+  // instruction cache.
 #pragma unroll 1
   for (int ci = 0; ci < 3; ++ci) {
     const int c = ci == 0 ? 1 : (ci == 1 ? 0 : 2);  // luma first: CfL needs it
@@ -492,6 +492,271 @@ __global__ void __launch_bounds__(128) k_render_vb(RenderArgs a, const uint32_t*
   }
 }
 
+// ---------------------------------------------------------------------------
+// R1, 8 x 8 — eight lanes per block, four blocks per warp, the three channels
+// together: all of a block's loads are in flight at once, its two passes
+// meet in shared memory within one warp, and no barrier of the block is
+// needed.  Bound by the reads of the coefficients and the writes of the
+// samples (24 bytes per sample of three channels).
+// ---------------------------------------------------------------------------
+
+__global__ void __launch_bounds__(128) k_render8(RenderArgs a, const uint32_t* __restrict__ list,
+                                                 int count) {
+  __shared__ float T[16][3][8][9];
+  const int g = threadIdx.x / 8, j = threadIdx.x % 8;
+  const int vi = blockIdx.x * 16 + g;
+  const bool active = vi < count;
+  const uint32_t packed = list[active ? vi : count - 1];  // idle lanes repeat the last block
+  const int bx = packed & 0xffff, by = packed >> 16;
+  const int x0 = bx * 8, y0 = by * 8;
+  const Geo& geo = a.geo;
+  const size_t cplane = (size_t)geo.W8 * geo.H8;
+  const size_t bplane = (size_t)geo.bw * geo.bh;
+  const size_t plane = (size_t)geo.w * geo.h;
+  const size_t bi = (size_t)by * geo.bw + bx;
+  int32_t q[3][8];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int y = 0; y < 8; ++y)
+      q[c][y] = a.qcoeff[cplane * c + (size_t)(y0 + y) * geo.W8 + x0 + j];
+  const float mul = hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[bi]);  // reconstruct.rs:27
+  const int tile = (by / 8) * geo.tw + bx / 8;
+  const float kx = 0.0f + (float)a.cfl_x[tile] / 84.0f;  // reconstruct.rs:96 cfl_factors
+  const float kb = 1.0f + (float)a.cfl_b[tile] / 84.0f;
+  // Dequantize column j (plan-render lib.rs:913: adjusted * (mul*qm) *
+  // matrix, left to right; lib.rs:1344 apply_hf_cfl).
+  float v[3][8];
+  const int off = dq_offset(0);
+#pragma unroll
+  for (int ci = 0; ci < 3; ++ci) {
+    const int c = ci == 0 ? 1 : (ci == 1 ? 0 : 2);  // luma first: CfL needs it
+    const float scale = mul * a.qs.qm[c], bias = c_quant_bias[c];
+    const float* m = a.dq + c * kDequantTableFloats + off + j;
+#pragma unroll
+    for (int y = 0; y < 8; ++y) {
+      const float d = bias_adjust_q(q[c][y], bias) * scale * __ldg(&m[y * 8]);
+      v[c][y] = c == 1 ? d : d + (c == 0 ? kx : kb) * v[1][y];
+    }
+  }
+  // The LLF sample (varblock.rs:817 llf_from_lf): LF dequantized
+  // (reconstruct.rs:84) with the LF CfL (plan-render lib.rs:1314), times
+  // scale_f(0) twice.
+  if (j == 0) {
+    float d[3];
+    if (a.lf_float) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[c] = a.lf_float[bplane * c + bi];
+    } else {
+      float k_x_lf = a.k_x_lf, k_b_lf = a.k_b_lf;
+      if (a.lf_factors_dev) {
+        k_x_lf = 0.0f + (float)a.lf_factors_dev[0] / 84.0f;
+        k_b_lf = 1.0f + (float)a.lf_factors_dev[1] / 84.0f;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[c] = a.qs.m_dc[c] * (float)a.lfq[bplane * c + bi] / 1.0f;
+      d[0] = d[0] + k_x_lf * d[1];
+      d[2] = d[2] + k_b_lf * d[1];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c][0] = d[c] * c_scale_f[0] * c_scale_f[0];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    idct_1d<8>(v[c]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) T[g][c][i][j] = v[c][i];
+  }
+  __syncwarp();
+  const int fx = x0 + j;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[c][i] = T[g][c][j][i];
+    idct_1d<8>(v[c]);
+    if (active && fx < geo.w) {
+      float* p = a.planes + plane * c + (size_t)y0 * geo.w + fx;
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (y0 + r < geo.h) p[(size_t)r * geo.w] = v[c][r];
+    }
+  }
+  // J.4.3 sigma (restoration.rs:338 vardct_sigma).
+  if (active && j == 0) {
+    int s = a.sharpness[bi];
+    s = s > 7 ? 7 : s;
+    const float lut = s == 7 ? 1.0f : (float)s / 7.0f;
+    a.sigma[bi] = mul * 0.46f * lut;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// R1, N x N (N = 16, 32) — the same block by N / 4 warps.  A transform of 16
+// or 32 points in one thread is a chain of several hundred dependent-issue
+// instructions behind a 254-register frame, and a frame has few such blocks:
+// the kernel was as long as one block (1920x1080 of mixed
+// squares: 80 us, now 43 with the 8x8 class beside it; 64x64: 24.2, now 18.3).  Here a warp takes a
+// share of each column (dct_share's split) and all three channels pass
+// through each phase together, so that between two barriers a warp has a
+// hundred or two independent instructions per channel.  The shares are dealt
+// so that the long ones (the odd half of the first level) spread over the
+// warps: (warp + 3 channel) mod N / 4.  Bound by the barriers' and the
+// dependent loads' latency at a few blocks, by the FP32 pipe at many.
+// A warp spans 32 / N blocks side by side; their rows of N + 1 floats keep
+// the column and the row reads free of bank conflicts.
+// ---------------------------------------------------------------------------
+
+template <int N>
+__global__ void __launch_bounds__(8 * N) k_render_sq(RenderArgs a, const uint32_t* __restrict__ list,
+                                                     int count) {
+  constexpr int kShares = N / 4, VPB = 32 / N, n = N / 8;
+  __shared__ float A[VPB][3][N][N + 1], B[VPB][3][N][N + 1];
+  __shared__ float rect[VPB][3][16];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int g = lane / N, j = lane % N;
+  const int vi = blockIdx.x * VPB + g;
+  const bool active = vi < count;
+  const uint32_t packed = list[active ? vi : count - 1];  // an idle half repeats the last block
+  const int bx = packed & 0xffff, by = packed >> 16;
+  const int x0 = bx * 8, y0 = by * 8;
+  const Geo& geo = a.geo;
+  const size_t cplane = (size_t)geo.W8 * geo.H8;
+  const size_t bplane = (size_t)geo.bw * geo.bh;
+  const size_t plane = (size_t)geo.w * geo.h;
+
+  // LF samples of the block, channel by channel (varblock.rs:817
+  // llf_from_lf; reconstruct.rs:84 with the LF CfL of plan-render
+  // lib.rs:1314): one thread per sample.
+  if (threadIdx.x < VPB * 3 * n * n) {
+    const int lg = threadIdx.x / (3 * n * n), c = threadIdx.x / (n * n) % 3;
+    const int i = threadIdx.x % (n * n);
+    const uint32_t pk = list[min((int)blockIdx.x * VPB + lg, count - 1)];
+    const size_t bi = (size_t)((pk >> 16) + i / n) * geo.bw + (pk & 0xffff) + i % n;
+    float v;
+    if (a.lf_float) {
+      v = a.lf_float[bplane * c + bi];  // dequantized, LF CfL and smoothing applied
+    } else {
+      float k_x_lf = a.k_x_lf, k_b_lf = a.k_b_lf;
+      if (a.lf_factors_dev) {
+        k_x_lf = 0.0f + (float)a.lf_factors_dev[0] / 84.0f;
+        k_b_lf = 1.0f + (float)a.lf_factors_dev[1] / 84.0f;
+      }
+      const float dY = a.qs.m_dc[1] * (float)a.lfq[bplane + bi] / 1.0f;
+      if (c == 1) {
+        v = dY;
+      } else {
+        const float d = a.qs.m_dc[c] * (float)a.lfq[bplane * c + bi] / 1.0f;
+        v = d + (c == 0 ? k_x_lf : k_b_lf) * dY;
+      }
+    }
+    rect[lg][c][i] = v;
+  }
+  const float mul = hf_multiplier(a.mul_table, a.qs.global_scale,
+                                  a.hf_mul[(size_t)by * geo.bw + bx]);  // reconstruct.rs:27
+  const int tile = (by / 8) * geo.tw + bx / 8;
+  const float kx = 0.0f + (float)a.cfl_x[tile] / 84.0f;  // reconstruct.rs:96 cfl_factors
+  const float kb = 1.0f + (float)a.cfl_b[tile] / 84.0f;
+  // Dequantize four rows of column j (plan-render lib.rs:913: adjusted *
+  // (mul*qm) * matrix, left to right; lib.rs:1344 apply_hf_cfl).
+  {
+    const int off = dq_offset(N == 16 ? 1 : 2);
+    int32_t q[3][4];
+    float m[3][4], dY[4];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int y = 4 * warp + i;
+        q[c][i] = a.qcoeff[cplane * c + (size_t)(y0 + y) * geo.W8 + x0 + j];
+        m[c][i] = __ldg(a.dq + c * kDequantTableFloats + off + y * N + j);
+      }
+#pragma unroll
+    for (int ci = 0; ci < 3; ++ci) {
+      const int c = ci == 0 ? 1 : (ci == 1 ? 0 : 2);  // luma first: CfL needs it
+      const float scale = mul * a.qs.qm[c], bias = c_quant_bias[c];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int y = 4 * warp + i;
+        float d = bias_adjust_q(q[c][i], bias) * scale * m[c][i];
+        if (c == 1) dY[i] = d;
+        else d = d + (c == 0 ? kx : kb) * dY[i];
+        if (y >= n || j >= n) A[g][c][y][j] = d;
+      }
+    }
+  }
+  __syncthreads();
+  // LLF corner: DCT_2D of the rectangle, times scale_f(y) * scale_f(x); one
+  // lane per (block, channel, column), then per row.
+  if (warp == 0) {
+    const int lg = lane / (3 * n), c = lane / n % 3, k = lane % n;
+    const float* sf = &c_scale_f[(n == 2 ? 1 : 2) * 8];
+    const bool on = lane < VPB * 3 * n;
+    float v[n];
+    if (on) {
+#pragma unroll
+      for (int r = 0; r < n; ++r) v[r] = rect[lg][c][r * n + k];
+      dct_1d<n>(v);
+#pragma unroll
+      for (int r = 0; r < n; ++r) rect[lg][c][r * n + k] = v[r];
+    }
+    __syncwarp();
+    if (on) {
+#pragma unroll
+      for (int r = 0; r < n; ++r) v[r] = rect[lg][c][k * n + r];
+      dct_1d<n>(v);
+#pragma unroll
+      for (int r = 0; r < n; ++r) A[lg][c][r][k] = v[r] * sf[r] * sf[k];
+    }
+  }
+  __syncthreads();
+  // IDCT_2D (dct.rs:982): the columns of the coefficient matrix, then the
+  // rows of the result, which become sample columns.
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c)
+    idct_share<N>((warp + 3 * c) % kShares, [&](int i) { return A[g][c][i][j]; },
+                  [&](int r, float v) { B[g][c][r][j] = v; });
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = warp + h * kShares;
+      float lo, hi;
+      idct_pair<N>(k, [&](int r) { return B[g][c][r][j]; }, &lo, &hi);
+      A[g][c][k][j] = lo;
+      A[g][c][N - 1 - k][j] = hi;
+    }
+  __syncthreads();
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c)
+    idct_share<N>((warp + 3 * c) % kShares, [&](int i) { return A[g][c][j][i]; },
+                  [&](int r, float v) { B[g][c][r][j] = v; });
+  __syncthreads();
+  if (!active) return;
+  const int fx = x0 + j;
+  if (fx < geo.w) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = warp + h * kShares;
+        float lo, hi;
+        idct_pair<N>(k, [&](int r) { return B[g][c][r][j]; }, &lo, &hi);
+        float* p = a.planes + plane * c + fx;
+        if (y0 + k < geo.h) p[(size_t)(y0 + k) * geo.w] = lo;
+        if (y0 + N - 1 - k < geo.h) p[(size_t)(y0 + N - 1 - k) * geo.w] = hi;
+      }
+  }
+  // J.4.3 sigma per block (restoration.rs:338 vardct_sigma).
+  if (warp == 0 && j < n * n) {
+    const size_t bi = (size_t)(by + j / n) * geo.bw + bx + j % n;
+    int s = a.sharpness[bi];
+    s = s > 7 ? 7 : s;
+    const float lut = s == 7 ? 1.0f : (float)s / 7.0f;
+    a.sigma[bi] = mul * 0.46f * lut;
+  }
+}
+
 // The LLF rectangles and EPF sigma of the square varblocks of size N that
 // the split-precision render (k_tc.cu) transforms: varblock.rs:817
 // llf_from_lf (LF dequantized by reconstruct.rs:84 with the LF CfL of
@@ -574,9 +839,10 @@ void launch_render_varblocks(const RenderArgs& a, const uint32_t* const* lists, 
                            128, 0, s[IDX]>>>(a, lists[IDX], counts[IDX]);
   // shape classes in kShapeSel order: DCT8, 16x16, 32x32, 16x8, 8x16, 32x8,
   // 8x32, 32x16, 16x32, DCT2x2, 64x64, 64x32, 32x64 (rows x cols of samples)
-  JPXLG_RV(0, 8, 8)
-  JPXLG_RV(1, 16, 16)
-  JPXLG_RV(2, 32, 32)
+  if (counts[0]) k_render8<<<(counts[0] + 15) / 16, 128, 0, s[0]>>>(a, lists[0], counts[0]);
+  if (counts[1])
+    k_render_sq<16><<<(counts[1] + 1) / 2, 128, 0, s[1]>>>(a, lists[1], counts[1]);
+  if (counts[2]) k_render_sq<32><<<counts[2], 256, 0, s[2]>>>(a, lists[2], counts[2]);
   JPXLG_RV(3, 16, 8)
   JPXLG_RV(4, 8, 16)
   JPXLG_RV(5, 32, 8)
