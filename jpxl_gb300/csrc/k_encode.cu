@@ -105,11 +105,14 @@ void launch_srgb_to_xyb(const void* rgb, int bits, size_t n, const float* lut, f
 
 // Tiling.  A CTA owns a 128 x 128 tile of one plane with a 12-sample halo
 // (104 x 104 outputs).  Lane l of warp v holds columns 4l .. 4l+3 of tile
-// rows 4v .. 4v+3 in registers for all twelve steps: west and east
-// neighbours come from the adjacent lanes by shuffle, the rows above and
-// below the warp's four from the neighbouring warps through shared memory
-// (double-buffered, one barrier per step), and the source plane F from
-// shared memory.  Every step updates the whole tile; a cell k samples from
+// rows 8v .. 8v+7, and the source plane's, in registers for all twelve
+// steps: west and east neighbours come from the adjacent lanes by shuffle,
+// the rows above and below the warp's eight from the neighbouring warps
+// through shared memory (double-buffered, one barrier per step).  Bound by
+// the issue of its sums and products; sixteen warps of eight rows against
+// thirty-two of four keep the source plane out of shared memory and halve
+// the exchanged rows (4096 x 3072: 452 us, then 433; a wider choice of
+// barriers, pairs of warps or rows at rest, gained nothing).  Every step updates the whole tile; a cell k samples from
 // the tile's edge is exact for k steps, so after twelve the inner 104 x 104
 // are, and no cell of the edge ring is ever read by one nearer the centre
 // than itself.
@@ -127,7 +130,8 @@ void launch_srgb_to_xyb(const void* rgb, int bits, size_t n, const float* lut, f
 constexpr int kPreOut = 104;
 constexpr int kPreHalo = 12;
 constexpr int kPreW = kPreOut + 2 * kPreHalo;  // 128: 32 lanes x 4 columns
-constexpr int kPreWarps = kPreW / 4;            // 32 warps of four rows
+constexpr int kPreRows = 8;                     // rows of a lane
+constexpr int kPreWarps = kPreW / kPreRows;    // 16
 constexpr int kPreThreads = 32 * kPreWarps;
 static_assert(kPreW == 128 && kPreHalo >= 12, "tile of the inverse Gaborish");
 // Tile rows in shared memory are kPreP floats apart: 16-byte aligned for the
@@ -135,15 +139,13 @@ static_assert(kPreW == 128 && kPreHalo >= 12, "tile of the inverse Gaborish");
 // banks for the ring's per-cell accesses (a pitch of 128 puts them all in
 // one).
 constexpr int kPreP = kPreW + 4;
-// F (the source tile, [kPreW][kPreP]), then the interior kernel's published
-// rows [2 parities][kPreWarps][first, last][kPreW], or the ring kernel's
-// step inputs [2 parities][kPreW][kPreP].
-constexpr size_t kPreSmem = (size_t)(kPreW * kPreP + 2 * kPreWarps * 2 * kPreW) * sizeof(float);
+// F (a ring tile's source, [kPreW][kPreP]), then an interior tile's published
+// rows [2 parities][kPreWarps][first, last][kPreW], or a ring tile's step
+// inputs [2 parities][kPreW][kPreP].
 constexpr size_t kPreRingSmem = (size_t)3 * kPreW * kPreP * sizeof(float);
 
 struct EncKernel {
   float centre, edge, corner, inv_c;
-  float neg_zero;  // -0.0f, the run-time addend of the paired products
 };
 
 // The tiles of a frame: a rectangle [fx0, fx1) x [fy0, fy1) of tiles with no
@@ -157,6 +159,18 @@ struct PreTiles {
 // weight; out of line so that the division is not evaluated for every cell.
 static __device__ __noinline__ float precondition_tail(float mm, float fv, float kx, float centre) {
   return mm + (fv - kx) / centre;
+}
+
+// The sums that take a neighbour one column over (pairs that straddle two
+// registers' alignment) and the products run as two scalar operations: a
+// paired sum of them costs register moves, a paired product a run-time
+// addend of -0 and an operand's bank conflict (4096 x 3072: 433 us all
+// paired, 396 all scalar, 388 mixed so).
+__device__ __forceinline__ f2 f2_add_lanes(f2 a, f2 b) {
+  return f2_pack(f2_lo(a) + f2_lo(b), f2_hi(a) + f2_hi(b));
+}
+__device__ __forceinline__ f2 f2_mul_lanes(f2 a, f2 b) {
+  return f2_pack(f2_lo(a) * f2_lo(b), f2_hi(a) * f2_hi(b));
 }
 
 // The three rows around a row of four cells, as lane pairs.  Columns are
@@ -189,21 +203,21 @@ __device__ __forceinline__ PreRows pre_rows(const float4& n, float nW, float nE,
 }
 
 // Interior rule: mm*c + (((N + S) + W) + E)*e + (((NW + NE) + SW) + SE)*k.
-__device__ __forceinline__ void pre_kx_interior(const PreRows& q, f2 c2, f2 e2, f2 k2, f2 nz,
-                                                f2& kxa, f2& kxb) {
-  const f2 s1a = f2_add(f2_add(f2_add(q.Mn0, q.Ms0), q.Wm), q.Cm);
-  const f2 s2a = f2_add(f2_add(f2_add(q.Wn, q.Cn), q.Ws), q.Cs);
-  const f2 s1b = f2_add(f2_add(f2_add(q.Mn1, q.Ms1), q.Cm), q.Em);
-  const f2 s2b = f2_add(f2_add(f2_add(q.Cn, q.En), q.Cs), q.Es);
-  kxa = f2_add(f2_add(f2_mul(q.Mm0, c2, nz), f2_mul(s1a, e2, nz)), f2_mul(s2a, k2, nz));
-  kxb = f2_add(f2_add(f2_mul(q.Mm1, c2, nz), f2_mul(s1b, e2, nz)), f2_mul(s2b, k2, nz));
+__device__ __forceinline__ void pre_kx_interior(const PreRows& q, f2 c2, f2 e2, f2 k2, f2& kxa,
+                                                f2& kxb) {
+  const f2 s1a = f2_add_lanes(f2_add_lanes(f2_add(q.Mn0, q.Ms0), q.Wm), q.Cm);
+  const f2 s2a = f2_add_lanes(f2_add_lanes(f2_add_lanes(q.Wn, q.Cn), q.Ws), q.Cs);
+  const f2 s1b = f2_add_lanes(f2_add_lanes(f2_add(q.Mn1, q.Ms1), q.Cm), q.Em);
+  const f2 s2b = f2_add_lanes(f2_add_lanes(f2_add_lanes(q.Cn, q.En), q.Cs), q.Es);
+  kxa = f2_add(f2_add(f2_mul_lanes(q.Mm0, c2), f2_mul_lanes(s1a, e2)), f2_mul_lanes(s2a, k2));
+  kxb = f2_add(f2_add(f2_mul_lanes(q.Mm1, c2), f2_mul_lanes(s1b, e2)), f2_mul_lanes(s2b, k2));
 }
 
 // mm + (f - kx) * (1/c).
 __device__ __forceinline__ float4 pre_update(const PreRows& q, const float4& f, f2 kxa, f2 kxb,
-                                             f2 i2, f2 nz) {
-  const f2 ya = f2_add(q.Mm0, f2_mul(f2_sub(f2_pack(f.x, f.y), kxa), i2, nz));
-  const f2 yb = f2_add(q.Mm1, f2_mul(f2_sub(f2_pack(f.z, f.w), kxb), i2, nz));
+                                             f2 i2) {
+  const f2 ya = f2_add(q.Mm0, f2_mul_lanes(f2_sub(f2_pack(f.x, f.y), kxa), i2));
+  const f2 yb = f2_add(q.Mm1, f2_mul_lanes(f2_sub(f2_pack(f.z, f.w), kxb), i2));
   return make_float4(f2_lo(ya), f2_hi(ya), f2_lo(yb), f2_hi(yb));
 }
 
@@ -345,34 +359,34 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tx0 = tile_x * kPreOut, ty0 = tile_y * kPreOut;
   const int gx0 = tx0 - kPreHalo, gy0 = ty0 - kPreHalo;
-  const int lx = 4 * lane, ly = 4 * warp;  // the thread's first column and row in the tile
+  const int lx = 4 * lane, ly = kPreRows * warp;  // the thread's first column and row in the tile
   const int gx = gx0 + lx, gy = gy0 + ly;  // ... in the frame
   // Load: tiles inside the frame with 16-byte aligned rows take 16-byte
   // loads; others clamp each coordinate (cells outside the frame are never
   // read by a cell inside it, so their values do not matter).
   const bool vec = gx0 >= 0 && gy0 >= 0 && gx0 + kPreW <= w && gy0 + kPreW <= h && (w % 4) == 0 &&
                    ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
-  float4 X[4];
+  float4 X[kPreRows];
   if (vec) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < kPreRows; ++r)
       X[r] = __ldg(reinterpret_cast<const float4*>(in + (size_t)(gy + r) * w + gx));
   } else {
     const int c0 = pre_clamp(gx, w), c1 = pre_clamp(gx + 1, w), c2 = pre_clamp(gx + 2, w),
               c3 = pre_clamp(gx + 3, w);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < kPreRows; ++r) {
       const float* row = in + (size_t)pre_clamp(gy + r, h) * w;
       X[r] = make_float4(__ldg(row + c0), __ldg(row + c1), __ldg(row + c2), __ldg(row + c3));
     }
   }
-#pragma unroll
-  for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(F + (ly + r) * kPreP + lx) = X[r];
   const f2 c2 = f2_pack(k.centre, k.centre), e2 = f2_pack(k.edge, k.edge);
   const f2 k2 = f2_pack(k.corner, k.corner), i2 = f2_pack(k.inv_c, k.inv_c);
-  const f2 nz = f2_pack(k.neg_zero, k.neg_zero);
   const unsigned full = 0xffffffffu;
   if (!kEdge) {
+    float4 Fr[kPreRows];
+#pragma unroll
+    for (int r = 0; r < kPreRows; ++r) Fr[r] = X[r];
     // The rows just above and below the warp's: the last row of the warp
     // above and the first of the warp below (the tile's edge rows for the
     // first and last warps, never read by an exact cell).
@@ -382,21 +396,21 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
     for (int it = 0; it < 12; ++it) {
       float* const S = xb + (it & 1) * (kPreWarps * 2 * kPreW);
       *reinterpret_cast<float4*>(S + (2 * warp) * kPreW + lx) = X[0];
-      *reinterpret_cast<float4*>(S + (2 * warp + 1) * kPreW + lx) = X[3];
+      *reinterpret_cast<float4*>(S + (2 * warp + 1) * kPreW + lx) = X[kPreRows - 1];
       __syncthreads();
       float4 prev = *reinterpret_cast<const float4*>(S + row_up);
       float pW = __shfl_up_sync(full, prev.w, 1), pE = __shfl_down_sync(full, prev.x, 1);
       float mW = __shfl_up_sync(full, X[0].w, 1), mE = __shfl_down_sync(full, X[0].x, 1);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
+      for (int r = 0; r < kPreRows; ++r) {
         const float4 nxt =
-            r < 3 ? X[r + 1 < 4 ? r + 1 : 3] : *reinterpret_cast<const float4*>(S + row_down);
+            r < kPreRows - 1 ? X[r + 1 < kPreRows ? r + 1 : r] : *reinterpret_cast<const float4*>(S + row_down);
         const float sW = __shfl_up_sync(full, nxt.w, 1), sE = __shfl_down_sync(full, nxt.x, 1);
-        const float4 f = *reinterpret_cast<const float4*>(F + (ly + r) * kPreP + lx);
+        const float4 f = Fr[r];
         f2 kxa, kxb;
         const PreRows q = pre_rows(prev, pW, pE, X[r], mW, mE, nxt, sW, sE);
-        pre_kx_interior(q, c2, e2, k2, nz, kxa, kxb);
-        const float4 y = pre_update(q, f, kxa, kxb, i2, nz);
+        pre_kx_interior(q, c2, e2, k2, kxa, kxb);
+        const float4 y = pre_update(q, f, kxa, kxb, i2);
         prev = X[r];
         pW = mW;
         pE = mE;
@@ -407,14 +421,24 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
     }
   } else {
     // Ring tiles keep the step's input in shared memory and write the
-    // step's output to the other buffer; each thread first finds its cell
-    // of another rule, if it has one.
+    // step's output to the other buffer; each thread first finds its cells
+    // of another rule (at most two, as a rule none).
     const PreRingCells rc = pre_ring_cells(w, h, gx0, gy0);
-    PreSpecial mine{0u, 0u};
-    if ((int)threadIdx.x < rc.count) mine = rc.special(threadIdx.x, w, h, gx0, gy0);
+    PreSpecial mine[2] = {{0u, 0u}, {0u, 0u}};
 #pragma unroll
-    for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(xb + (ly + r) * kPreP + lx) = X[r];
+    for (int s = 0; s < 2; ++s) {
+      const int i = threadIdx.x + s * kPreThreads;
+      if (i < rc.count) mine[s] = rc.special(i, w, h, gx0, gy0);
+    }
+#pragma unroll
+    for (int r = 0; r < kPreRows; ++r) {
+      *reinterpret_cast<float4*>(F + (ly + r) * kPreP + lx) = X[r];
+      *reinterpret_cast<float4*>(xb + (ly + r) * kPreP + lx) = X[r];
+    }
     const int row_up = max(ly - 1, 0) * kPreP + lx;
+    // Rows wholly outside the frame are read by no cell inside it (64 x 64:
+    // half of the tile; 30 us with them, 23 without).
+    const bool live = gy + kPreRows - 1 >= 0 && gy < h;
 #pragma unroll 1
     for (int it = 0; it < 12; ++it) {
       const float* const S = xb + (it & 1) * (kPreW * kPreP);
@@ -423,21 +447,21 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
       // A warp whose four rows have all left the exact region [1 + it,
       // 127 - it) rests; its rows in the step buffers are read only by
       // cells that are no longer exact either.
-      if (!(4 * warp + 3 < 1 + it || 4 * warp >= kPreW - 1 - it)) {
+      if (live && !(ly + kPreRows - 1 < 1 + it || ly >= kPreW - 1 - it)) {
         float4 prev = *reinterpret_cast<const float4*>(S + row_up);
         float4 cur = *reinterpret_cast<const float4*>(S + ly * kPreP + lx);
         float pW = __shfl_up_sync(full, prev.w, 1), pE = __shfl_down_sync(full, prev.x, 1);
         float mW = __shfl_up_sync(full, cur.w, 1), mE = __shfl_down_sync(full, cur.x, 1);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < kPreRows; ++r) {
           const float4 nxt =
               *reinterpret_cast<const float4*>(S + min(ly + r + 1, kPreW - 1) * kPreP + lx);
           const float sW = __shfl_up_sync(full, nxt.w, 1), sE = __shfl_down_sync(full, nxt.x, 1);
           const float4 f = *reinterpret_cast<const float4*>(F + (ly + r) * kPreP + lx);
           f2 kxa, kxb;
           const PreRows q = pre_rows(prev, pW, pE, cur, mW, mE, nxt, sW, sE);
-          pre_kx_interior(q, c2, e2, k2, nz, kxa, kxb);
-          *reinterpret_cast<float4*>(Sn + (ly + r) * kPreP + lx) = pre_update(q, f, kxa, kxb, i2, nz);
+          pre_kx_interior(q, c2, e2, k2, kxa, kxb);
+          *reinterpret_cast<float4*>(Sn + (ly + r) * kPreP + lx) = pre_update(q, f, kxa, kxb, i2);
           prev = cur;
           pW = mW;
           pE = mE;
@@ -447,27 +471,28 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
         }
       }
       __syncthreads();
-      if (mine.b) pre_special_step(mine, S, F, Sn, k);
-      // More cells than threads (none for frames at least 4 samples wide).
-      if (rc.count > kPreThreads) {
+      if (mine[0].b) pre_special_step(mine[0], S, F, Sn, k);
+      if (mine[1].b) pre_special_step(mine[1], S, F, Sn, k);
+      // More cells than two per thread (none for frames at least 4 samples wide).
+      if (rc.count > 2 * kPreThreads) {
         const PreRingCells more = pre_ring_cells(w, h, gx0, gy0);
-        for (int i = threadIdx.x + kPreThreads; i < more.count; i += kPreThreads)
+        for (int i = threadIdx.x + 2 * kPreThreads; i < more.count; i += kPreThreads)
           pre_special_step(more.special(i, w, h, gx0, gy0), S, F, Sn, k);
       }
     }
     __syncthreads();
     // Twelve steps end in buffer 0; each thread reads back its own rows.
 #pragma unroll
-    for (int r = 0; r < 4; ++r) X[r] = *reinterpret_cast<const float4*>(xb + (ly + r) * kPreP + lx);
+    for (int r = 0; r < kPreRows; ++r) X[r] = *reinterpret_cast<const float4*>(xb + (ly + r) * kPreP + lx);
   }
-  // The inner 104 x 104: lanes 3 .. 28 of warps 3 .. 28.
+  // The inner 104 x 104: lanes 3 .. 28 of rows 12 .. 115.
   const int oh = kPreHalo / 4;
-  if (lane >= oh && lane < 32 - oh && warp >= oh && warp < kPreWarps - oh) {
+  if (lane >= oh && lane < 32 - oh) {
     const bool vec_out =
         gx + 3 < w && (w % 4) == 0 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (gy + r >= h) break;
+    for (int r = 0; r < kPreRows; ++r) {
+      if (ly + r < kPreHalo || ly + r >= kPreW - kPreHalo || gy + r >= h) continue;
       float* row = out + (size_t)(gy + r) * w;
       if (vec_out) {
         *reinterpret_cast<float4*>(row + gx) = X[r];
@@ -497,7 +522,7 @@ int launch_precondition(const float* in, float* out, int w, int h, cudaStream_t 
   // gaborish.rs:31 GaborKernel::new, normalised without FMA.
   float unnorm = 1.0f + 4.0f * w1 + 4.0f * w2;
   float scale = 1.0f / unnorm;
-  EncKernel k{scale, w1 * scale, w2 * scale, 1.0f / scale, -0.0f};
+  EncKernel k{scale, w1 * scale, w2 * scale, 1.0f / scale};
   PreTiles pt{(w + kPreOut - 1) / kPreOut, (h + kPreOut - 1) / kPreOut, 0, 0, 0, 0};
   // Columns and rows of cells with another rule: 0, [cb, w) and 0, [rb, h)
   // (the frame border, the columns past the groups of four, the rows of
