@@ -381,7 +381,7 @@ __device__ __forceinline__ void idct_1d(float* v) {
   for (int i = 0; i < N; ++i) v[i] *= f;
 }
 
-// ---- one DCT shared by a group of warps (N = 16, 32) ------------------------
+// ---- one DCT shared by a group of warps -------------------------------------
 // A 1-D transform of N points falls apart into dot products: with
 // i = (2u + 1) 2^t, the odd half of level t of the recursion is dct_iv of
 // N >> (t + 1) points, each output of which is independent of the others.
@@ -468,9 +468,12 @@ __device__ __forceinline__ void dct_share(int g, Get get, Put put) {
   }
 }
 
+// Levels of odd halves of two and more points below an N-point transform.
+__host__ __device__ constexpr int dct_levels(int n) { return n <= 4 ? 1 : 1 + dct_levels(n / 2); }
+
 // Inverse, first half: share `g`'s dot products from get(0 .. N-1) into
 // put(row, value): the odd half of level t at rows N - (N >> t) ..., the last
-// pair in rows N - 2, N - 1.
+// pair in rows N - 2, N - 1.  N = 8, 16, 32.
 template <int N, typename Get, typename Put>
 __device__ __forceinline__ void idct_share(int g, Get get, Put put) {
   auto level = [&](auto lt, int share) {
@@ -487,18 +490,20 @@ __device__ __forceinline__ void idct_share(int g, Get get, Put put) {
     return;
   }
   g -= N / 8;
-  if (g < N / 16) {
-    level(std::integral_constant<int, 1>{}, g);
-    return;
+  if constexpr (N >= 16) {
+    if (g < N / 16) {
+      level(std::integral_constant<int, 1>{}, g);
+      return;
+    }
+    g -= N / 16;
   }
-  g -= N / 16;
   if constexpr (N == 32) {
     if (g < 1) {
       level(std::integral_constant<int, 2>{}, 0);
       return;
     }
   }
-  constexpr int T = N == 32 ? 4 : 3;
+  constexpr int T = dct_levels(N);
   float odd[2] = {scale_half<T>(get(N / 4)), scale_half<T>(get(3 * N / 4))};
   dct_iv<2>(odd);
   float even[2] = {scale_half<T>(get(0)), scale_half<T>(get(N / 2))};
@@ -514,14 +519,15 @@ __device__ __forceinline__ void idct_share(int g, Get get, Put put) {
 // idct_share, scaled as idct_1d.
 template <int N, typename Get>
 __device__ __forceinline__ void idct_pair(int k, Get get, float* lo, float* hi) {
-  // the even half at k, from the last pair outwards
-  auto fold = [](int i, int m) { return i < m ? i : 2 * m - 1 - i; };
-  int at[4];  // position within the half of level t
-  constexpr int kLevels = N == 32 ? 4 : 3;
+  constexpr int kLevels = dct_levels(N);
+  int at[kLevels];  // position within the half of level t
   at[0] = k;
 #pragma unroll
-  for (int t = 1; t < kLevels; ++t) at[t] = fold(at[t - 1], N >> (t + 1));
-  // innermost: two points
+  for (int t = 1; t < kLevels; ++t) {
+    const int m = N >> (t + 1);
+    at[t] = at[t - 1] < m ? at[t - 1] : 2 * m - 1 - at[t - 1];
+  }
+  // from the last pair outwards
   float even = get(N - 2 + at[kLevels - 1]);
 #pragma unroll
   for (int t = kLevels - 1; t >= 1; --t) {

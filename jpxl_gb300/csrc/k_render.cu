@@ -1,5 +1,6 @@
 // k_render.cu — sm_103a kernels of the plan renderer / decoder tail:
-//   R1 k_render8, k_render_sq<N>, k_render_vb<R,C>  dequantize, HF CfL, LLF from the LF planes, IDCT_2D,
+//   R1 k_render8<kind>, k_render_rect<R,C>, k_render_64<R,C>
+//                        dequantize, HF CfL, LLF from the LF planes, IDCT_2D,
 //                        in-frame scatter and the per-block EPF sigma
 //   R2 k_gaborish        J.3 3x3 with FMA, mirrored borders
 //   R3 k_epf<step>       J.4 steps 0/1/2
@@ -23,17 +24,22 @@ __constant__ float c_opsin_m[9];
 __constant__ float c_opsin_bias[3];
 __constant__ float c_opsin_bias_cbrt[3];
 // dct.rs:631 the 64-point DCT-II matrix (rows u, columns x), f32 entries.
-__device__ float g_dct64[64 * 64];
+__device__ __align__(16) float g_dct64[64 * 64];
 
 // dct.rs:678 matrix_pass for N = 64 (the reference's transforms above 32
 // points): each output an f64 dot product of f32 entries, rounded once, then
 // the normative factor sqrt(64) = 8.  The dot product runs in double-float on
 // the FP32 pipe (GB300's FP64 rate is a small fraction of its FP32 rate):
-// each product is exact as p + e (e from one FMA), four independent
-// compensated partial sums carry the rest, and one rounding to f32 ends it.
-// Both that sum and the reference's sequential f64 sum lie within ~1e-15
-// (relative) of the exact dot product, so they round to the same f32 unless
-// the exact value lies that close to a rounding midpoint.
+// each product is exact as p + e (e from one FMA) and a compensated sum
+// carries the rest, rounded to f32 once at the end.  Both that sum and the
+// reference's sequential f64 sum lie within ~1e-15 (relative) of the exact
+// dot product, so they round to the same f32 unless the exact value lies
+// that close to a rounding midpoint.
+//
+// The matrix's f32 entries are exactly symmetric, M[u][63 - x] = +-M[u][x]
+// by u's parity, and so are its even rows again over half the columns, and
+// so on: the sum falls apart by levels as idct_share's does, odd multiples of
+// 2^t at level t, which leaves 1366 products of 4096 per column.
 __device__ __forceinline__ void df_acc(float& hi, float& lo, float a, float b) {
   const float p = a * b;
   const float e = __fmaf_rn(a, b, -p);  // a*b = p + e exactly
@@ -43,32 +49,75 @@ __device__ __forceinline__ void df_acc(float& hi, float& lo, float a, float b) {
   hi = s;
   lo = lo + (err + e);
 }
+__device__ __forceinline__ float2 df_sum(float2 a, float2 b) {
+  const float s = a.x + b.x;
+  const float bb = s - a.x;
+  const float err = (a.x - (s - bb)) + (b.x - bb);
+  return make_float2(s, a.y + (err + b.y));
+}
+__device__ __forceinline__ float2 df_neg(float2 a) { return make_float2(-a.x, -a.y); }
 
-__device__ __forceinline__ void idct_64(float* v) {
-  float out[64];
-#pragma unroll 1
-  for (int k = 0; k < 64; ++k) {
+// Share `g` < 16 of a column's 64-point inverse: put(row, double-float) in
+// idct_share's rows; rows 62 and 63 hold the products of inputs 32 and 0.
+template <typename Get, typename Put>
+__device__ __forceinline__ void idct64_share(int g, Get get, Put put) {
+  if (g < 15) {
+    // level t: 64 >> (t + 1) outputs, four per share, of as many terms
+    const int t = g < 8 ? 0 : (g < 12 ? 1 : (g < 14 ? 2 : 3));
+    const int k = 4 * (g < 8 ? g : (g < 12 ? g - 8 : (g < 14 ? g - 12 : 0)));
+    const int terms = 32 >> t;
     float h[4] = {0.0f, 0.0f, 0.0f, 0.0f}, l[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int j = 0; j < 64; j += 4)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) df_acc(h[i], l[i], g_dct64[(j + i) * 64 + k], v[j + i]);
-    // combine the four partial sums (double-float additions)
-    float hi = h[0], lo = l[0];
-#pragma unroll
-    for (int i = 1; i < 4; ++i) {
-      const float s = hi + h[i];
-      const float bb = s - hi;
-      const float err = (hi - (s - bb)) + (h[i] - bb);
-      hi = s;
-      lo = lo + (err + l[i]);
+#pragma unroll 4
+    for (int m = 0; m < terms; ++m) {
+      const int u = (2 * m + 1) << t;
+      const float4 row = __ldg(reinterpret_cast<const float4*>(g_dct64 + u * 64 + k));
+      const float x = get(u);
+      df_acc(h[0], l[0], row.x, x);
+      df_acc(h[1], l[1], row.y, x);
+      df_acc(h[2], l[2], row.z, x);
+      df_acc(h[3], l[3], row.w, x);
     }
-    const float r = hi + lo;
-    // one correct rounding of hi + lo: r is f32(hi + lo) (round to nearest)
-    out[k] = r;
-  }
 #pragma unroll
-  for (int k = 0; k < 64; ++k) v[k] = out[k] * 8.0f;
+    for (int i = 0; i < 4; ++i) put(64 - (64 >> t) + k + i, make_float2(h[i], l[i]));
+    return;
+  }
+  // level 4 (inputs 16 and 48, two outputs) and the last two products
+  const float x16 = get(16), x48 = get(48), x32 = get(32), x0 = get(0);
+  float2 o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    df_acc(o[i].x, o[i].y, g_dct64[16 * 64 + i], x16);
+    df_acc(o[i].x, o[i].y, g_dct64[48 * 64 + i], x48);
+  }
+  df_acc(o[2].x, o[2].y, g_dct64[32 * 64], x32);
+  df_acc(o[3].x, o[3].y, g_dct64[0], x0);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) put(60 + i, o[i]);
+}
+
+// Outputs k and 63 - k (k < 32) from the rows of idct64_share.
+template <typename Get>
+__device__ __forceinline__ void idct64_pair(int k, Get get, float* lo, float* hi) {
+  int at[6];
+  at[0] = k;
+#pragma unroll
+  for (int t = 1; t < 6; ++t) {
+    const int m = 64 >> (t + 1);
+    at[t] = at[t - 1] < m ? at[t - 1] : 2 * m - 1 - at[t - 1];
+  }
+  float2 even = get(63);
+#pragma unroll
+  for (int t = 5; t >= 1; --t) {
+    const float2 odd = get(64 - (64 >> t) + at[t]);
+    even = df_sum(even, at[t - 1] < (64 >> (t + 1)) ? odd : df_neg(odd));
+  }
+  const float2 odd = get(at[0]);
+  const float2 a = df_sum(even, odd), b = df_sum(even, df_neg(odd));
+  // one correct rounding of the double-float sum, then the factor 8
+  *lo = (a.x + a.y) * 8.0f;
+  *hi = (b.x + b.y) * 8.0f;
 }
 
 // jpxl-core dct.rs:982 idct_2d_in_place for the small shapes of the 8x8
@@ -249,260 +298,23 @@ __device__ __forceinline__ void special_block(const float* b, float* o) {
   }
 }
 
-template <int N>
-__device__ __forceinline__ void idct_n(float* v) {
-  if constexpr (N == 64) idct_64(v);
-  else idct_1d<N>(v);
-}
-
-// ---------------------------------------------------------------------------
-// R1 — one varblock of R x C samples per group of T = max(R, C) threads.
-// Landscape coefficients are crows = min x ccols = max.  IDCT_2D
-// (dct.rs:982): scratch S (C x R) is L transposed when C > R, else L; step A
-// runs length-C IDCTs down S's R columns; step B runs length-R IDCTs along
-// the C rows of the result, producing sample column i in thread i.
-// ---------------------------------------------------------------------------
-
-// KIND 1: DCT2x2 (R = C = 8): the dequantized block goes through the three
-// aux_idct_2x2 stages of jpxl-core varblock.rs:917 instead of IDCT_2D.
-template <int R, int C, int KIND = 0>
-__global__ void __launch_bounds__(128) k_render_vb(RenderArgs a, const uint32_t* __restrict__ list,
-                                                   int count) {
-  constexpr int T = R > C ? R : C;
-  constexpr int CR = R < C ? R : C;   // landscape rows
-  constexpr int CC = T;               // landscape cols
-  constexpr bool portrait = R > C;
-  constexpr int BR = R / 8, BC = C / 8;
-  constexpr int LY = CR / 8, LX = CC / 8;  // LLF corner
-  constexpr int VPB = 128 / T;
-  __shared__ float L[VPB][CR][CC + 1];
-  __shared__ float LLF[VPB][3][64];
-  const int g = threadIdx.x / T, j = threadIdx.x % T;
-  const int vi = blockIdx.x * VPB + g;
-  const bool active = vi < count;
-  const uint32_t packed = active ? list[vi] : 0u;
-  const int bx = packed & 0xffff, by = packed >> 16;
-  const int x0 = bx * 8, y0 = by * 8;
-  const Geo& geo = a.geo;
-  const size_t cplane = (size_t)geo.W8 * geo.H8;
-  const size_t bplane = (size_t)geo.bw * geo.bh;
-  const size_t plane = (size_t)geo.w * geo.h;
-
-  float mul = 0.0f, kx = 0.0f, kb = 0.0f;
-  if (active) {
-    mul = hf_multiplier(a.mul_table, a.qs.global_scale,
-                        a.hf_mul[(size_t)by * geo.bw + bx]);  // reconstruct.rs:27
-    const int tile = (by / 8) * geo.tw + bx / 8;
-    kx = 0.0f + (float)a.cfl_x[tile] / 84.0f;  // reconstruct.rs:96 cfl_factors
-    kb = 1.0f + (float)a.cfl_b[tile] / 84.0f;
-    // LLF rectangles (varblock.rs:817 llf_from_lf) of the three channels:
-    // LF dequantized (reconstruct.rs:84) with the LF CfL (plan-render
-    // lib.rs:1314), laid out landscape, DCT_2D, times scale_f(y)*scale_f(x).
-    if (j < 3) {
-      const int c = j;
-      float k_x_lf = a.k_x_lf, k_b_lf = a.k_b_lf;
-      if (a.lf_factors_dev) {
-        k_x_lf = 0.0f + (float)a.lf_factors_dev[0] / 84.0f;
-        k_b_lf = 1.0f + (float)a.lf_factors_dev[1] / 84.0f;
-      }
-      float rect[64];
-      for (int dy = 0; dy < BR; ++dy)
-        for (int dx = 0; dx < BC; ++dx) {
-          size_t bi = (size_t)(by + dy) * geo.bw + bx + dx;
-          float v;
-          if (a.lf_float) {
-            v = a.lf_float[bplane * c + bi];  // dequantized, LF CfL and smoothing applied
-          } else {
-            float dY = a.qs.m_dc[1] * (float)a.lfq[bplane + bi] / 1.0f;
-            if (c == 1) v = dY;
-            else {
-              float d = a.qs.m_dc[c] * (float)a.lfq[bplane * c + bi] / 1.0f;
-              v = d + (c == 0 ? k_x_lf : k_b_lf) * dY;
-            }
-          }
-          if (portrait) rect[dx * BR + dy] = v; else rect[dy * BC + dx] = v;
-        }
-      if (LY * LX > 1) dct2d_small(rect, LY, LX);
-      constexpr int sfiy = LY == 1 ? 0 : (LY == 2 ? 1 : (LY == 4 ? 2 : 3));
-      constexpr int sfix = LX == 1 ? 0 : (LX == 2 ? 1 : (LX == 4 ? 2 : 3));
-      const float* sfy = &c_scale_f[sfiy * 8];
-      const float* sfx = &c_scale_f[sfix * 8];
-      for (int y = 0; y < LY; ++y)
-        for (int x = 0; x < LX; ++x) LLF[g][c][y * LX + x] = rect[y * LX + x] * sfy[y] * sfx[x];
-    }
-  }
-  __syncthreads();
-
-  // Dequantize landscape column x = j of each channel (plan-render
-  // lib.rs:913: adjusted * (mul*qm) * matrix, left to right).
-  float dY[CR];
-  // compact dequant slot of this shape (the plain squares up to 32 have kernels
-  // of their own)
-  constexpr int slot = KIND == 1 ? 6
-                       : KIND == 2 ? 9
-                       : KIND == 3 ? 10
-                       : (KIND == 4 || KIND == 5) ? 11
-                       : KIND >= 6 ? 12
-                       : (R == 64 && C == 64) ? 7
-                       : (T == 64) ? 8
-                                   : (CC == 16 ? 3 : (CR == 8 ? 4 : 5));
-  const int off = dq_offset(slot);
-  // The channel loop stays rolled, and for 64 x 64 both IDCT passes run
-  // through one copy of the transform: inlined six times it does not fit the
-  // instruction cache.
-#pragma unroll 1
-  for (int ci = 0; ci < 3; ++ci) {
-    const int c = ci == 0 ? 1 : (ci == 1 ? 0 : 2);  // luma first: CfL needs it
-    if (active) {
-      const float scale = mul * a.qs.qm[c];
-      const float bias = c_quant_bias[c];
-      const float* m = a.dq + c * kDequantTableFloats + off;
-      const float kc = c == 0 ? kx : kb;
-#pragma unroll
-      for (int y = 0; y < CR; ++y) {
-        const int x = j;
-        size_t pos = portrait ? (size_t)(y0 + x) * geo.W8 + x0 + y : (size_t)(y0 + y) * geo.W8 + x0 + x;
-        int32_t q = a.qcoeff[cplane * c + pos];
-        float d = bias_adjust_q(q, bias) * scale * __ldg(&m[y * CC + x]);
-        if (c == 1) dY[y] = d;
-        else d = d + kc * dY[y];  // lib.rs:1344 apply_hf_cfl
-        if (y < LY && x < LX) d = LLF[g][c][y * LX + x];
-        L[g][y][x] = d;
-      }
-    }
-    __syncthreads();
-    float v[T];
-    if constexpr (KIND >= 2) {
-      // thread 0 of the group reconstructs the block, then thread j writes
-      // sample column j.
-      if (active && j == 0) {
-        float b[64], o[64];
-#pragma unroll
-        for (int i = 0; i < 64; ++i) b[i] = L[g][i / 8][i % 8];
-        special_block<KIND>(b, o);
-#pragma unroll
-        for (int i = 0; i < 64; ++i) L[g][i / 8][i % 8] = o[i];
-      }
-      __syncthreads();
-      if (active) {
-        const int fx = x0 + j;
-        if (fx < geo.w) {
-#pragma unroll
-          for (int rr = 0; rr < 8; ++rr) {
-            const int fy = y0 + rr;
-            if (fy < geo.h) a.planes[plane * c + (size_t)fy * geo.w + fx] = L[g][rr][j];
-          }
-        }
-      }
-      __syncthreads();
-    } else if constexpr (KIND == 1) {
-      // varblock.rs:895 aux_idct_2x2 with s = 2, 4, 8, each stage reading the
-      // previous one; thread 0 of the group runs the cascade, then thread j
-      // writes sample column j.
-      if (active && j == 0) {
-        float b[64];
-#pragma unroll
-        for (int i = 0; i < 64; ++i) b[i] = L[g][i / 8][i % 8];
-        dct2x2_block(b);
-#pragma unroll
-        for (int i = 0; i < 64; ++i) L[g][i / 8][i % 8] = b[i];
-      }
-      __syncthreads();
-      if (active) {
-        const int fx = x0 + j;
-        if (fx < geo.w) {
-#pragma unroll
-          for (int rr = 0; rr < 8; ++rr) {
-            const int fy = y0 + rr;
-            if (fy < geo.h) a.planes[plane * c + (size_t)fy * geo.w + fx] = L[g][rr][j];
-          }
-        }
-      }
-      __syncthreads();
-    } else if constexpr (R == C) {
-      // Step A (st = 0): thread j transforms column j of L in place.
-      // Step B (st = 1): thread j transforms row j of the result into sample
-      // column j and scatters it inside the frame.
-#pragma unroll 1
-      for (int st = 0; st < 2; ++st) {
-        if (active) {
-#pragma unroll
-          for (int i = 0; i < T; ++i) v[i] = st == 0 ? L[g][i][j] : L[g][j][i];
-          idct_n<T>(v);
-        }
-        if (st == 0) {
-          __syncthreads();
-          if (active) {
-#pragma unroll
-            for (int i = 0; i < T; ++i) L[g][i][j] = v[i];
-          }
-        } else if (active) {
-          const int fx = x0 + j;
-          if (fx < geo.w) {
-#pragma unroll
-            for (int r = 0; r < T; ++r) {
-              const int fy = y0 + r;
-              if (fy < geo.h) a.planes[plane * c + (size_t)fy * geo.w + fx] = v[r];
-            }
-          }
-        }
-        __syncthreads();
-      }
-    } else {
-      // Step A: thread jj < R transforms column jj of S (length C).
-      if (active && j < R) {
-#pragma unroll
-        for (int i = 0; i < C; ++i) v[i] = (C > R) ? L[g][j][i] : L[g][i][j];
-        idct_n<C>(v);
-      }
-      __syncthreads();
-      if (active && j < R) {
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-          if (C > R) L[g][j][i] = v[i]; else L[g][i][j] = v[i];
-        }
-      }
-      __syncthreads();
-      // Step B: thread i < C transforms row i of the step-A result (length R)
-      // into sample column i and scatters it inside the frame.
-      if (active && j < C) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = (C > R) ? L[g][r][j] : L[g][j][r];
-        idct_n<R>(v);
-        const int fx = x0 + j;
-        if (fx < geo.w) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int fy = y0 + r;
-            if (fy < geo.h) a.planes[plane * c + (size_t)fy * geo.w + fx] = v[r];
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // J.4.3 sigma per block (restoration.rs:338 vardct_sigma).
-  if (active && j < BR * BC) {
-    const int dy = j / BC, dx = j % BC;
-    size_t bi = (size_t)(by + dy) * geo.bw + bx + dx;
-    int s = a.sharpness[bi];
-    s = s > 7 ? 7 : s;
-    const float lut = s == 7 ? 1.0f : (float)s / 7.0f;
-    a.sigma[bi] = mul * 0.46f * lut;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // R1, 8 x 8 — eight lanes per block, four blocks per warp, the three channels
 // together: all of a block's loads are in flight at once, its two passes
 // meet in shared memory within one warp, and no barrier of the block is
-// needed.  Bound by the reads of the coefficients and the writes of the
+// needed.  KIND 0 is DCT8; KIND 1 (DCT2x2) and 2 .. 9 (special_block) run in
+// the block's first three lanes, one channel each (a 128 x 128 stream's:
+// 22.5 us with the channels in turn, now 15).  Bound by the reads of the coefficients and the writes of the
 // samples (24 bytes per sample of three channels).
 // ---------------------------------------------------------------------------
 
+template <int KIND>
 __global__ void __launch_bounds__(128) k_render8(RenderArgs a, const uint32_t* __restrict__ list,
                                                  int count) {
   __shared__ float T[16][3][8][9];
+  // compact dequant slot of this transform
+  constexpr int slot = KIND == 0 ? 0 : KIND == 1 ? 6 : KIND == 2 ? 9 : KIND == 3 ? 10
+                       : KIND <= 5 ? 11 : 12;
   const int g = threadIdx.x / 8, j = threadIdx.x % 8;
   const int vi = blockIdx.x * 16 + g;
   const bool active = vi < count;
@@ -527,7 +339,7 @@ __global__ void __launch_bounds__(128) k_render8(RenderArgs a, const uint32_t* _
   // Dequantize column j (plan-render lib.rs:913: adjusted * (mul*qm) *
   // matrix, left to right; lib.rs:1344 apply_hf_cfl).
   float v[3][8];
-  const int off = dq_offset(0);
+  const int off = dq_offset(slot);
 #pragma unroll
   for (int ci = 0; ci < 3; ++ci) {
     const int c = ci == 0 ? 1 : (ci == 1 ? 0 : 2);  // luma first: CfL needs it
@@ -563,17 +375,34 @@ __global__ void __launch_bounds__(128) k_render8(RenderArgs a, const uint32_t* _
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    idct_1d<8>(v[c]);
+    if constexpr (KIND == 0) idct_1d<8>(v[c]);
 #pragma unroll
     for (int i = 0; i < 8; ++i) T[g][c][i][j] = v[c][i];
   }
   __syncwarp();
+  if constexpr (KIND != 0) {
+    if (j < 3) {
+      float b[64], o[64];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) b[i] = T[g][j][i / 8][i % 8];
+      if constexpr (KIND == 1) {
+        dct2x2_block(b);
+#pragma unroll
+        for (int i = 0; i < 64; ++i) o[i] = b[i];
+      } else {
+        special_block<KIND>(b, o);
+      }
+#pragma unroll
+      for (int i = 0; i < 64; ++i) T[g][j][i / 8][i % 8] = o[i];
+    }
+    __syncwarp();
+  }
   const int fx = x0 + j;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[c][i] = T[g][c][j][i];
-    idct_1d<8>(v[c]);
+    for (int i = 0; i < 8; ++i) v[c][i] = KIND == 0 ? T[g][c][j][i] : T[g][c][i][j];
+    if constexpr (KIND == 0) idct_1d<8>(v[c]);
     if (active && fx < geo.w) {
       float* p = a.planes + plane * c + (size_t)y0 * geo.w + fx;
 #pragma unroll
@@ -591,169 +420,339 @@ __global__ void __launch_bounds__(128) k_render8(RenderArgs a, const uint32_t* _
 }
 
 // ---------------------------------------------------------------------------
-// R1, N x N (N = 16, 32) — the same block by N / 4 warps.  A transform of 16
-// or 32 points in one thread is a chain of several hundred dependent-issue
+// R1, R x C with a side of 16 or 32 — one varblock by R C / 4 threads.
+// Landscape coefficients L are crows = min x ccols = max.  IDCT_2D
+// (dct.rs:982): scratch S (C x R) is L transposed when C > R, else L; step A
+// runs length-C IDCTs down S's R columns; step B runs length-R IDCTs along
+// the C rows of the result, producing sample column i from row i.
+//
+// A transform of 16 or 32 points in one thread is a chain of several hundred
 // instructions behind a 254-register frame, and a frame has few such blocks:
-// the kernel was as long as one block (1920x1080 of mixed
-// squares: 80 us, now 43 with the 8x8 class beside it; 64x64: 24.2, now 18.3).  Here a warp takes a
-// share of each column (dct_share's split) and all three channels pass
-// through each phase together, so that between two barriers a warp has a
-// hundred or two independent instructions per channel.  The shares are dealt
-// so that the long ones (the odd half of the first level) spread over the
-// warps: (warp + 3 channel) mod N / 4.  Bound by the barriers' and the
-// dependent loads' latency at a few blocks, by the FP32 pipe at many.
-// A warp spans 32 / N blocks side by side; their rows of N + 1 floats keep
-// the column and the row reads free of bank conflicts.
+// the kernel was as long as one block (1920x1080 of mixed squares: 80 us, now
+// 34 with the 8x8 class beside it; 64x64: 24, now 17).  Here a warp takes a
+// share of 32 columns (idct_share's split; as many blocks side by side as 32
+// columns need) and all three channels pass through each phase together, so
+// that between two barriers a warp has a hundred or two independent
+// instructions per channel.  The shares are dealt so that the long ones (the
+// odd half of the first level) spread over the warps.  Bound by the barriers'
+// and the dependent loads' latency at a few blocks, by the FP32 pipe at many.
+// Rows one float longer than the matrix keep the column and the row reads
+// free of bank conflicts.
 // ---------------------------------------------------------------------------
 
-template <int N>
-__global__ void __launch_bounds__(8 * N) k_render_sq(RenderArgs a, const uint32_t* __restrict__ list,
-                                                     int count) {
-  constexpr int kShares = N / 4, VPB = 32 / N, n = N / 8;
-  __shared__ float A[VPB][3][N][N + 1], B[VPB][3][N][N + 1];
-  __shared__ float rect[VPB][3][16];
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int g = lane / N, j = lane % N;
-  const int vi = blockIdx.x * VPB + g;
-  const bool active = vi < count;
-  const uint32_t packed = list[active ? vi : count - 1];  // an idle half repeats the last block
-  const int bx = packed & 0xffff, by = packed >> 16;
-  const int x0 = bx * 8, y0 = by * 8;
+template <int R, int C>
+struct RectShape {
+  static constexpr int CR = R < C ? R : C, CC = R < C ? C : R;  // landscape rows, columns
+  static constexpr bool portrait = R > C;
+  static constexpr int BR = R / 8, BC = C / 8;
+  static constexpr int LY = CR / 8, LX = CC / 8;  // LLF corner
+  // compact dequant slot
+  static constexpr int slot = CC == 64 ? (CR == 64 ? 7 : 8)
+                              : R == C ? (R == 16 ? 1 : 2)
+                                       : (CC == 16 ? 3 : (CR == 8 ? 4 : 5));
+  // rows of c_scale_f
+  static constexpr int SY = LY == 1 ? 0 : (LY == 2 ? 1 : (LY == 4 ? 2 : 3));
+  static constexpr int SX = LX == 1 ? 0 : (LX == 2 ? 1 : (LX == 4 ? 2 : 3));
+};
+
+// An LF sample of channel c at block bi: as it stands in a decoded frame's LF
+// image, else dequantized (reconstruct.rs:84) with the LF CfL (plan-render
+// lib.rs:1314).
+__device__ __forceinline__ float lf_sample(const RenderArgs& a, size_t bplane, int c, size_t bi) {
+  if (a.lf_float) return a.lf_float[bplane * c + bi];
+  const float dY = a.qs.m_dc[1] * (float)a.lfq[bplane + bi] / 1.0f;
+  if (c == 1) return dY;
+  float k = c == 0 ? a.k_x_lf : a.k_b_lf;
+  if (a.lf_factors_dev)
+    k = (c == 0 ? 0.0f : 1.0f) + (float)a.lf_factors_dev[c == 0 ? 0 : 1] / 84.0f;
+  const float d = a.qs.m_dc[c] * (float)a.lfq[bplane * c + bi] / 1.0f;
+  return d + k * dY;
+}
+
+// J.4.3 sigma of a block (restoration.rs:338 vardct_sigma).
+__device__ __forceinline__ float block_sigma(const RenderArgs& a, float mul, size_t bi) {
+  int s = a.sharpness[bi];
+  s = s > 7 ? 7 : s;
+  const float lut = s == 7 ? 1.0f : (float)s / 7.0f;
+  return mul * 0.46f * lut;
+}
+
+// The LLF corner (varblock.rs:817 llf_from_lf) of one channel from its LF
+// rectangle `rect` (landscape LY x LX): DCT_2D, times scale_f(y) *
+// scale_f(x), by LX lanes and then LY lanes of one warp; put(y, x, value).
+template <typename S, typename Put>
+__device__ __forceinline__ void llf_corner(float* rect, int k, bool on, Put put) {
+  constexpr int LY = S::LY, LX = S::LX;
+  const float* sfy = &c_scale_f[S::SY * 8];
+  const float* sfx = &c_scale_f[S::SX * 8];
+  if (on && k < LX) {
+    float v[LY];
+#pragma unroll
+    for (int r = 0; r < LY; ++r) v[r] = rect[r * LX + k];
+    if constexpr (LY > 1) dct_1d<LY>(v);
+#pragma unroll
+    for (int r = 0; r < LY; ++r) rect[r * LX + k] = v[r];
+  }
+  __syncwarp();
+  if (on && k < LY) {
+    float v[LX];
+#pragma unroll
+    for (int r = 0; r < LX; ++r) v[r] = rect[k * LX + r];
+    dct_1d<LX>(v);
+    // a square's second pass leaves the matrix transposed (dct.rs:956)
+#pragma unroll
+    for (int r = 0; r < LX; ++r) {
+      const int y = LX == LY ? r : k, x = LX == LY ? k : r;
+      put(y, x, v[r] * sfy[y] * sfx[x]);
+    }
+  }
+}
+
+template <int R, int C>
+__global__ void __launch_bounds__(R* C / 4 * (32 / (R < C ? R : C)))
+    k_render_rect(RenderArgs a, const uint32_t* __restrict__ list, int count) {
+  using S = RectShape<R, C>;
+  constexpr int VPB = 32 / S::CR;                       // blocks per CTA
+  constexpr int kWarpsA = VPB * R / 32, kWarpsB = VPB * C / 32;  // column groups of 32
+  constexpr int kLlf = S::LY * S::LX;
+  __shared__ float A[VPB][3][C][R + 1];
+  __shared__ float B[VPB * 3 * (C * (R + 1) > R * (C + 1) ? C * (R + 1) : R * (C + 1))];
+  __shared__ float rect[VPB][3][kLlf];
+  const int t = threadIdx.x, warp = t / 32, lane = t % 32;
   const Geo& geo = a.geo;
   const size_t cplane = (size_t)geo.W8 * geo.H8;
   const size_t bplane = (size_t)geo.bw * geo.bh;
   const size_t plane = (size_t)geo.w * geo.h;
-
-  // LF samples of the block, channel by channel (varblock.rs:817
-  // llf_from_lf; reconstruct.rs:84 with the LF CfL of plan-render
-  // lib.rs:1314): one thread per sample.
-  if (threadIdx.x < VPB * 3 * n * n) {
-    const int lg = threadIdx.x / (3 * n * n), c = threadIdx.x / (n * n) % 3;
-    const int i = threadIdx.x % (n * n);
-    const uint32_t pk = list[min((int)blockIdx.x * VPB + lg, count - 1)];
-    const size_t bi = (size_t)((pk >> 16) + i / n) * geo.bw + (pk & 0xffff) + i % n;
-    float v;
-    if (a.lf_float) {
-      v = a.lf_float[bplane * c + bi];  // dequantized, LF CfL and smoothing applied
-    } else {
-      float k_x_lf = a.k_x_lf, k_b_lf = a.k_b_lf;
-      if (a.lf_factors_dev) {
-        k_x_lf = 0.0f + (float)a.lf_factors_dev[0] / 84.0f;
-        k_b_lf = 1.0f + (float)a.lf_factors_dev[1] / 84.0f;
-      }
-      const float dY = a.qs.m_dc[1] * (float)a.lfq[bplane + bi] / 1.0f;
-      if (c == 1) {
-        v = dY;
-      } else {
-        const float d = a.qs.m_dc[c] * (float)a.lfq[bplane * c + bi] / 1.0f;
-        v = d + (c == 0 ? k_x_lf : k_b_lf) * dY;
-      }
-    }
-    rect[lg][c][i] = v;
+  const int v0 = blockIdx.x * VPB;
+  // an idle place repeats the last block
+  auto block = [&](int g) { return list[min(v0 + g, count - 1)]; };
+  auto to_s = [](int y, int x, float(&m)[C][R + 1], float d) {
+    if constexpr (C > R) m[x][y] = d;
+    else m[y][x] = d;
+  };
+  // The LF rectangles, one thread per sample.
+  if (t < VPB * 3 * kLlf) {
+    const int g = t / (3 * kLlf), c = t / kLlf % 3, i = t % kLlf;
+    const uint32_t pk = block(g);
+    const int dy = i / S::BC, dx = i % S::BC;
+    const size_t bi = (size_t)((pk >> 16) + dy) * geo.bw + (pk & 0xffff) + dx;
+    rect[g][c][S::portrait ? dx * S::BR + dy : i] = lf_sample(a, bplane, c, bi);
   }
-  const float mul = hf_multiplier(a.mul_table, a.qs.global_scale,
-                                  a.hf_mul[(size_t)by * geo.bw + bx]);  // reconstruct.rs:27
-  const int tile = (by / 8) * geo.tw + bx / 8;
-  const float kx = 0.0f + (float)a.cfl_x[tile] / 84.0f;  // reconstruct.rs:96 cfl_factors
-  const float kb = 1.0f + (float)a.cfl_b[tile] / 84.0f;
-  // Dequantize four rows of column j (plan-render lib.rs:913: adjusted *
-  // (mul*qm) * matrix, left to right; lib.rs:1344 apply_hf_cfl).
+  // Dequantize four rows of landscape column x (plan-render lib.rs:913:
+  // adjusted * (mul*qm) * matrix, left to right; lib.rs:1344 apply_hf_cfl).
   {
-    const int off = dq_offset(N == 16 ? 1 : 2);
+    const int x = t % S::CC, yg = t / S::CC % (S::CR / 4), g = t / (S::CC * S::CR / 4);
+    const uint32_t pk = block(g);
+    const int bx = pk & 0xffff, by = pk >> 16;
     int32_t q[3][4];
     float m[3][4], dY[4];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int y = 4 * warp + i;
-        q[c][i] = a.qcoeff[cplane * c + (size_t)(y0 + y) * geo.W8 + x0 + j];
-        m[c][i] = __ldg(a.dq + c * kDequantTableFloats + off + y * N + j);
+        const int y = 4 * yg + i;
+        const size_t pos = S::portrait ? (size_t)(by * 8 + x) * geo.W8 + bx * 8 + y
+                                       : (size_t)(by * 8 + y) * geo.W8 + bx * 8 + x;
+        q[c][i] = a.qcoeff[cplane * c + pos];
+        m[c][i] = __ldg(a.dq + c * kDequantTableFloats + dq_offset(S::slot) + y * S::CC + x);
       }
+    const float mul = hf_multiplier(a.mul_table, a.qs.global_scale,
+                                    a.hf_mul[(size_t)by * geo.bw + bx]);  // reconstruct.rs:27
+    const int tile = (by / 8) * geo.tw + bx / 8;
+    const float kx = 0.0f + (float)a.cfl_x[tile] / 84.0f;  // reconstruct.rs:96 cfl_factors
+    const float kb = 1.0f + (float)a.cfl_b[tile] / 84.0f;
 #pragma unroll
     for (int ci = 0; ci < 3; ++ci) {
       const int c = ci == 0 ? 1 : (ci == 1 ? 0 : 2);  // luma first: CfL needs it
       const float scale = mul * a.qs.qm[c], bias = c_quant_bias[c];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int y = 4 * warp + i;
+        const int y = 4 * yg + i;
         float d = bias_adjust_q(q[c][i], bias) * scale * m[c][i];
         if (c == 1) dY[i] = d;
         else d = d + (c == 0 ? kx : kb) * dY[i];
-        if (y >= n || j >= n) A[g][c][y][j] = d;
+        if (y >= S::LY || x >= S::LX) to_s(y, x, A[g][c], d);
       }
     }
   }
   __syncthreads();
-  // LLF corner: DCT_2D of the rectangle, times scale_f(y) * scale_f(x); one
-  // lane per (block, channel, column), then per row.
   if (warp == 0) {
-    const int lg = lane / (3 * n), c = lane / n % 3, k = lane % n;
-    const float* sf = &c_scale_f[(n == 2 ? 1 : 2) * 8];
-    const bool on = lane < VPB * 3 * n;
-    float v[n];
-    if (on) {
-#pragma unroll
-      for (int r = 0; r < n; ++r) v[r] = rect[lg][c][r * n + k];
-      dct_1d<n>(v);
-#pragma unroll
-      for (int r = 0; r < n; ++r) rect[lg][c][r * n + k] = v[r];
-    }
-    __syncwarp();
-    if (on) {
-#pragma unroll
-      for (int r = 0; r < n; ++r) v[r] = rect[lg][c][k * n + r];
-      dct_1d<n>(v);
-#pragma unroll
-      for (int r = 0; r < n; ++r) A[lg][c][r][k] = v[r] * sf[r] * sf[k];
+    const int g = lane / (3 * S::LX), c = lane / S::LX % 3, k = lane % S::LX;
+    static_assert(VPB * 3 * S::LX <= 64);
+    llf_corner<S>(rect[min(g, VPB - 1)][c], k, g < VPB,
+                  [&](int y, int x, float d) { to_s(y, x, A[g][c], d); });
+    if constexpr (VPB * 3 * S::LX > 32) {  // 32 x 8: a second round of lanes
+      const int l2 = lane + 32;
+      const int g2 = l2 / (3 * S::LX), c2 = l2 / S::LX % 3, k2 = l2 % S::LX;
+      __syncwarp();
+      llf_corner<S>(rect[min(g2, VPB - 1)][c2], k2, g2 < VPB,
+                    [&](int y, int x, float d) { to_s(y, x, A[g2][c2], d); });
     }
   }
   __syncthreads();
-  // IDCT_2D (dct.rs:982): the columns of the coefficient matrix, then the
-  // rows of the result, which become sample columns.
+  // Step A: length C down R columns.
+  const int shA = warp / kWarpsA, qa = (warp % kWarpsA) * 32 + lane, ga = qa / R, ja = qa % R;
 #pragma unroll 1
-  for (int c = 0; c < 3; ++c)
-    idct_share<N>((warp + 3 * c) % kShares, [&](int i) { return A[g][c][i][j]; },
-                  [&](int r, float v) { B[g][c][r][j] = v; });
+  for (int c = 0; c < 3; ++c) {
+    float* const b = B + (ga * 3 + c) * C * (R + 1) + ja;
+    idct_share<C>((shA + 3 * c) % (C / 4), [&](int i) { return A[ga][c][i][ja]; },
+                  [&](int r, float v) { b[r * (R + 1)] = v; });
+  }
   __syncthreads();
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int k = warp + h * kShares;
+      const int k = shA + h * (C / 4);
+      const float* const b = B + (ga * 3 + c) * C * (R + 1) + ja;
       float lo, hi;
-      idct_pair<N>(k, [&](int r) { return B[g][c][r][j]; }, &lo, &hi);
-      A[g][c][k][j] = lo;
-      A[g][c][N - 1 - k][j] = hi;
+      idct_pair<C>(k, [&](int r) { return b[r * (R + 1)]; }, &lo, &hi);
+      A[ga][c][k][ja] = lo;
+      A[ga][c][C - 1 - k][ja] = hi;
     }
   __syncthreads();
+  // Step B: length R along C rows, into sample columns.
+  const int shB = warp / kWarpsB, qb = (warp % kWarpsB) * 32 + lane, gb = qb / C, jb = qb % C;
 #pragma unroll 1
-  for (int c = 0; c < 3; ++c)
-    idct_share<N>((warp + 3 * c) % kShares, [&](int i) { return A[g][c][j][i]; },
-                  [&](int r, float v) { B[g][c][r][j] = v; });
-  __syncthreads();
-  if (!active) return;
-  const int fx = x0 + j;
-  if (fx < geo.w) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int k = warp + h * kShares;
-        float lo, hi;
-        idct_pair<N>(k, [&](int r) { return B[g][c][r][j]; }, &lo, &hi);
-        float* p = a.planes + plane * c + fx;
-        if (y0 + k < geo.h) p[(size_t)(y0 + k) * geo.w] = lo;
-        if (y0 + N - 1 - k < geo.h) p[(size_t)(y0 + N - 1 - k) * geo.w] = hi;
-      }
+  for (int c = 0; c < 3; ++c) {
+    float* const b = B + (gb * 3 + c) * R * (C + 1) + jb;
+    idct_share<R>((shB + 3 * c) % (R / 4), [&](int i) { return A[gb][c][jb][i]; },
+                  [&](int r, float v) { b[r * (C + 1)] = v; });
   }
-  // J.4.3 sigma per block (restoration.rs:338 vardct_sigma).
-  if (warp == 0 && j < n * n) {
-    const size_t bi = (size_t)(by + j / n) * geo.bw + bx + j % n;
-    int s = a.sharpness[bi];
-    s = s > 7 ? 7 : s;
-    const float lut = s == 7 ? 1.0f : (float)s / 7.0f;
-    a.sigma[bi] = mul * 0.46f * lut;
+  __syncthreads();
+  {
+    const uint32_t pk = block(gb);
+    const int fx = (pk & 0xffff) * 8 + jb, y0 = (pk >> 16) * 8;
+    if (v0 + gb < count && fx < geo.w) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int k = shB + h * (R / 4);
+          const float* const b = B + (gb * 3 + c) * R * (C + 1) + jb;
+          float lo, hi;
+          idct_pair<R>(k, [&](int r) { return b[r * (C + 1)]; }, &lo, &hi);
+          float* p = a.planes + plane * c + fx;
+          if (y0 + k < geo.h) p[(size_t)(y0 + k) * geo.w] = lo;
+          if (y0 + R - 1 - k < geo.h) p[(size_t)(y0 + R - 1 - k) * geo.w] = hi;
+        }
+    }
+  }
+  if (t < VPB * S::BR * S::BC) {
+    const int g = t / (S::BR * S::BC), i = t % (S::BR * S::BC);
+    if (v0 + g < count) {
+      const uint32_t pk = block(g);
+      const size_t b0 = (size_t)(pk >> 16) * geo.bw + (pk & 0xffff);
+      const size_t bi = b0 + (size_t)(i / S::BC) * geo.bw + i % S::BC;
+      a.sigma[bi] = block_sigma(a, hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[b0]), bi);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// R1 with a side of 64 — one channel of one varblock per CTA of 512 threads
+// (a chroma channel dequantizes its luma again for the CfL), the same two
+// steps; the 64-point ones in double-float (idct64_share).  A thread's whole
+// 64-point column was 41000 dependent-issue operations, six times in a row:
+// 375 us however few the blocks; a 64 x 64 block now takes 28 us, a
+// 64 x 32 one 17 (185).
+// Bound by the FP32 pipe of the SMs that hold its three CTAs.
+// ---------------------------------------------------------------------------
+
+template <int R, int C>
+struct Rect64Smem {
+  float A[C][R + 1];
+  float2 B[C * (R + 1) > R * (C + 1) ? C * (R + 1) : R * (C + 1)];
+  float rect[RectShape<R, C>::LY * RectShape<R, C>::LX];
+};
+
+// One length-N transform of `cols` columns by 16 warps: get(i, column),
+// put(k, column, value); B holds N x (cols + 1).
+template <int N, int COLS, typename Get, typename Put>
+__device__ __forceinline__ void rect64_pass(float2* B, int warp, int lane, Get get, Put put) {
+  constexpr int kHalves = COLS / 32, kShares = N / 4, kItems = kHalves * kShares;
+  float* const Bf = reinterpret_cast<float*>(B);
+#pragma unroll 1
+  for (int item = warp; item < kItems; item += 16) {
+    // column half by half; the second half's shares start half way round, so
+    // that a warp's two shares are a long and a short one
+    const int half = item / kShares, j = half * 32 + lane;
+    const int sh = (item + half * (kShares / 2)) % kShares;
+    if constexpr (N == 64)
+      idct64_share(sh, [&](int i) { return get(i, j); },
+                   [&](int r, float2 v) { B[r * (COLS + 1) + j] = v; });
+    else
+      idct_share<N>(sh, [&](int i) { return get(i, j); },
+                    [&](int r, float v) { Bf[r * (COLS + 1) + j] = v; });
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int item = warp; item < kHalves * N / 2; item += 16) {
+    const int j = item / (N / 2) * 32 + lane, k = item % (N / 2);
+    float lo, hi;
+    if constexpr (N == 64)
+      idct64_pair(k, [&](int r) { return B[r * (COLS + 1) + j]; }, &lo, &hi);
+    else
+      idct_pair<N>(k, [&](int r) { return Bf[r * (COLS + 1) + j]; }, &lo, &hi);
+    put(k, j, lo);
+    put(N - 1 - k, j, hi);
+  }
+}
+
+template <int R, int C>
+__global__ void __launch_bounds__(512) k_render_64(RenderArgs a, const uint32_t* __restrict__ list) {
+  using S = RectShape<R, C>;
+  extern __shared__ __align__(16) unsigned char smem64[];
+  auto& sm = *reinterpret_cast<Rect64Smem<R, C>*>(smem64);
+  const int t = threadIdx.x, warp = t / 32, lane = t % 32, c = blockIdx.y;
+  const uint32_t pk = list[blockIdx.x];
+  const int bx = pk & 0xffff, by = pk >> 16, x0 = bx * 8, y0 = by * 8;
+  const Geo& geo = a.geo;
+  const size_t cplane = (size_t)geo.W8 * geo.H8;
+  const size_t bplane = (size_t)geo.bw * geo.bh;
+  const size_t plane = (size_t)geo.w * geo.h;
+  const size_t b0 = (size_t)by * geo.bw + bx;
+  constexpr int kLlf = S::LY * S::LX;
+  if (t < kLlf) {
+    const int dy = t / S::BC, dx = t % S::BC;
+    sm.rect[S::portrait ? dx * S::BR + dy : t] =
+        lf_sample(a, bplane, c, b0 + (size_t)dy * geo.bw + dx);
+  }
+  const float mul = hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[b0]);  // reconstruct.rs:27
+  const int tile = (by / 8) * geo.tw + bx / 8;
+  const float kc = c == 0 ? 0.0f + (float)a.cfl_x[tile] / 84.0f   // reconstruct.rs:96 cfl_factors
+                          : 1.0f + (float)a.cfl_b[tile] / 84.0f;
+  auto to_s = [&](int y, int x, float d) {
+    if constexpr (C > R) sm.A[x][y] = d;
+    else sm.A[y][x] = d;
+  };
+  auto dequant = [&](int ch, size_t pos, int cell) {
+    return bias_adjust_q(a.qcoeff[cplane * ch + pos], c_quant_bias[ch]) * (mul * a.qs.qm[ch]) *
+           __ldg(a.dq + ch * kDequantTableFloats + dq_offset(S::slot) + cell);
+  };
+#pragma unroll 4
+  for (int i = t; i < R * C; i += 512) {
+    const int y = i / S::CC, x = i % S::CC;
+    const size_t pos = S::portrait ? (size_t)(y0 + x) * geo.W8 + x0 + y
+                                   : (size_t)(y0 + y) * geo.W8 + x0 + x;
+    float d = dequant(c, pos, i);
+    if (c != 1) d = d + kc * dequant(1, pos, i);  // lib.rs:1344 apply_hf_cfl
+    if (y >= S::LY || x >= S::LX) to_s(y, x, d);
+  }
+  __syncthreads();
+  if (warp == 0) llf_corner<S>(sm.rect, lane, true, to_s);
+  __syncthreads();
+  rect64_pass<C, R>(sm.B, warp, lane, [&](int i, int j) { return sm.A[i][j]; },
+                    [&](int k, int j, float v) { sm.A[k][j] = v; });
+  __syncthreads();
+  rect64_pass<R, C>(sm.B, warp, lane, [&](int i, int j) { return sm.A[j][i]; },
+                    [&](int k, int j, float v) {
+                      if (x0 + j < geo.w && y0 + k < geo.h)
+                        a.planes[plane * c + (size_t)(y0 + k) * geo.w + x0 + j] = v;
+                    });
+  if (c == 1 && t < S::BR * S::BC) {
+    const size_t bi = b0 + (size_t)(t / S::BC) * geo.bw + t % S::BC;
+    a.sigma[bi] = block_sigma(a, mul, bi);
   }
 }
 
@@ -761,7 +760,7 @@ __global__ void __launch_bounds__(8 * N) k_render_sq(RenderArgs a, const uint32_
 // the split-precision render (k_tc.cu) transforms: varblock.rs:817
 // llf_from_lf (LF dequantized by reconstruct.rs:84 with the LF CfL of
 // plan-render lib.rs:1314, DCT_2D, times scale_f) and restoration.rs:338
-// vardct_sigma, exactly as k_render_vb forms them.  One thread per
+// vardct_sigma, exactly as k_render_rect forms them.  One thread per
 // (varblock, channel); llf receives 16 floats per channel per varblock.
 template <int N>
 __global__ void __launch_bounds__(128) k_llf_sigma(RenderArgs a, const uint32_t* __restrict__ list,
@@ -827,42 +826,44 @@ int launch_llf_sigma(const RenderArgs& a, const uint32_t* const* lists, const in
 
 void launch_render_varblocks(const RenderArgs& a, const uint32_t* const* lists, const int* counts,
                              const cudaStream_t* s) {
-#define JPXLG_RV(IDX, R, C)                                                              \
-  if (counts[IDX])                                                                       \
-    k_render_vb<R, C><<<(counts[IDX] + (128 / ((R) > (C) ? (R) : (C))) - 1) /            \
-                            (128 / ((R) > (C) ? (R) : (C))),                             \
-                        128, 0, s[IDX]>>>(a, lists[IDX], counts[IDX]);
-#define JPXLG_RVK(IDX, R, C, K)                                                          \
-  if (counts[IDX])                                                                       \
-    k_render_vb<R, C, K><<<(counts[IDX] + (128 / ((R) > (C) ? (R) : (C))) - 1) /         \
-                               (128 / ((R) > (C) ? (R) : (C))),                          \
-                           128, 0, s[IDX]>>>(a, lists[IDX], counts[IDX]);
+  auto n8 = [&](int i) { return (counts[i] + 15) / 16; };
+#define JPXLG_R8(IDX, KIND) \
+  if (counts[IDX]) k_render8<KIND><<<n8(IDX), 128, 0, s[IDX]>>>(a, lists[IDX], counts[IDX]);
+#define JPXLG_RECT(IDX, R, C)                                                                   \
+  if (counts[IDX]) {                                                                            \
+    constexpr int vpb = 32 / ((R) < (C) ? (R) : (C));                                           \
+    k_render_rect<R, C><<<(counts[IDX] + vpb - 1) / vpb, (R) * (C) / 4 * vpb, 0, s[IDX]>>>(     \
+        a, lists[IDX], counts[IDX]);                                                            \
+  }
+#define JPXLG_R64(IDX, R, C) \
+  if (counts[IDX])           \
+    k_render_64<R, C><<<dim3(counts[IDX], 3), 512, sizeof(Rect64Smem<R, C>), s[IDX]>>>(a, lists[IDX]);
   // shape classes in kShapeSel order: DCT8, 16x16, 32x32, 16x8, 8x16, 32x8,
   // 8x32, 32x16, 16x32, DCT2x2, 64x64, 64x32, 32x64 (rows x cols of samples)
-  if (counts[0]) k_render8<<<(counts[0] + 15) / 16, 128, 0, s[0]>>>(a, lists[0], counts[0]);
-  if (counts[1])
-    k_render_sq<16><<<(counts[1] + 1) / 2, 128, 0, s[1]>>>(a, lists[1], counts[1]);
-  if (counts[2]) k_render_sq<32><<<counts[2], 256, 0, s[2]>>>(a, lists[2], counts[2]);
-  JPXLG_RV(3, 16, 8)
-  JPXLG_RV(4, 8, 16)
-  JPXLG_RV(5, 32, 8)
-  JPXLG_RV(6, 8, 32)
-  JPXLG_RV(7, 32, 16)
-  JPXLG_RV(8, 16, 32)
-  JPXLG_RVK(9, 8, 8, 1)
-  JPXLG_RV(10, 64, 64)
-  JPXLG_RV(11, 64, 32)
-  JPXLG_RV(12, 32, 64)
-  JPXLG_RVK(13, 8, 8, 2)  // Hornuss
-  JPXLG_RVK(14, 8, 8, 3)  // DCT4x4
-  JPXLG_RVK(15, 8, 8, 4)  // DCT8x4
-  JPXLG_RVK(16, 8, 8, 5)  // DCT4x8
-  JPXLG_RVK(17, 8, 8, 6)  // AFV0..AFV3
-  JPXLG_RVK(18, 8, 8, 7)
-  JPXLG_RVK(19, 8, 8, 8)
-  JPXLG_RVK(20, 8, 8, 9)
-#undef JPXLG_RV
-#undef JPXLG_RVK
+  JPXLG_R8(0, 0)
+  JPXLG_RECT(1, 16, 16)
+  JPXLG_RECT(2, 32, 32)
+  JPXLG_RECT(3, 16, 8)
+  JPXLG_RECT(4, 8, 16)
+  JPXLG_RECT(5, 32, 8)
+  JPXLG_RECT(6, 8, 32)
+  JPXLG_RECT(7, 32, 16)
+  JPXLG_RECT(8, 16, 32)
+  JPXLG_R8(9, 1)
+  JPXLG_R64(10, 64, 64)
+  JPXLG_R64(11, 64, 32)
+  JPXLG_R64(12, 32, 64)
+  JPXLG_R8(13, 2)  // Hornuss
+  JPXLG_R8(14, 3)  // DCT4x4
+  JPXLG_R8(15, 4)  // DCT8x4
+  JPXLG_R8(16, 5)  // DCT4x8
+  JPXLG_R8(17, 6)  // AFV0..AFV3
+  JPXLG_R8(18, 7)
+  JPXLG_R8(19, 8)
+  JPXLG_R8(20, 9)
+#undef JPXLG_R8
+#undef JPXLG_RECT
+#undef JPXLG_R64
 }
 
 // ---------------------------------------------------------------------------
@@ -1373,7 +1374,10 @@ cudaError_t configure_render_kernels() {
   cudaError_t e;
   if ((e = allow(k_epf<0>, sizeof(EpfSmem<0>))) != cudaSuccess) return e;
   if ((e = allow(k_epf<1>, sizeof(EpfSmem<1>))) != cudaSuccess) return e;
-  return allow(k_epf<2>, sizeof(EpfSmem<2>));
+  if ((e = allow(k_epf<2>, sizeof(EpfSmem<2>))) != cudaSuccess) return e;
+  if ((e = allow(k_render_64<64, 64>, sizeof(Rect64Smem<64, 64>))) != cudaSuccess) return e;
+  if ((e = allow(k_render_64<64, 32>, sizeof(Rect64Smem<64, 32>))) != cudaSuccess) return e;
+  return allow(k_render_64<32, 64>, sizeof(Rect64Smem<32, 64>));
 }
 
 // ---------------------------------------------------------------------------
