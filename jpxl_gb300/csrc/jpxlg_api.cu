@@ -330,7 +330,7 @@ int check_params(jpxlg_ctx* ctx, const jpxlg_params* p) {
 // (K1), preconditioned by the inverse Gaborish (K2) when the decoder will
 // run Gaborish.  Also resets and sets the context's not-grey word.
 int transform_frame(jpxlg_ctx* ctx, const Geo& g, const void* rgb_dev, int bits,
-                    const jpxlg_params* p, const float** pre_out) {
+                    const jpxlg_params* p, float* mul_table, const float** pre_out) {
   const size_t n = (size_t)g.w * g.h;
   CK(ctx->xyb.ensure(3 * n * sizeof(float)));
   const float* lut = get_lut(ctx, bits);
@@ -339,7 +339,7 @@ int transform_frame(jpxlg_ctx* ctx, const Geo& g, const void* rgb_dev, int bits,
   float* xyb = ctx->xyb.as<float>();
   stage_begin(ctx, JPXLG_STAGE_XYB);
   launch_srgb_to_xyb(rgb_dev, bits, n, lut, xyb, xyb + n, xyb + 2 * n, ctx->d_words + 1,
-                     ctx->num_sms, ctx->stream);
+                     p->global_scale, mul_table, ctx->num_sms, ctx->stream);
   int rc = after_launch(ctx, 1);
   stage_end(ctx);
   if (rc) return rc;
@@ -373,7 +373,7 @@ int encode_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const void* rgb_dev, in
   CK(ctx->lf_seed.ensure(4 * sizeof(int)));
   CK(ctx->lf_part.ensure(kCflScratchBytes));
   const float* pre = nullptr;
-  int rc = transform_frame(ctx, g, rgb_dev, bits, p, &pre);
+  int rc = transform_frame(ctx, g, rgb_dev, bits, p, ctx->d_mul, &pre);
   if (rc) return rc;
   EncArgs a;
   a.geo = g;
@@ -399,16 +399,15 @@ int encode_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const void* rgb_dev, in
   a.cfl_fallbacks = ctx->d_words + 2;
   // square classes only: DCT8, DCT16, DCT32 are shape classes 0..2
   stage_begin(ctx, JPXLG_STAGE_FDCT_LUMA);
-  launch_mul_table(p->global_scale, ctx->d_mul, ctx->stream);
   {
     const ClassStreams cs = class_fork(ctx, L->counts, 3);
     if (p->precision == JPXLG_PRECISION_FP32) {
-      rc = after_launch(ctx, 1 + launch_fdct_luma(a, L->lists, L->counts, cs.s));
+      rc = after_launch(ctx, launch_fdct_luma(a, L->lists, L->counts, cs.s));
     } else {
       // split-precision forward transform of all three channels on the
       // tensor cores, then the luma quantization from the coefficient image
       const int terms = p->precision == JPXLG_PRECISION_BF16X3 ? 2 : 3;
-      int k = 1 + launch_fdct_tc(a, L->lists, L->counts, terms, ctx->num_sms, cs.s);
+      int k = launch_fdct_tc(a, L->lists, L->counts, terms, ctx->num_sms, cs.s);
       rc = after_launch(ctx, k + launch_luma_from_image(a, L->lists, L->counts, cs.s));
     }
     class_join(ctx, cs);
@@ -440,7 +439,7 @@ int render_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const int32_t* qcoeff,
                   const int32_t* lfq, const int8_t* cflx, const int8_t* cflb, int fx_biased,
                   int fb_biased, const int* lf_dev_unbiased, const jpxlg_params* p, int out_kind,
                   int bits, void* out_dev, float* pxyb_dev = nullptr,
-                  const float* lf_float = nullptr) {
+                  const float* lf_float = nullptr, bool mul_ready = false) {
   const Geo& g = L->geo;
   const size_t n = (size_t)g.w * g.h, nb = (size_t)g.bw * g.bh;
   if (p->precision != JPXLG_PRECISION_FP32 && (uintptr_t)qcoeff % 16 != 0)
@@ -468,8 +467,11 @@ int render_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const int32_t* qcoeff,
   a.lf_float = lf_float;
   a.err = ctx->d_words;
   stage_begin(ctx, JPXLG_STAGE_RENDER_VARBLOCKS);
-  launch_mul_table(p->global_scale, ctx->d_mul, ctx->stream);
-  uint64_t k = 1;
+  uint64_t k = 0;
+  if (!mul_ready) {
+    launch_mul_table(p->global_scale, ctx->d_mul, ctx->stream);
+    k = 1;
+  }
   const ClassStreams cs = class_fork(ctx, L->counts, kNumShapes);
   if (p->precision == JPXLG_PRECISION_FP32) {
     launch_render_varblocks(a, L->lists, L->counts, cs.s);
@@ -1226,7 +1228,8 @@ int jpxlg_probe(jpxlg_ctx* ctx, const jpxlg_layout* L, const jpxlg_ref* R, const
   if (rc) return rc;
   rc = render_device(ctx, L, ctx->qcoeff.as<int32_t>(), ctx->lfq.as<int32_t>(),
                      ctx->cflx.as<int8_t>(), ctx->cflb.as<int8_t>(), 128, 128, ctx->d_lf, p,
-                     JPXLG_OUT_LINEAR_DEPTH, bits, ctx->out.p, ctx->cxyb.as<float>());
+                     JPXLG_OUT_LINEAR_DEPTH, bits, ctx->out.p, ctx->cxyb.as<float>(), nullptr,
+                     true /* the encode left the multipliers of this scale */);
   if (rc) return rc;
   // The finish kernel fills the context's 128-double buffer (score, raw
   // error, terms); the caller's slot receives the score alone.
@@ -1269,7 +1272,7 @@ extern "C" int jpxlg_select_blocks(jpxlg_ctx* ctx, int width, int height, const 
     src = ctx->rgb.p;
   }
   const float* pre = nullptr;
-  rc = transform_frame(ctx, g, src, bits, p, &pre);
+  rc = transform_frame(ctx, g, src, bits, p, nullptr, &pre);
   if (rc) return rc;
   uint8_t* map = block_map;
   if (mem == JPXLG_MEM_HOST) {
@@ -1604,7 +1607,7 @@ namespace {
 struct DecodeStage {
   jpxlg_layout* L = nullptr;
   jpxlg_params p{};
-  size_t n = 0, n8 = 0, nb = 0, nt = 0;
+  size_t n = 0, n8 = 0, nb = 0, nt = 0, bytes = 0;
   void* host = nullptr;
   bool pinned = false;
   int32_t* q = nullptr;
@@ -1682,7 +1685,7 @@ int decode_stage(jpxlg_ctx* ctx, const jpxlg_codestream* cs, int out_kind, bool 
       if (v.lf_frame[c].size() != st.nb) return fail(ctx, JPXLG_ERR_STREAM, "LF frame size");
   const size_t qb = 3 * st.n8 * sizeof(int32_t), lb = 3 * st.nb * sizeof(int32_t);
   const size_t fb = v.lf_from_frame ? 3 * st.nb * sizeof(float) : 0;
-  const size_t bytes = qb + lb + fb + 2 * st.nt;
+  const size_t bytes = st.bytes = qb + lb + fb + 2 * st.nt;
   st.pinned = pinned;
   if (pinned) CK(cudaMallocHost(&st.host, bytes));
   else if (!(st.host = std::malloc(bytes)))
@@ -1718,30 +1721,29 @@ int decode_stage(jpxlg_ctx* ctx, const jpxlg_codestream* cs, int out_kind, bool 
 // context's buffers have grown to the frame.
 int decode_enqueue(jpxlg_ctx* ctx, const DecodeStage& st, int out_kind, void* out_dev) {
   const Geo& g = st.L->geo;
-  CK(ctx->qcoeff.ensure(3 * st.n8 * sizeof(int32_t)));
-  CK(ctx->lfq.ensure(3 * st.nb * sizeof(int32_t)));
-  CK(ctx->cflx.ensure(st.nt));
-  CK(ctx->cflb.ensure(st.nt));
+  CK(ctx->qcoeff.ensure(st.bytes));
   CK(ctx->lfs.ensure(3 * st.nb * sizeof(float)));
-  CK(ctx->aux.ensure(3 * std::max(st.n, st.nb) * sizeof(float)));
-  CK(cudaMemcpyAsync(ctx->qcoeff.p, st.q, 3 * st.n8 * sizeof(int32_t), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  CK(cudaMemcpyAsync(ctx->lfq.p, st.lfq, 3 * st.nb * sizeof(int32_t), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  CK(cudaMemcpyAsync(ctx->cflx.p, st.cflx, st.nt, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->cflb.p, st.cflb, st.nt, cudaMemcpyHostToDevice, ctx->stream));
+  // The staged planes are one block on the host and on the device: one copy
+  // (four to six of a few microseconds each on the copy engine bound a batch
+  // of small streams).
+  CK(cudaMemcpyAsync(ctx->qcoeff.p, st.host, st.bytes, cudaMemcpyHostToDevice, ctx->stream));
+  auto staged = [&](const void* h) {
+    return ctx->qcoeff.as<char>() + ((const char*)h - (const char*)st.host);
+  };
+  const int32_t* lfq = (const int32_t*)staged(st.lfq);
+  const float* lf = ctx->lfs.as<float>();
   int rc;
   if (st.lf_frame) {
-    CK(cudaMemcpyAsync(ctx->lfs.p, st.lf_frame, 3 * st.nb * sizeof(float),
-                       cudaMemcpyHostToDevice, ctx->stream));
+    lf = (const float*)staged(st.lf_frame);
   } else {
-    launch_lf_prepare(ctx->lfq.as<int32_t>(), g.bw, g.bh, st.m, st.div, st.kx, st.kb, st.smooth,
-                      ctx->aux.as<float>(), ctx->lfs.as<float>(), ctx->num_sms, ctx->stream);
-    if ((rc = after_launch(ctx, st.smooth ? 2 : 1))) return rc;
+    launch_lf_prepare(lfq, g.bw, g.bh, st.m, st.div, st.kx, st.kb, st.smooth,
+                      ctx->lfs.as<float>(), st.p.global_scale, ctx->d_mul, ctx->num_sms,
+                      ctx->stream);
+    if ((rc = after_launch(ctx, 1))) return rc;
   }
-  return render_device(ctx, st.L, ctx->qcoeff.as<int32_t>(), ctx->lfq.as<int32_t>(),
-                       ctx->cflx.as<int8_t>(), ctx->cflb.as<int8_t>(), st.fx, st.fb, nullptr,
-                       &st.p, out_kind, 8, out_dev, nullptr, ctx->lfs.as<float>());
+  return render_device(ctx, st.L, ctx->qcoeff.as<int32_t>(), lfq, (const int8_t*)staged(st.cflx),
+                       (const int8_t*)staged(st.cflb), st.fx, st.fb, nullptr, &st.p, out_kind, 8,
+                       out_dev, nullptr, lf, !st.lf_frame);
 }
 
 size_t decode_out_bytes(const DecodeStage& st, int out_kind) {
@@ -1781,6 +1783,11 @@ struct jpxlg_decode_batch {
   std::vector<size_t> out_bytes, out_off;
   uint8_t* d_out = nullptr;  // every item's pixels, back to back
   uint8_t* h_out = nullptr;  // pinned mirror, filled inside the graph
+  // One word per item, pinned: kPending from before a launch until the item's
+  // pixels stand in h_out, then its lane's device error word (a few flag
+  // bits, never kPending).
+  static constexpr uint32_t kPending = 0xffffffffu;
+  uint32_t* h_done = nullptr;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> joins;
   cudaGraph_t graph = nullptr;
@@ -1799,10 +1806,12 @@ void decode_batch_free(jpxlg_decode_batch* b) {
   for (jpxlg_ctx* l : b->lanes) jpxlg_ctx_destroy(l);
   cudaFree(b->d_out);
   cudaFreeHost(b->h_out);
+  cudaFreeHost(b->h_done);
   delete b;
 }
 
-// Item i on lane i % lanes: its render, then its pixels to the pinned mirror.
+// Item i on lane i % lanes: its render, then its pixels to the pinned mirror
+// and its word.
 int decode_batch_enqueue(jpxlg_ctx* ctx, jpxlg_decode_batch* b) {
   const size_t L = b->lanes.size();
   for (size_t i = 0; i < b->items.size(); ++i) {
@@ -1811,12 +1820,19 @@ int decode_batch_enqueue(jpxlg_ctx* ctx, jpxlg_decode_batch* b) {
     if (rc) return fail(ctx, rc, "decode batch item %zu: %s", i, lane->last_error.c_str());
     CK(cudaMemcpyAsync(b->h_out + b->out_off[i], b->d_out + b->out_off[i], b->out_bytes[i],
                        cudaMemcpyDeviceToHost, lane->stream));
+    launch_publish(lane->d_words, b->h_done + i, lane->stream);
+    if ((rc = after_launch(lane, 1)))
+      return fail(ctx, rc, "decode batch item %zu: %s", i, lane->last_error.c_str());
   }
   return JPXLG_OK;
 }
 
+// Waits for the lanes and reads the device error words that their items'
+// words say are set.
 int decode_batch_check(jpxlg_ctx* ctx, jpxlg_decode_batch* b) {
-  for (jpxlg_ctx* lane : b->lanes) {
+  for (size_t i = 0; i < b->items.size(); ++i) {
+    if (!b->h_done[i]) continue;
+    jpxlg_ctx* lane = b->lanes[i % b->lanes.size()];
     int rc = sync_and_check(lane);
     if (rc) return fail(ctx, rc, "decode batch lane: %s", lane->last_error.c_str());
   }
@@ -1876,9 +1892,12 @@ extern "C" int jpxlg_decode_batch_create(jpxlg_ctx* ctx, int n, const jpxlg_code
   CK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
   CK(cudaMalloc(&b->d_out, total));
   CK(cudaMallocHost(&b->h_out, total));
+  CK(cudaMallocHost(&b->h_done, n * sizeof(uint32_t)));
+  std::fill_n(b->h_done, n, jpxlg_decode_batch::kPending);
   // Warm-up: the lanes' buffers grow to their largest frame here.
   int rc = decode_batch_enqueue(ctx, b.get());
   if (rc) return rc;
+  for (jpxlg_ctx* lane : b->lanes) CK(cudaStreamSynchronize(lane->stream));
   if ((rc = decode_batch_check(ctx, b.get()))) return rc;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   cudaEventRecord(b->fork, ctx->stream);
@@ -1902,6 +1921,11 @@ extern "C" int jpxlg_decode_batch_run(jpxlg_ctx* ctx, jpxlg_decode_batch* b, voi
   if (!ctx || !b) return fail(ctx, JPXLG_ERR_ARGUMENT, "null argument");
   if (b->owner != ctx) return fail(ctx, JPXLG_ERR_ARGUMENT, "batch belongs to another context");
   CK(cudaSetDevice(ctx->device));
+  if (mem != JPXLG_MEM_DEVICE) {
+    // An earlier run without a wait may still be writing the words.
+    CK(cudaStreamSynchronize(ctx->stream));
+    std::fill_n(b->h_done, b->items.size(), jpxlg_decode_batch::kPending);
+  }
   CK(cudaGraphLaunch(b->exec, ctx->stream));
   if (mem == JPXLG_MEM_DEVICE) {
     if (outs)
@@ -1911,13 +1935,28 @@ extern "C" int jpxlg_decode_batch_run(jpxlg_ctx* ctx, jpxlg_decode_batch* b, voi
                              cudaMemcpyDeviceToDevice, ctx->stream));
     return JPXLG_OK;
   }
-  CK(cudaStreamSynchronize(ctx->stream));
-  int rc = decode_batch_check(ctx, b);
-  if (rc) return rc;
+  // Each item's pixels as they arrive, while the rest renders; items of a
+  // lane finish in order, so a pass over the pending ones meets the done ones
+  // soon.  The stream's own end bounds the wait.
+  std::vector<size_t> pending;
   if (outs)
     for (size_t i = 0; i < b->items.size(); ++i)
-      if (outs[i]) std::memcpy(outs[i], b->h_out + b->out_off[i], b->out_bytes[i]);
-  return JPXLG_OK;
+      if (outs[i]) pending.push_back(i);
+  bool running = true, clean = true;
+  while (clean && !pending.empty() && running) {
+    running = cudaStreamQuery(ctx->stream) == cudaErrorNotReady;
+    size_t kept = 0;
+    for (size_t k = 0; k < pending.size() && clean; ++k) {
+      const size_t i = pending[k];
+      const uint32_t word = __atomic_load_n(&b->h_done[i], __ATOMIC_ACQUIRE);
+      if (word == jpxlg_decode_batch::kPending) pending[kept++] = i;
+      else if (word) clean = false;
+      else std::memcpy(outs[i], b->h_out + b->out_off[i], b->out_bytes[i]);
+    }
+    pending.resize(clean ? kept : 0);
+  }
+  CK(cudaStreamSynchronize(ctx->stream));
+  return decode_batch_check(ctx, b);
 }
 
 extern "C" int jpxlg_decode_batch_destroy(jpxlg_decode_batch* b) {

@@ -90,6 +90,10 @@ __device__ __forceinline__ float hf_multiplier_f64(uint32_t global_scale, uint32
   const double denom = (double)global_scale * (double)hf_mul;
   return denom <= 0.0 ? 0.0f : (float)(65536.0 / denom);
 }
+// The table, by a CTA of kMulTableN threads.
+__device__ __forceinline__ void fill_mul_table(uint32_t global_scale, float* table) {
+  table[threadIdx.x] = hf_multiplier_f64(global_scale, threadIdx.x);
+}
 __device__ __forceinline__ float hf_multiplier(const float* table, uint32_t global_scale,
                                                uint32_t hf_mul) {
   return hf_mul < (uint32_t)kMulTableN ? __ldg(&table[hf_mul])

@@ -56,10 +56,13 @@ struct RenderArgs {
 };
 
 // LF of a decoded frame: dequantize, LF CfL and (smooth) adaptive smoothing
-// into out [3][bw*bh]; tmp holds as much when smoothing.
+// into out [3][bw*bh]; also the table of HF multipliers for global_scale.
 void launch_lf_prepare(const int32_t* lfq, int bw, int bh, const float m[3], float div, float kx,
-                       float kb, bool smooth, float* tmp, float* out, int num_sms,
-                       cudaStream_t s);
+                       float kb, bool smooth, float* out, uint32_t global_scale, float* mul_table,
+                       int num_sms, cudaStream_t s);
+// One finished stream of a batch: its lane's device error word to `flag`, in
+// pinned host memory, after everything its stream has written before.
+void launch_publish(const uint32_t* err, uint32_t* flag, cudaStream_t s);
 void upload_dct64(const float* matrix, cudaStream_t s);
 void upload_afv(const double* basis, cudaStream_t s);
 bool launch_special_diag(int kind, const float* coef, int n, float* out, cudaStream_t s);
@@ -74,8 +77,10 @@ cudaError_t configure_render_kernels();
 
 void upload_dct_constants(const float* iv4, const float* iv8, const float* iv16,
                           const float* scale_f, cudaStream_t s);
+// mul_table (or null): also the table of HF multipliers for global_scale.
 void launch_srgb_to_xyb(const void* rgb, int bits, size_t n, const float* lut, float* x, float* y,
-                        float* b, uint32_t* not_gray, int num_sms, cudaStream_t s);
+                        float* b, uint32_t* not_gray, uint32_t global_scale, float* mul_table,
+                        int num_sms, cudaStream_t s);
 // One launch (the ring of tiles along the frame's rows and columns of other
 // rules, then the tiles inside it); returns 1.
 int launch_precondition(const float* in, float* out, int w, int h, cudaStream_t s);

@@ -51,8 +51,13 @@ __global__ void __launch_bounds__(256, 8) k_srgb_to_xyb(const T* __restrict__ rg
                                                      float* __restrict__ px,
                                                      float* __restrict__ py,
                                                      float* __restrict__ pb,
-                                                     uint32_t* __restrict__ not_gray) {
+                                                     uint32_t* __restrict__ not_gray,
+                                                     uint32_t global_scale,
+                                                     float* __restrict__ mul_table) {
   constexpr bool kByte = sizeof(T) == 1;
+  // The transform's table of HF multipliers, where it follows: the last CTA's
+  // threads, beside its pixels (a launch of its own cost 2.9 us).
+  if (mul_table && blockIdx.x == gridDim.x - 1) fill_mul_table(global_scale, mul_table);
   __shared__ float slut[kByte ? 256 : 1];
   if (kByte) {
     slut[threadIdx.x] = __ldg(lut + threadIdx.x);
@@ -75,14 +80,16 @@ __global__ void __launch_bounds__(256, 8) k_srgb_to_xyb(const T* __restrict__ rg
 }
 
 void launch_srgb_to_xyb(const void* rgb, int bits, size_t n, const float* lut, float* x, float* y,
-                        float* b, uint32_t* not_gray, int num_sms, cudaStream_t s) {
+                        float* b, uint32_t* not_gray, uint32_t global_scale, float* mul_table,
+                        int num_sms, cudaStream_t s) {
   const int blocks = (int)std::max<size_t>(
       1, std::min<size_t>((n + 255) / 256, (size_t)num_sms * 16));
   if (bits == 8)
-    k_srgb_to_xyb<uint8_t><<<blocks, 256, 0, s>>>((const uint8_t*)rgb, n, lut, x, y, b, not_gray);
+    k_srgb_to_xyb<uint8_t><<<blocks, 256, 0, s>>>((const uint8_t*)rgb, n, lut, x, y, b, not_gray,
+                                                  global_scale, mul_table);
   else
     k_srgb_to_xyb<uint16_t><<<blocks, 256, 0, s>>>((const uint16_t*)rgb, n, lut, x, y, b,
-                                                   not_gray);
+                                                   not_gray, global_scale, mul_table);
 }
 
 // ---------------------------------------------------------------------------
@@ -1491,9 +1498,8 @@ int launch_cfl_chroma(const EncArgs& a, int* lf_seeds, void* lf_scratch, cudaStr
   return 4;
 }
 
-__global__ void k_mul_table(uint32_t global_scale, float* table) {
-  const int h = threadIdx.x;
-  if (h < kMulTableN) table[h] = hf_multiplier_f64(global_scale, (uint32_t)h);
+__global__ void __launch_bounds__(kMulTableN) k_mul_table(uint32_t global_scale, float* table) {
+  fill_mul_table(global_scale, table);
 }
 
 void launch_mul_table(uint32_t global_scale, float* table, cudaStream_t s) {

@@ -1386,54 +1386,80 @@ cudaError_t configure_render_kernels() {
 // (m * q / 2^extra_precision), apply the LF CfL, then smooth interior cells.
 // ---------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(256) k_lf_dequant(const int32_t* __restrict__ lfq, size_t nb,
+// A cell dequantizes its own neighbours again: thirty multiplications and
+// divisions against a second launch and a plane between them (11.8 us in three
+// launches with the multipliers' table, 9 in one).
+__global__ void __launch_bounds__(256) k_lf_prepare(const int32_t* __restrict__ lfq, int bw, int bh,
                                                     float m0, float m1, float m2, float div,
-                                                    float kx, float kb, float* __restrict__ out) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const float dx = m0 * (float)lfq[i] / div;
-    const float dy = m1 * (float)lfq[nb + i] / div;
-    const float db = m2 * (float)lfq[2 * nb + i] / div;
-    out[i] = dx + kx * dy;
-    out[nb + i] = dy;
-    out[2 * nb + i] = db + kb * dy;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_lf_smooth(const float* __restrict__ in, int bw, int bh,
-                                                   float m0, float m1, float m2,
-                                                   float* __restrict__ out) {
+                                                    float kx, float kb, bool smooth,
+                                                    float* __restrict__ out, uint32_t global_scale,
+                                                    float* __restrict__ mul_table) {
+  if (blockIdx.x == gridDim.x - 1) fill_mul_table(global_scale, mul_table);
   const size_t nb = (size_t)bw * bh;
+  const float m[3] = {m0, m1, m2};
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb;
        i += (size_t)gridDim.x * blockDim.x) {
     const int x = (int)(i % bw), y = (int)(i / bw);
-    if (x == 0 || y == 0 || x == bw - 1 || y == bh - 1) {
-      for (int c = 0; c < 3; ++c) out[c * nb + i] = in[c * nb + i];
+    auto lf = [&](size_t at, float* v) {
+      const float dx = m0 * (float)lfq[at] / div;
+      const float dy = m1 * (float)lfq[nb + at] / div;
+      const float db = m2 * (float)lfq[2 * nb + at] / div;
+      v[0] = dx + kx * dy;
+      v[1] = dy;
+      v[2] = db + kb * dy;
+    };
+    float sv[3];
+    lf(i, sv);
+    if (!smooth || x == 0 || y == 0 || x == bw - 1 || y == bh - 1) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) out[c * nb + i] = sv[c];
       continue;
     }
-    float wa[3], sv[3];
-    for (int c = 0; c < 3; ++c) {
-      const float* p = in + c * nb;
-      auto g = [&](int dx, int dy) { return p[(size_t)(y + dy) * bw + x + dx]; };
-      sv[c] = g(0, 0);
-      wa[c] = (0.052262735f * sv[c] + 0.2034514f * (((g(-1, 0) + g(1, 0)) + g(0, -1)) + g(0, 1))) +
-              0.03348292f * (((g(-1, -1) + g(1, -1)) + g(-1, 1)) + g(1, 1));
+    // in the reference's order: W + E + N + S, NW + NE + SW + SE
+    const int side[4][2] = {{-1, 0}, {1, 0}, {0, -1}, {0, 1}};
+    const int diag[4][2] = {{-1, -1}, {1, -1}, {-1, 1}, {1, 1}};
+    float se[3], sd[3];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float e[3], d[3];
+      lf((size_t)(y + side[k][1]) * bw + x + side[k][0], e);
+      lf((size_t)(y + diag[k][1]) * bw + x + diag[k][0], d);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        se[c] = k == 0 ? e[c] : se[c] + e[c];
+        sd[c] = k == 0 ? d[c] : sd[c] + d[c];
+      }
     }
-    const float m[3] = {m0, m1, m2};
-    float gap = 0.5f;
-    for (int c = 0; c < 3; ++c) gap = fmaxf(gap, fabsf(wa[c] - sv[c]) / m[c]);
+    float wa[3], gap = 0.5f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      wa[c] = (0.052262735f * sv[c] + 0.2034514f * se[c]) + 0.03348292f * sd[c];
+      gap = fmaxf(gap, fabsf(wa[c] - sv[c]) / m[c]);
+    }
     const float factor = fmaxf(3.0f - 4.0f * gap, 0.0f);
+#pragma unroll
     for (int c = 0; c < 3; ++c) out[c * nb + i] = (wa[c] - sv[c]) * factor + sv[c];
   }
 }
 
 void launch_lf_prepare(const int32_t* lfq, int bw, int bh, const float m[3], float div, float kx,
-                       float kb, bool smooth, float* tmp, float* out, int num_sms,
-                       cudaStream_t s) {
+                       float kb, bool smooth, float* out, uint32_t global_scale, float* mul_table,
+                       int num_sms, cudaStream_t s) {
   const size_t nb = (size_t)bw * bh;
   const int blocks = (int)std::max<size_t>(1, std::min<size_t>((nb + 255) / 256, num_sms * 4));
-  k_lf_dequant<<<blocks, 256, 0, s>>>(lfq, nb, m[0], m[1], m[2], div, kx, kb, smooth ? tmp : out);
-  if (smooth) k_lf_smooth<<<blocks, 256, 0, s>>>(tmp, bw, bh, m[0], m[1], m[2], out);
+  k_lf_prepare<<<blocks, 256, 0, s>>>(lfq, bw, bh, m[0], m[1], m[2], div, kx, kb, smooth, out,
+                                      global_scale, mul_table);
+}
+
+// The stream's earlier work is visible to this thread, and the release makes
+// it visible to the host that reads the flag.
+__global__ void k_publish(const uint32_t* __restrict__ err, uint32_t* flag) {
+  const uint32_t e = *err;
+  asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(flag), "r"(e) : "memory");
+}
+
+void launch_publish(const uint32_t* err, uint32_t* flag, cudaStream_t s) {
+  k_publish<<<1, 1, 0, s>>>(err, flag);
 }
 
 // The special transforms on given blocks, one thread per block (a
