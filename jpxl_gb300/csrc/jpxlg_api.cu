@@ -347,7 +347,8 @@ int transform_frame(jpxlg_ctx* ctx, const Geo& g, const void* rgb_dev, int bits,
   if (p->gaborish) {
     CK(ctx->pre.ensure(3 * n * sizeof(float)));
     stage_begin(ctx, JPXLG_STAGE_PRECONDITION);
-    rc = after_launch(ctx, launch_precondition(xyb, ctx->pre.as<float>(), g.w, g.h, ctx->stream));
+    rc = after_launch(ctx, launch_precondition(xyb, ctx->pre.as<float>(), g.w, g.h, ctx->num_sms,
+                                              ctx->stream));
     stage_end(ctx);
     if (rc) return rc;
     pre = ctx->pre.as<float>();
@@ -420,8 +421,8 @@ int encode_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const void* rgb_dev, in
   {
     const int chains[2] = {2, 1};  // the tiles on the context's stream, the LF chain beside
     const ClassStreams cs = class_fork(ctx, chains, 2);
-    rc = after_launch(ctx, launch_cfl_chroma(a, ctx->lf_seed.as<int>(), ctx->lf_part.p, cs.s[0],
-                                             cs.s[1]));
+    rc = after_launch(ctx, launch_cfl_chroma(a, ctx->lf_seed.as<int>(), ctx->lf_part.p, ctx->num_sms,
+                                             cs.s[0], cs.s[1]));
     class_join(ctx, cs);
   }
   stage_end(ctx);
@@ -552,11 +553,25 @@ int ensure_blur_scratch(jpxlg_ctx* ctx, const int (*dims)[2], int n, int nq) {
 // aligned.
 size_t plane_set_floats(int w, int h) { return (3 * (size_t)w * h + 3) & ~(size_t)3; }
 
+// Whether a kernel may store a double to a caller's address: memory of this
+// device, aligned.  Anything else goes through a copy, which checks it.
+bool device_double(const jpxlg_ctx* ctx, const double* p) {
+  if (!p || (uintptr_t)p % sizeof(double) != 0) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+}
+
 // Candidate side of SSIMULACRA2 against `ref`: cand_dev is the candidate's
 // linear RGB; cand_xyb (optional) its positive XYB, when the producer of the
-// pixels already formed it.
+// pixels already formed it.  score and raw (each may be null) receive the
+// first two of out_dev's doubles as well.
 int score_device(jpxlg_ctx* ctx, const jpxlg_ref* ref, const float* cand_dev,
-                 const float* cand_xyb, double* out_dev) {
+                 const float* cand_xyb, double* out_dev, double* score = nullptr,
+                 double* raw = nullptr) {
   const int w = ref->w, h = ref->h, ns = ref->nscales;
   int dims[kMaxScales][2], ctas[kMaxScales], pixels[kMaxScales];
   size_t pyr = 0, ctas_total = 0;
@@ -598,7 +613,8 @@ int score_device(jpxlg_ctx* ctx, const jpxlg_ref* ref, const float* cand_dev,
   // the hook counts the blur's kernels
   launch_score_scales(bs, ns, 0, 3, ctx->hpl.as<float>(), ctx->bcarry.p, ctx->d_words,
                       ctx->stream, ssim_stage_hook, ctx);
-  k += launch_score_finish(ctx->partial.as<DF>(), ctas, ns, pixels, out_dev, ctx->stream);
+  k += launch_score_finish(ctx->partial.as<DF>(), ctas, ns, pixels, ctx->bcarry.p, out_dev, score,
+                           raw, ctx->stream);
   rc = after_launch(ctx, k);
   stage_end(ctx);
   return rc;
@@ -1147,13 +1163,16 @@ int jpxlg_ssim2_score(jpxlg_ctx* ctx, const jpxlg_ref* R, const float* rgb, uint
   }
   // The finish kernel writes score, raw error and every term into the
   // context's own buffer; callers receive only the outputs they asked for.
-  int rc = score_device(ctx, R, cand, nullptr, ctx->score.as<double>());
+  const bool dev = mem == JPXLG_MEM_DEVICE;
+  const bool sd = dev && device_double(ctx, score), rd = dev && device_double(ctx, raw_error);
+  int rc = score_device(ctx, R, cand, nullptr, ctx->score.as<double>(), sd ? score : nullptr,
+                        rd ? raw_error : nullptr);
   if (rc) return rc;
-  if (mem == JPXLG_MEM_DEVICE) {
+  if (dev) {
     const double* s = ctx->score.as<double>();
-    if (score)
+    if (score && !sd)
       CK(cudaMemcpyAsync(score, s, sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-    if (raw_error)
+    if (raw_error && !rd)
       CK(cudaMemcpyAsync(raw_error, s + 1, sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     if (terms)
       CK(cudaMemcpyAsync(terms, s + 2, R->nscales * 18 * sizeof(double), cudaMemcpyDeviceToDevice,
@@ -1233,10 +1252,13 @@ int jpxlg_probe(jpxlg_ctx* ctx, const jpxlg_layout* L, const jpxlg_ref* R, const
   if (rc) return rc;
   // The finish kernel fills the context's 128-double buffer (score, raw
   // error, terms); the caller's slot receives the score alone.
-  rc = score_device(ctx, R, ctx->out.as<float>(), ctx->cxyb.as<float>(), ctx->score.as<double>());
+  const bool direct = mem == JPXLG_MEM_DEVICE && device_double(ctx, score);
+  rc = score_device(ctx, R, ctx->out.as<float>(), ctx->cxyb.as<float>(), ctx->score.as<double>(),
+                    direct ? score : nullptr);
   if (rc) return rc;
   if (mem == JPXLG_MEM_DEVICE) {
-    CK(cudaMemcpyAsync(score, ctx->score.p, sizeof(double), cudaMemcpyDeviceToDevice,
+    if (!direct)
+      CK(cudaMemcpyAsync(score, ctx->score.p, sizeof(double), cudaMemcpyDeviceToDevice,
                        ctx->stream));
     return JPXLG_OK;
   }
@@ -1590,7 +1612,8 @@ extern "C" int jpxlg_ssim2_score_static(jpxlg_ctx* ctx, const jpxlg_ref* ref,
     pixels[s] = rs.w * rs.h;
     part += (size_t)ctas[s] * 18;
   }
-  k += launch_score_finish(part0, ctas, ref->nscales, pixels, out_dev, ctx->stream);
+  k += launch_score_finish(part0, ctas, ref->nscales, pixels, carry, out_dev, nullptr, nullptr,
+                           ctx->stream);
   return after_launch(ctx, k);
 }
 

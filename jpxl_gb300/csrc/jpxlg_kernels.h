@@ -83,7 +83,7 @@ void launch_srgb_to_xyb(const void* rgb, int bits, size_t n, const float* lut, f
                         int num_sms, cudaStream_t s);
 // One launch (the ring of tiles along the frame's rows and columns of other
 // rules, then the tiles inside it); returns 1.
-int launch_precondition(const float* in, float* out, int w, int h, cudaStream_t s);
+int launch_precondition(const float* in, float* out, int w, int h, int num_sms, cudaStream_t s);
 // The per-shape-class launchers take one stream per class (s[i] for class
 // i), so that independent classes can run side by side.  Each returns the
 // number of kernels it launched.
@@ -95,7 +95,7 @@ constexpr size_t kCflScratchBytes = (size_t)kLfCtas * (7 * 8 + 8 * 4);
 // CfL estimation and the chroma quantization: the tiles' kernel on s, the
 // LF factors' chain and the chroma LF on lf_s (it reads only the LF planes);
 // the caller joins lf_s back.  Returns the number of kernels.
-int launch_cfl_chroma(const EncArgs& a, int* lf_seeds, void* lf_scratch, cudaStream_t s,
+int launch_cfl_chroma(const EncArgs& a, int* lf_seeds, void* lf_scratch, int num_sms, cudaStream_t s,
                       cudaStream_t lf_s);
 
 void launch_render_varblocks(const RenderArgs& a, const uint32_t* const* lists,
@@ -210,9 +210,14 @@ using ScaleHook = void (*)(void* user, int part);
 int launch_score_scales(const BlurScale* scales, int n, int c0, int nch, float* hpl, void* carry,
                         uint32_t* err, cudaStream_t s, ScaleHook hook = nullptr,
                         void* user = nullptr);
-// Two launches (the per-scale sums, then the score); returns 2.  The sums
-// overwrite row 0 of each scale's partial rows.
+// The per-scale sums, then the score, in one launch; returns 1.  The sums
+// overwrite row 0 of each scale's partial rows; `carry` is the buffer that
+// launch_score_scales used.  out receives the score, the raw error and the
+// terms; score and raw (each may be null) the first two as well.
 int launch_score_finish(DF* partials, const int* ctas_per_scale, int nscales,
-                        const int* pixels_per_scale, double* out, cudaStream_t s);
+                        const int* pixels_per_scale, void* carry, double* out, double* score,
+                        double* raw, cudaStream_t s);
+// The word of a scan buffer's header that counts finished CTAs.
+uint32_t* blur_ticket(void* carry);
 
 }  // namespace jpxlg

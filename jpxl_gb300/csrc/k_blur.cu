@@ -254,9 +254,13 @@ __device__ __forceinline__ f2 ripple_hom2(int u, const f2* ep, const f2* eq, f2 
 // ---------------------------------------------------------------------------
 
 struct ScanHeader {
-  uint32_t epoch, counter, finished, pad[13];
+  uint32_t epoch, counter, finished;
+  uint32_t ticket;  // the score's last CTA; zero between launches
+  uint32_t pad[12];
 };
 static_assert(sizeof(ScanHeader) == 64, "scan header");
+
+uint32_t* blur_ticket(void* carry) { return &static_cast<ScanHeader*>(carry)->ticket; }
 
 __device__ __forceinline__ void scan_store(uint4* p, float a, float b, float c, uint32_t tag) {
   const unsigned long long lo =

@@ -134,11 +134,10 @@ void launch_srgb_to_xyb(const void* rgb, int bits, size_t n, const float* lut, f
 // frame coordinates (always among the cell's own 3 x 3 neighbourhood).  One
 // launch holds both: the ring's CTAs first (they take longer), then the
 // interior's, which fill the SMs around them.
-constexpr int kPreOut = 104;
+constexpr int kPreOut = 104;                   // outputs across
 constexpr int kPreHalo = 12;
 constexpr int kPreW = kPreOut + 2 * kPreHalo;  // 128: 32 lanes x 4 columns
-constexpr int kPreRows = 8;                     // rows of a lane
-constexpr int kPreWarps = kPreW / kPreRows;    // 16
+constexpr int kPreWarps = 16;                  // of ROWS = 8 or 4 rows
 constexpr int kPreThreads = 32 * kPreWarps;
 static_assert(kPreW == 128 && kPreHalo >= 12, "tile of the inverse Gaborish");
 // Tile rows in shared memory are kPreP floats apart: 16-byte aligned for the
@@ -146,10 +145,15 @@ static_assert(kPreW == 128 && kPreHalo >= 12, "tile of the inverse Gaborish");
 // banks for the ring's per-cell accesses (a pitch of 128 puts them all in
 // one).
 constexpr int kPreP = kPreW + 4;
-// F (a ring tile's source, [kPreW][kPreP]), then an interior tile's published
+// F (a ring tile's source, [H][kPreP]), then an interior tile's published
 // rows [2 parities][kPreWarps][first, last][kPreW], or a ring tile's step
-// inputs [2 parities][kPreW][kPreP].
-constexpr size_t kPreRingSmem = (size_t)3 * kPreW * kPreP * sizeof(float);
+// inputs [2 parities][H][kPreP].
+template <int ROWS>
+struct PreTile {
+  static constexpr int H = ROWS * kPreWarps;         // 128 or 64 rows
+  static constexpr int kOut = H - 2 * kPreHalo;      // 104 or 40 of them outputs
+  static constexpr size_t kSmem = (size_t)3 * H * kPreP * sizeof(float);
+};
 
 struct EncKernel {
   float centre, edge, corner, inv_c;
@@ -234,11 +238,13 @@ struct PreSpecial {
   uint32_t a;  // tx | xm << 7 | xp << 14 | ty << 21
   uint32_t b;  // ym | yp << 7 | seq << 14 | div << 15 | valid << 16
 };
+template <int H>
 __device__ __forceinline__ PreSpecial pre_special(int ty, int tx, int cx, int cy, int gx0, int gy0,
                                                   int w, int h, bool seq, bool div) {
-  auto clampt = [](int v) { return min(max(v, 0), kPreW - 1); };
-  const int xm = clampt(mirror1d(cx - 1, w) - gx0), xp = clampt(mirror1d(cx + 1, w) - gx0);
-  const int ym = clampt(mirror1d(cy - 1, h) - gy0), yp = clampt(mirror1d(cy + 1, h) - gy0);
+  auto clampt = [](int v, int n) { return min(max(v, 0), n - 1); };
+  const int xm = clampt(mirror1d(cx - 1, w) - gx0, kPreW),
+            xp = clampt(mirror1d(cx + 1, w) - gx0, kPreW);
+  const int ym = clampt(mirror1d(cy - 1, h) - gy0, H), yp = clampt(mirror1d(cy + 1, h) - gy0, H);
   return {(uint32_t)tx | (uint32_t)xm << 7 | (uint32_t)xp << 14 | (uint32_t)ty << 21,
           (uint32_t)ym | (uint32_t)yp << 7 | (uint32_t)seq << 14 | (uint32_t)div << 15 | 1u << 16};
 }
@@ -277,6 +283,7 @@ __device__ __forceinline__ void pre_special_step(const PreSpecial& c, const floa
 // in-frame columns, then the special columns (0 and [cb, w)) down its other
 // in-frame rows; rb and cb as the reference's groups of four and division
 // tail place them.
+template <int H>
 struct PreRingCells {
   int cx0, ncin, rB0, nr0, nrin, cB0, nrow_cells, count, groups;
   bool r0, c0;
@@ -295,12 +302,13 @@ struct PreRingCells {
     }
     const int cx = gx0 + tx, cy = gy0 + ty;
     const bool border = cx == 0 || cx == w - 1 || cy == 0 || cy == h - 1;
-    return pre_special(ty, tx, cx, cy, gx0, gy0, w, h, border || cx - 1 >= 4 * groups,
+    return pre_special<H>(ty, tx, cx, cy, gx0, gy0, w, h, border || cx - 1 >= 4 * groups,
                        (size_t)cy * w + cx >= bulk);
   }
 };
-__device__ __forceinline__ PreRingCells pre_ring_cells(int w, int h, int gx0, int gy0) {
-  PreRingCells g;
+template <int H>
+__device__ __forceinline__ PreRingCells<H> pre_ring_cells(int w, int h, int gx0, int gy0) {
+  PreRingCells<H> g;
   const size_t plane = (size_t)w * h;
   g.groups = (w >= 3 && h >= 3) ? (w - 2) / 4 : 0;
   g.bulk = plane - plane % 4;
@@ -309,7 +317,7 @@ __device__ __forceinline__ PreRingCells pre_ring_cells(int w, int h, int gx0, in
   const int cb = max(min(w - 1, 4 * g.groups + 1), 1);
   g.cx0 = max(0, -gx0);
   g.ncin = max(0, min(kPreW, w - gx0) - g.cx0);
-  const int ry0 = max(0, -gy0), ry1 = min(kPreW, h - gy0), cx1 = g.cx0 + g.ncin;
+  const int ry0 = max(0, -gy0), ry1 = min(H, h - gy0), cx1 = g.cx0 + g.ncin;
   g.r0 = -gy0 >= ry0 && -gy0 < ry1;
   g.rB0 = max(ry0, rb - gy0);
   const int nsr = (g.r0 ? 1 : 0) + max(0, ry1 - g.rB0);
@@ -327,14 +335,15 @@ __device__ __forceinline__ int pre_clamp(int c, int size) { return min(max(c, 0)
 
 // One tile: item is the tile's index among the interior tiles (row-major
 // over the rectangle) or among the ring tiles.
-template <bool kEdge>
+template <int ROWS, bool kEdge>
 __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
                                                   float* __restrict__ out, int w, int h,
                                                   const EncKernel& k, const PreTiles& pt,
                                                   int item) {
   extern __shared__ __align__(16) float pre_smem[];
-  float* const F = pre_smem;                   // [kPreW][kPreP]
-  float* const xb = pre_smem + kPreW * kPreP;  // published rows, or the ring's step inputs
+  constexpr int H = PreTile<ROWS>::H;
+  float* const F = pre_smem;               // [H][kPreP]
+  float* const xb = pre_smem + H * kPreP;  // published rows, or the ring's step inputs
   const size_t plane = (size_t)w * h;
   in += plane * blockIdx.z;
   out += plane * blockIdx.z;
@@ -364,25 +373,25 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int tx0 = tile_x * kPreOut, ty0 = tile_y * kPreOut;
+  const int tx0 = tile_x * kPreOut, ty0 = tile_y * PreTile<ROWS>::kOut;
   const int gx0 = tx0 - kPreHalo, gy0 = ty0 - kPreHalo;
-  const int lx = 4 * lane, ly = kPreRows * warp;  // the thread's first column and row in the tile
+  const int lx = 4 * lane, ly = ROWS * warp;  // the thread's first column and row in the tile
   const int gx = gx0 + lx, gy = gy0 + ly;  // ... in the frame
   // Load: tiles inside the frame with 16-byte aligned rows take 16-byte
   // loads; others clamp each coordinate (cells outside the frame are never
   // read by a cell inside it, so their values do not matter).
-  const bool vec = gx0 >= 0 && gy0 >= 0 && gx0 + kPreW <= w && gy0 + kPreW <= h && (w % 4) == 0 &&
+  const bool vec = gx0 >= 0 && gy0 >= 0 && gx0 + kPreW <= w && gy0 + H <= h && (w % 4) == 0 &&
                    ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
-  float4 X[kPreRows];
+  float4 X[ROWS];
   if (vec) {
 #pragma unroll
-    for (int r = 0; r < kPreRows; ++r)
+    for (int r = 0; r < ROWS; ++r)
       X[r] = __ldg(reinterpret_cast<const float4*>(in + (size_t)(gy + r) * w + gx));
   } else {
     const int c0 = pre_clamp(gx, w), c1 = pre_clamp(gx + 1, w), c2 = pre_clamp(gx + 2, w),
               c3 = pre_clamp(gx + 3, w);
 #pragma unroll
-    for (int r = 0; r < kPreRows; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
       const float* row = in + (size_t)pre_clamp(gy + r, h) * w;
       X[r] = make_float4(__ldg(row + c0), __ldg(row + c1), __ldg(row + c2), __ldg(row + c3));
     }
@@ -391,9 +400,9 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
   const f2 k2 = f2_pack(k.corner, k.corner), i2 = f2_pack(k.inv_c, k.inv_c);
   const unsigned full = 0xffffffffu;
   if (!kEdge) {
-    float4 Fr[kPreRows];
+    float4 Fr[ROWS];
 #pragma unroll
-    for (int r = 0; r < kPreRows; ++r) Fr[r] = X[r];
+    for (int r = 0; r < ROWS; ++r) Fr[r] = X[r];
     // The rows just above and below the warp's: the last row of the warp
     // above and the first of the warp below (the tile's edge rows for the
     // first and last warps, never read by an exact cell).
@@ -403,15 +412,15 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
     for (int it = 0; it < 12; ++it) {
       float* const S = xb + (it & 1) * (kPreWarps * 2 * kPreW);
       *reinterpret_cast<float4*>(S + (2 * warp) * kPreW + lx) = X[0];
-      *reinterpret_cast<float4*>(S + (2 * warp + 1) * kPreW + lx) = X[kPreRows - 1];
+      *reinterpret_cast<float4*>(S + (2 * warp + 1) * kPreW + lx) = X[ROWS - 1];
       __syncthreads();
       float4 prev = *reinterpret_cast<const float4*>(S + row_up);
       float pW = __shfl_up_sync(full, prev.w, 1), pE = __shfl_down_sync(full, prev.x, 1);
       float mW = __shfl_up_sync(full, X[0].w, 1), mE = __shfl_down_sync(full, X[0].x, 1);
 #pragma unroll
-      for (int r = 0; r < kPreRows; ++r) {
+      for (int r = 0; r < ROWS; ++r) {
         const float4 nxt =
-            r < kPreRows - 1 ? X[r + 1 < kPreRows ? r + 1 : r] : *reinterpret_cast<const float4*>(S + row_down);
+            r < ROWS - 1 ? X[r + 1 < ROWS ? r + 1 : r] : *reinterpret_cast<const float4*>(S + row_down);
         const float sW = __shfl_up_sync(full, nxt.w, 1), sE = __shfl_down_sync(full, nxt.x, 1);
         const float4 f = Fr[r];
         f2 kxa, kxb;
@@ -430,7 +439,7 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
     // Ring tiles keep the step's input in shared memory and write the
     // step's output to the other buffer; each thread first finds its cells
     // of another rule (at most two, as a rule none).
-    const PreRingCells rc = pre_ring_cells(w, h, gx0, gy0);
+    const PreRingCells<H> rc = pre_ring_cells<H>(w, h, gx0, gy0);
     PreSpecial mine[2] = {{0u, 0u}, {0u, 0u}};
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
@@ -438,31 +447,31 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
       if (i < rc.count) mine[s] = rc.special(i, w, h, gx0, gy0);
     }
 #pragma unroll
-    for (int r = 0; r < kPreRows; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
       *reinterpret_cast<float4*>(F + (ly + r) * kPreP + lx) = X[r];
       *reinterpret_cast<float4*>(xb + (ly + r) * kPreP + lx) = X[r];
     }
     const int row_up = max(ly - 1, 0) * kPreP + lx;
     // Rows wholly outside the frame are read by no cell inside it (64 x 64:
     // half of the tile; 30 us with them, 23 without).
-    const bool live = gy + kPreRows - 1 >= 0 && gy < h;
+    const bool live = gy + ROWS - 1 >= 0 && gy < h;
 #pragma unroll 1
     for (int it = 0; it < 12; ++it) {
-      const float* const S = xb + (it & 1) * (kPreW * kPreP);
-      float* const Sn = xb + ((it + 1) & 1) * (kPreW * kPreP);
+      const float* const S = xb + (it & 1) * (H * kPreP);
+      float* const Sn = xb + ((it + 1) & 1) * (H * kPreP);
       __syncthreads();
       // A warp whose four rows have all left the exact region [1 + it,
-      // 127 - it) rests; its rows in the step buffers are read only by
+      // H - 1 - it) rests; its rows in the step buffers are read only by
       // cells that are no longer exact either.
-      if (live && !(ly + kPreRows - 1 < 1 + it || ly >= kPreW - 1 - it)) {
+      if (live && !(ly + ROWS - 1 < 1 + it || ly >= H - 1 - it)) {
         float4 prev = *reinterpret_cast<const float4*>(S + row_up);
         float4 cur = *reinterpret_cast<const float4*>(S + ly * kPreP + lx);
         float pW = __shfl_up_sync(full, prev.w, 1), pE = __shfl_down_sync(full, prev.x, 1);
         float mW = __shfl_up_sync(full, cur.w, 1), mE = __shfl_down_sync(full, cur.x, 1);
 #pragma unroll
-        for (int r = 0; r < kPreRows; ++r) {
+        for (int r = 0; r < ROWS; ++r) {
           const float4 nxt =
-              *reinterpret_cast<const float4*>(S + min(ly + r + 1, kPreW - 1) * kPreP + lx);
+              *reinterpret_cast<const float4*>(S + min(ly + r + 1, H - 1) * kPreP + lx);
           const float sW = __shfl_up_sync(full, nxt.w, 1), sE = __shfl_down_sync(full, nxt.x, 1);
           const float4 f = *reinterpret_cast<const float4*>(F + (ly + r) * kPreP + lx);
           f2 kxa, kxb;
@@ -482,7 +491,7 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
       if (mine[1].b) pre_special_step(mine[1], S, F, Sn, k);
       // More cells than two per thread (none for frames at least 4 samples wide).
       if (rc.count > 2 * kPreThreads) {
-        const PreRingCells more = pre_ring_cells(w, h, gx0, gy0);
+        const PreRingCells<H> more = pre_ring_cells<H>(w, h, gx0, gy0);
         for (int i = threadIdx.x + 2 * kPreThreads; i < more.count; i += kPreThreads)
           pre_special_step(more.special(i, w, h, gx0, gy0), S, F, Sn, k);
       }
@@ -490,16 +499,16 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
     __syncthreads();
     // Twelve steps end in buffer 0; each thread reads back its own rows.
 #pragma unroll
-    for (int r = 0; r < kPreRows; ++r) X[r] = *reinterpret_cast<const float4*>(xb + (ly + r) * kPreP + lx);
+    for (int r = 0; r < ROWS; ++r) X[r] = *reinterpret_cast<const float4*>(xb + (ly + r) * kPreP + lx);
   }
-  // The inner 104 x 104: lanes 3 .. 28 of rows 12 .. 115.
+  // The inner rows and columns: lanes 3 .. 28 of rows 12 .. H - 13.
   const int oh = kPreHalo / 4;
   if (lane >= oh && lane < 32 - oh) {
     const bool vec_out =
         gx + 3 < w && (w % 4) == 0 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
 #pragma unroll
-    for (int r = 0; r < kPreRows; ++r) {
-      if (ly + r < kPreHalo || ly + r >= kPreW - kPreHalo || gy + r >= h) continue;
+    for (int r = 0; r < ROWS; ++r) {
+      if (ly + r < kPreHalo || ly + r >= H - kPreHalo || gy + r >= h) continue;
       float* row = out + (size_t)(gy + r) * w;
       if (vec_out) {
         *reinterpret_cast<float4*>(row + gx) = X[r];
@@ -515,34 +524,38 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
 
 // Both kinds of tile in one launch: the ring tiles at blockIdx.x < nedge,
 // then the interior tiles.
+template <int ROWS>
 __global__ void __launch_bounds__(kPreThreads, 1) k_precondition(const float* __restrict__ in,
                                                               float* __restrict__ out, int w,
                                                               int h, EncKernel k, PreTiles pt,
                                                               int nedge) {
   const int i = (int)blockIdx.x;
-  if (i < nedge) precondition_tile<true>(in, out, w, h, k, pt, i);
-  else precondition_tile<false>(in, out, w, h, k, pt, i - nedge);
+  if (i < nedge) precondition_tile<ROWS, true>(in, out, w, h, k, pt, i);
+  else precondition_tile<ROWS, false>(in, out, w, h, k, pt, i - nedge);
 }
 
-int launch_precondition(const float* in, float* out, int w, int h, cudaStream_t s) {
+template <int ROWS>
+static int precondition_rows(const float* in, float* out, int w, int h, cudaStream_t s) {
+  using Tile = PreTile<ROWS>;
   const float w1 = 0.115169525f, w2 = 0.061248592f;
   // gaborish.rs:31 GaborKernel::new, normalised without FMA.
   float unnorm = 1.0f + 4.0f * w1 + 4.0f * w2;
   float scale = 1.0f / unnorm;
   EncKernel k{scale, w1 * scale, w2 * scale, 1.0f / scale};
-  PreTiles pt{(w + kPreOut - 1) / kPreOut, (h + kPreOut - 1) / kPreOut, 0, 0, 0, 0};
+  PreTiles pt{(w + kPreOut - 1) / kPreOut, (h + Tile::kOut - 1) / Tile::kOut, 0, 0, 0, 0};
   // Columns and rows of cells with another rule: 0, [cb, w) and 0, [rb, h)
   // (the frame border, the columns past the groups of four, the rows of
   // the division tail).  A tile is in the rectangle when its haloed extent
-  // [t*104 - 12, t*104 + 116) lies inside [1, cb) and [1, rb).
+  // [t*104 - 12, t*104 + 116), down [t*kOut - 12, (t+1)*kOut + 12), lies inside
+  // [1, cb) and [1, rb).
   const long long n = (long long)w * h;
   const int groups = (w >= 3 && h >= 3) ? (w - 2) / 4 : 0;
   const int cb = std::max(std::min(w - 1, 4 * groups + 1), 1);
   const int row_end = n % 4 == 0 ? h - 1 : (int)std::min<long long>(h - 1, (n - n % 4) / w);
   const int rb = std::max(row_end, 1);
-  const int reach = kPreW - kPreHalo;  // 116
+  const int reach = kPreW - kPreHalo, reach_y = Tile::H - kPreHalo;
   const int fx1 = cb >= reach ? std::min((cb - reach) / kPreOut + 1, pt.tx) : 0;
-  const int fy1 = rb >= reach ? std::min((rb - reach) / kPreOut + 1, pt.ty) : 0;
+  const int fy1 = rb >= reach_y ? std::min((rb - reach_y) / Tile::kOut + 1, pt.ty) : 0;
   if (fx1 > 1 && fy1 > 1) {
     pt.fx0 = 1;
     pt.fx1 = fx1;
@@ -551,9 +564,20 @@ int launch_precondition(const float* in, float* out, int w, int h, cudaStream_t 
   }
   const int nfast = (pt.fx1 - pt.fx0) * (pt.fy1 - pt.fy0);
   const int nedge = pt.tx * pt.ty - nfast;
-  k_precondition<<<dim3(nedge + nfast, 1, 3), kPreThreads, kPreRingSmem, s>>>(in, out, w, h, k,
-                                                                             pt, nedge);
+  k_precondition<ROWS><<<dim3(nedge + nfast, 1, 3), kPreThreads, Tile::kSmem, s>>>(in, out, w, h, k,
+                                                                                  pt, nedge);
   return 1;
+}
+
+// Tiles of 64 rows compute 1.3 times as many cells per output as tiles of 128
+// and take two thirds of their time each: they are the better ones as long as
+// every one has an SM of its own (64x64: 24.5 us, 18.3 with them; 501x333: 30.7,
+// 20.2).
+int launch_precondition(const float* in, float* out, int w, int h, int num_sms, cudaStream_t s) {
+  const long long across = (w + kPreOut - 1) / kPreOut;
+  const long long down = (h + PreTile<4>::kOut - 1) / PreTile<4>::kOut;
+  return 3 * across * down <= num_sms ? precondition_rows<4>(in, out, w, h, s)
+                                      : precondition_rows<8>(in, out, w, h, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -940,8 +964,6 @@ __device__ __forceinline__ uint32_t factor_bits(int32_t f) {
   return (32u - __clz(af)) + 2u;
 }
 
-constexpr int kCflThreads = 256;
-
 // One CTA per 64x64 tile, from the coefficients to the quantized chroma:
 // (1) the HF regression sums (X and B against source Y) in double-float;
 // (2) the seeds; (3) the residual bit costs of the candidate windows and the
@@ -950,15 +972,19 @@ constexpr int kCflThreads = 256;
 // steps' latencies (the seeds' f64 chain above all) hide behind the SM's
 // other tiles.
 // Bound: issue slots (ten quantizer choices a cell).  Measured, with the LF
-// chain beside it: MEASURED_CFL
+// chain beside it: 193 us, now 109 (2048x2048), 452, now 275 (4096x3072).
+// Where every tile has an SM of its own the CTA's own chain is the time, and
+// 512 threads shorten it (64x64: 32.5 us, 28.5 with 512); beyond that three
+// CTAs of 256 to an SM hide one another's chains (2048x2048: 109 against 118).
 constexpr int kCflSide = 64;
+template <int THREADS>
 struct CflSmem {
   float p[4][kCflSide][kCflSide];        // X, Y, B coefficients, reconstructed luma
   float step[2][64], rstep[2][64];       // baseline quantizer, DCT8x8 cells
   float mul[64];                         // hf multiplier of each 8x8 block's varblock
   uint8_t lg[64];                        // log2 of its side in blocks
-  DF part[kCflThreads / 32][8];
-  uint32_t bits[kCflThreads / 32][8];
+  DF part[THREADS / 32][8];
+  uint32_t bits[THREADS / 32][8];
   int seed[2], factor[2];
 };
 
@@ -988,9 +1014,11 @@ __device__ __forceinline__ DF warp_sum8(DF* v, int lane, int* q) {
   return x;
 }
 
-__global__ void __launch_bounds__(kCflThreads, 3) k_cfl_tile(const __grid_constant__ EncArgs a) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
+    k_cfl_tile(const __grid_constant__ EncArgs a) {
   extern __shared__ __align__(16) unsigned char cfl_smem[];
-  CflSmem& sm = *reinterpret_cast<CflSmem*>(cfl_smem);
+  auto& sm = *reinterpret_cast<CflSmem<THREADS>*>(cfl_smem);
   const Geo& geo = a.geo;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int tx = blockIdx.x, ty = blockIdx.y, tile = ty * geo.tw + tx;
@@ -998,7 +1026,7 @@ __global__ void __launch_bounds__(kCflThreads, 3) k_cfl_tile(const __grid_consta
   const int px0 = tx * kCflSide, py0 = ty * kCflSide;
   const int pw = min(kCflSide, geo.W8 - px0), ph = min(kCflSide, geo.H8 - py0);
   const size_t origin = (size_t)py0 * geo.W8 + px0;
-  for (int i = t; i < 4 * kCflSide * kCflSide / 4; i += kCflThreads) {
+  for (int i = t; i < 4 * kCflSide * kCflSide / 4; i += THREADS) {
     const int x = 4 * (i % (kCflSide / 4)), y = i / (kCflSide / 4) % kCflSide,
               c = i / (kCflSide * kCflSide / 4);
     if (x >= pw || y >= ph) continue;
@@ -1023,7 +1051,7 @@ __global__ void __launch_bounds__(kCflThreads, 3) k_cfl_tile(const __grid_consta
     sm.mul[t] = mul;
   }
   // Baseline steps of the 64 folded cells and their reciprocals.
-  if (t >= 128) {
+  if (t >= 128 && t < 256) {
     const int ch = (t - 128) / 64, cell = t % 64;
     const float scale = a.base_mul * a.qs.qm[ch == 0 ? 0 : 2];
     const float st = scale * a.dq[(ch == 0 ? 0 : 2) * kDequantTableFloats + cell];
@@ -1033,9 +1061,9 @@ __global__ void __launch_bounds__(kCflThreads, 3) k_cfl_tile(const __grid_consta
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const bool on = *a.not_gray != 0u && a.cfl_enabled;
-  // Thread t covers column t % 64 of rows t / 64, t / 64 + 4, ...
+  // Thread t covers column t % 64 of rows t / 64, t / 64 + kStep, ...
   const int col = t % kCflSide, row0 = t / kCflSide;
-  constexpr int kStep = kCflThreads / kCflSide;
+  constexpr int kStep = THREADS / kCflSide;
   int seed[2] = {0, 0};
   if (on) {
     // (1) s_yy, s_yx, s_xx, s_yb, s_bb, sum|yx|, sum|yb|, count.
@@ -1065,7 +1093,7 @@ __global__ void __launch_bounds__(kCflThreads, 3) k_cfl_tile(const __grid_consta
     // then coefficient rows and columns).
     if (warp == 0) {
       DF sum = sm.part[0][lane & 7];
-      for (int i = 1; i < kCflThreads / 32; ++i) sum = df_add(sum, sm.part[i][lane & 7]);
+      for (int i = 1; i < THREADS / 32; ++i) sum = df_add(sum, sm.part[i][lane & 7]);
       const double value = df_value(sum);
       auto total = [&](int k) { return __shfl_sync(0xffffffffu, value, k); };
       const int ch = lane >> 3 & 1;
@@ -1178,7 +1206,7 @@ __global__ void __launch_bounds__(kCflThreads, 3) k_cfl_tile(const __grid_consta
       uint32_t tot[4];
       for (int c = 0; c < 4; ++c) {
         tot[c] = 0;
-        for (int i = 0; i < kCflThreads / 32; ++i) tot[c] += sm.bits[i][ch * 4 + c];
+        for (int i = 0; i < THREADS / 32; ++i) tot[c] += sm.bits[i][ch * 4 + c];
       }
       int result = 0;
       if (seed[ch] != 0) {
@@ -1484,9 +1512,13 @@ int launch_luma_from_image(const EncArgs& a, const uint32_t* const* lists, const
   return k;
 }
 
-int launch_cfl_chroma(const EncArgs& a, int* lf_seeds, void* lf_scratch, cudaStream_t s,
+int launch_cfl_chroma(const EncArgs& a, int* lf_seeds, void* lf_scratch, int num_sms, cudaStream_t s,
                       cudaStream_t lf_s) {
-  k_cfl_tile<<<dim3(a.geo.tw, a.geo.th), kCflThreads, sizeof(CflSmem), s>>>(a);
+  const dim3 tiles(a.geo.tw, a.geo.th);
+  if (a.geo.tw * a.geo.th <= num_sms)
+    k_cfl_tile<512><<<tiles, 512, sizeof(CflSmem<512>), s>>>(a);
+  else
+    k_cfl_tile<256><<<tiles, 256, sizeof(CflSmem<256>), s>>>(a);
   DF* sums = (DF*)lf_scratch;
   uint32_t* bits = (uint32_t*)((char*)lf_scratch + kLfCtas * 7 * sizeof(DF));
   // The LF chain reads only the LF planes: on its own stream.
@@ -1507,11 +1539,14 @@ void launch_mul_table(uint32_t global_scale, float* table, cudaStream_t s) {
 }
 
 cudaError_t configure_encode_kernels() {
-  const cudaError_t e = cudaFuncSetAttribute(
-      k_precondition, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPreRingSmem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_cfl_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(CflSmem));
+  auto allow = [](auto* kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  cudaError_t e;
+  if ((e = allow(k_precondition<4>, PreTile<4>::kSmem)) != cudaSuccess) return e;
+  if ((e = allow(k_precondition<8>, PreTile<8>::kSmem)) != cudaSuccess) return e;
+  if ((e = allow(k_cfl_tile<256>, sizeof(CflSmem<256>))) != cudaSuccess) return e;
+  return allow(k_cfl_tile<512>, sizeof(CflSmem<512>));
 }
 
 void upload_dct_constants(const float* iv4, const float* iv8, const float* iv16,

@@ -2,8 +2,8 @@
 // blur (k_blur.cu):
 //   S1, S2 k_pyramid       pyramid.rs:19 2x2 means, edge replicated, and
 //                          color.rs:66 positive XYB (reproducible cube root)
-//   S5 k_score_reduce      the partial rows' sums per scale and quantity
-//      k_score_finish      norms, 108 weights, remap (ssimulacra2.rs:509/:531)
+//   S5 k_score_finish      the partial rows' sums per scale and quantity, norms,
+//                          108 weights, remap (ssimulacra2.rs:509/:531)
 //
 // The per-strip partial sums that S5 folds come from k_blur_cols (f32 per
 // 32 rows of a column, double-float above that, fixed order).
@@ -130,17 +130,28 @@ struct FinishArgs {
 };
 
 constexpr int kReduceThreads = 256;
-constexpr int kFinishThreads = 128;
 
-// S5a: one CTA per (quantity, scale): thread t sums the quantity's tile rows
+// S5 — one CTA per (quantity, scale): thread t sums the quantity's tile rows
 // t, t + 256, ... of the scale in order in double-float, then the threads'
 // sums meet in a fixed tree (warps, then warps in order).  The total goes to
 // row 0 of the scale's partial rows, column k (only this CTA reads that
 // column).  Deterministic for a given frame size; every load of a scale is
 // in flight at once instead of behind one CTA's sequential chains.
-__global__ void __launch_bounds__(kReduceThreads) k_score_reduce(DF* __restrict__ partials,
-                                                                 FinishArgs fa) {
+//
+// The CTA that finishes last (`ticket`, zero between launches) goes on to
+// the norms, weights and remap of the 6 x 18 totals, a thread per term.
+// Bound by the latency of its double-precision chain (two square roots, the
+// weighted sum, one power): 3 + 13.6 us as two launches whose second took a
+// channel's six terms in one thread, 12.5 us in one.
+__global__ void __launch_bounds__(kReduceThreads) k_score_finish(DF* __restrict__ partials,
+                                                                 FinishArgs fa,
+                                                                 uint32_t* __restrict__ ticket,
+                                                                 double* __restrict__ out,
+                                                                 double* __restrict__ score,
+                                                                 double* __restrict__ raw) {
   __shared__ DF wsum[kReduceThreads / 32];
+  __shared__ double wterm[108];
+  __shared__ bool last;
   const int k = blockIdx.x, s = blockIdx.y, t = threadIdx.x;
   size_t base = 0;
   for (int i = 0; i < s; ++i) base += fa.ctas[i];
@@ -155,74 +166,57 @@ __global__ void __launch_bounds__(kReduceThreads) k_score_reduce(DF* __restrict_
     DF tot = wsum[0];
     for (int i = 1; i < kReduceThreads / 32; ++i) tot = df_add(tot, wsum[i]);
     partials[base * 18 + k] = tot;
-  }
-}
-
-// S5b: the norms, weights and remap from the 6 x 18 sums.
-__global__ void __launch_bounds__(kFinishThreads) k_score_finish(const DF* __restrict__ partials,
-                                                                 FinishArgs fa,
-                                                                 double* __restrict__ out) {
-  __shared__ double scale_sums[6][18];
-  __shared__ double terms[6][3][6];
-  __shared__ double wterm[108];
-  if (threadIdx.x < 18) {
-    size_t base = 0;
-    for (int s = 0; s < fa.nscales; ++s) {
-      scale_sums[s][threadIdx.x] = df_value(partials[base * 18 + threadIdx.x]);
-      base += fa.ctas[s];
-    }
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1;
   }
   __syncthreads();
-  // pool.rs:60 norms, one (scale, channel) per thread.
-  if (threadIdx.x < fa.nscales * 3) {
-    const int s = threadIdx.x / 3, c = threadIdx.x % 3;
-    const double inv = 1.0 / (double)(fa.pixels[s] > 0 ? fa.pixels[s] : 1);
-    const double* q = &scale_sums[s][c * 6];
-    terms[s][c][0] = inv * q[0];
-    terms[s][c][1] = inv * q[2];
-    terms[s][c][2] = inv * q[4];
-    terms[s][c][3] = sqrt(sqrt(inv * q[1]));
-    terms[s][c][4] = sqrt(sqrt(inv * q[3]));
-    terms[s][c][5] = sqrt(sqrt(inv * q[5]));
-  }
-  __syncthreads();
+  if (!last) return;
+  __threadfence();
   // ssimulacra2.rs:509 weighted error: weight i belongs to channel c, scale
-  // s, norm nn, map m with i = ((c * scales + s) * 2 + nn) * 3 + m.
-  if (threadIdx.x < 108) {
-    const int i = threadIdx.x;
-    const int m = i % 3, nn = (i / 3) % 2, cs = i / 6;
-    const int c = cs / fa.nscales, s = cs % fa.nscales;
-    wterm[i] = c < 3 ? c_weights[i] * fabs(terms[s][c][nn * 3 + m]) : 0.0;
+  // sc, norm nn, map m with i = ((c * scales + sc) * 2 + nn) * 3 + m; the norm
+  // itself is pool.rs:60's (mean, or fourth root of the mean).
+  if (t < 3 * fa.nscales * 6) {
+    const int m = t % 3, nn = (t / 3) % 2, c = t / 6 / fa.nscales, sc = t / 6 % fa.nscales;
+    size_t b = 0;
+    for (int i = 0; i < sc; ++i) b += fa.ctas[i];
+    const float2 p = __ldcg(reinterpret_cast<const float2*>(partials) + b * 18 + c * 6 + 2 * m + nn);
+    const double inv = 1.0 / (double)(fa.pixels[sc] > 0 ? fa.pixels[sc] : 1);
+    double term = inv * df_value(DF{p.x, p.y});
+    if (nn) term = sqrt(sqrt(term));
+    out[2 + (sc * 3 + c) * 6 + nn * 3 + m] = term;
+    wterm[t] = c_weights[t] * fabs(term);
   }
+  if (t == 0) *ticket = 0;
   __syncthreads();
-  if (threadIdx.x >= 32) return;
+  if (t >= 32) return;
   double part = 0.0;
-  for (int i = threadIdx.x; i < 3 * fa.nscales * 6; i += 32) part += wterm[i];
+  for (int i = t; i < 3 * fa.nscales * 6; i += 32) part += wterm[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if (threadIdx.x != 0) return;
+  if (t != 0) return;
   const double err = part;
   double sc = err * 0.9562382616834844;
   sc = 6.248496625763138e-5 * sc * sc * sc + 2.326765642916932 * sc -
        0.020884521182843837 * sc * sc;
-  out[0] = sc > 0.0 ? 100.0 - 10.0 * pow(sc, 0.6276336467831387) : 100.0;
+  const double value = sc > 0.0 ? 100.0 - 10.0 * pow(sc, 0.6276336467831387) : 100.0;
+  out[0] = value;
   out[1] = err;
-  for (int s = 0; s < fa.nscales; ++s)
-    for (int c = 0; c < 3; ++c)
-      for (int m = 0; m < 6; ++m) out[2 + (s * 3 + c) * 6 + m] = terms[s][c][m];
+  if (score) *score = value;
+  if (raw) *raw = err;
 }
 
 int launch_score_finish(DF* partials, const int* ctas_per_scale, int nscales,
-                        const int* pixels_per_scale, double* out, cudaStream_t s) {
+                        const int* pixels_per_scale, void* carry, double* out, double* score,
+                        double* raw, cudaStream_t s) {
   FinishArgs fa;
   fa.nscales = nscales;
   for (int i = 0; i < 6; ++i) {
     fa.ctas[i] = i < nscales ? ctas_per_scale[i] : 0;
     fa.pixels[i] = i < nscales ? pixels_per_scale[i] : 0;
   }
-  k_score_reduce<<<dim3(18, nscales), kReduceThreads, 0, s>>>(partials, fa);
-  k_score_finish<<<1, kFinishThreads, 0, s>>>(partials, fa, out);
-  return 2;
+  k_score_finish<<<dim3(18, nscales), kReduceThreads, 0, s>>>(partials, fa, blur_ticket(carry), out,
+                                                              score, raw);
+  return 1;
 }
 
 
