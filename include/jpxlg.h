@@ -209,8 +209,9 @@ int jpxlg_encode_stages(jpxlg_ctx* ctx, const jpxlg_layout* layout, const void* 
 /* Launch tunables (no reference counterpart), process-wide, for the
  * autotuner (jpxl_gb300/tune.py):
  *   JPXLG_TUNE_TC_CTAS_PER_SM  persistent CTAs per SM of the split-precision
- *                              tensor-core kernels, 1..4 (default 4: four
- *                              128-column TMEM allocations fill an SM).
+ *                              tensor-core kernels, in quarters of those
+ *                              that fit (three to eight by block size),
+ *                              1..4 (default 4).
  * jpxlg_tune_set returns the previous value (JPXLG_ERR_ARGUMENT for an
  * unknown knob or a value out of range); launches queued afterwards use the
  * new value (a batch captures it when it is created). */

@@ -25,15 +25,21 @@
 //
 // Tile: 128 rows = 128/N varblocks of one size N, one row of one varblock
 // per thread (thread t = (b, r): block b = t / N, row r = t % N).
-//   pass 1  A1 = the N x N transform matrix stacked 128/N times (constant),
-//           B1 = the tile's data rows (row t from thread t, K-major), so
-//           D1[(j, r)][(b, r')] = sum_k M[r][k] X_b[r'][k] for every block
-//           pair; thread (j, r) reads its own block's N columns (b = j).
-//   pass 2  A2 = those rows (written by the thread that read them, into the
-//           B1 buffer, which pass 1 has finished with), B2 = the transform
-//           matrix (constant); D2[(j, r)][k] is row r of block j's result.
+//   pass 1  A = the tile's data rows (row t from thread t, K-major), B = the
+//           N x N transform matrix (constant): D[(b, r')][u] = sum_k
+//           X_b[r'][k] M[u][k]; thread (b, r') reads its N columns, and the
+//           N lanes of a block exchange them (an N x N transpose by
+//           shuffles), so that thread (b, r) holds D[(b, r')][r] for all r'.
+//   pass 2  A = those rows (into the buffer that pass 1 has finished with),
+//           the same B; D[(j, r)][k] is row r of block j's result.
 // No transpose goes through shared memory: every operand row is written as
-// 16-byte K-major chunks by the thread that owns it.  Forward (M = D): X
+// 16-byte K-major chunks by the thread that owns it.  (Pass 1 with the matrix
+// stacked as A and the data as B needs no transpose, but computes every pair
+// of blocks for the sake of the diagonal: 16 times the products at N = 8, and
+// 128 TMEM columns a CTA, which held an SM to four CTAs of 128 threads.
+// Bound by the latency of the two passes' chain, which more CTAs cover: the
+// 8 x 8 blocks of 2048x2048 forward 64 us, now 42, render 71, now 47; of
+// 4096x3072 forward 188, now 121.)  Forward (M = D): X
 // rows are sample rows y, D2 rows are landscape coefficient rows v.  Inverse
 // (M = I): X rows are landscape coefficient rows v, D2 rows are sample rows
 // y.  Square shapes keep the coefficient matrix in the transposed
@@ -44,7 +50,7 @@
 // matrices of 8 rows x 16 bytes (128 contiguous bytes), the K-direction
 // core-matrix stride in the descriptor's leading-byte-offset field and the
 // 8-row-group stride (128 bytes) in its stride-byte-offset field.  The
-// kernels are persistent (grid-stride over tiles); each CTA allocates 128
+// kernels are persistent (grid-stride over tiles); each CTA allocates 32
 // TMEM columns once, loads the constant operands once, and frees the TMEM on
 // every exit path.  Every wait on the MMA's mbarrier is bounded; a wait that
 // runs out raises kDevTcTimeout in the error word, waits once more (bounded)
@@ -83,18 +89,17 @@ namespace tc {
 
 constexpr int kThreads = 128;
 constexpr uint32_t kWaitLimit = 1u << 24;
-constexpr int kTmemCols = 128;  // pass 1's accumulator, reused by pass 2
+constexpr int kTmemCols = 32;  // pass 1's accumulator, reused by pass 2
 
 template <int N, int TERMS>
 struct Tile {
   static constexpr int kVpt = 128 / N;           // varblocks per tile
   static constexpr int kKp = N < 16 ? 16 : N;    // contraction length padded to a bf16 MMA's 16
-  static constexpr int kNp = N < 16 ? 16 : N;    // pass-2 width (M = 128 needs a multiple of 16)
+  static constexpr int kNp = N < 16 ? 16 : N;    // width (M = 128 needs a multiple of 16)
   static constexpr int kOpTerm = 128 * kKp * 2;  // bytes of one term of a 128-row operand
   static constexpr int kB2Term = kNp * kKp * 2;
-  static constexpr int kA1 = 0;
-  static constexpr int kB1 = TERMS * kOpTerm;
-  static constexpr int kB2 = 2 * TERMS * kOpTerm;
+  static constexpr int kOp = 0;             // the 128-row operand of either pass
+  static constexpr int kB2 = TERMS * kOpTerm;  // the matrix
   static constexpr int kBytes = kB2 + TERMS * kB2Term;
   static constexpr uint32_t kLbo128 = (128 / 8) * 128;  // K-direction core-matrix stride
   static constexpr uint32_t kLboB2 = (kNp / 8) * 128;
@@ -247,19 +252,22 @@ __device__ __forceinline__ void store_row(uint8_t* region, int term_bytes, int r
 }
 
 // The products of one contraction, smallest terms first: A term pa[p] times
-// B term pb[p].  Issued by one thread.
+// B term pb[p]; of two products of the same order pass 1 takes the matrix's
+// smaller term first, pass 2 the data's.  Issued by one thread.
 template <int TERMS>
 __device__ __forceinline__ void issue_split(uint32_t tmem, uint32_t a_base, uint32_t a_term,
                                             uint32_t a_lbo, uint32_t b_base, uint32_t b_term,
-                                            uint32_t b_lbo, int ksteps, uint32_t idesc) {
+                                            uint32_t b_lbo, int ksteps, uint32_t idesc,
+                                            bool pass1) {
   const int np = TERMS == 2 ? 3 : 6;
-  const int pa[6] = {TERMS == 2 ? 1 : 2, TERMS == 2 ? 0 : 1, 0, 1, 0, 0};
-  const int pb[6] = {0, 1, TERMS == 2 ? 0 : 2, 0, 1, 0};
+  const int hi[6] = {TERMS == 2 ? 1 : 2, TERMS == 2 ? 0 : 1, 0, 1, 0, 0};
+  const int lo[6] = {0, 1, TERMS == 2 ? 0 : 2, 0, 1, 0};
   uint32_t acc = 0;
   for (int p = 0; p < np; ++p)
     for (int ks = 0; ks < ksteps; ++ks) {
-      const uint64_t da = sdesc(a_base + pa[p] * a_term + ks * 2 * a_lbo, a_lbo, 128);
-      const uint64_t db = sdesc(b_base + pb[p] * b_term + ks * 2 * b_lbo, b_lbo, 128);
+      const int pa = pass1 ? lo[p] : hi[p], pb = pass1 ? hi[p] : lo[p];
+      const uint64_t da = sdesc(a_base + pa * a_term + ks * 2 * a_lbo, a_lbo, 128);
+      const uint64_t db = sdesc(b_base + pb * b_term + ks * 2 * b_lbo, b_lbo, 128);
       mma_bf16(tmem, da, db, idesc, acc);
       acc = 1;
     }
@@ -283,21 +291,34 @@ struct State {
   bool ok;
 };
 
-// Loads the constant operands: A1 row t = M[t % N], B2 row r = M[r] (zero
-// rows past N); M = the inverse (dir 0) or forward (dir 1) matrix.
+// Loads the constant operand: B row r = M[r] (zero rows past N); M = the
+// inverse (dir 0) or forward (dir 1) matrix.
 template <int N, int TERMS>
 __device__ __forceinline__ void load_basis(uint8_t* smem, int dir) {
   using T = Tile<N, TERMS>;
   const float* m = g_tc_basis[dir][T::kSizeIdx];
   const int t = threadIdx.x;
-  float row[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) row[k] = m[(t % N) * N + k];
-  store_row<N, TERMS, T::kKp>(smem + T::kA1, T::kOpTerm, t, 128, row);
   if (t < T::kNp) {
+    float row[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) row[k] = t < N ? m[t * N + k] : 0.0f;
     store_row<N, TERMS, T::kKp>(smem + T::kB2, T::kB2Term, t, T::kNp, row);
+  }
+}
+
+// The N x N matrix whose row r lane r of a group of N holds, transposed.
+template <int N>
+__device__ __forceinline__ void transpose_lanes(float* v, int lane) {
+#pragma unroll
+  for (int o = N / 2; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if ((i & o) == 0) {
+        const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i | o], o);
+        if (up) v[i] = got;
+        else v[i | o] = got;
+      }
   }
 }
 
@@ -310,64 +331,35 @@ __device__ __forceinline__ void transform_rows(uint8_t* smem, uint64_t* mbar, St
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
   const uint32_t s0 = smem_u32(smem);
-  // pass 1
-  store_row<N, TERMS, T::kKp>(smem + T::kB1, T::kOpTerm, t, 128, row);
-  fence_async_smem();
-  before_sync();
-  __syncthreads();
-  after_sync();
-  if (t == 0) {
-    issue_split<TERMS>(st.tmem, s0 + T::kA1, T::kOpTerm, T::kLbo128, s0 + T::kB1, T::kOpTerm,
-                       T::kLbo128, T::kKp / 16, idesc_bf16(128, 128));
-    mma_commit(mbar);
-  }
-  bool ok = mbar_wait(mbar, st.phase);
-  st.phase ^= 1u;
-  if (__syncthreads_or(!ok)) {
-    st.ok = false;
-    return;
-  }
-  after_sync();
-  {
-    // This warp's 32 columns hold its lanes' blocks (warp w: blocks
-    // 32w/N .. 32(w+1)/N - 1); each lane keeps its own block's N.
-    uint32_t r[32];
-    tmem_ld32(st.tmem + lane_base + (uint32_t)(warp * 32), r);
-    const int off = lane - lane % N;
-#pragma unroll
-    for (int s = 0; s < 32 / N; ++s)
-      if (off == s * N) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) row[i] = __uint_as_float(r[s * N + i]);
-      }
-  }
-  // pass 2: A2 is written into B1's buffer, which pass 1 has consumed.
-  store_row<N, TERMS, T::kKp>(smem + T::kB1, T::kOpTerm, t, 128, row);
-  fence_async_smem();
-  before_sync();
-  __syncthreads();
-  after_sync();
-  if (t == 0) {
-    issue_split<TERMS>(st.tmem, s0 + T::kB1, T::kOpTerm, T::kLbo128, s0 + T::kB2, T::kB2Term,
-                       T::kLboB2, T::kKp / 16, idesc_bf16(128, T::kNp));
-    mma_commit(mbar);
-  }
-  ok = mbar_wait(mbar, st.phase);
-  st.phase ^= 1u;
-  if (__syncthreads_or(!ok)) {
-    st.ok = false;
-    return;
-  }
-  after_sync();
-  {
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    // pass 2's rows go where pass 1's were, which its products have consumed
+    store_row<N, TERMS, T::kKp>(smem + T::kOp, T::kOpTerm, t, 128, row);
+    fence_async_smem();
+    before_sync();
+    __syncthreads();
+    after_sync();
+    if (t == 0) {
+      issue_split<TERMS>(st.tmem, s0 + T::kOp, T::kOpTerm, T::kLbo128, s0 + T::kB2, T::kB2Term,
+                         T::kLboB2, T::kKp / 16, idesc_bf16(128, T::kNp), pass == 0);
+      mma_commit(mbar);
+    }
+    const bool ok = mbar_wait(mbar, st.phase);
+    st.phase ^= 1u;
+    if (__syncthreads_or(!ok)) {
+      st.ok = false;
+      return;
+    }
+    after_sync();
     uint32_t r[N];
     if constexpr (N == 32) tmem_ld32(st.tmem + lane_base, r);
     else if constexpr (N == 16) tmem_ld16(st.tmem + lane_base, r);
     else tmem_ld8(st.tmem + lane_base, r);
 #pragma unroll
     for (int i = 0; i < N; ++i) row[i] = __uint_as_float(r[i]);
+    before_sync();
+    if (pass == 0) transpose_lanes<N>(row, lane);
   }
-  before_sync();
 }
 
 __device__ __forceinline__ void begin(uint32_t* slot, uint64_t* mbar) {
@@ -398,13 +390,20 @@ namespace {
 
 using namespace tc;
 
+// Persistent CTAs that an SM holds by their registers: forward, render.
+template <int N>
+constexpr int kFit = N == 32 ? 4 : 8;
+template <int N>
+constexpr int kFitRender = N == 32 ? 3 : (N == 16 ? 5 : 8);
+
 // ---------------------------------------------------------------------------
 // T1 — forward DCT_2D of the square varblocks of size N into the
 // coefficient image (all three channels).
 // ---------------------------------------------------------------------------
 template <int N, int TERMS>
-__global__ void __launch_bounds__(kThreads) k_fdct_tc(EncArgs a, const uint32_t* __restrict__ list,
-                                                       int count, int ntiles) {
+__global__ void __launch_bounds__(kThreads, kFit<N>) k_fdct_tc(EncArgs a,
+                                                               const uint32_t* __restrict__ list,
+                                                               int count, int nitems) {
   using T = Tile<N, TERMS>;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t mbar;
@@ -420,14 +419,15 @@ __global__ void __launch_bounds__(kThreads) k_fdct_tc(EncArgs a, const uint32_t*
   const Geo& geo = a.geo;
   const size_t plane = (size_t)geo.w * geo.h;
   const size_t cplane = (size_t)geo.W8 * geo.H8;
-  // The varblock of this thread's row in a tile, and its sample row r of one
-  // channel, edges replicated (lib.rs:3008); zeros past the list's end.
+  // Items are (tile, channel) pairs, the channel fastest.  The varblock of
+  // this thread's row in an item, and its sample row r, edges replicated
+  // (lib.rs:3008); zeros past the list's end.
   struct Src {
     bool active;
     int x0, y0;
   };
-  auto locate = [&](int tile) {
-    const int vi = tile * T::kVpt + b;
+  auto locate = [&](int item) {
+    const int vi = item / 3 * T::kVpt + b;
     const bool active = vi < count;
     const uint32_t packed = active ? __ldg(&list[vi]) : 0u;
     return Src{active, (int)(packed & 0xffff) * 8, (int)(packed >> 16) * 8};
@@ -458,28 +458,26 @@ __global__ void __launch_bounds__(kThreads) k_fdct_tc(EncArgs a, const uint32_t*
       for (int x = 0; x < N; ++x) row[x] = 0.0f;
     }
   };
-  // (tile, channel) steps in order; the next step's row is loaded before
-  // this step's transform, so that its latency overlaps the MMAs, and the
-  // next tile's varblock a tile ahead, so that those loads never wait on it.
+  // The next item's row is loaded before this item's transform, so that its
+  // latency overlaps the MMAs, and the list entry an item ahead of that, so
+  // that those loads never wait on it.
   const Src none{false, 0, 0};
-  int tile = blockIdx.x, c = 0;
-  Src cur = tile < ntiles ? locate(tile) : none;
-  Src after = tile + (int)gridDim.x < ntiles ? locate(tile + gridDim.x) : none;
+  int item = blockIdx.x;
+  const int stride = gridDim.x;
+  Src cur = item < nitems ? locate(item) : none;
+  Src after = item + stride < nitems ? locate(item + stride) : none;
   float nxt[N];
-  if (tile < ntiles) load_row(cur, 0, nxt);
-  while (tile < ntiles && st.ok) {
+  if (item < nitems) load_row(cur, item % 3, nxt);
+  while (item < nitems && st.ok) {
     float row[N];
 #pragma unroll
     for (int x = 0; x < N; ++x) row[x] = nxt[x];
     const Src here = cur;
-    const int ch = c;
-    if (++c == 3) {
-      c = 0;
-      tile += gridDim.x;
-      cur = after;
-      if (tile + (int)gridDim.x < ntiles) after = locate(tile + gridDim.x);
-    }
-    if (tile < ntiles) load_row(cur, c, nxt);
+    const int ch = item % 3;
+    item += stride;
+    cur = after;
+    if (item + stride < nitems) after = locate(item + stride);
+    if (item < nitems) load_row(cur, item % 3, nxt);
     transform_rows<N, TERMS>(smem, &mbar, st, row);
     if (!st.ok) break;
     if (here.active) {
@@ -498,10 +496,10 @@ __global__ void __launch_bounds__(kThreads) k_fdct_tc(EncArgs a, const uint32_t*
 // IDCT_2D, scatter, sigma.
 // ---------------------------------------------------------------------------
 template <int N, int TERMS>
-__global__ void __launch_bounds__(kThreads) k_render_tc(RenderArgs a,
-                                                        const uint32_t* __restrict__ list,
-                                                        int count, int ntiles,
-                                                        const float* __restrict__ llf) {
+__global__ void __launch_bounds__(kThreads, kFitRender<N>) k_render_tc(RenderArgs a,
+                                                                 const uint32_t* __restrict__ list,
+                                                                 int count, int ntiles,
+                                                                 const float* __restrict__ llf) {
   using T = Tile<N, TERMS>;
   constexpr int n = N / 8;  // LLF corner side in blocks
   extern __shared__ __align__(128) uint8_t smem[];
@@ -661,9 +659,85 @@ __global__ void __launch_bounds__(kThreads) k_render_tc(RenderArgs a,
   end(st, &mbar, a.err);
 }
 
-// Persistent CTAs per SM of the tensor-core kernels: at most four, whose
-// 128-column TMEM allocations fill an SM's 512; a tunable (tc_ctas_per_sm).
+// T2 where the tiles are few: one CTA per (tile, channel), a chroma channel
+// dequantizing its luma again, instead of a tile's three channels in turn.
+template <int N, int TERMS>
+__global__ void __launch_bounds__(kThreads) k_render_tc_split(RenderArgs a,
+                                                              const uint32_t* __restrict__ list,
+                                                              int count,
+                                                              const float* __restrict__ llf) {
+  using T = Tile<N, TERMS>;
+  constexpr int n = N / 8;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ uint32_t tmem_slot;
+  const int t = threadIdx.x, b = t / N, r = t % N, c = blockIdx.y;
+  const Geo& geo = a.geo;
+  const size_t cplane = (size_t)geo.W8 * geo.H8;
+  const size_t plane = (size_t)geo.w * geo.h;
+  const int vi = blockIdx.x * T::kVpt + b;
+  const bool active = vi < count;
+  const uint32_t packed = __ldg(&list[min(vi, count - 1)]);
+  const int bx = packed & 0xffff, by = packed >> 16, x0 = bx * 8, y0 = by * 8;
+  const int* qp = a.qcoeff + (size_t)(y0 + r) * geo.W8 + x0;
+  int4 q[N / 4], ql[N / 4];
+#pragma unroll
+  for (int u = 0; u < N / 4; ++u) {
+    q[u] = __ldg(reinterpret_cast<const int4*>(qp + cplane * c) + u);
+    ql[u] = c == 1 ? q[u] : __ldg(reinterpret_cast<const int4*>(qp + cplane) + u);
+  }
+  const float mul = hf_multiplier(a.mul_table, a.qs.global_scale,
+                                  a.hf_mul[(size_t)by * geo.bw + bx]);  // reconstruct.rs:27
+  const int tile64 = (by / 8) * geo.tw + bx / 8;
+  const float kc = c == 0 ? 0.0f + (float)a.cfl_x[tile64] / 84.0f   // reconstruct.rs:96
+                          : 1.0f + (float)a.cfl_b[tile64] / 84.0f;
+  begin(&tmem_slot, &mbar);
+  load_basis<N, TERMS>(smem, 0);
+  before_sync();
+  __syncthreads();
+  after_sync();
+  State st{tmem_slot, 0u, true};
+  constexpr int slot = N == 8 ? 0 : (N == 16 ? 1 : 2);
+  const float* m = a.dq + dq_offset(slot) + r * N;
+  float row[N];
+#pragma unroll
+  for (int u4 = 0; u4 < N / 4; ++u4) {
+    const float4 mc = __ldg(reinterpret_cast<const float4*>(m + c * kDequantTableFloats) + u4);
+    const float4 ml = __ldg(reinterpret_cast<const float4*>(m + kDequantTableFloats) + u4);
+    const float mcs[4] = {mc.x, mc.y, mc.z, mc.w}, mls[4] = {ml.x, ml.y, ml.z, ml.w};
+    const int qs[4] = {q[u4].x, q[u4].y, q[u4].z, q[u4].w};
+    const int qls[4] = {ql[u4].x, ql[u4].y, ql[u4].z, ql[u4].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int u = u4 * 4 + i;
+      float d = bias_adjust(qs[i], c_tc_bias[c]) * (mul * a.qs.qm[c]) * mcs[i];
+      if (c != 1) d = d + kc * (bias_adjust(qls[i], c_tc_bias[1]) * (mul * a.qs.qm[1]) * mls[i]);
+      if (r < n && u < n) d = __ldg(&llf[(size_t)min(vi, count - 1) * 48 + c * 16 + r * n + u]);
+      row[u] = active ? d : 0.0f;
+    }
+  }
+  transform_rows<N, TERMS>(smem, &mbar, st, row);
+  if (st.ok && active && y0 + r < geo.h) {
+    float* o = a.planes + plane * c + (size_t)(y0 + r) * geo.w + x0;
+    if (x0 + N <= geo.w && (geo.w & 3) == 0) {
+#pragma unroll
+      for (int x = 0; x < N; x += 4)
+        *reinterpret_cast<float4*>(o + x) = make_float4(row[x], row[x + 1], row[x + 2], row[x + 3]);
+    } else {
+#pragma unroll
+      for (int x = 0; x < N; ++x)
+        if (x0 + x < geo.w) o[x] = row[x];
+    }
+  }
+  end(st, &mbar, a.err);
+}
+
+// Share of the CTAs that fit that the persistent grids take, in quarters: a
+// tunable (tc_ctas_per_sm), 1 to 4.
 std::atomic<int> g_tc_ctas_per_sm{4};
+int tc_grid(int num_sms, int fit) {
+  return num_sms * std::max(1, fit * g_tc_ctas_per_sm.load() / 4);
+}
 
 template <typename K>
 cudaError_t set_smem(K kernel, int bytes) {
@@ -673,9 +747,9 @@ cudaError_t set_smem(K kernel, int bytes) {
 template <int N, int TERMS>
 int launch_fdct_one(const EncArgs& a, const uint32_t* list, int count, int num_sms,
                     cudaStream_t s) {
-  const int ntiles = (count + Tile<N, TERMS>::kVpt - 1) / Tile<N, TERMS>::kVpt;
-  const int grid = std::min(ntiles, num_sms * g_tc_ctas_per_sm.load());
-  k_fdct_tc<N, TERMS><<<grid, kThreads, Tile<N, TERMS>::kBytes, s>>>(a, list, count, ntiles);
+  const int nitems = 3 * ((count + Tile<N, TERMS>::kVpt - 1) / Tile<N, TERMS>::kVpt);
+  const int grid = std::min(nitems, tc_grid(num_sms, kFit<N>));
+  k_fdct_tc<N, TERMS><<<grid, kThreads, Tile<N, TERMS>::kBytes, s>>>(a, list, count, nitems);
   return 1;
 }
 
@@ -683,7 +757,14 @@ template <int N, int TERMS>
 int launch_render_one(const RenderArgs& a, const uint32_t* list, int count, const float* llf,
                       int num_sms, cudaStream_t s) {
   const int ntiles = (count + Tile<N, TERMS>::kVpt - 1) / Tile<N, TERMS>::kVpt;
-  const int grid = std::min(ntiles, num_sms * g_tc_ctas_per_sm.load());
+  if (3 * ntiles <= num_sms) {
+    // Each (tile, channel) on an SM of its own (10 tiles of 32 x 32: 34 us in
+    // turn, 17 so; 39 of 16 x 16: 18.5, 10.3).
+    k_render_tc_split<N, TERMS><<<dim3(ntiles, 3), kThreads, Tile<N, TERMS>::kBytes, s>>>(
+        a, list, count, llf);
+    return 1;
+  }
+  const int grid = std::min(ntiles, tc_grid(num_sms, kFitRender<N>));
   k_render_tc<N, TERMS><<<grid, kThreads, Tile<N, TERMS>::kBytes, s>>>(a, list, count, ntiles,
                                                                          llf);
   return 1;
@@ -701,7 +782,8 @@ cudaError_t configure_tc_kernels() {
   cudaError_t e = cudaSuccess;
 #define JPXLG_TC_ATTR(N, T)                                                          \
   if (e == cudaSuccess) e = set_smem(k_fdct_tc<N, T>, Tile<N, T>::kBytes);          \
-  if (e == cudaSuccess) e = set_smem(k_render_tc<N, T>, Tile<N, T>::kBytes);
+  if (e == cudaSuccess) e = set_smem(k_render_tc<N, T>, Tile<N, T>::kBytes);        \
+  if (e == cudaSuccess) e = set_smem(k_render_tc_split<N, T>, Tile<N, T>::kBytes);
   JPXLG_TC_ATTR(8, 2)
   JPXLG_TC_ATTR(16, 2)
   JPXLG_TC_ATTR(32, 2)

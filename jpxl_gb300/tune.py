@@ -4,7 +4,7 @@ A batch of probes (BatchProbe, one CUDA graph) has two run-time knobs that
 change its speed but not its results: how many lanes (internal contexts,
 each with its own stream and workspace) the probes are spread over, and how
 many persistent CTAs per SM the split-precision tensor-core kernels take
-(JPXLG_TUNE_TC_CTAS_PER_SM).  `tune_batch` times every combination on the
+(JPXLG_TUNE_TC_CTAS_PER_SM, in quarters of those that fit).  `tune_batch` times every combination on the
 caller's own items (each a fresh graph, warmed up, then timed over several
 launches with the device synchronised around them), keeps the fastest and
 caches it in a JSON file under a key made of the device, the precision and
