@@ -967,20 +967,26 @@ __device__ __forceinline__ uint32_t factor_bits(int32_t f) {
 // One CTA per 64x64 tile, from the coefficients to the quantized chroma:
 // (1) the HF regression sums (X and B against source Y) in double-float;
 // (2) the seeds; (3) the residual bit costs of the candidate windows and the
-// choice; (4) K5, the X and B cells against the chosen factors.  The tile's
-// four planes arrive once, by cp.async, and stay in shared memory; the
+// choice; (4) K5, the X and B cells against the chosen factors.  X, Y and B
+// arrive once, by cp.async, and stay in shared memory; the reconstructed luma
+// of (3) and (4) takes Y's place behind (1) and arrives while (2) runs.  The
 // steps' latencies (the seeds' f64 chain above all) hide behind the SM's
 // other tiles.
-// Bound: issue slots (ten quantizer choices a cell).  Measured, with the LF
-// chain beside it: 193 us, now 109 (2048x2048), 452, now 275 (4096x3072).
+// Bound: issue slots and, with 32 warps to an SM, the steps' latencies.  Three
+// planes instead of four let an SM hold four tiles; a cell whose candidates
+// all fall under the zero threshold (most of a photograph's chroma) skips its
+// ten quantizer choices.  Measured, with the LF chain beside it: 4096x3072
+// 452 us, then 280 (one kernel), 255 (skips), 226 (four tiles); 1920x1080 66,
+// then 57, 51.
 // Where every tile has an SM of its own the CTA's own chain is the time, and
-// 512 threads shorten it (64x64: 32.5 us, 28.5 with 512); beyond that three
-// CTAs of 256 to an SM hide one another's chains (2048x2048: 109 against 118).
+// 512 threads shorten it (64x64: 32.5 us, 28.5 with 512); beyond that CTAs of
+// 256 hide one another's chains (2048x2048 at three to an SM: 109 against 118).
 constexpr int kCflSide = 64;
 template <int THREADS>
 struct CflSmem {
-  float p[4][kCflSide][kCflSide];        // X, Y, B coefficients, reconstructed luma
+  float p[3][kCflSide][kCflSide];        // X, Y, B coefficients; Y, then reconstructed luma
   float step[2][64], rstep[2][64];       // baseline quantizer, DCT8x8 cells
+  float half[2][64];                     // its zero threshold, -1 for a step out of range
   float mul[64];                         // hf multiplier of each 8x8 block's varblock
   uint8_t lg[64];                        // log2 of its side in blocks
   DF part[THREADS / 32][8];
@@ -1015,7 +1021,7 @@ __device__ __forceinline__ DF warp_sum8(DF* v, int lane, int* q) {
 }
 
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 4 : 1)
     k_cfl_tile(const __grid_constant__ EncArgs a) {
   extern __shared__ __align__(16) unsigned char cfl_smem[];
   auto& sm = *reinterpret_cast<CflSmem<THREADS>*>(cfl_smem);
@@ -1026,14 +1032,16 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
   const int px0 = tx * kCflSide, py0 = ty * kCflSide;
   const int pw = min(kCflSide, geo.W8 - px0), ph = min(kCflSide, geo.H8 - py0);
   const size_t origin = (size_t)py0 * geo.W8 + px0;
-  for (int i = t; i < 4 * kCflSide * kCflSide / 4; i += THREADS) {
-    const int x = 4 * (i % (kCflSide / 4)), y = i / (kCflSide / 4) % kCflSide,
-              c = i / (kCflSide * kCflSide / 4);
-    if (x >= pw || y >= ph) continue;
-    const float* src = (c < 3 ? a.coeff + cplane * c : a.dyhf) + origin + (size_t)y * geo.W8 + x;
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.p[c][y][x]);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-  }
+  auto fetch = [&](const float* plane, float(&to)[kCflSide][kCflSide]) {
+    for (int i = t; i < kCflSide * kCflSide / 4; i += THREADS) {
+      const int x = 4 * (i % (kCflSide / 4)), y = i / (kCflSide / 4);
+      if (x >= pw || y >= ph) continue;
+      const float* src = plane + origin + (size_t)y * geo.W8 + x;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&to[y][x]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    }
+  };
+  for (int c = 0; c < 3; ++c) fetch(a.coeff + cplane * c, sm.p[c]);
   // Each block's varblock (square, naturally aligned: its origin is the
   // block position with the low bits cleared).
   if (t < 64) {
@@ -1057,6 +1065,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
     const float st = scale * a.dq[(ch == 0 ? 0 : 2) * kDequantTableFloats + cell];
     sm.step[ch][cell] = st;
     sm.rstep[ch][cell] = 1.0f / st;
+    sm.half[ch][cell] = st > 0.0f && st < __int_as_float(0x7f800000)
+                            ? 0.5f * c_quant_bias[ch == 0 ? 0 : 2] * st
+                            : -1.0f;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
@@ -1087,6 +1098,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
     const DF w = warp_sum8(v, lane, &q);
     if ((lane & 3) == 0) sm.part[warp][q] = w;
     __syncthreads();
+    fetch(a.dyhf, sm.p[1]);
     // (2) Eight lanes for X's seed, eight for B's; a seed the bound cannot
     // settle is recomputed from the tile's coefficients in the reference's
     // order (varblocks in raster order of their origins within the tile,
@@ -1118,7 +1130,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
             const int nb = 1 << sm.lg[by * 8 + bx], side = nb * 8;
             for (int row = 0; row < side; ++row)
               for (int cc = (row < nb ? nb : 0); cc < side; ++cc) {
-                const double y = (double)sm.p[1][by * 8 + row][bx * 8 + cc];
+                const double y = (double)a.coeff[cplane + origin + (size_t)(by * 8 + row) * geo.W8 +
+                                                 bx * 8 + cc];
                 const double c = (double)sm.p[ch ? 2 : 0][by * 8 + row][bx * 8 + cc];
                 e.s_yy += y * y;
                 e.s_yc += y * c;
@@ -1131,9 +1144,14 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
       }
       if ((lane & 7) == 0 && lane < 16) sm.seed[ch] = sd;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     seed[0] = sm.seed[0];
     seed[1] = sm.seed[1];
+  } else {
+    fetch(a.dyhf, sm.p[1]);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
   }
   // (3) Residual bits of every candidate through the DCT8x8 baseline quantizer
   // (cells folded onto the 8x8 grid, lib.rs:3585), then the choice.
@@ -1162,21 +1180,32 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
       kx[i] = 0.0f + (float)cands[0][i < ncand[0] ? i : 0] / 84.0f;
       kb[i] = 1.0f + (float)cands[1][i < ncand[1] ? i : 0] / 84.0f;
     }
+    // lanes by frequency: a warp takes the same four of eight columns of each
+    // block, so that its cells fall under the threshold together
+    const int col = t % 8 * 8 + t / 8 % 8;
     if (col < pw)
 #pragma unroll 1
       for (int row = row0; row < ph; row += kStep) {
         const int l = sm.lg[(row >> 3) * 8 + (col >> 3)], mask = (8 << l) - 1;
         if ((col & mask) < (1 << l) && (row & mask) < (1 << l)) continue;  // LLF
         const int cell8 = ((row & mask) >> l) * 8 + ((col & mask) >> l);
-        const float x = sm.p[0][row][col], b = sm.p[2][row][col], dy = sm.p[3][row][col];
+        const float x = sm.p[0][row][col], b = sm.p[2][row][col], dy = sm.p[1][row][col];
         const float step_x = sm.step[0][cell8], rstep_x = sm.rstep[0][cell8];
         const float step_b = sm.step[1][cell8], rstep_b = sm.rstep[1][cell8];
-        auto cost = [&](int ch, float v, const float* k, float step, float rstep) {
+        auto cost = [&](int ch, float v, const float* k, float step, float rstep, float half) {
           bool ok = true;
           uint32_t n[4];
+          float target[4];
+          bool zeros = true;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const Choice q(ch, v - k[c] * dy, step, rstep);
+            target[c] = v - k[c] * dy;
+            zeros = zeros && fabsf(target[c]) <= half;
+          }
+          if (zeros) return;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const Choice q(ch, target[c], step, rstep);
             ok = ok && q.ok;
             n[c] = q.bits();
           }
@@ -1185,13 +1214,13 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
             for (int c = 0; c < 4; ++c) {
               float rc;
               n[c] = residual_bits(
-                  choose_general(v - k[c] * dy, step, c_quant_bias[ch], a.err, &rc));
+                  choose_general(target[c], step, c_quant_bias[ch], a.err, &rc));
             }
 #pragma unroll
           for (int c = 0; c < 4; ++c) bits[ch / 2][c] += n[c];
         };
-        if (seed[0] != 0) cost(0, x, kx, step_x, rstep_x);
-        if (seed[1] != 0) cost(2, b, kb, step_b, rstep_b);
+        if (seed[0] != 0) cost(0, x, kx, step_x, rstep_x, sm.half[0][cell8]);
+        if (seed[1] != 0) cost(2, b, kb, step_b, rstep_b, sm.half[1][cell8]);
       }
     // Integer sums, exact in any order.  A tile holds at most 4096 cells of at
     // most 22 bits, so 32 bits suffice.
@@ -1250,18 +1279,24 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
     const int l = sm.lg[blk], mask = (8 << l) - 1, k = row & mask, j = col & mask;
     int32_t qx = 0, qb = 0;
     if (!(k < (1 << l) && j < (1 << l))) {
-      const float mul = sm.mul[blk], dy = sm.p[3][row][col];
+      const float mul = sm.mul[blk], dy = sm.p[1][row][col];
       const float* m = a.dq + dq_offset(l) + (k << (3 + l)) + j;  // slots 0, 1, 2: the squares
       const float step_x = mul * qm_x * __ldg(m);
       const float step_b = mul * qm_b * __ldg(m + 2 * kDequantTableFloats);
       const float vx = sm.p[0][row][col] - k_x * dy, vb = sm.p[2][row][col] - k_b * dy;
-      const Choice cx(0, vx, step_x, approx_rcp(step_x)), cb(2, vb, step_b, approx_rcp(step_b));
-      qx = cx.q(vx);
-      qb = cb.q(vb);
-      if (!(cx.ok && cb.ok)) {
-        float rc;
-        qx = choose_general(vx, step_x, c_quant_bias[0], a.err, &rc);
-        qb = choose_general(vb, step_b, c_quant_bias[2], a.err, &rc);
+      const float inf = __int_as_float(0x7f800000);
+      const bool zeros = step_x > 0.0f && step_x < inf && step_b > 0.0f && step_b < inf &&
+                         fabsf(vx) <= 0.5f * c_quant_bias[0] * step_x &&
+                         fabsf(vb) <= 0.5f * c_quant_bias[2] * step_b;
+      if (!zeros) {
+        const Choice cx(0, vx, step_x, approx_rcp(step_x)), cb(2, vb, step_b, approx_rcp(step_b));
+        qx = cx.q(vx);
+        qb = cb.q(vb);
+        if (!(cx.ok && cb.ok)) {
+          float rc;
+          qx = choose_general(vx, step_x, c_quant_bias[0], a.err, &rc);
+          qb = choose_general(vb, step_b, c_quant_bias[2], a.err, &rc);
+        }
       }
     }
     const size_t ci = origin + (size_t)row * geo.W8 + col;
