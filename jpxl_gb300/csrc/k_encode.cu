@@ -137,7 +137,7 @@ void launch_srgb_to_xyb(const void* rgb, int bits, size_t n, const float* lut, f
 constexpr int kPreOut = 104;                   // outputs across
 constexpr int kPreHalo = 12;
 constexpr int kPreW = kPreOut + 2 * kPreHalo;  // 128: 32 lanes x 4 columns
-constexpr int kPreWarps = 16;                  // of ROWS = 8 or 4 rows
+constexpr int kPreWarps = 16;                  // of ROWS = 2, 3, 4 or 8 rows
 constexpr int kPreThreads = 32 * kPreWarps;
 static_assert(kPreW == 128 && kPreHalo >= 12, "tile of the inverse Gaborish");
 // Tile rows in shared memory are kPreP floats apart: 16-byte aligned for the
@@ -150,8 +150,8 @@ constexpr int kPreP = kPreW + 4;
 // inputs [2 parities][H][kPreP].
 template <int ROWS>
 struct PreTile {
-  static constexpr int H = ROWS * kPreWarps;         // 128 or 64 rows
-  static constexpr int kOut = H - 2 * kPreHalo;      // 104 or 40 of them outputs
+  static constexpr int H = ROWS * kPreWarps;         // up to 128 rows
+  static constexpr int kOut = H - 2 * kPreHalo;      // of them outputs
   static constexpr size_t kSmem = (size_t)3 * H * kPreP * sizeof(float);
 };
 
@@ -569,15 +569,21 @@ static int precondition_rows(const float* in, float* out, int w, int h, cudaStre
   return 1;
 }
 
-// Tiles of 64 rows compute 1.3 times as many cells per output as tiles of 128
-// and take two thirds of their time each: they are the better ones as long as
-// every one has an SM of its own (64x64: 24.5 us, 18.3 with them; 501x333: 30.7,
-// 20.2).
+// Rows per lane: the fewest with which every tile still has an SM of its own,
+// else eight.  A short tile computes more cells per output but ends sooner
+// (64x64: 24.5 us with eight rows, 18.3 with four, 14.2 with two; 501x333:
+// 30.7, 20.2 with four); beyond a tile to an SM the work is the time, and
+// choosing rows to fill the last round better gained nothing (1920x1080 with
+// seven: 81.8 us, 81.0 with eight).
 int launch_precondition(const float* in, float* out, int w, int h, int num_sms, cudaStream_t s) {
-  const long long across = (w + kPreOut - 1) / kPreOut;
-  const long long down = (h + PreTile<4>::kOut - 1) / PreTile<4>::kOut;
-  return 3 * across * down <= num_sms ? precondition_rows<4>(in, out, w, h, s)
-                                      : precondition_rows<8>(in, out, w, h, s);
+  auto fits = [&](int outs) {
+    const long long across = (w + kPreOut - 1) / kPreOut, down = (h + outs - 1) / outs;
+    return 3 * across * down <= num_sms;
+  };
+  if (fits(PreTile<2>::kOut)) return precondition_rows<2>(in, out, w, h, s);
+  if (fits(PreTile<3>::kOut)) return precondition_rows<3>(in, out, w, h, s);
+  if (fits(PreTile<4>::kOut)) return precondition_rows<4>(in, out, w, h, s);
+  return precondition_rows<8>(in, out, w, h, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1578,6 +1584,8 @@ cudaError_t configure_encode_kernels() {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
   cudaError_t e;
+  if ((e = allow(k_precondition<2>, PreTile<2>::kSmem)) != cudaSuccess) return e;
+  if ((e = allow(k_precondition<3>, PreTile<3>::kSmem)) != cudaSuccess) return e;
   if ((e = allow(k_precondition<4>, PreTile<4>::kSmem)) != cudaSuccess) return e;
   if ((e = allow(k_precondition<8>, PreTile<8>::kSmem)) != cudaSuccess) return e;
   if ((e = allow(k_cfl_tile<256>, sizeof(CflSmem<256>))) != cudaSuccess) return e;

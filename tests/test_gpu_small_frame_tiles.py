@@ -1,8 +1,9 @@
 """The encoder at the sizes where its tiling changes, bit for bit against the
-restatement: inverse Gaborish tiles of 64 rows (outputs 104 x 40) up to the
-largest frame that gives each an SM of its own and tiles of 128 beyond it,
-their edges and remainders, frames of one row or column; chroma-from-luma
-CTAs of 512 threads up to a tile per SM and of 256 beyond."""
+restatement: inverse Gaborish tiles of 32, 48 and 64 rows (8, 24 and 40 of
+outputs, 104 across) up to the largest frame that gives each an SM of its own
+and tiles of 128 beyond it, their edges and remainders, frames of one row or
+column; chroma-from-luma CTAs of 512 threads up to a tile per SM and of 256
+beyond."""
 import numpy as np
 import pytest
 
@@ -12,7 +13,8 @@ from jpxl_gb300 import synth
 pytestmark = pytest.mark.gpu
 
 SIZES = [(1, 90), (90, 1), (2, 41), (3, 200), (200, 3), (103, 39), (104, 40), (105, 41), (107, 80),
-         (116, 52), (128, 64), (129, 65), (211, 121), (520, 400), (521, 401), (832, 1000)]
+         (116, 52), (128, 64), (129, 65), (211, 121), (208, 200), (209, 201), (312, 384),
+         (313, 385), (520, 400), (521, 401), (832, 1000)]
 
 
 @pytest.mark.parametrize("w,h", SIZES)
