@@ -1626,14 +1626,17 @@ namespace {
 
 // A parsed VarDCT frame staged for the GPU render: its layout and
 // parameters, and in one host block (pinned for batches) the coefficient
-// image, the LF planes, the CfL tiles and (an LF frame) the LF XYB planes.
+// image, in the narrowest of 1, 2 and 4 bytes that holds every value, then
+// the LF planes, (an LF frame) the LF XYB planes and the CfL tiles, padded to
+// 16 bytes.  k_unstage lays it out on the device.
 struct DecodeStage {
   jpxlg_layout* L = nullptr;
   jpxlg_params p{};
-  size_t n = 0, n8 = 0, nb = 0, nt = 0, bytes = 0;
+  size_t n = 0, n8 = 0, nb = 0, nt = 0;
+  int q_bytes = 4;             // of a staged coefficient
+  size_t bytes = 0, rest = 0;  // of the block, and of what follows the coefficients
   void* host = nullptr;
   bool pinned = false;
-  int32_t* q = nullptr;
   int32_t* lfq = nullptr;
   int8_t* cflx = nullptr;
   int8_t* cflb = nullptr;
@@ -1706,20 +1709,27 @@ int decode_stage(jpxlg_ctx* ctx, const jpxlg_codestream* cs, int out_kind, bool 
   if (v.lf_from_frame)
     for (int c = 0; c < 3; ++c)
       if (v.lf_frame[c].size() != st.nb) return fail(ctx, JPXLG_ERR_STREAM, "LF frame size");
-  const size_t qb = 3 * st.n8 * sizeof(int32_t), lb = 3 * st.nb * sizeof(int32_t);
+  std::vector<int32_t> q(3 * st.n8);
+  if ((rc = jpxlg_codestream_coefficients(cs, q.data()))) return rc;
+  uint32_t span = 0;  // bits of the magnitudes, two's complement
+  for (int32_t x : q) span |= (uint32_t)(x ^ (x >> 31));
+  st.q_bytes = span < 0x80u ? 1 : (span < 0x8000u ? 2 : 4);
+  const size_t qb = 3 * st.n8 * st.q_bytes, lb = 3 * st.nb * sizeof(int32_t);
   const size_t fb = v.lf_from_frame ? 3 * st.nb * sizeof(float) : 0;
-  const size_t bytes = st.bytes = qb + lb + fb + 2 * st.nt;
+  st.rest = (lb + fb + 2 * st.nt + 15) & ~(size_t)15;
+  const size_t bytes = st.bytes = qb + st.rest;
   st.pinned = pinned;
   if (pinned) CK(cudaMallocHost(&st.host, bytes));
   else if (!(st.host = std::malloc(bytes)))
     return fail(ctx, JPXLG_ERR_CUDA, "host staging of %zu bytes", bytes);
   char* h = (char*)st.host;
-  st.q = (int32_t*)h;
   st.lfq = (int32_t*)(h + qb);
   st.lf_frame = fb ? (float*)(h + qb + lb) : nullptr;
   st.cflx = (int8_t*)(h + qb + lb + fb);
   st.cflb = st.cflx + st.nt;
-  if ((rc = jpxlg_codestream_coefficients(cs, st.q))) return rc;
+  if (st.q_bytes == 1) std::copy(q.begin(), q.end(), (int8_t*)h);
+  else if (st.q_bytes == 2) std::copy(q.begin(), q.end(), (int16_t*)h);
+  else std::copy(q.begin(), q.end(), (int32_t*)h);
   for (int c = 0; c < 3; ++c) {
     std::copy(v.lf[c].begin(), v.lf[c].end(), st.lfq + c * st.nb);
     if (st.lf_frame) std::copy(v.lf_frame[c].begin(), v.lf_frame[c].end(), st.lf_frame + c * st.nb);
@@ -1744,14 +1754,22 @@ int decode_stage(jpxlg_ctx* ctx, const jpxlg_codestream* cs, int out_kind, bool 
 // context's buffers have grown to the frame.
 int decode_enqueue(jpxlg_ctx* ctx, const DecodeStage& st, int out_kind, void* out_dev) {
   const Geo& g = st.L->geo;
-  CK(ctx->qcoeff.ensure(st.bytes));
+  const size_t wide = 3 * st.n8 * sizeof(int32_t);
+  CK(ctx->qcoeff.ensure(wide + st.rest));
   CK(ctx->lfs.ensure(3 * st.nb * sizeof(float)));
-  // The staged planes are one block on the host and on the device: one copy
-  // (four to six of a few microseconds each on the copy engine bound a batch
-  // of small streams).
-  CK(cudaMemcpyAsync(ctx->qcoeff.p, st.host, st.bytes, cudaMemcpyHostToDevice, ctx->stream));
+  // The block goes up narrow: pinned, the kernel that widens it reads it where
+  // it is (many streams' copies of a few microseconds each bound a batch on
+  // the copy engine); else by a copy into planes that the render uses later.
+  const void* src = st.host;
+  if (!st.pinned) {
+    CK(ctx->aux.ensure(std::max(3 * st.n * sizeof(float), st.bytes)));
+    CK(cudaMemcpyAsync(ctx->aux.p, st.host, st.bytes, cudaMemcpyHostToDevice, ctx->stream));
+    src = ctx->aux.p;
+  }
+  launch_unstage(src, st.q_bytes, 3 * st.n8, st.rest, ctx->qcoeff.p, ctx->num_sms, ctx->stream);
+  const char* rest = (const char*)st.host + 3 * st.n8 * st.q_bytes;
   auto staged = [&](const void* h) {
-    return ctx->qcoeff.as<char>() + ((const char*)h - (const char*)st.host);
+    return ctx->qcoeff.as<char>() + wide + ((const char*)h - rest);
   };
   const int32_t* lfq = (const int32_t*)staged(st.lfq);
   const float* lf = ctx->lfs.as<float>();
@@ -1762,8 +1780,8 @@ int decode_enqueue(jpxlg_ctx* ctx, const DecodeStage& st, int out_kind, void* ou
     launch_lf_prepare(lfq, g.bw, g.bh, st.m, st.div, st.kx, st.kb, st.smooth,
                       ctx->lfs.as<float>(), st.p.global_scale, ctx->d_mul, ctx->num_sms,
                       ctx->stream);
-    if ((rc = after_launch(ctx, 1))) return rc;
   }
+  if ((rc = after_launch(ctx, st.lf_frame ? 1 : 2))) return rc;
   return render_device(ctx, st.L, ctx->qcoeff.as<int32_t>(), lfq, (const int8_t*)staged(st.cflx),
                        (const int8_t*)staged(st.cflb), st.fx, st.fb, nullptr, &st.p, out_kind, 8,
                        out_dev, nullptr, lf, !st.lf_frame);

@@ -60,6 +60,11 @@ struct RenderArgs {
 void launch_lf_prepare(const int32_t* lfq, int bw, int bh, const float m[3], float div, float kx,
                        float kb, bool smooth, float* out, uint32_t global_scale, float* mul_table,
                        int num_sms, cudaStream_t s);
+// A staged stream's block (device or pinned host memory, 16-byte aligned): n
+// coefficients of q_bytes each (n a multiple of 64) widened to int32 at dst,
+// then `rest` bytes (a multiple of 16) as they are behind them.
+void launch_unstage(const void* src, int q_bytes, size_t n, size_t rest, void* dst, int num_sms,
+                    cudaStream_t s);
 // One finished stream of a batch: its lane's device error word to `flag`, in
 // pinned host memory, after everything its stream has written before.
 void launch_publish(const uint32_t* err, uint32_t* flag, cudaStream_t s);

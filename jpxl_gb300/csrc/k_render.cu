@@ -1451,6 +1451,45 @@ void launch_lf_prepare(const int32_t* lfq, int bw, int bh, const float m[3], flo
                                       global_scale, mul_table);
 }
 
+// A thread moves 16 bytes of the block at a time, several loads in flight:
+// bound by the host link where the block is pinned host memory (about 2 us of
+// latency, 200 GB/s).  48 small streams: 659 us with each block copied whole,
+// 625 copied narrow and widened, 599 read in place.
+template <typename Q>
+__global__ void __launch_bounds__(256) k_unstage(const uint4* __restrict__ src, size_t nq,
+                                                 size_t nrest, uint4* __restrict__ dst) {
+  constexpr int kPer = 16 / sizeof(Q);  // coefficients of a load
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq + nrest; i += stride) {
+    const uint4 v = src[i];
+    if (i >= nq) {
+      dst[nq * (kPer / 4) + (i - nq)] = v;
+      continue;
+    }
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    int32_t q[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      q[k] = (int32_t)(Q)(w[k * sizeof(Q) / 4] >> (8 * (k * sizeof(Q) % 4)));
+#pragma unroll
+    for (int k = 0; k < kPer / 4; ++k)
+      dst[i * (kPer / 4) + k] = make_uint4(q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]);
+  }
+}
+
+void launch_unstage(const void* src, int q_bytes, size_t n, size_t rest, void* dst, int num_sms,
+                    cudaStream_t s) {
+  const size_t nq = n * q_bytes / 16, nr = rest / 16;
+  const int blocks = (int)std::max<size_t>(1, std::min<size_t>((nq + nr + 255) / 256, num_sms * 4));
+  auto go = [&](auto q) {
+    k_unstage<decltype(q)><<<blocks, 256, 0, s>>>((const uint4*)src, nq, nr, (uint4*)dst);
+  };
+  if (q_bytes == 1) go(int8_t{});
+  else if (q_bytes == 2) go(int16_t{});
+  else go(int32_t{});
+}
+
 // The stream's earlier work is visible to this thread, and the release makes
 // it visible to the host that reads the flag.
 __global__ void k_publish(const uint32_t* __restrict__ err, uint32_t* flag) {
