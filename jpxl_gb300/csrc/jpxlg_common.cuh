@@ -363,10 +363,6 @@ __device__ __forceinline__ void dct_iii(float* v) {
 // dct.rs:731/749: normative scaling after the butterfly.  The factors are
 // 1/sqrtf(N) and sqrtf(N) in f32, as the reference computes them.
 template <int N>
-__device__ __forceinline__ float fwd_factor() {
-  return 1.0f / sqrtf((float)N);
-}
-template <int N>
 __device__ __forceinline__ void dct_1d(float* v) {
   dct_ii<N>(v);
   const float f = 1.0f / __fsqrt_rn((float)N);
@@ -538,44 +534,5 @@ __device__ __forceinline__ void idct_pair(int k, Get get, float* lo, float* hi) 
   *lo = (even + odd) * f;
   *hi = (even - odd) * f;
 }
-
-// ---- LF rectangles (dct.rs:956 on the LLF corner of a varblock) -------------
-template <int N>
-__device__ __forceinline__ void dct_small(float* v) {
-  if (N == 2) dct_1d<2>(v);
-  else if (N == 4) dct_1d<4>(v);
-  else if (N == 8) dct_1d<8>(v);
-}
-
-// dct.rs:956 DCT_2D of an LF rectangle cy x cx (cy <= cx, both <= 8) in place.
-__device__ __forceinline__ void dct2d_small(float* m, int rows, int cols) {
-  float col[8], s[64];
-  // column pass (length rows) on rows x cols
-  for (int c = 0; c < cols; ++c) {
-    for (int r = 0; r < rows; ++r) col[r] = m[r * cols + c];
-    if (rows == 2) dct_small<2>(col);
-    else if (rows == 4) dct_small<4>(col);
-    else if (rows == 8) dct_small<8>(col);
-    for (int r = 0; r < rows; ++r) m[r * cols + c] = col[r];
-  }
-  // transpose to cols x rows, column pass (length cols)
-  for (int r = 0; r < rows; ++r)
-    for (int c = 0; c < cols; ++c) s[c * rows + r] = m[r * cols + c];
-  for (int r = 0; r < rows; ++r) {
-    for (int c = 0; c < cols; ++c) col[c] = s[c * rows + r];
-    if (cols == 2) dct_small<2>(col);
-    else if (cols == 4) dct_small<4>(col);
-    else if (cols == 8) dct_small<8>(col);
-    for (int c = 0; c < cols; ++c) s[c * rows + r] = col[c];
-  }
-  // cols x rows result; landscape => transpose back when cols > rows
-  if (cols <= rows) {
-    for (int i = 0; i < rows * cols; ++i) m[i] = s[i];
-  } else {
-    for (int c = 0; c < cols; ++c)
-      for (int r = 0; r < rows; ++r) m[r * cols + c] = s[c * rows + r];
-  }
-}
-
 
 }  // namespace jpxlg

@@ -757,70 +757,70 @@ __global__ void __launch_bounds__(512) k_render_64(RenderArgs a, const uint32_t*
 }
 
 // The LLF rectangles and EPF sigma of the square varblocks of size N that
-// the split-precision render (k_tc.cu) transforms: varblock.rs:817
-// llf_from_lf (LF dequantized by reconstruct.rs:84 with the LF CfL of
-// plan-render lib.rs:1314, DCT_2D, times scale_f) and restoration.rs:338
-// vardct_sigma, exactly as k_render_rect forms them.  One thread per
-// (varblock, channel); llf receives 16 floats per channel per varblock.
+// the split-precision render (k_tc.cu) transforms, exactly as k_render_rect
+// forms them: one thread per LF sample, then one per column and per row of a
+// rectangle (one thread per rectangle took 8.5 us for ten tiles of 32 x 32,
+// 5.2 so: the loads' latency once instead of sixteen blocks' sigma in
+// turn).  llf receives 16 floats per channel per varblock.
+constexpr int kLlfThreads = 128;
 template <int N>
-__global__ void __launch_bounds__(128) k_llf_sigma(RenderArgs a, const uint32_t* __restrict__ list,
-                                                   int count, float* __restrict__ llf) {
-  constexpr int n = N / 8;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= count * 3) return;
-  const int vi = idx / 3, c = idx % 3;
-  const uint32_t packed = list[vi];
-  const int bx = packed & 0xffff, by = packed >> 16;
+__global__ void __launch_bounds__(kLlfThreads) k_llf_sigma(RenderArgs a,
+                                                           const uint32_t* __restrict__ list,
+                                                           int count, float* __restrict__ llf) {
+  using S = RectShape<N, N>;
+  constexpr int n = N / 8, kPer = 3 * n * n, kBlocks = kLlfThreads / kPer;
+  __shared__ float rect[kBlocks][3][n * n];
   const Geo& geo = a.geo;
   const size_t bplane = (size_t)geo.bw * geo.bh;
-  float k_x_lf = a.k_x_lf, k_b_lf = a.k_b_lf;
-  if (a.lf_factors_dev) {
-    k_x_lf = 0.0f + (float)a.lf_factors_dev[0] / 84.0f;
-    k_b_lf = 1.0f + (float)a.lf_factors_dev[1] / 84.0f;
-  }
-  if (c == 0) {
-    const float mul = hf_multiplier(a.mul_table, a.qs.global_scale,
-                                    a.hf_mul[(size_t)by * geo.bw + bx]);
-    for (int i = 0; i < n * n; ++i) {
-      const size_t bi = (size_t)(by + i / n) * geo.bw + bx + i % n;
-      int sh = a.sharpness[bi];
-      sh = sh > 7 ? 7 : sh;
-      const float lut = sh == 7 ? 1.0f : (float)sh / 7.0f;
-      a.sigma[bi] = mul * 0.46f * lut;
+  const int t = threadIdx.x, v0 = blockIdx.x * kBlocks;
+  const float* sf = &c_scale_f[S::SX * 8];
+  {
+    const int g = t / kPer, c = t / (n * n) % 3, i = t % (n * n);
+    if (g < kBlocks && v0 + g < count) {
+      const uint32_t pk = list[v0 + g];
+      const size_t b0 = (size_t)(pk >> 16) * geo.bw + (pk & 0xffff);
+      const size_t bi = b0 + (size_t)(i / n) * geo.bw + i % n;
+      rect[g][c][i] = lf_sample(a, bplane, c, bi);
+      if (c == 0)
+        a.sigma[bi] = block_sigma(a, hf_multiplier(a.mul_table, a.qs.global_scale, a.hf_mul[b0]), bi);
     }
   }
-  float rect[64];
-  for (int dy = 0; dy < n; ++dy)
-    for (int dx = 0; dx < n; ++dx) {
-      const size_t bi = (size_t)(by + dy) * geo.bw + bx + dx;
-      float v;
-      if (a.lf_float) {
-        v = a.lf_float[bplane * c + bi];
-      } else {
-        const float dY = a.qs.m_dc[1] * (float)a.lfq[bplane + bi] / 1.0f;
-        if (c == 1) {
-          v = dY;
-        } else {
-          const float d = a.qs.m_dc[c] * (float)a.lfq[bplane * c + bi] / 1.0f;
-          v = d + (c == 0 ? k_x_lf : k_b_lf) * dY;
-        }
-      }
-      rect[dy * n + dx] = v;
+  __syncthreads();
+  const int g = t / (3 * n), c = t / n % 3, k = t % n;
+  const bool on = g < kBlocks && v0 + g < count;
+  float v[n];
+  if constexpr (n > 1) {
+    if (on) {
+#pragma unroll
+      for (int r = 0; r < n; ++r) v[r] = rect[g][c][r * n + k];
+      dct_1d<n>(v);
+#pragma unroll
+      for (int r = 0; r < n; ++r) rect[g][c][r * n + k] = v[r];
     }
-  if (n > 1) dct2d_small(rect, n, n);
-  constexpr int sfi = n == 1 ? 0 : (n == 2 ? 1 : (n == 4 ? 2 : 3));
-  const float* sf = &c_scale_f[sfi * 8];
-  float* o = llf + (size_t)vi * 48 + c * 16;
-  for (int y = 0; y < n; ++y)
-    for (int x = 0; x < n; ++x) o[y * n + x] = rect[y * n + x] * sf[y] * sf[x];
+    __syncthreads();
+  }
+  if (!on) return;
+#pragma unroll
+  for (int r = 0; r < n; ++r) v[r] = rect[g][c][k * n + r];
+  if constexpr (n > 1) dct_1d<n>(v);
+  // the second pass leaves the matrix transposed (dct.rs:956)
+  float* o = llf + (size_t)(v0 + g) * 48 + c * 16;
+#pragma unroll
+  for (int r = 0; r < n; ++r) o[r * n + k] = v[r] * sf[r] * sf[k];
 }
 
 int launch_llf_sigma(const RenderArgs& a, const uint32_t* const* lists, const int* counts,
                      float* const* llf, const cudaStream_t* s) {
   int k = 0;
-  if (counts[0]) { k_llf_sigma<8><<<(3 * counts[0] + 127) / 128, 128, 0, s[0]>>>(a, lists[0], counts[0], llf[0]); ++k; }
-  if (counts[1]) { k_llf_sigma<16><<<(3 * counts[1] + 127) / 128, 128, 0, s[1]>>>(a, lists[1], counts[1], llf[1]); ++k; }
-  if (counts[2]) { k_llf_sigma<32><<<(3 * counts[2] + 127) / 128, 128, 0, s[2]>>>(a, lists[2], counts[2], llf[2]); ++k; }
+  auto go = [&](auto kernel, int i, int blocks) {
+    if (!counts[i]) return;
+    kernel<<<(counts[i] + blocks - 1) / blocks, kLlfThreads, 0, s[i]>>>(a, lists[i], counts[i],
+                                                                       llf[i]);
+    ++k;
+  };
+  go(k_llf_sigma<8>, 0, kLlfThreads / 3);
+  go(k_llf_sigma<16>, 1, kLlfThreads / 12);
+  go(k_llf_sigma<32>, 2, kLlfThreads / 48);
   return k;
 }
 
