@@ -68,12 +68,12 @@ STAGE_GROUP = {"xyb": "encode", "precondition": "encode", "fdct_luma": "encode",
 # The metric's blur kernels, each timed under its own stage: algorithmic bytes
 # per pixel of every pyramid scale (f32 planes read and written once):
 # k_blur_rows<3> reads the candidate's and the reference's positive XYB and
-# writes the nine row-pass planes (15 planes); k_blur_col_out<3> (the column
+# writes the nine row-pass planes (15 planes); k_blur_cols<3> (the column
 # pass with the ripple's segment scan inside) reads the nine and the
-# reference's mu, sigma11 and XYB and the candidate's XYB (21).  The column
-# ripple's stage now holds only the reset of the scan's flags.
+# reference's mu, sigma11 and XYB and the candidate's XYB (21).  Each is one
+# launch over every scale; the column ripple's stage is empty.
 KERNEL_STAGES = {"ssim_rows": ("k_blur_rows<3>", 60.0),
-                 "ssim_col_out": ("k_blur_col_out<3>", 84.0)}
+                 "ssim_col_out": ("k_blur_cols<3>", 84.0)}
 
 
 def pyramid_pixels(w: int, h: int) -> int:
