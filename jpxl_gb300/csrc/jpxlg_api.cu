@@ -512,7 +512,7 @@ int render_device(jpxlg_ctx* ctx, const jpxlg_layout* L, const int32_t* qcoeff,
   for (int s = 0; s < 3; ++s) {
     int step = steps_for[p->epf_iters][s];
     if (step < 0) break;
-    launch_epf_step(step, cur, nxt, ctx->sigma.as<float>(), g.w, g.h, ctx->stream);
+    launch_epf_step(step, cur, nxt, ctx->sigma.as<float>(), g.w, g.h, ctx->num_sms, ctx->stream);
     std::swap(cur, nxt);
     if ((rc = after_launch(ctx, 1))) return rc;
   }

@@ -130,7 +130,7 @@ int launch_luma_from_image(const EncArgs& a, const uint32_t* const* lists, const
                            const cudaStream_t* s);
 void launch_gaborish(const float* in, float* out, int w, int h, cudaStream_t s);
 void launch_epf_step(int step, const float* in, float* out, const float* sigma, int w, int h,
-                     cudaStream_t s);
+                     int num_sms, cudaStream_t s);
 // out_kind: 1 linear f32 planes, 2 sRGB8 interleaved, 3 linear at depth
 // pxyb (optional, out_kind 3 only): also the SSIMULACRA2 positive XYB planes
 // of the output pixels.

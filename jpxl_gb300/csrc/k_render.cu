@@ -963,7 +963,8 @@ void launch_gaborish(const float* in, float* out, int w, int h, cudaStream_t s) 
 // d_-k(p) = sum |t(p+q) - t(p-k+q)| has d_k(p-k)'s terms in the same order,
 // |a - b| being |b - a| to the bit.  So step 0's twelve taps need six
 // distance fields and step 1's four need two.  A CTA forms the fields of a
-// 64 x 24 region in shared memory, a thread six rows of one column: each
+// 64 x 24 region in shared memory, a thread six rows of one column (RUN; two
+// or four in regions of 8 or 16 rows for small frames): each
 // |t - t'| of a column serves the three crosses above one another that hold
 // it, and the lanes' consecutive columns read without conflicts.  It then
 // weighs the taps of the region's inner pixels (a field is read at most two
@@ -974,22 +975,21 @@ void launch_gaborish(const float* in, float* out, int w, int h, cudaStream_t s) 
 // Runs of four or eight rows and regions of 20 to 40 rows measured 160 to
 // 166 us at 2048x2048; taller regions leave 1920x1080 a nearly empty wave.
 constexpr int kEpfCols = 64;                     // region columns, a thread each
-constexpr int kEpfRun = 6;                       // region rows of a thread
-constexpr int kEpfRows = 4 * kEpfRun;            // region rows
-constexpr int kEpfThreads = kEpfCols * kEpfRows / kEpfRun;
+constexpr int kEpfThreads = 256;                 // four runs of rows
 constexpr int kEpfTileW = kEpfCols + 8;          // 16-byte columns around the region
-constexpr int kEpfTileH = kEpfRows + 4;          // region rows -1 .. kEpfRows + 2
 
-template <int STEP>
+template <int STEP, int RUN>
 struct EpfSmem {
+  static constexpr int kRows = 4 * RUN;   // region rows, RUN a thread
+  static constexpr int kTileH = kRows + 4;  // region rows -1 .. kRows + 2
   static constexpr int kFields = STEP == 0 ? 6 : (STEP == 1 ? 2 : 0);
   // Pixels written: the region's columns 2 .. 61 and rows from 2 where fields
   // are read to their left, right and above, all of it in step 2.
   static constexpr int kEdge = STEP < 2 ? 2 : 0;
-  static constexpr int kOutW = STEP < 2 ? kEpfCols - 4 : kEpfCols, kOutH = kEpfRows - kEdge;
+  static constexpr int kOutW = STEP < 2 ? kEpfCols - 4 : kEpfCols, kOutH = kRows - kEdge;
   static constexpr int kBlocksW = kOutW / 8 + 2, kBlocksH = kOutH / 8 + 2;
-  float t[3][kEpfTileH][kEpfTileW];
-  float d[kFields > 0 ? kFields : 1][kFields > 0 ? kEpfRows : 1][kEpfCols];
+  float t[3][kTileH][kEpfTileW];
+  float d[kFields > 0 ? kFields : 1][kFields > 0 ? kRows : 1][kEpfCols];
   float sigma[kBlocksH][kBlocksW], inv[kBlocksH][kBlocksW];  // of the 8x8 blocks under the tile
 };
 
@@ -1002,16 +1002,16 @@ __device__ __forceinline__ constexpr float epf_scale(int c) {
 // step 0, (1,1), (-1,1), (2,0), (0,2).  Row by row, a cross's north, centre
 // row and south terms enter its sum in the order centre, west, east, north,
 // south.
-template <int STEP>
-__device__ __forceinline__ void epf_fields(EpfSmem<STEP>& sm, int x, int y) {
-  constexpr int NF = EpfSmem<STEP>::kFields;
+template <int STEP, int RUN>
+__device__ __forceinline__ void epf_fields(EpfSmem<STEP, RUN>& sm, int x, int y) {
+  constexpr int NF = EpfSmem<STEP, RUN>::kFields;
   constexpr int kAhead = STEP == 0 ? 2 : 1;  // rows a tap reaches down
   constexpr int fx[6] = {1, 0, 1, -1, 2, 0}, fy[6] = {0, 1, 1, 1, 0, 2};
-  float d[NF][kEpfRun];
+  float d[NF][RUN];
 #pragma unroll
   for (int k = 0; k < NF; ++k)
 #pragma unroll
-    for (int i = 0; i < kEpfRun; ++i) d[k][i] = 0.0f;
+    for (int i = 0; i < RUN; ++i) d[k][i] = 0.0f;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const float s = epf_scale(c);
@@ -1024,14 +1024,14 @@ __device__ __forceinline__ void epf_fields(EpfSmem<STEP>& sm, int x, int y) {
     for (int j = 0; j < kAhead; ++j) fetch(r[j], j);
     float north[NF];
 #pragma unroll
-    for (int j = 0; j < kEpfRun + 2; ++j) {  // run row j - 1
-      if (j + kAhead < kEpfRun + 2 + kAhead) fetch(r[kAhead], j + kAhead);
+    for (int j = 0; j < RUN + 2; ++j) {  // run row j - 1
+      if (j + kAhead < RUN + 2 + kAhead) fetch(r[kAhead], j + kAhead);
 #pragma unroll
       for (int k = 0; k < NF; ++k) {
         auto diff = [&](int q) { return fabsf(r[0][q] - r[fy[k]][q + fx[k]]); };
         const float centre = diff(2);
         if (j >= 2) d[k][j - 2] = __fmaf_rn(centre, s, d[k][j - 2]);
-        if (j >= 1 && j <= kEpfRun) {
+        if (j >= 1 && j <= RUN) {
           float& a = d[k][j - 1];
           a = __fmaf_rn(centre, s, a);
           a = __fmaf_rn(diff(1), s, a);
@@ -1049,17 +1049,18 @@ __device__ __forceinline__ void epf_fields(EpfSmem<STEP>& sm, int x, int y) {
 #pragma unroll
   for (int k = 0; k < NF; ++k)
 #pragma unroll
-    for (int i = 0; i < kEpfRun; ++i) sm.d[k][y + i][x] = d[k][i];
+    for (int i = 0; i < RUN; ++i) sm.d[k][y + i][x] = d[k][i];
 }
 
-template <int STEP>
+template <int STEP, int RUN>
 __global__ void __launch_bounds__(kEpfThreads, STEP == 0 ? 3 : 4)
     k_epf(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ sigma,
           int w, int h, float step_mul4) {
   extern __shared__ __align__(16) unsigned char epf_smem[];
-  EpfSmem<STEP>& sm = *reinterpret_cast<EpfSmem<STEP>*>(epf_smem);
+  using Smem = EpfSmem<STEP, RUN>;
+  Smem& sm = *reinterpret_cast<Smem*>(epf_smem);
+  constexpr int kEpfTileH = Smem::kTileH;
   const size_t plane = (size_t)w * h;
-  using Smem = EpfSmem<STEP>;
   constexpr int kEdge = Smem::kEdge;
   const int x0 = blockIdx.x * Smem::kOutW, y0 = blockIdx.y * Smem::kOutH;
   // Tile columns x0-4 .., region rows -1 ..: 16 bytes at a time inside the frame,
@@ -1103,9 +1104,9 @@ __global__ void __launch_bounds__(kEpfThreads, STEP == 0 ? 3 : 4)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  const int rx = threadIdx.x % kEpfCols, ry = threadIdx.x / kEpfCols * kEpfRun;
+  const int rx = threadIdx.x % kEpfCols, ry = threadIdx.x / kEpfCols * RUN;
   if constexpr (STEP < 2) {
-    epf_fields<STEP>(sm, rx, ry);
+    epf_fields<STEP, RUN>(sm, rx, ry);
     __syncthreads();
   }
   const int gx = x0 - kEdge + rx;
@@ -1122,7 +1123,7 @@ __global__ void __launch_bounds__(kEpfThreads, STEP == 0 ? 3 : 4)
   const bool side = (gx & 7) == 0 || (gx & 7) == 7;
   const int bcol = gx / 8 - x0 / 8;
 #pragma unroll 1
-  for (int i = 0; i < kEpfRun; ++i) {
+  for (int i = 0; i < RUN; ++i) {
     const int cy = ry + i, gy = y0 - kEdge + cy;
     if (cy < kEdge || gy >= h) continue;
     auto at = [&](int c, int dx, int dy) { return sm.t[c][cy + 1 + dy][rx + 4 - kEdge + dx]; };
@@ -1180,21 +1181,38 @@ __global__ void __launch_bounds__(kEpfThreads, STEP == 0 ? 3 : 4)
 }
 
 void launch_epf_step(int step, const float* in, float* out, const float* sigma, int w, int h,
-                     cudaStream_t s) {
+                     int num_sms, cudaStream_t s) {
   // restoration.rs:356 epf_inv_sigma: step_multiplier * 4 * (1 - sqrt(0.5)) / sigma,
   // evaluated left to right; the numerator is formed here once.
   float sc = step == 0 ? 0.9f : (step == 1 ? 1.0f : 6.5f);
   float sm = 1.65f * sc;
   float num = sm * 4.0f * (1.0f - sqrtf(0.5f));
   auto run = [&](auto* kernel, auto smem) {
-    using Smem = decltype(smem);
-    const dim3 grid((w + Smem::type::kOutW - 1) / Smem::type::kOutW,
-                    (h + Smem::type::kOutH - 1) / Smem::type::kOutH);
-    kernel<<<grid, kEpfThreads, sizeof(typename Smem::type), s>>>(in, out, sigma, w, h, num);
+    using Smem = typename decltype(smem)::type;
+    const dim3 grid((w + Smem::kOutW - 1) / Smem::kOutW, (h + Smem::kOutH - 1) / Smem::kOutH);
+    kernel<<<grid, kEpfThreads, sizeof(Smem), s>>>(in, out, sigma, w, h, num);
   };
-  if (step == 0) run(k_epf<0>, std::common_type<EpfSmem<0>>{});
-  else if (step == 1) run(k_epf<1>, std::common_type<EpfSmem<1>>{});
-  else run(k_epf<2>, std::common_type<EpfSmem<2>>{});
+  // Rows of a thread: two or four where at most two CTAs come to an SM, else
+  // six.  A short run computes more of its fields twice but ends sooner (the
+  // three steps of 64x64: 26.7 us with six rows, 20.4 with two; of 501x333:
+  // 27.5, 26.4 with four); beyond that the work is the time.
+  auto pick = [&](auto st) {
+    constexpr int STEP = decltype(st)::value;
+    auto fits = [&](auto smem) {
+      using Smem = typename decltype(smem)::type;
+      return (long long)((w + Smem::kOutW - 1) / Smem::kOutW) *
+                 ((h + Smem::kOutH - 1) / Smem::kOutH) <= 2LL * num_sms;
+    };
+    const std::common_type<EpfSmem<STEP, 2>> two;
+    const std::common_type<EpfSmem<STEP, 4>> four;
+    const std::common_type<EpfSmem<STEP, 6>> six;
+    if (fits(two)) run(k_epf<STEP, 2>, two);
+    else if (fits(four)) run(k_epf<STEP, 4>, four);
+    else run(k_epf<STEP, 6>, six);
+  };
+  if (step == 0) pick(std::integral_constant<int, 0>{});
+  else if (step == 1) pick(std::integral_constant<int, 1>{});
+  else pick(std::integral_constant<int, 2>{});
 }
 
 // ---------------------------------------------------------------------------
@@ -1372,9 +1390,15 @@ cudaError_t configure_render_kernels() {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
   cudaError_t e;
-  if ((e = allow(k_epf<0>, sizeof(EpfSmem<0>))) != cudaSuccess) return e;
-  if ((e = allow(k_epf<1>, sizeof(EpfSmem<1>))) != cudaSuccess) return e;
-  if ((e = allow(k_epf<2>, sizeof(EpfSmem<2>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<0, 2>, sizeof(EpfSmem<0, 2>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<0, 4>, sizeof(EpfSmem<0, 4>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<0, 6>, sizeof(EpfSmem<0, 6>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<1, 2>, sizeof(EpfSmem<1, 2>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<1, 4>, sizeof(EpfSmem<1, 4>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<1, 6>, sizeof(EpfSmem<1, 6>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<2, 2>, sizeof(EpfSmem<2, 2>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<2, 4>, sizeof(EpfSmem<2, 4>))) != cudaSuccess) return e;
+  if ((e = allow(k_epf<2, 6>, sizeof(EpfSmem<2, 6>))) != cudaSuccess) return e;
   if ((e = allow(k_render_64<64, 64>, sizeof(Rect64Smem<64, 64>))) != cudaSuccess) return e;
   if ((e = allow(k_render_64<64, 32>, sizeof(Rect64Smem<64, 32>))) != cudaSuccess) return e;
   return allow(k_render_64<32, 64>, sizeof(Rect64Smem<32, 64>));

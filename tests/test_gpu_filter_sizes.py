@@ -2,7 +2,8 @@
 restatement's XYB planes.
 
 Widths around the EPF's 60 and 64 pixel columns and the 16-byte rows that
-the tiles and Gaborish load at once, heights around its 22 and 24 rows and
+the tiles and Gaborish load at once, heights around its 6 and 8, 14 and 16, 22
+and 24 rows (runs of two, four and six rows by the frame's size) and
 Gaborish's runs of eight; every step count, sharpness 0 .. 7 (blocks that
 are copied among them) and uneven hf_mul.
 """
@@ -15,7 +16,8 @@ from jpxl_gb300 import synth
 pytestmark = pytest.mark.gpu
 
 SIZES = [(1, 1), (3, 2), (8, 8), (60, 22), (61, 23), (64, 24), (65, 25), (68, 45), (72, 50),
-         (123, 44), (124, 47), (128, 96), (131, 73), (192, 71), (200, 120), (252, 68)]
+         (123, 44), (124, 47), (128, 96), (131, 73), (192, 71), (200, 120), (252, 68),
+         (240, 362), (253, 378), (601, 425), (640, 462)]
 
 
 @pytest.mark.parametrize("epf", [1, 2, 3])
