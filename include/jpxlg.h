@@ -458,6 +458,10 @@ int jpxlg_decode_batch_destroy(jpxlg_decode_batch* batch);
  * library's module loads, whether or not this entry point is called. */
 int jpxlg_ssim2_score_static(jpxlg_ctx* ctx, const jpxlg_ref* ref,
                              const float* linear_rgb_dev, double* out_dev);
+/* Diagnostic: leaves in the scoring scratch of ctx and of its device the
+ * counts that calls in flight at the same time can leave there (queued on
+ * ctx's stream).  The scores of later calls do not depend on them. */
+int jpxlg_diag_scan_words(jpxlg_ctx* ctx);
 
 #ifdef __cplusplus
 }

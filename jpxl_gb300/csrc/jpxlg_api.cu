@@ -1617,6 +1617,17 @@ extern "C" int jpxlg_ssim2_score_static(jpxlg_ctx* ctx, const jpxlg_ref* ref,
   return after_launch(ctx, k);
 }
 
+extern "C" int jpxlg_diag_scan_words(jpxlg_ctx* ctx) {
+  if (!ctx) return JPXLG_ERR_ARGUMENT;
+  CK(cudaSetDevice(ctx->device));
+  unsigned char* scratch = nullptr;
+  int rc = static_scratch(ctx, &scratch);
+  if (rc) return rc;
+  CK(blur_disturb((float*)scratch + kStaticFloats - kStaticCarryFloats, ctx->stream));
+  if (ctx->bcarry.p) CK(blur_disturb(ctx->bcarry.p, ctx->stream));
+  return JPXLG_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Decoded codestreams: the frame's integer content from the host reader,
 // reconstructed by the same kernels as a plan (decode.rs:2700-3061).

@@ -224,5 +224,7 @@ int launch_score_finish(DF* partials, const int* ctas_per_scale, int nscales,
                         double* raw, cudaStream_t s);
 // The word of a scan buffer's header that counts finished CTAs.
 uint32_t* blur_ticket(void* carry);
+// Leaves counts in the header as calls that raced on the buffer may.
+cudaError_t blur_disturb(void* carry, cudaStream_t s);
 
 }  // namespace jpxlg

@@ -253,14 +253,22 @@ __device__ __forceinline__ f2 ripple_hom2(int u, const f2* ep, const f2* eq, f2 
 // stale word can carry the current one.
 // ---------------------------------------------------------------------------
 
+// counter: the column pass's segments handed out.  ticket: the score's CTAs
+// that have finished.  Both are zeroed by the row pass of every blur, so that
+// whatever an earlier call left in them (calls that raced on one buffer lose
+// counts) ends with that call.
 struct ScanHeader {
-  uint32_t epoch, counter, finished;
-  uint32_t ticket;  // the score's last CTA; zero between launches
-  uint32_t pad[12];
+  uint32_t epoch, counter, ticket;
+  uint32_t pad[13];
 };
 static_assert(sizeof(ScanHeader) == 64, "scan header");
 
 uint32_t* blur_ticket(void* carry) { return &static_cast<ScanHeader*>(carry)->ticket; }
+
+cudaError_t blur_disturb(void* carry, cudaStream_t s) {
+  ScanHeader* const h = static_cast<ScanHeader*>(carry);
+  return cudaMemsetAsync(&h->counter, 0x35, sizeof h->counter + sizeof h->ticket, s);
+}
 
 __device__ __forceinline__ void scan_store(uint4* p, float a, float b, float c, uint32_t tag) {
   const unsigned long long lo =
@@ -325,10 +333,12 @@ __global__ void __launch_bounds__(kRowThreads, 5) k_blur_rows(const __grid_const
   extern __shared__ __align__(16) f2 bsm2[];
   __shared__ f2 carry[6][kRowThreads];
   const int t = threadIdx.x;
-  // The column pass that follows starts a new epoch and work count.
+  // The column pass that follows starts a new epoch and work count, and the
+  // score's end a new count of its CTAs.
   if (blockIdx.x == 0 && t == 0) {
-    a.scan->epoch += 1;
+    atomicAdd(&a.scan->epoch, 1u);
     a.scan->counter = 0;
+    a.scan->ticket = 0;
   }
   int si = 0;
   while (si + 1 < a.n && (int)blockIdx.x >= a.s[si + 1].first) ++si;
@@ -539,7 +549,7 @@ struct ColArgs {
   ColScale s[kMaxScales];
   ScanHeader* scan;
   uint32_t* err;  // the context's device error word
-  int n, c0, nch;
+  int n, c0, nch, items;  // items: segments of all scales
   float nz;
   float pw[3][4];  // M_k^kTileH
 };
@@ -602,6 +612,9 @@ __global__ void __launch_bounds__(kColThreads, 3) k_blur_cols(const __grid_const
   const uint32_t epoch = a.scan->epoch;
   __syncthreads();
   const int gitem = sm.item;
+  // A count past the last segment: another call runs on this buffer at the
+  // same time.  The scores are spoilt, the accesses stay inside it.
+  if (gitem >= a.items) return;
   int si = 0;
   while (si + 1 < a.n && gitem >= a.s[si + 1].first) ++si;
   const ColScale& sc = a.s[si];
@@ -930,6 +943,7 @@ void launch_blur(const BlurScale* scales, int n, int c0, int nch, float* hpl, vo
     cols += c.strips * c.nseg * nch;
     states += (size_t)nch * c.nseg * NQ * 2 * b.w;
   }
+  ca.items = cols;
   if (hook) hook(user, 0);
   // scale 0 has the longest lines
   k_blur_rows<NQ><<<rows, kRowThreads, row_smem(scales[0].w), s>>>(ra);

@@ -138,7 +138,7 @@ constexpr int kReduceThreads = 256;
 // column).  Deterministic for a given frame size; every load of a scale is
 // in flight at once instead of behind one CTA's sequential chains.
 //
-// The CTA that finishes last (`ticket`, zero between launches) goes on to
+// The CTA that finishes last (`ticket`, zeroed by the blur before) goes on to
 // the norms, weights and remap of the 6 x 18 totals, a thread per term.
 // Bound by the latency of its double-precision chain (two square roots, the
 // weighted sum, one power): 3 + 13.6 us as two launches whose second took a
@@ -186,7 +186,6 @@ __global__ void __launch_bounds__(kReduceThreads) k_score_finish(DF* __restrict_
     out[2 + (sc * 3 + c) * 6 + nn * 3 + m] = term;
     wterm[t] = c_weights[t] * fabs(term);
   }
-  if (t == 0) *ticket = 0;
   __syncthreads();
   if (t >= 32) return;
   double part = 0.0;
