@@ -1864,6 +1864,41 @@ void decode(const uint8_t* data, size_t size, Decoded* out) {
 }
 
 
+int coefficient_bytes(const VarDctFrame& v) {
+  uint32_t span = 0;  // bits of the magnitudes, two's complement
+  for (const std::vector<int32_t>& c : v.coeffs)
+    for (int32_t x : c) span |= (uint32_t)(x ^ (x >> 31));
+  return span < 0x80u ? 1 : (span < 0x8000u ? 2 : 4);
+}
+
+namespace {
+
+template <typename T>
+void place_coefficients(const VarDctFrame& v, T* out) {
+  const size_t W8 = (size_t)v.bw * 8, H8 = (size_t)v.bh * 8, plane = W8 * H8;
+  std::fill_n(out, 3 * plane, (T)0);
+  for (const Varblock& vb : v.varblocks) {
+    const TransformShape s = transform_shape(vb.transform);
+    const uint32_t cr = std::min(s.rows, s.cols) * 8, cc = std::max(s.rows, s.cols) * 8;
+    const bool portrait = s.rows > s.cols;
+    for (int c = 0; c < 3; ++c)
+      for (uint32_t y = 0; y < cr; ++y)
+        for (uint32_t x = 0; x < cc; ++x) {
+          const size_t pos = portrait ? (size_t)(vb.by * 8 + x) * W8 + vb.bx * 8 + y
+                                      : (size_t)(vb.by * 8 + y) * W8 + vb.bx * 8 + x;
+          out[c * plane + pos] = (T)v.coeffs[c][vb.coeff_offset + y * cc + x];
+        }
+  }
+}
+
+}  // namespace
+
+void stage_coefficients(const VarDctFrame& v, int q_bytes, void* out) {
+  if (q_bytes == 1) place_coefficients(v, static_cast<int8_t*>(out));
+  else if (q_bytes == 2) place_coefficients(v, static_cast<int16_t*>(out));
+  else place_coefficients(v, static_cast<int32_t*>(out));
+}
+
 }  // namespace cs
 }  // namespace jpxlg
 
@@ -1969,21 +2004,7 @@ extern "C" int jpxlg_codestream_blocks(const jpxlg_codestream* cs, int32_t* lf, 
 // portrait varblock's matrix transposed.
 extern "C" int jpxlg_codestream_coefficients(const jpxlg_codestream* cs, int32_t* out) {
   if (!cs || !out) return JPXLG_ERR_ARGUMENT;
-  const jpxlg::cs::VarDctFrame& v = cs->d.vardct;
-  const size_t W8 = (size_t)v.bw * 8, H8 = (size_t)v.bh * 8, plane = W8 * H8;
-  std::memset(out, 0, 3 * plane * sizeof(int32_t));
-  for (const jpxlg::cs::Varblock& vb : v.varblocks) {
-    const jpxlg::cs::TransformShape s = jpxlg::cs::transform_shape(vb.transform);
-    const uint32_t cr = std::min(s.rows, s.cols) * 8, cc = std::max(s.rows, s.cols) * 8;
-    const bool portrait = s.rows > s.cols;
-    for (int c = 0; c < 3; ++c)
-      for (uint32_t y = 0; y < cr; ++y)
-        for (uint32_t x = 0; x < cc; ++x) {
-          const size_t pos = portrait ? (size_t)(vb.by * 8 + x) * W8 + vb.bx * 8 + y
-                                      : (size_t)(vb.by * 8 + y) * W8 + vb.bx * 8 + x;
-          out[c * plane + pos] = v.coeffs[c][vb.coeff_offset + y * cc + x];
-        }
-  }
+  jpxlg::cs::stage_coefficients(cs->d.vardct, sizeof(int32_t), out);
   return JPXLG_OK;
 }
 

@@ -123,6 +123,12 @@ struct TransformShape {
 };
 TransformShape transform_shape(uint8_t dct_select);
 
+// The narrowest of 1, 2 and 4 bytes that holds every coefficient of a frame,
+// and the frame's coefficient image (3 x (8*bh) x (8*bw)) in integers of that
+// width.  Neither allocates: they run behind C entries.
+int coefficient_bytes(const VarDctFrame& v);
+void stage_coefficients(const VarDctFrame& v, int q_bytes, void* out);
+
 // Parses the codestream (a bare one, starting 0xFF 0x0A) and decodes the
 // integer content of its first frame.  Throws Malformed.
 void decode(const uint8_t* data, size_t size, Decoded* out);

@@ -1720,11 +1720,7 @@ int decode_stage(jpxlg_ctx* ctx, const jpxlg_codestream* cs, int out_kind, bool 
   if (v.lf_from_frame)
     for (int c = 0; c < 3; ++c)
       if (v.lf_frame[c].size() != st.nb) return fail(ctx, JPXLG_ERR_STREAM, "LF frame size");
-  std::vector<int32_t> q(3 * st.n8);
-  if ((rc = jpxlg_codestream_coefficients(cs, q.data()))) return rc;
-  uint32_t span = 0;  // bits of the magnitudes, two's complement
-  for (int32_t x : q) span |= (uint32_t)(x ^ (x >> 31));
-  st.q_bytes = span < 0x80u ? 1 : (span < 0x8000u ? 2 : 4);
+  st.q_bytes = jpxlg::cs::coefficient_bytes(v);
   const size_t qb = 3 * st.n8 * st.q_bytes, lb = 3 * st.nb * sizeof(int32_t);
   const size_t fb = v.lf_from_frame ? 3 * st.nb * sizeof(float) : 0;
   st.rest = (lb + fb + 2 * st.nt + 15) & ~(size_t)15;
@@ -1738,9 +1734,7 @@ int decode_stage(jpxlg_ctx* ctx, const jpxlg_codestream* cs, int out_kind, bool 
   st.lf_frame = fb ? (float*)(h + qb + lb) : nullptr;
   st.cflx = (int8_t*)(h + qb + lb + fb);
   st.cflb = st.cflx + st.nt;
-  if (st.q_bytes == 1) std::copy(q.begin(), q.end(), (int8_t*)h);
-  else if (st.q_bytes == 2) std::copy(q.begin(), q.end(), (int16_t*)h);
-  else std::copy(q.begin(), q.end(), (int32_t*)h);
+  jpxlg::cs::stage_coefficients(v, st.q_bytes, h);
   for (int c = 0; c < 3; ++c) {
     std::copy(v.lf[c].begin(), v.lf[c].end(), st.lfq + c * st.nb);
     if (st.lf_frame) std::copy(v.lf_frame[c].begin(), v.lf_frame[c].end(), st.lf_frame + c * st.nb);
@@ -1840,6 +1834,7 @@ struct jpxlg_decode_batch {
   // bits, never kPending).
   static constexpr uint32_t kPending = 0xffffffffu;
   uint32_t* h_done = nullptr;
+  std::vector<size_t> pending;  // run's items to copy out; its room is made at creation
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> joins;
   cudaGraph_t graph = nullptr;
@@ -1946,6 +1941,7 @@ extern "C" int jpxlg_decode_batch_create(jpxlg_ctx* ctx, int n, const jpxlg_code
   CK(cudaMallocHost(&b->h_out, total));
   CK(cudaMallocHost(&b->h_done, n * sizeof(uint32_t)));
   std::fill_n(b->h_done, n, jpxlg_decode_batch::kPending);
+  b->pending.reserve(n);
   // Warm-up: the lanes' buffers grow to their largest frame here.
   int rc = decode_batch_enqueue(ctx, b.get());
   if (rc) return rc;
@@ -1990,7 +1986,8 @@ extern "C" int jpxlg_decode_batch_run(jpxlg_ctx* ctx, jpxlg_decode_batch* b, voi
   // Each item's pixels as they arrive, while the rest renders; items of a
   // lane finish in order, so a pass over the pending ones meets the done ones
   // soon.  The stream's own end bounds the wait.
-  std::vector<size_t> pending;
+  std::vector<size_t>& pending = b->pending;
+  pending.clear();
   if (outs)
     for (size_t i = 0; i < b->items.size(); ++i)
       if (outs[i]) pending.push_back(i);
