@@ -423,15 +423,18 @@ int jpxlg_codestream_render(jpxlg_ctx* ctx, const jpxlg_codestream* cs, int out_
  * are large: each lane keeps a workspace of about 64 bytes per pixel of its
  * largest frame, held to 16 GiB in all), renders each once to
  * size the workspaces, and captures one CUDA graph on ctx's stream: per
- * stream, the staged planes to the device, LF preparation, the render into
- * `out_kind` (as jpxlg_codestream_render) and the pixels back to a pinned
- * host buffer.  `precision` (JPXLG_PRECISION_*) picks how the square
+ * stream, a kernel that reads the staged block where it stands and lays it
+ * out on the device (the coefficients are staged in the narrowest of 1, 2 and
+ * 4 bytes that holds them), LF preparation, the render into `out_kind` (as
+ * jpxlg_codestream_render) and the pixels back to a pinned host buffer.  `precision` (JPXLG_PRECISION_*) picks how the square
  * DCT8/16/32 varblocks' IDCTs run; every other transform renders through
  * the FP32 kernels.  The streams must stay open while the batch lives.
- * jpxlg_decode_batch_run launches the graph; with JPXLG_MEM_HOST it waits
- * and copies stream i's pixels to outs[i] (host; NULL entries, or outs
- * NULL, skip the copy); with JPXLG_MEM_DEVICE it queues device-to-device
- * copies to outs[i] and returns without waiting.  Streams the renderer does
+ * jpxlg_decode_batch_run launches the graph; with JPXLG_MEM_HOST it copies
+ * stream i's pixels to outs[i] (host; NULL entries, or outs NULL, skip the
+ * copy) as each stream finishes and returns when all have; if it returns an
+ * error, some of the arrays may have been written and others not.  With
+ * JPXLG_MEM_DEVICE it queues device-to-device copies to outs[i] and returns
+ * without waiting.  Streams the renderer does
  * not carry fail creation with JPXLG_ERR_STREAM, naming the stream. */
 typedef struct jpxlg_decode_batch jpxlg_decode_batch;
 int jpxlg_decode_batch_create(jpxlg_ctx* ctx, int n, const jpxlg_codestream* const* streams,

@@ -11,6 +11,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/jpxlg.h"
@@ -1985,15 +1986,21 @@ extern "C" int jpxlg_decode_batch_run(jpxlg_ctx* ctx, jpxlg_decode_batch* b, voi
   }
   // Each item's pixels as they arrive, while the rest renders; items of a
   // lane finish in order, so a pass over the pending ones meets the done ones
-  // soon.  The stream's own end bounds the wait.
+  // soon.  A pass that finds none gives way to other threads; the stream,
+  // whose end bounds the wait, is asked only after a run of such passes.
   std::vector<size_t>& pending = b->pending;
   pending.clear();
   if (outs)
     for (size_t i = 0; i < b->items.size(); ++i)
       if (outs[i]) pending.push_back(i);
+  constexpr int kIdlePasses = 64;
+  int idle = 0;
   bool running = true, clean = true;
   while (clean && !pending.empty() && running) {
-    running = cudaStreamQuery(ctx->stream) == cudaErrorNotReady;
+    if (idle == kIdlePasses) {
+      running = cudaStreamQuery(ctx->stream) == cudaErrorNotReady;
+      idle = 0;
+    }
     size_t kept = 0;
     for (size_t k = 0; k < pending.size() && clean; ++k) {
       const size_t i = pending[k];
@@ -2001,6 +2008,12 @@ extern "C" int jpxlg_decode_batch_run(jpxlg_ctx* ctx, jpxlg_decode_batch* b, voi
       if (word == jpxlg_decode_batch::kPending) pending[kept++] = i;
       else if (word) clean = false;
       else std::memcpy(outs[i], b->h_out + b->out_off[i], b->out_bytes[i]);
+    }
+    if (kept == pending.size()) {
+      ++idle;
+      std::this_thread::yield();
+    } else {
+      idle = 0;
     }
     pending.resize(clean ? kept : 0);
   }
