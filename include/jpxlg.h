@@ -228,6 +228,15 @@ int jpxlg_tune_get(int knob);
 int jpxlg_diag_special_blocks(jpxlg_ctx* ctx, int kind, const float* coef, int n, float* out,
                               uint32_t mem);
 
+/* Diagnostic: the kernels' short forms of a rule against the rule itself, for
+ * every float of bit patterns first .. first + count - 1 (2^32 in all): the
+ * codec's and the metric's cube root (jpxl-core simd.rs:36, jpxl-perceptual
+ * color.rs:46: the f64 iterations), or the output level of a linear sample at
+ * a depth of 1..16 bits (JPXLG_SWEEP_LEVELS + bits: its thresholds).  *wrong
+ * receives the number of results that differ in any bit.  Synchronizes. */
+enum { JPXLG_SWEEP_CBRT_CORE = 0, JPXLG_SWEEP_CBRT_METRIC = 1, JPXLG_SWEEP_LEVELS = 100 };
+int jpxlg_diag_sweep(jpxlg_ctx* ctx, int what, uint32_t first, uint64_t count, uint64_t* wrong);
+
 /* Quantized plan -> pixels.  `out` sizes: JPXLG_OUT_SRGB8 w*h*3 bytes, other
  * kinds 3*w*h floats.  `bits` is the depth of JPXLG_OUT_LINEAR_DEPTH. */
 int jpxlg_reconstruct(jpxlg_ctx* ctx, const jpxlg_layout* layout, const jpxlg_plan* plan,

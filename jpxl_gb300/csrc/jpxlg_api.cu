@@ -971,6 +971,34 @@ int jpxlg_diag_special_blocks(jpxlg_ctx* ctx, int kind, const float* coef, int n
   return JPXLG_OK;
 }
 
+int jpxlg_diag_sweep(jpxlg_ctx* ctx, int what, uint32_t first, uint64_t count, uint64_t* wrong) {
+  if (!ctx || !wrong) return fail(ctx, JPXLG_ERR_ARGUMENT, "null argument");
+  const int bits = what - JPXLG_SWEEP_LEVELS;
+  const bool cbrt = what == JPXLG_SWEEP_CBRT_CORE || what == JPXLG_SWEEP_CBRT_METRIC;
+  if (!cbrt && !(bits >= 1 && bits <= 16))
+    return fail(ctx, JPXLG_ERR_ARGUMENT, "no such sweep: %d", what);
+  if (count > ((uint64_t)1 << 32) - first)
+    return fail(ctx, JPXLG_ERR_ARGUMENT, "a float has 32 bits");
+  CK(cudaSetDevice(ctx->device));
+  DepthTable none;
+  const DepthTable* t = cbrt ? &none : get_depth(ctx, bits);
+  if (!t) return fail(ctx, JPXLG_ERR_CUDA, "depth table");
+  CK(ctx->score.ensure(128 * sizeof(double)));
+  unsigned long long* const d = ctx->score.as<unsigned long long>();
+  CK(cudaMemsetAsync(d, 0, sizeof *d, ctx->stream));
+  for (uint64_t done = 0; done < count;) {
+    const uint32_t n = (uint32_t)std::min<uint64_t>(count - done, 1u << 28);
+    launch_sweep_diag(what, first + (uint32_t)done, n, t->thr, t->lev, t->bracket, t->levels, d,
+                      ctx->num_sms, ctx->stream);
+    int rc = after_launch(ctx, 1);
+    if (rc) return rc;
+    done += n;
+  }
+  CK(cudaMemcpyAsync(wrong, d, sizeof *d, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return JPXLG_OK;
+}
+
 int jpxlg_encode_stages(jpxlg_ctx* ctx, const jpxlg_layout* L, const void* rgb, int bits,
                         const jpxlg_params* p, float* xyb, float* pre, float* coeff) {
   if (!ctx || !L || !rgb) return fail(ctx, JPXLG_ERR_ARGUMENT, "null argument");

@@ -34,10 +34,12 @@ __device__ __forceinline__ int mirror1d(int c, int size) {
 // exact cube root, i.e. they return the correctly rounded cube root unless
 // the exact root lies within that distance of a rounding midpoint.  The fast
 // paths below find the correctly rounded root in f32 arithmetic (an estimate,
-// then a double-float residual that places the exact root to within 2^-19
-// ulp); where the root lies within 2^-17 ulp of a midpoint, or the input is
-// outside the verified range, the reference's own f64 iteration runs, so the
-// result is the reference's bit for bit either way.
+// then a double-float residual that places the exact root to within 2^-17.7
+// ulp from the short path's estimate, 2^-20 ulp from the wide one's); where
+// the root lies within 2^-17 ulp of a midpoint, or the input is outside the
+// paths' ranges, the reference's own f64 iteration runs, so the result is the
+// reference's bit for bit either way (test_gpu_sweeps.py compares them for
+// every float).
 
 static __device__ __noinline__ float cbrt_core_f64(float value) {
   const uint32_t B1 = 709958130u, B2 = 642849266u;
@@ -114,12 +116,15 @@ static __device__ __noinline__ float cbrt_general(float v) {
 
 // Correctly rounded cbrt of v in [2^-10, 2^10] (where an opsin mix of
 // in-gamut light lies: 0.0038 to 1.004).  The estimate y = 2^(log2(a) / 3)
-// is within 2^-20 of the root, log2 losing 2^-22.6 of at most 10; the
-// residual a - y^3 is formed to 2^-48 of a, and with its second-order term
-// places the root to 2^-42 of itself, 2^-18 ulp.  z is the nearest float to
-// y plus that correction; it is certain unless the remainder is within 2^-17
-// ulp of half an ulp, or z a power of two (where the ulp changes).  Checked
-// against the f64 iterations for every float of the range.
+// is within 2^-20.5 of the root: log2 loses 2^-22.6 of at most 10, a third of
+// it by ln 2 is 2^-21.4, and the product and the power add 2^-21.6.  The
+// residual a - y^3 is formed to 2^-48 of a; the correction from it, with its
+// second-order term, is at most as large as the estimate's error and loses
+// seven times 2^-24 of itself (d, p, 3p, two for the reciprocal, d1, d2), so
+// that it places the root to 2^-41.7 of itself, 2^-17.7 ulp below a power of
+// two.  z is the nearest float to y plus the correction; it is certain unless
+// the remainder is within 2^-17 ulp of half an ulp, or z a power of two (where
+// the ulp changes).
 // Measured against a library root with its residual, by itself: XYB of a
 // 4096x3072 frame 122 -> 102 us, colour output of a 2048x2048 one 77 -> 71.
 template <bool kMetric>

@@ -70,6 +70,12 @@ void launch_unstage(const void* src, int q_bytes, size_t n, size_t rest, void* d
 void launch_publish(const uint32_t* err, uint32_t* flag, cudaStream_t s);
 void upload_dct64(const float* matrix, cudaStream_t s);
 void upload_afv(const double* basis, cudaStream_t s);
+// Differences over count floats (count + 2^20 at most 2^32) from bit pattern
+// `first`: what 0 and 1 the cube roots, else the output levels of the given
+// tables.
+void launch_sweep_diag(int what, uint32_t first, uint32_t count, const float* thr,
+                       const float* levels, const float4* bracket, int nlev,
+                       unsigned long long* wrong, int num_sms, cudaStream_t s);
 bool launch_special_diag(int kind, const float* coef, int n, float* out, cudaStream_t s);
 
 // Fills table[h] = hf_multiplier_f64(global_scale, h) for h < kMulTableN.

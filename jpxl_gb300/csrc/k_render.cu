@@ -1248,6 +1248,16 @@ __device__ __forceinline__ int level_estimate(float x, float maxv, float margin,
   return (int)fminf(fmaxf(k, 0.0f), maxv);
 }
 
+// x's level by the estimate where it is certain, else by its n thresholds.
+__device__ __forceinline__ int shallow_level(float x, float maxv, float margin, const float* thr,
+                                             int n) {
+  bool certain;
+  const int k = level_estimate(x, maxv, margin, &certain);
+  return certain ? k : level_of(x, thr, n);
+}
+
+__device__ __forceinline__ float level_margin(float maxv) { return 1e-3f + 1e-6f * maxv; }
+
 // The linear value of x's level for deep outputs (more than 256 levels) where
 // the bracket of the estimated level does not hold x: stepping by one, then
 // by binary search.  The thresholds decide, so the result is exactly the
@@ -1265,6 +1275,14 @@ static __device__ __noinline__ float level_value_search(float x, int est,
     est += lo_ok ? 1 : -1;
   }
   return __ldg(&levels[level_of(x, thr, n)]);
+}
+
+// The same from v, the bracket of the estimated level est.
+__device__ __forceinline__ float deep_level_value(float x, int est, const float4& v,
+                                                  const float4* __restrict__ br,
+                                                  const float* __restrict__ thr,
+                                                  const float* __restrict__ levels, int n) {
+  return v.x <= x && x < v.y ? v.z : level_value_search(x, est, br, thr, levels, n);
 }
 
 // Bound: issue slots (the powf's, the metric's cube roots).  An 8-bit level
@@ -1288,12 +1306,8 @@ __global__ void __launch_bounds__(kColourThreads, 6)
     for (int i = threadIdx.x; i < nlev; i += blockDim.x) s_lev[i] = levels[i];
     __syncthreads();
   }
-  const float maxv = (float)(nlev - 1), margin = 1e-3f + 1e-6f * maxv;
-  auto shallow_level = [&](float x) {
-    bool certain;
-    const int k = level_estimate(x, maxv, margin, &certain);
-    return certain ? k : level_of(x, s_thr, nlev - 1);
-  };
+  const float maxv = (float)(nlev - 1), margin = level_margin(maxv);
+  auto level = [&](float x) { return shallow_level(x, maxv, margin, s_thr, nlev - 1); };
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     float x = xyb[i], y = xyb[n + i], b = xyb[2 * n + i];
@@ -1329,12 +1343,12 @@ __global__ void __launch_bounds__(kColourThreads, 6)
     } else if (KIND == 2) {
       uint8_t* o = (uint8_t*)out;
 #pragma unroll
-      for (int q = 0; q < 3; ++q) o[3 * i + q] = (uint8_t)shallow_level(rgb[q]);
+      for (int q = 0; q < 3; ++q) o[3 * i + q] = (uint8_t)level(rgb[q]);
     } else {
       float lin[3];
       if (shallow) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) lin[q] = s_lev[shallow_level(rgb[q])];
+        for (int q = 0; q < 3; ++q) lin[q] = s_lev[level(rgb[q])];
       } else {
         // One 16-byte load of the bracket table gives a level's thresholds and
         // value, the three channels' at once.
@@ -1347,11 +1361,8 @@ __global__ void __launch_bounds__(kColourThreads, 6)
           v[q] = __ldg(&bracket[k[q]]);
         }
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          lin[q] = v[q].z;
-          if (!(v[q].x <= rgb[q] && rgb[q] < v[q].y))
-            lin[q] = level_value_search(rgb[q], k[q], bracket, thr, levels, nlev - 1);
-        }
+        for (int q = 0; q < 3; ++q)
+          lin[q] = deep_level_value(rgb[q], k[q], v[q], bracket, thr, levels, nlev - 1);
       }
       float* o = (float*)out;
       o[i] = lin[0];
@@ -1561,6 +1572,51 @@ bool launch_special_diag(int kind, const float* coef, int n, float* out, cudaStr
     case 9: k_special_diag<9><<<blocks, 64, 0, s>>>(coef, n, out); return true;
     default: return false;
   }
+}
+
+// The short forms of a rule against the rule itself over the floats of bit
+// patterns first .. first + count - 1 (a diagnostic of jpxlg_diag_sweep):
+// WHAT 0 the codec's cube root, 1 the metric's, 2 an output level by the
+// estimate, 3 a deep level's value.  Counts the differences.
+template <int WHAT>
+__global__ void __launch_bounds__(256) k_sweep_diag(uint32_t first, uint32_t count,
+                                                    const float* __restrict__ thr,
+                                                    const float* __restrict__ levels,
+                                                    const float4* __restrict__ bracket, int nlev,
+                                                    unsigned long long* __restrict__ wrong) {
+  const float maxv = (float)(nlev - 1), margin = level_margin(maxv);
+  for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < count; i += gridDim.x * 256u) {
+    const float x = __uint_as_float(first + i);
+    float got, want;
+    if constexpr (WHAT == 0) {
+      got = cbrt_core(x);
+      want = cbrt_core_f64(x);
+    } else if constexpr (WHAT == 1) {
+      got = cbrt_perceptual(x);
+      want = cbrt_perceptual_f64(x);
+    } else if constexpr (WHAT == 2) {
+      got = (float)shallow_level(x, maxv, margin, thr, nlev - 1);
+      want = (float)level_of(x, thr, nlev - 1);
+    } else {
+      bool unused;
+      const int k = level_estimate(x, maxv, margin, &unused);
+      got = deep_level_value(x, k, __ldg(&bracket[k]), bracket, thr, levels, nlev - 1);
+      want = __ldg(&levels[level_of(x, thr, nlev - 1)]);
+    }
+    if (__float_as_uint(got) != __float_as_uint(want)) atomicAdd(wrong, 1ull);
+  }
+}
+
+void launch_sweep_diag(int what, uint32_t first, uint32_t count, const float* thr,
+                       const float* levels, const float4* bracket, int nlev,
+                       unsigned long long* wrong, int num_sms, cudaStream_t s) {
+  auto run = [&](auto* kernel) {
+    kernel<<<num_sms * 8, 256, 0, s>>>(first, count, thr, levels, bracket, nlev, wrong);
+  };
+  if (what == 0) run(k_sweep_diag<0>);
+  else if (what == 1) run(k_sweep_diag<1>);
+  else if (nlev <= 256) run(k_sweep_diag<2>);
+  else run(k_sweep_diag<3>);
 }
 
 void upload_afv(const double* basis, cudaStream_t s) {
