@@ -237,6 +237,20 @@ int jpxlg_diag_special_blocks(jpxlg_ctx* ctx, int kind, const float* coef, int n
 enum { JPXLG_SWEEP_CBRT_CORE = 0, JPXLG_SWEEP_CBRT_METRIC = 1, JPXLG_SWEEP_LEVELS = 100 };
 int jpxlg_diag_sweep(jpxlg_ctx* ctx, int what, uint32_t first, uint64_t count, uint64_t* wrong);
 
+/* Diagnostic: a host table as the kernels receive it (no device needed):
+ * which 0, the dequantization matrices of the 13 kinds of transform, 3
+ * channels of 8704 floats; which 1, the 64-point DCT-II matrix, 4096 floats.
+ * Returns the floats of the table (0: no such table) and, unless out is NULL,
+ * writes them. */
+size_t jpxlg_diag_table(int which, float* out);
+
+/* Diagnostic: the kernel that lays a staged stream out on the device, on a
+ * block in host memory: n coefficients (a multiple of 64) of q_bytes (1, 2 or
+ * 4) each and `rest` bytes (a multiple of 16) behind them, into n int32 and
+ * the same bytes behind those. */
+int jpxlg_diag_unstage(jpxlg_ctx* ctx, int q_bytes, const void* src, size_t n, size_t rest,
+                       void* dst);
+
 /* Quantized plan -> pixels.  `out` sizes: JPXLG_OUT_SRGB8 w*h*3 bytes, other
  * kinds 3*w*h floats.  `bits` is the depth of JPXLG_OUT_LINEAR_DEPTH. */
 int jpxlg_reconstruct(jpxlg_ctx* ctx, const jpxlg_layout* layout, const jpxlg_plan* plan,

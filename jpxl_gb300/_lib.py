@@ -33,6 +33,8 @@ SIGNATURES: dict[str, tuple] = {
     "jpxlg_encode_transform": (_I, [_P, _P, _P, _I, _P, _P, _U32]),
     "jpxlg_encode_stages": (_I, [_P, _P, _P, _I, _P, _P, _P, _P]),
     "jpxlg_diag_special_blocks": (_I, [_P, _I, _P, _I, _P, _U32]),
+    "jpxlg_diag_table": (C.c_size_t, [_I, _P]),
+    "jpxlg_diag_unstage": (_I, [_P, _I, _P, C.c_size_t, C.c_size_t, _P]),
     "jpxlg_diag_sweep": (_I, [_P, _I, _U32, C.c_uint64, C.POINTER(C.c_uint64)]),
     "jpxlg_tune_set": (_I, [_I, _I]),
     "jpxlg_tune_get": (_I, [_I]),

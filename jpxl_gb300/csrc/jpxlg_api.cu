@@ -971,6 +971,36 @@ int jpxlg_diag_special_blocks(jpxlg_ctx* ctx, int kind, const float* coef, int n
   return JPXLG_OK;
 }
 
+size_t jpxlg_diag_table(int which, float* out) {
+  if (which == 0) {
+    if (out) build_dequant_tables(out);
+    return 3 * (size_t)kDequantTableFloats;
+  }
+  if (which == 1) {
+    if (out) build_dct64_matrix(out);
+    return 64 * 64;
+  }
+  return 0;
+}
+
+int jpxlg_diag_unstage(jpxlg_ctx* ctx, int q_bytes, const void* src, size_t n, size_t rest,
+                       void* dst) {
+  if (!ctx || !src || !dst) return fail(ctx, JPXLG_ERR_ARGUMENT, "null argument");
+  if ((q_bytes != 1 && q_bytes != 2 && q_bytes != 4) || n == 0 || n % 64 != 0 || rest % 16 != 0)
+    return fail(ctx, JPXLG_ERR_ARGUMENT, "no such staged block");
+  CK(cudaSetDevice(ctx->device));
+  const size_t in = n * q_bytes + rest, out = n * sizeof(int32_t) + rest;
+  CK(ctx->coeff.ensure(in));
+  CK(ctx->out.ensure(out));
+  CK(cudaMemcpyAsync(ctx->coeff.p, src, in, cudaMemcpyHostToDevice, ctx->stream));
+  launch_unstage(ctx->coeff.p, q_bytes, n, rest, ctx->out.p, ctx->num_sms, ctx->stream);
+  int rc = after_launch(ctx, 1);
+  if (rc) return rc;
+  CK(cudaMemcpyAsync(dst, ctx->out.p, out, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return JPXLG_OK;
+}
+
 int jpxlg_diag_sweep(jpxlg_ctx* ctx, int what, uint32_t first, uint64_t count, uint64_t* wrong) {
   if (!ctx || !wrong) return fail(ctx, JPXLG_ERR_ARGUMENT, "null argument");
   const int bits = what - JPXLG_SWEEP_LEVELS;
