@@ -168,16 +168,17 @@ enum {
   JPXLG_STAGE_XYB = 0,          /* K1 RGB -> XYB */
   JPXLG_STAGE_PRECONDITION,     /* K2 inverse Gaborish, 12 steps */
   JPXLG_STAGE_FDCT_LUMA,        /* K3 forward DCT, LF, luma quantization */
-  JPXLG_STAGE_CFL,              /* K4 CfL estimation */
-  JPXLG_STAGE_QUANT_CHROMA,     /* K5 chroma quantization */
+  JPXLG_STAGE_CFL,              /* K4 CfL estimation and K5 chroma quantization: one kernel
+                                   per tile does both */
+  JPXLG_STAGE_QUANT_CHROMA,     /* empty: always 0 (its work is timed under JPXLG_STAGE_CFL) */
   JPXLG_STAGE_RENDER_VARBLOCKS, /* R1 dequant, CfL, LLF, IDCT */
   JPXLG_STAGE_GABORISH,         /* R2 */
   JPXLG_STAGE_EPF,              /* R3, all steps */
   JPXLG_STAGE_COLOUR,           /* R4 */
   JPXLG_STAGE_SSIM,             /* S1-S5 candidate side, but for the three below */
   JPXLG_STAGE_SSIM_ROWS,        /* S3 blur row pass (every scale) */
-  JPXLG_STAGE_SSIM_COL_RIPPLE,  /* S3 the reset of the column scan's flags (the ripple's
-                                   segment scan runs inside the column pass) */
+  JPXLG_STAGE_SSIM_COL_RIPPLE,  /* empty: always 0 (the ripple's segment scan runs inside the
+                                   column pass, and its states need no reset) */
   JPXLG_STAGE_SSIM_COL_OUT,     /* S3/S4 blur column pass with the per-pixel terms */
   JPXLG_STAGE_COUNT
 };
@@ -269,7 +270,7 @@ int jpxlg_ssim2_ref_destroy(jpxlg_ref* ref);
 int jpxlg_ssim2_score(jpxlg_ctx* ctx, const jpxlg_ref* ref, const float* linear_rgb,
                       uint32_t mem, double* score, double* raw_error, double* terms);
 /* One-shot pair score.  The reference side is built in a device buffer the
- * context keeps for the next call (its pyramid: about 64 bytes per source
+ * context keeps for the next call (its pyramid: about 48 bytes per source
  * pixel), freed with the context. */
 int jpxlg_score_pair(jpxlg_ctx* ctx, const float* ref_rgb, const float* cand_rgb, int width,
                      int height, uint32_t mem, double* score);
@@ -480,7 +481,7 @@ int jpxlg_decode_batch_destroy(jpxlg_decode_batch* batch);
  * JPXLG_ERR_ARGUMENT); the first call on a device resolves the scratch
  * address and should come before any stream capture; there is one scratch
  * per device, so calls in flight at the same time on one device race.  The
- * scratch is a 137 MB __device__ array, resident on every device where the
+ * scratch is a 125 MB __device__ array, resident on every device where the
  * library's module loads, whether or not this entry point is called. */
 int jpxlg_ssim2_score_static(jpxlg_ctx* ctx, const jpxlg_ref* ref,
                              const float* linear_rgb_dev, double* out_dev);

@@ -255,9 +255,10 @@ __device__ double exact_node(const CoverArgs& a, const CoverSmem& sm, int bx, in
 // Bound: issue slots and the quantizer's latency (three shapes, three
 // channels a cell).  Measured at 1536x1024: 402 us as three scoring kernels
 // (the DCT32 one 136, 32 cells a thread and channel) and one thread of serial
-// f64 per region (170, twelve CTAs); 104 us now, nothing but the map in
-// memory.  Four CTAs an SM spill some of the DCT32's registers and are still
-// faster than three or two (217, 221, 241 us the whole call).
+// f64 per region (170, twelve CTAs); 104 us now of the call's 182 (112 by
+// itself, from a cold cache), nothing but the map in memory.  Four CTAs an SM
+// spill some of the DCT32's registers and are still faster than three or two
+// (the whole call as it was then: 217, 221, 241 us).
 __global__ void __launch_bounds__(kCoverThreads, 4) k_cover(const __grid_constant__ CoverArgs a) {
   extern __shared__ __align__(16) unsigned char cover_smem[];
   CoverSmem& sm = *reinterpret_cast<CoverSmem*>(cover_smem);

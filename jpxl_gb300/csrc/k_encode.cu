@@ -460,7 +460,7 @@ __device__ __forceinline__ void precondition_tile(const float* __restrict__ in,
       const float* const S = xb + (it & 1) * (H * kPreP);
       float* const Sn = xb + ((it + 1) & 1) * (H * kPreP);
       __syncthreads();
-      // A warp whose four rows have all left the exact region [1 + it,
+      // A warp whose rows have all left the exact region [1 + it,
       // H - 1 - it) rests; its rows in the step buffers are read only by
       // cells that are no longer exact either.
       if (live && !(ly + ROWS - 1 < 1 + it || ly >= H - 1 - it)) {
@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(128) k_fdct8(EncArgs a, const uint32_t* __rest
 
 // K3, N = 16 and 32 — the same block by N / 4 warps, a share of each column
 // per warp and the three channels together through each phase: the split of
-// k_render_sq, for the same reason (the luma stage at 1920x1080: 47 us, now
+// k_render_rect, for the same reason (the luma stage at 1920x1080: 47 us, now
 // 34; at 64x64 14.9, now 13.3).
 template <int N, bool FROM_IMAGE = false>
 __global__ void __launch_bounds__(8 * N) k_fdct_sq(EncArgs a, const uint32_t* __restrict__ list,

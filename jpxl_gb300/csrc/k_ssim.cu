@@ -141,8 +141,9 @@ constexpr int kReduceThreads = 256;
 // The CTA that finishes last (`ticket`, zeroed by the blur before) goes on to
 // the norms, weights and remap of the 6 x 18 totals, a thread per term.
 // Bound by the latency of its double-precision chain (two square roots, the
-// weighted sum, one power): 3 + 13.6 us as two launches whose second took a
-// channel's six terms in one thread, 12.5 us in one.
+// weighted sum, one power): 3 + 13.6 us at 64x64 as two launches whose second
+// took a channel's six terms in one thread, 12.5 us in one (13 by itself, 17 at
+// 2048x2048, from a cold cache).
 __global__ void __launch_bounds__(kReduceThreads) k_score_finish(DF* __restrict__ partials,
                                                                  FinishArgs fa,
                                                                  uint32_t* __restrict__ ticket,
